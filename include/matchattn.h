@@ -318,7 +318,7 @@ MATCHATTN_API int matchattn_local_disparity(const void *volume, void *flow, void
  *   blur_max    [2B, N]        or NULL: the pooled maximum (tests)
  *   centre      [2B, N] int32  or NULL: the clamped window centre as y*W + x (tests)
  *   scratch     at least matchattn_flow_init_scratch_bytes(B, H, W) bytes of device memory, 16-byte aligned
- * H, W >= 5.  Allocates nothing; five kernels on `cuda_stream`.
+ * H, W >= 5.  Allocates nothing; four kernels on `cuda_stream`.
  */
 MATCHATTN_API size_t matchattn_flow_init_scratch_bytes(int B, int H, int W);
 MATCHATTN_API int matchattn_flow_init(const void *correlation, void *prob, void *flow, void *blur_max, int *centre,

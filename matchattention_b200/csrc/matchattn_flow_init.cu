@@ -1,5 +1,5 @@
 // Flow branch of GlobalCorrelation after its matmul, with local_flow_estimator
-// (models/cost_volume.py:61-69 and :71-121), as five kernels and no temporaries beyond a small scratch:
+// (models/cost_volume.py:61-69 and :71-121), as four kernels:
 //
 //   corr [B, N, N] (N = H*W; scaled q.k^T, reference token then target token)
 //   prob [2B, N, N]   written: softmax over the last axis of corr[b] and of corr[b]^T
@@ -7,14 +7,27 @@
 //
 // The reference materialises the concatenation [corr; corr^T] (2 x N^2), its softmax, the 5x5-pooled copy
 // (avg_pool2d over the N x N "image"), arg max, a [2B, N, 25, 2] gather of coordinates and a dozen
-// elementwise temporaries.  Here: row softmax of corr; column statistics of corr and a tiled transposed
-// normalise for the second half; one pass that pools and takes the arg max without storing the pooled
-// volume; one thread per token for the 5x5 window estimate.
+// elementwise temporaries.  Here:
+//   1. flow_max_kernel        one read of corr: partial maxima of rows AND columns
+//   2. flow_sum_kernel        one read for the rows, one for the columns: maximum and sum of exponentials
+//   3. flow_prob_pool_kernel  reads corr again, writes both halves of prob and, from the values in registers,
+//                             the maximum of the 5x5 box sums per (token, chunk of targets); no second pass over prob
+//   4. flow_window_kernel     per token: the chunks that can hold the arg max are pooled once more to find it, then
+//                             the 5x5 window estimate
+// The window hangs on an arg max, and box averages that differ in their last bit are common in the 16-bit types; so
+// prob and the deciding averages are formed in one fixed order (sums of exponentials in 256 interleaved partial sums
+// per row and four per column, box sums row by row) whatever the split of the work, and only the screening in step 3
+// adds in another.
+// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.22 ms = 0.09 + 0.34 +
+// 0.72 + 0.08; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
+// the pooling took 4.1.  48x48 tokens: 56 us, before 189.
 // Rounding of the 16-bit types as eager PyTorch on the GPU: softmax, pooling and sums accumulate in float32
 // and round once, every elementwise op rounds.
 #include "../../include/matchattn.h"
 
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "matchattn_kernels.cuh"
 
@@ -22,240 +35,757 @@ namespace matchattn {
 namespace {
 
 constexpr int kFlowThreads = 256;
+constexpr int kFlowWarps = kFlowThreads / 32;
+constexpr int kLaneCols = 4;                          // consecutive columns of corr that a lane owns
+constexpr int kWarpCols = 32 * kLaneCols;
+constexpr int kMaxRows = 16;                          // rows of corr that a lane holds at a time in the maximum pass
+constexpr int kPoolCols = kWarpCols - 2 * kLaneCols;  // columns a warp pools: its outer lanes are the halo
+constexpr int kPoolStep = 8;                          // rows per unrolled step of the pooling kernel (two halves of four)
+constexpr int kTransBytes = 64, kTransPitch = kTransBytes + 16;   // run of a prob row that a transposed store writes; its slot in shared memory
+constexpr int kPoolSmemPerWarp = kWarpCols * kTransPitch;
+constexpr int kPoolWarps = 4;                         // warps per block of the pooling kernel
+constexpr int kSumGroups = 4;                         // interleaved partial sums per column
+constexpr int kWindowTokens = kFlowWarps;             // tokens per block of the window kernel: one per warp
 
-__device__ __forceinline__ float block_reduce_max(float v, float *sm)
+// Sizes and scratch areas of one call, computed alike by the size query and the launcher.
+struct FlowPlan {
+    int64_t N;
+    int max_rows;       // rows per warp of the maximum kernel
+    int row_parts;      // partials per row of corr (one per kWarpCols columns)
+    int col_parts;      // partials per column of corr (one per max_rows rows)
+    int band;           // rows per warp of the pooling kernel
+    int chunks, bands;  // chunks of kPoolCols columns, bands of rows
+    size_t off_col, off_stats, off_row_max, off_col_max, bytes;
+};
+
+FlowPlan flow_plan(int B, int H, int W)
 {
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = sm[0];
-    for (int w = 1; w < (blockDim.x >> 5); ++w) r = fmaxf(r, sm[w]);
-    __syncthreads();
+    FlowPlan pl{};
+    pl.N = static_cast<int64_t>(H) * W;
+    const auto parts = [&](int64_t of) { return static_cast<int>((pl.N + of - 1) / of); };
+    // Rows per warp: long columns amortise the start of a warp (the halo rows, the merges of the partials); below
+    // about 5000 tokens there are not enough warps to fill the chip with long ones.
+    pl.max_rows = pl.N >= 5000 ? 128 : 32;
+    pl.band = pl.N >= 5000 ? 64 : 32;
+    pl.row_parts = parts(kWarpCols);
+    pl.col_parts = parts(pl.max_rows);
+    pl.chunks = parts(kPoolCols);
+    pl.bands = parts(pl.band);
+    const auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
+    const size_t n = static_cast<size_t>(B) * pl.N;
+    size_t off = up(n * pl.row_parts * sizeof(float));
+    pl.off_col = off;     off = up(off + n * pl.col_parts * sizeof(float));
+    pl.off_stats = off;   off = up(off + 2 * n * sizeof(float2));
+    pl.off_row_max = off; off = up(off + n * pl.chunks * sizeof(float));
+    pl.off_col_max = off; off = up(off + n * pl.bands * sizeof(float));
+    pl.bytes = off;
+    return pl;
+}
+
+// maximum over a warp in one instruction (PTX ISA 8.6, sm_100a)
+__device__ __forceinline__ float warp_max(float v)
+{
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
-
-__device__ __forceinline__ float block_reduce_sum(float v, float *sm)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = 0.f;
-    for (int w = 0; w < (blockDim.x >> 5); ++w) r += sm[w];
-    __syncthreads();
-    return r;
-}
-
-// prob[b, i, :] = softmax(corr[b, i, :]); one block per row
+// Four consecutive elements of a row of corr, raw (two words of pairs, or four words).  VEC: rows start 16-byte
+// aligned, so a lane's group is one load.  FULL: the group lies inside the row; otherwise columns outside [0, N) and
+// rows outside [0, N) read as -infinity (probability 0).
 template <typename T>
-__global__ void __launch_bounds__(kFlowThreads) flow_row_softmax_kernel(const T *__restrict__ corr, T *__restrict__ prob, int64_t N)
+__device__ __forceinline__ uint32_t word_max(uint32_t a, uint32_t b)
 {
-    __shared__ float sm[kFlowThreads / 32];
-    const T *src = corr + (static_cast<int64_t>(blockIdx.y) * N + blockIdx.x) * N;
-    T *dst = prob + (static_cast<int64_t>(blockIdx.y) * N + blockIdx.x) * N;
-    float mx = -INFINITY;
-    for (int64_t j = threadIdx.x; j < N; j += blockDim.x) mx = fmaxf(mx, load_one<T>(src + j));
-    mx = block_reduce_max(mx, sm);
-    float den = 0.f;
-    for (int64_t j = threadIdx.x; j < N; j += blockDim.x) den += expf(load_one<T>(src + j) - mx);
-    den = block_reduce_sum(den, sm);
-    for (int64_t j = threadIdx.x; j < N; j += blockDim.x) store_one<T>(dst + j, __fdiv_rn(expf(load_one<T>(src + j) - mx), den));
-}
-
-// column maximum and sum of exponentials of corr[b]: 64 columns per block, four row groups
-template <typename T>
-__global__ void __launch_bounds__(kFlowThreads) flow_col_stats_kernel(const T *__restrict__ corr, float *__restrict__ cmax,
-                                                                       float *__restrict__ csum, int64_t N)
-{
-    __shared__ float sm[4][64];
-    const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
-    const int64_t col = static_cast<int64_t>(blockIdx.x) * 64 + c;
-    const T *src = corr + static_cast<int64_t>(blockIdx.y) * N * N;
-    float mx = -INFINITY;
-    if (col < N)
-        for (int64_t j = g; j < N; j += 4) mx = fmaxf(mx, load_one<T>(src + j * N + col));
-    sm[g][c] = mx;
-    __syncthreads();
-    mx = fmaxf(fmaxf(sm[0][c], sm[1][c]), fmaxf(sm[2][c], sm[3][c]));
-    __syncthreads();
-    float den = 0.f;
-    if (col < N)
-        for (int64_t j = g; j < N; j += 4) den += expf(load_one<T>(src + j * N + col) - mx);
-    sm[g][c] = den;
-    __syncthreads();
-    if (g == 0 && col < N) {
-        cmax[blockIdx.y * N + col] = mx;
-        csum[blockIdx.y * N + col] = (sm[0][c] + sm[1][c]) + (sm[2][c] + sm[3][c]);
+    if constexpr (sizeof(T) == 4) {
+        return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
+    } else if constexpr (std::is_same_v<T, __half>) {
+        const __half2 m = __hmax2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+        return *reinterpret_cast<const uint32_t *>(&m);
+    } else {
+        const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162 *>(&a), *reinterpret_cast<const __nv_bfloat162 *>(&b));
+        return *reinterpret_cast<const uint32_t *>(&m);
     }
 }
 
-// prob[B + b, i, j] = exp(corr[b, j, i] - cmax[i]) / csum[i], through a 32 x 32 shared-memory tile
 template <typename T>
-__global__ void __launch_bounds__(kFlowThreads) flow_transposed_softmax_kernel(const T *__restrict__ corr, const float *__restrict__ cmax,
-                                                                                const float *__restrict__ csum, T *__restrict__ prob_t,
-                                                                                int64_t N)
-{
-    __shared__ float tile[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;       // 32 x 8
-    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32, j0 = static_cast<int64_t>(blockIdx.y) * 32;
-    const T *src = corr + static_cast<int64_t>(blockIdx.z) * N * N;
-    T *dst = prob_t + static_cast<int64_t>(blockIdx.z) * N * N;
-    for (int k = ty; k < 32; k += 8) {
-        const int64_t j = j0 + k, i = i0 + tx;
-        tile[k][tx] = (j < N && i < N) ? load_one<T>(src + j * N + i) : 0.f;
-    }
-    __syncthreads();
-    for (int k = ty; k < 32; k += 8) {
-        const int64_t i = i0 + k, j = j0 + tx;
-        if (i < N && j < N)
-            store_one<T>(dst + i * N + j, __fdiv_rn(expf(tile[tx][k] - cmax[blockIdx.z * N + i]), csum[blockIdx.z * N + i]));
-    }
-}
-
-// per (b2, i): maximum over j of the 5 x 5 box average of prob[b2] around (i, j), and its first arg max.
-// A block takes kPoolRows consecutive rows i: the kPoolRows + 4 rows of probabilities they need are staged
-// once per column chunk in shared memory (1.5 reads per element instead of 5), every thread keeps the
-// 12 x 5 neighbourhood of its column in registers and forms the 25-term sums of its eight outputs from
-// them, in the reference's order (row-major over the window, out-of-range taps skipped).
-constexpr int kPoolRows = 8;
-
-template <typename T>
-__global__ void __launch_bounds__(kFlowThreads) flow_pool_argmax_kernel(const T *__restrict__ prob, T *__restrict__ blur_max,
-                                                                         int *__restrict__ arg_out, int64_t N)
-{
-    __shared__ float rows[kPoolRows + 4][kFlowThreads + 4];
-    __shared__ float best_v[kPoolRows][kFlowThreads / 32];
-    __shared__ int best_j[kPoolRows][kFlowThreads / 32];
-    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * kPoolRows;
-    const T *base = prob + static_cast<int64_t>(blockIdx.y) * N * N;
-    float best[kPoolRows];
-    int arg[kPoolRows];
+struct Group {
+    uint32_t w[kLaneCols / DT<T>::kElemsPerWord];
+    __device__ __forceinline__ float get(int k) const { return DT<T>::unpack(w[k / DT<T>::kElemsPerWord], k % DT<T>::kElemsPerWord); }
+    __device__ __forceinline__ void max_with(const Group &o)      // element by element
+    {
 #pragma unroll
-    for (int r = 0; r < kPoolRows; ++r) {
-        best[r] = -INFINITY;
-        arg[r] = 0x7fffffff;
+        for (int i = 0; i < kLaneCols / DT<T>::kElemsPerWord; ++i) w[i] = word_max<T>(w[i], o.w[i]);
     }
-    for (int64_t c0 = 0; c0 < N; c0 += kFlowThreads) {
-        for (int e = threadIdx.x; e < (kPoolRows + 4) * (kFlowThreads + 4); e += kFlowThreads) {
-            const int di = e / (kFlowThreads + 4), cc = e - di * (kFlowThreads + 4);
-            const int64_t ii = i0 + di - 2, jj = c0 + cc - 2;
-            rows[di][cc] = (ii >= 0 && ii < N && jj >= 0 && jj < N) ? load_one<T>(base + ii * N + jj) : 0.f;
+    __device__ __forceinline__ float max4() const
+    {
+        if constexpr (sizeof(T) == 4) return fmaxf(fmaxf(get(0), get(1)), fmaxf(get(2), get(3)));
+        const uint32_t m = word_max<T>(w[0], w[1]);
+        return fmaxf(DT<T>::unpack(m, 0), DT<T>::unpack(m, 1));
+    }
+    __device__ __forceinline__ void mask()
+    {
+        constexpr uint32_t kMinusInf = sizeof(T) == 4 ? 0xff800000u : std::is_same_v<T, __nv_bfloat16> ? 0xff80ff80u : 0xfc00fc00u;
+#pragma unroll
+        for (uint32_t &x : w) x = kMinusInf;
+    }
+};
+
+__device__ __forceinline__ float to_float(float x) { return x; }
+__device__ __forceinline__ float to_float(__half x) { return __half2float(x); }
+__device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
+
+template <typename T>
+__device__ __forceinline__ uint32_t raw_bits(const T *p)
+{
+    if constexpr (sizeof(T) == 4) return __ldg(reinterpret_cast<const uint32_t *>(p));
+    else return __ldg(reinterpret_cast<const unsigned short *>(p));
+}
+
+template <typename T, bool VEC, bool FULL>
+__device__ __forceinline__ Group<T> load_group(const T *row, int64_t col, int64_t N, bool row_ok)
+{
+    Group<T> g;
+    constexpr int EPW = DT<T>::kElemsPerWord;
+    if constexpr (FULL || VEC) {
+        if (!FULL && (!row_ok || col < 0 || col >= N)) {
+            g.mask();
+            return g;
         }
+        if constexpr (!VEC) {
+#pragma unroll
+            for (int k = 0; k < kLaneCols; k += EPW) {
+                uint32_t w = raw_bits(row + col + k);
+                if constexpr (EPW == 2) w |= raw_bits(row + col + k + 1) << 16;
+                g.w[k / EPW] = w;
+            }
+        } else if constexpr (EPW == 1) {
+            const uint4 t = __ldg(reinterpret_cast<const uint4 *>(row + col));
+            g.w[0] = t.x; g.w[1] = t.y; g.w[2] = t.z; g.w[3] = t.w;
+        } else {
+            const uint2 t = __ldg(reinterpret_cast<const uint2 *>(row + col));
+            g.w[0] = t.x; g.w[1] = t.y;
+        }
+    } else {
+        g.mask();
+        if (!row_ok) return g;
+#pragma unroll
+        for (int k = 0; k < kLaneCols; ++k)
+            if (col + k >= 0 && col + k < N) {
+                const uint32_t w = raw_bits(row + col + k);
+                if constexpr (EPW == 1) g.w[k] = w;
+                else g.w[k / 2] = (k & 1) ? __byte_perm(g.w[k / 2], w, 0x5410) : __byte_perm(g.w[k / 2], w, 0x3254);
+            }
+    }
+    return g;
+}
+
+// Partial maxima of the rows and columns of corr.  A warp takes 128 columns (four per lane) and walks down its rows,
+// sixteen at a time; the maxima are taken on pairs of 16-bit values.  Memory-bound.
+template <typename T, bool VEC, bool FULL>
+__device__ __forceinline__ void max_tile(const T *src, int64_t col, int64_t r0, int64_t last, int64_t N, Group<T> &cm, float *row_part, int lane)
+{
+    Group<T> g[kMaxRows];
+#pragma unroll
+    for (int r = 0; r < kMaxRows; ++r) g[r] = load_group<T, VEC, FULL>(src + (r0 + r) * N, col, N, r0 + r < last);
+    float mine = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kMaxRows; ++r) {
+        const float m = warp_max(g[r].max4());
+        mine = lane == r ? m : mine;
+        cm.max_with(g[r]);
+    }
+    if (lane < kMaxRows && r0 + lane < last) row_part[r0 + lane] = mine;
+}
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kFlowThreads) flow_max_kernel(const T *__restrict__ corr, float *__restrict__ row_part,
+                                                                float *__restrict__ col_part, int64_t N, int rows_per_warp,
+                                                                int row_parts, int col_parts)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t unit = static_cast<int64_t>(blockIdx.x) * kFlowWarps + (threadIdx.x >> 5);
+    const int band = static_cast<int>(unit / row_parts), chunk = static_cast<int>(unit - static_cast<int64_t>(band) * row_parts);
+    if (band >= col_parts) return;
+    const int64_t b = blockIdx.y;
+    const T *src = corr + b * N * N;
+    const int64_t col0 = static_cast<int64_t>(chunk) * kWarpCols, col = col0 + lane * kLaneCols;
+    const int64_t first = static_cast<int64_t>(band) * rows_per_warp, last = min(first + rows_per_warp, N);
+    float *rows = row_part + (b * row_parts + chunk) * N;
+    Group<T> cm;
+    cm.mask();
+    for (int64_t r0 = first; r0 < last; r0 += kMaxRows) {
+        if (col0 + kWarpCols <= N && r0 + kMaxRows <= last) max_tile<T, VEC, true>(src, col, r0, last, N, cm, rows, lane);
+        else max_tile<T, VEC, false>(src, col, r0, last, N, cm, rows, lane);
+    }
+#pragma unroll
+    for (int k = 0; k < kLaneCols; ++k)
+        if (col + k < N) col_part[(b * col_parts + band) * N + col + k] = cm.get(k);
+}
+
+// stats[half, b, token] = (maximum, sum of exp(x - maximum)) of row `token` of corr[b] (half 0) or of column `token`
+// (half 1).  The first blocks serve COLUMNS columns each, four threads per column, every fourth row per thread, BATCH
+// rows read ahead; the others serve one row per warp: 256 partial sums (element j goes to sum j mod 256), then a tree
+// over each 32 of them and a running sum over the eight results.
+// Bound by instruction issue on large maps (one exponential per element and half; the column blocks, few and long,
+// start first), on small ones by the latency of a column's chain of reads: narrower blocks with more rows in flight.
+template <typename T, bool VEC, int COLUMNS, int BATCH>
+__global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T *__restrict__ corr, const float *__restrict__ row_part,
+                                                                const float *__restrict__ col_part, float2 *__restrict__ stats,
+                                                                int64_t N, int row_parts, int col_parts, int col_blocks)
+{
+    const int64_t b = blockIdx.y;
+    const T *src = corr + b * N * N;
+    if (static_cast<int>(blockIdx.x) < col_blocks) {
+        __shared__ float sm[kSumGroups][COLUMNS];
+        const int c = threadIdx.x % COLUMNS, g = threadIdx.x / COLUMNS;
+        const int64_t col = static_cast<int64_t>(blockIdx.x) * COLUMNS + c;
+        float mx = -INFINITY;
+        if (col < N) {
+#pragma unroll 8
+            for (int i = g; i < col_parts; i += kSumGroups) mx = fmaxf(mx, col_part[(b * col_parts + i) * N + col]);
+        }
+        sm[g][c] = mx;
         __syncthreads();
-        const int64_t j = c0 + threadIdx.x;
-        if (j < N) {
-            float w[kPoolRows + 4][5];
 #pragma unroll
-            for (int di = 0; di < kPoolRows + 4; ++di)
+        for (int i = 0; i < kSumGroups; ++i) mx = fmaxf(mx, sm[i][c]);
+        __syncthreads();
+        float den = 0.f;
+        if (col < N) {
+            const T *p = src + g * N + col;
+            const int64_t step = kSumGroups * N;
+            int64_t left = (N - g + kSumGroups - 1) / kSumGroups;
+            T now[BATCH], next[BATCH];      // the next batch is read while this one is summed
+            if (left >= BATCH) {
 #pragma unroll
-                for (int dj = 0; dj < 5; ++dj) w[di][dj] = rows[di][threadIdx.x + dj];
+                for (int i = 0; i < BATCH; ++i) now[i] = p[i * step];
+                while (left >= BATCH) {
+                    p += BATCH * step;
+                    left -= BATCH;
+                    const bool more = left >= BATCH;
+                    if (more) {
 #pragma unroll
-            for (int r = 0; r < kPoolRows; ++r) {
-                const int64_t i = i0 + r;
-                if (i >= N) break;
-                float acc = 0.f;
-#pragma unroll
-                for (int di = 0; di < 5; ++di)
-#pragma unroll
-                    for (int dj = 0; dj < 5; ++dj) {
-                        const int64_t ii = i + di - 2, jj = j + dj - 2;
-                        if (ii >= 0 && ii < N && jj >= 0 && jj < N) acc += w[r + di][dj];
+                        for (int i = 0; i < BATCH; ++i) next[i] = p[i * step];
                     }
-                const float bl = DT<T>::rnd(__fdiv_rn(acc, 25.f));
-                if (bl > best[r]) {
-                    best[r] = bl;
-                    arg[r] = static_cast<int>(j);
+#pragma unroll
+                    for (int i = 0; i < BATCH; ++i) den += expf(to_float(now[i]) - mx);
+                    if (more) {
+#pragma unroll
+                        for (int i = 0; i < BATCH; ++i) now[i] = next[i];
+                    }
                 }
             }
+            for (; left > 0; --left, p += step) den += expf(load_one<T>(p) - mx);
         }
+        sm[g][c] = den;
         __syncthreads();
+        if (g == 0 && col < N)
+            stats[(gridDim.y + b) * N + col] = make_float2(mx, (sm[0][c] + sm[1][c]) + (sm[2][c] + sm[3][c]));
+        return;
     }
-    // block arg max per row: larger value wins, equal values keep the smaller index
+    const int lane = threadIdx.x & 31;
+    const int64_t row = static_cast<int64_t>(blockIdx.x - col_blocks) * (COLUMNS * kSumGroups / 32) + (threadIdx.x >> 5);
+    if (row >= N) return;
+    float mx = -INFINITY;
+    for (int i = lane; i < row_parts; i += 32) mx = fmaxf(mx, row_part[(b * row_parts + i) * N + row]);
+    mx = warp_max(mx);
+    const T *p = src + row * N;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float total = 0.f;
+    if constexpr (VEC) {      // lane l holds the partial sums 8 l .. 8 l + 7
+#pragma unroll 4
+        for (int64_t j = lane * 8; j < N; j += 256) {
+            const Group<T> g0 = load_group<T, true, true>(p, j, N, true), g1 = load_group<T, true, true>(p, j + 4, N, true);
 #pragma unroll
-    for (int r = 0; r < kPoolRows; ++r) {
-        float bv = best[r];
-        int bj = arg[r];
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-            if (ov > bv || (ov == bv && oj < bj)) {
-                bv = ov;
-                bj = oj;
+            for (int k = 0; k < 4; ++k) {
+                s[k] += expf(g0.get(k) - mx);
+                s[k + 4] += expf(g1.get(k) - mx);
             }
         }
-        if ((threadIdx.x & 31) == 0) {
-            best_v[r][threadIdx.x >> 5] = bv;
-            best_j[r][threadIdx.x >> 5] = bj;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            s[k] += __shfl_xor_sync(0xffffffffu, s[k], 2);
+            s[k] += __shfl_xor_sync(0xffffffffu, s[k], 1);
+        }
+        const float sum = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+#pragma unroll
+        for (int w = 0; w < 8; ++w) total += __shfl_sync(0xffffffffu, sum, 4 * w);
+    } else {                  // lane l holds the partial sums l, l + 32, .. l + 224
+        int64_t j = lane;
+        for (; j + 224 < N; j += 256) {
+            float x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = load_one<T>(p + j + 32 * k);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s[k] += expf(x[k] - mx);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (j + 32 * k < N) s[k] += expf(load_one<T>(p + j + 32 * k) - mx);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+            total += s[k];
         }
     }
-    __syncthreads();
-    if (threadIdx.x < kPoolRows && i0 + threadIdx.x < N) {
-        const int r = threadIdx.x;
-        float bv = best_v[r][0];
-        int bj = best_j[r][0];
-        for (int w = 1; w < kFlowThreads / 32; ++w)
-            if (best_v[r][w] > bv || (best_v[r][w] == bv && best_j[r][w] < bj)) {
-                bv = best_v[r][w];
-                bj = best_j[r][w];
+    if (lane == 0) stats[b * N + row] = make_float2(mx, total);
+}
+
+// Softmax of an element: the quotient exp(x - max) / sum, to the last bit, by one Newton step on the product with the
+// rounded reciprocal (Markstein, IBM J. Res. Dev. 34, 1990).
+struct Softmax {
+    float max, sum, inv;
+    __device__ __forceinline__ float operator()(float x) const
+    {
+        const float e = expf(x - max), q = e * inv;
+        return fmaf(fmaf(-q, sum, e), inv, q);
+    }
+};
+
+template <typename T>
+__device__ __forceinline__ Softmax softmax_of(float2 st) { return Softmax{st.x, st.y, __frcp_rn(st.y)}; }
+
+// Sliding 5-sum down the rows of a pair of columns: push(p) returns p(a-4) + .. + p(a), from the pair sums it keeps.
+struct PairSums {
+    float2 p1, s1, s2, s3;   // p(a-1); pair sums ending at a-1, a-2, a-3
+    __device__ __forceinline__ void reset() { p1 = s1 = s2 = s3 = make_float2(0.f, 0.f); }
+    __device__ __forceinline__ float2 push(float2 p)
+    {
+        const float2 v = add_f32x2(add_f32x2(s3, s1), p);
+        s3 = s2;
+        s2 = s1;
+        s1 = add_f32x2(p1, p);
+        p1 = p;
+        return v;
+    }
+};
+
+// box[k] = v(c-2) + .. + v(c+2) around the lane's column k; the outer two columns come from the neighbouring lanes
+__device__ __forceinline__ void box_sums(const float2 a, const float2 b, float (&box)[kLaneCols])
+{
+    const float pa = a.x + a.y, pb = b.x + b.y;
+    const float left2 = __shfl_up_sync(0xffffffffu, pb, 1), left1 = __shfl_up_sync(0xffffffffu, b.y, 1);
+    const float right1 = __shfl_down_sync(0xffffffffu, a.x, 1), right2 = __shfl_down_sync(0xffffffffu, pa, 1);
+    const float mid = pa + pb;
+    box[0] = (left2 + pa) + b.x;
+    box[1] = left1 + mid;
+    box[2] = mid + right1;
+    box[3] = (a.y + pb) + right2;
+}
+
+struct PoolParams {
+    const float2 *stats;
+    float *row_max, *col_max;
+    int64_t N;
+    int B, band_rows, chunks, bands;
+};
+
+// role "rows": prob[b][row][col], statistics per row; the box maximum per (row, chunk) by a warp reduction
+template <typename T, bool VEC, bool FULL>
+__device__ __forceinline__ void pool_rows(const PoolParams &pp, const T *src, T *dst, char *smem, int64_t b, int64_t a0, int64_t c0, int chunk, int lane)
+{
+    const int64_t N = pp.N;
+    float4 *st = reinterpret_cast<float4 *>(smem);          // rows a0 - 2 .. a0 + band_rows + 1: maximum, sum, reciprocal
+    float *row_max = reinterpret_cast<float *>(st + pp.band_rows + 4);
+    for (int i = lane; i < pp.band_rows + 4; i += 32) {
+        const int64_t a = a0 - 2 + i;
+        const Softmax s = softmax_of<T>(FULL || (a >= 0 && a < N) ? __ldg(pp.stats + b * N + a) : make_float2(0.f, 1.f));
+        st[i] = make_float4(s.max, s.sum, s.inv, 0.f);
+    }
+    __syncwarp();
+    const bool inner = lane != 0 && lane != 31;
+    PairSums lo, hi;
+    lo.reset();
+    hi.reset();
+    // one row: probabilities, store, box sums of the row two above, their maximum over the warp
+    const auto row_step = [&](const Group<T> &g, const Softmax &sm, int64_t a, bool store, bool pool) {
+        float2 p01 = make_float2(sm(g.get(0)), sm(g.get(1))), p23 = make_float2(sm(g.get(2)), sm(g.get(3)));
+        uint32_t w[kLaneCols / DT<T>::kElemsPerWord];
+        if constexpr (sizeof(T) == 2) {
+            w[0] = DT<T>::aw_from(p01.x, p01.y);
+            w[1] = DT<T>::aw_from(p23.x, p23.y);
+            p01 = make_float2(DT<T>::unpack(w[0], 0), DT<T>::unpack(w[0], 1));
+            p23 = make_float2(DT<T>::unpack(w[1], 0), DT<T>::unpack(w[1], 1));
+        } else {
+            w[0] = __float_as_uint(p01.x); w[1] = __float_as_uint(p01.y);
+            w[2] = __float_as_uint(p23.x); w[3] = __float_as_uint(p23.y);
+        }
+        if (store && inner && (FULL || a < N)) {
+            T *out = dst + a * N + c0;
+            if constexpr (VEC) {
+                if (FULL || c0 < N) store_words<kLaneCols / DT<T>::kElemsPerWord>(out, w);
+            } else {
+                const float p[kLaneCols] = {p01.x, p01.y, p23.x, p23.y};
+#pragma unroll
+                for (int k = 0; k < kLaneCols; ++k)
+                    if (FULL || c0 + k < N) store_one<T>(out + k, p[k]);
             }
-        arg_out[blockIdx.y * N + i0 + r] = bj;
-        if (blur_max != nullptr) store_one<T>(blur_max + blockIdx.y * N + i0 + r, bv);
+        }
+        const float2 va = lo.push(p01), vb = hi.push(p23);
+        if (!pool) return;
+        float box[kLaneCols];
+        box_sums(va, vb, box);
+        float m;
+        if constexpr (FULL || VEC) m = fmaxf(fmaxf(box[0], box[1]), fmaxf(box[2], box[3]));
+        else {
+            m = 0.f;
+#pragma unroll
+            for (int k = 0; k < kLaneCols; ++k) m = c0 + k < N ? fmaxf(m, box[k]) : m;
+        }
+        m = warp_max(inner && (FULL || c0 < N) ? m : 0.f);
+        if (lane == 0) row_max[a - 2 - a0] = m;
+    };
+    const auto load = [&](int64_t a) {
+        return load_group<T, VEC, FULL>(src + (FULL ? min(a, N - 1) : a) * N, c0, N, a >= 0 && a < N);
+    };
+    const auto stat = [&](int64_t a) {
+        const float4 v = st[a - (a0 - 2)];
+        return Softmax{v.x, v.y, v.z};
+    };
+    Group<T> now[kPoolStep / 2], next[kPoolStep / 2];     // corr is read four rows ahead
+#pragma unroll
+    for (int i = 0; i < 2; ++i) next[i] = load(a0 - 2 + i);
+#pragma unroll
+    for (int i = 0; i < kPoolStep / 2; ++i) now[i] = load(a0 + i);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) row_step(next[i], stat(a0 - 2 + i), a0 - 2 + i, false, false);
+    for (int64_t a = a0; a < a0 + pp.band_rows; a += kPoolStep) {
+#pragma unroll
+        for (int i = 0; i < kPoolStep / 2; ++i) next[i] = load(a + kPoolStep / 2 + i);
+#pragma unroll
+        for (int i = 0; i < kPoolStep / 2; ++i) row_step(now[i], stat(a + i), a + i, true, i >= 2 || a > a0);
+#pragma unroll
+        for (int i = 0; i < kPoolStep / 2; ++i) now[i] = load(a + kPoolStep + i);
+#pragma unroll
+        for (int i = 0; i < kPoolStep / 2; ++i) row_step(next[i], stat(a + kPoolStep / 2 + i), a + kPoolStep / 2 + i, true, true);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) row_step(now[i], stat(a0 + pp.band_rows + i), a0 + pp.band_rows + i, false, true);
+    __syncwarp();
+    for (int i = lane; i < pp.band_rows; i += 32)
+        if (FULL || a0 + i < N) pp.row_max[(b * pp.chunks + chunk) * N + a0 + i] = row_max[i];
+}
+
+// role "columns": prob[B + b][col][row], statistics per column; the box maximum per (column, band) stays in the lane
+template <typename T, bool VEC, bool FULL>
+__device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T *dst, char *smem, int64_t b, int64_t a0, int64_t c0,
+                                          int chunk, int band, int lane)
+{
+    constexpr int kPerStore = 16 / sizeof(T);               // rows of a column in 16 bytes
+    constexpr int kTransRows = kTransBytes / sizeof(T);     // rows gathered before a transposed store
+    const int64_t N = pp.N;
+    const bool inner = lane != 0 && lane != 31;
+    PairSums lo, hi;
+    lo.reset();
+    hi.reset();
+    Softmax sm[kLaneCols];
+    float best[kLaneCols];
+#pragma unroll
+    for (int k = 0; k < kLaneCols; ++k) {
+        sm[k] = softmax_of<T>(FULL || (c0 + k >= 0 && c0 + k < N) ? __ldg(pp.stats + (pp.B + b) * N + c0 + k) : make_float2(0.f, 1.f));
+        best[k] = 0.f;
+    }
+    // probabilities of two rows (16-bit types: a word per column, first row low), then the box sums two rows above each
+    const auto two_rows = [&](const Group<T> &g0, const Group<T> &g1, int64_t a, bool pool, uint32_t (&w)[kLaneCols][2]) {
+        float2 p[2][2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            p[0][k] = make_float2(sm[2 * k](g0.get(2 * k)), sm[2 * k + 1](g0.get(2 * k + 1)));
+            p[1][k] = make_float2(sm[2 * k](g1.get(2 * k)), sm[2 * k + 1](g1.get(2 * k + 1)));
+            if constexpr (sizeof(T) == 2) {
+                const uint32_t wx = DT<T>::aw_from(p[0][k].x, p[1][k].x), wy = DT<T>::aw_from(p[0][k].y, p[1][k].y);
+                w[2 * k][0] = wx;
+                w[2 * k + 1][0] = wy;
+                p[0][k] = make_float2(DT<T>::unpack(wx, 0), DT<T>::unpack(wy, 0));
+                p[1][k] = make_float2(DT<T>::unpack(wx, 1), DT<T>::unpack(wy, 1));
+            } else {
+                w[2 * k][0] = __float_as_uint(p[0][k].x);
+                w[2 * k][1] = __float_as_uint(p[1][k].x);
+                w[2 * k + 1][0] = __float_as_uint(p[0][k].y);
+                w[2 * k + 1][1] = __float_as_uint(p[1][k].y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float2 va = lo.push(p[i][0]), vb = hi.push(p[i][1]);
+            if (!pool) continue;
+            float box[kLaneCols];
+            box_sums(va, vb, box);
+#pragma unroll
+            for (int k = 0; k < kLaneCols; ++k)
+                if (FULL || a + i - 2 < N) best[k] = fmaxf(best[k], box[k]);
+        }
+    };
+    const auto load = [&](int64_t a) {
+        return load_group<T, VEC, FULL>(src + (FULL ? min(a, N - 1) : a) * N, c0, N, a >= 0 && a < N);
+    };
+    uint32_t w[kLaneCols][2];
+    Group<T> now[kPoolStep / 2], next[kPoolStep / 2];     // corr is read four rows ahead
+    next[0] = load(a0 - 2);
+    next[1] = load(a0 - 1);
+#pragma unroll
+    for (int i = 0; i < kPoolStep / 2; ++i) now[i] = load(a0 + i);
+    two_rows(next[0], next[1], a0 - 2, false, w);
+    for (int64_t a = a0; a < a0 + pp.band_rows; a += kPoolStep) {
+#pragma unroll
+        for (int i = 0; i < kPoolStep / 2; ++i) next[i] = load(a + kPoolStep / 2 + i);
+        uint32_t pend[kLaneCols][4];      // 16 bytes of rows of every column
+#pragma unroll
+        for (int i = 0; i < kPoolStep; i += 2) {
+            // the first two box sums of a band belong to the rows above it
+            if (i < kPoolStep / 2) {
+                two_rows(now[i % 4], now[i % 4 + 1], a + i, i > 0 || a > a0, w);
+            } else {
+                if (i == kPoolStep / 2) {
+#pragma unroll
+                    for (int j = 0; j < kPoolStep / 2; ++j) now[j] = load(a + kPoolStep + j);
+                }
+                two_rows(next[i % 4], next[i % 4 + 1], a + i, true, w);
+            }
+#pragma unroll
+            for (int k = 0; k < kLaneCols; ++k) {
+                if constexpr (sizeof(T) == 2) {
+                    pend[k][i / 2] = w[k][0];
+                } else {
+                    pend[k][i & 3] = w[k][0];
+                    pend[k][(i & 3) + 1] = w[k][1];
+                }
+            }
+            if ((i + 2) % kPerStore == 0) {
+                // column k of lane l in slot k * 32 + l: eight lanes' 16-byte pieces fall into different banks
+                const int at = static_cast<int>(a + i + 2 - kPerStore - a0) & (kTransRows - 1);
+#pragma unroll
+                for (int k = 0; k < kLaneCols; ++k)
+                    *reinterpret_cast<uint4 *>(smem + (k * 32 + lane) * kTransPitch + at * sizeof(T)) =
+                        make_uint4(pend[k][0], pend[k][1], pend[k][2], pend[k][3]);
+            }
+        }
+        if ((static_cast<int>(a + kPoolStep - a0) & (kTransRows - 1)) == 0) {
+            __syncwarp();
+            const int64_t row0 = a + kPoolStep - kTransRows, token0 = static_cast<int64_t>(chunk) * kPoolCols - kLaneCols;
+            if constexpr (VEC) {      // four lanes per column, eight columns per store
+                const int64_t row = row0 + (lane & 3) * kPerStore;
+#pragma unroll 4
+                for (int u = 0; u < kWarpCols; u += 8) {
+                    const int l = (u + (lane >> 2)) & 31, k = u >> 5;
+                    const int64_t token = token0 + l * kLaneCols + k;
+                    const uint4 v = *reinterpret_cast<const uint4 *>(smem + (k * 32 + l) * kTransPitch + (lane & 3) * 16);
+                    if (l != 0 && l != 31 && (FULL || (token < N && row < N))) *reinterpret_cast<uint4 *>(dst + token * N + row) = v;
+                }
+            } else {                  // 2-byte types: one column per store, float32: two
+                const int r = lane & (kTransRows - 1);
+#pragma unroll 4
+                for (int c = kLaneCols + lane / kTransRows; c < kWarpCols - kLaneCols; c += 32 / kTransRows) {
+                    const int64_t token = token0 + c;
+                    const T v = *reinterpret_cast<const T *>(smem + ((c & 3) * 32 + (c >> 2)) * kTransPitch + r * sizeof(T));
+                    if (FULL || (token < N && row0 + r < N)) dst[token * N + row0 + r] = v;
+                }
+            }
+            __syncwarp();
+        }
+    }
+    two_rows(now[0], now[1], a0 + pp.band_rows, true, w);
+    if (inner) {
+#pragma unroll
+        for (int k = 0; k < kLaneCols; ++k)
+            if (FULL || c0 + k < N) pp.col_max[(b * pp.bands + band) * N + c0 + k] = best[k];
     }
 }
 
-// per (b2, i): 5 x 5 window of probabilities around the clamped arg max -> expected target position - own position
-template <typename T>
-__global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__restrict__ prob, const int *__restrict__ arg_in,
-                                                                    T *__restrict__ flow, int *__restrict__ centre_out, int H, int W,
-                                                                    int64_t total, float tiny)
+// Both halves of prob and the maxima of the 5x5 box sums.  A warp takes 128 columns of corr (120 pooled, the outer
+// lanes are the halo) and walks down a band of rows (two more on either side); every lane keeps the running pair
+// sums of its four columns, so a box sum costs about four additions.  Blocks come in two roles that differ in what
+// the softmax runs over (pool_rows, pool_cols); a lane of the second gathers eight rows of its columns and stores
+// them as 16 bytes of a prob row, or, where rows of prob are not 16-byte aligned, through shared memory.
+// Eight consecutive blocks (four of either role) cover one 4-band x 4-chunk region, so the second role finds corr in L2.
+// Bound by instruction issue (about 25 per element and role, a third of them the exponential; 60 % of the slots busy).
+// Measured, float16, 16384 x 16384: 0.72 ms.  With 16-byte stores straight from the registers to 32 rows of prob the
+// second role alone took 0.67 ms; five blocks of four warps hold 20 warps per SM (0.75 ms with four blocks).
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(32 * kPoolWarps, 5) flow_prob_pool_kernel(const T *__restrict__ corr, T *__restrict__ prob, const PoolParams pp)
 {
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    const int64_t N = static_cast<int64_t>(H) * W;
-    const int64_t b2 = t / N, i = t - b2 * N;
-    const int arg = arg_in[t];
-    const int cy = min(max(arg / W, 2), H - 3), cx = min(max(arg % W, 2), W - 3);
-    const T *row = prob + (b2 * N + i) * N;
-    const float mean = DT<T>::rnd(static_cast<float>(1.0 / static_cast<double>(N)));   // the scalar is converted to T first
-    float p[25], sum = 0.f;
-#pragma unroll
-    for (int k = 0; k < 25; ++k) {
-        p[k] = load_one<T>(row + static_cast<int64_t>(cy + k / 5 - 2) * W + (cx + k % 5 - 2));
-        if (p[k] < mean) p[k] = 0.f;
-        sum += p[k];
+    extern __shared__ __align__(16) char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int chunk_groups = (pp.chunks + kPoolWarps - 1) / kPoolWarps;
+    const int region = blockIdx.x / (2 * kPoolWarps), within = blockIdx.x - region * 2 * kPoolWarps;
+    const int bg = region / chunk_groups, cg = region - bg * chunk_groups;
+    const bool cols = within >= kPoolWarps;
+    const int band = bg * kPoolWarps + (cols ? warp : within);
+    const int chunk = cg * kPoolWarps + (cols ? within - kPoolWarps : warp);
+    if (band >= pp.bands || chunk >= pp.chunks) return;
+    const int64_t b = blockIdx.y, N = pp.N;
+    const T *src = corr + b * N * N;
+    const int64_t a0 = static_cast<int64_t>(band) * pp.band_rows;
+    const int64_t first = static_cast<int64_t>(chunk) * kPoolCols - kLaneCols, c0 = first + lane * kLaneCols;
+    char *smem = smem_raw + warp * kPoolSmemPerWarp;
+    const bool full = a0 >= 2 && a0 + pp.band_rows + 2 <= N && first >= 0 && first + kWarpCols <= N;
+    if (!cols) {
+        T *dst = prob + b * N * N;
+        if (full) pool_rows<T, VEC, true>(pp, src, dst, smem, b, a0, c0, chunk, lane);
+        else pool_rows<T, VEC, false>(pp, src, dst, smem, b, a0, c0, chunk, lane);
+    } else {
+        T *dst = prob + (pp.B + b) * N * N;
+        if (full) pool_cols<T, VEC, true>(pp, src, dst, smem, b, a0, c0, chunk, band, lane);
+        else pool_cols<T, VEC, false>(pp, src, dst, smem, b, a0, c0, chunk, band, lane);
     }
+}
+
+// Per token (b2, i): the first target j whose 5x5 box average, rounded to T, is the largest, and the expected target
+// position within the 5x5 window of probabilities around it (clamped to the map) minus the token's own position.
+// The box maxima per chunk of targets screen the chunks: the average is monotone in the box sum, and the screening
+// sums are within kScreen of the ones that decide.  A block takes eight tokens: its threads scan the chunk maxima of
+// all of them, then every warp serves one: it sums the boxes of the chunks that pass (as a rule one) from prob, row by
+// row, lanes = targets, then takes the window, lanes = its 25 elements.  Latency-bound: a few dependent reads.
+constexpr float kScreen = 4e-6f;      // 24 float32 additions of positive terms in two different orders
+
+template <typename T>
+__global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__restrict__ prob, const float *__restrict__ row_max,
+                                                                   const float *__restrict__ col_max, T *__restrict__ flow,
+                                                                   T *__restrict__ blur_max, int *__restrict__ centre_out, int B, int H,
+                                                                   int W, int chunks, int bands, int band_rows, float tiny)
+{
+    constexpr int kGroups = kFlowThreads / kWindowTokens;
+    __shared__ float top[kWindowTokens][kGroups + 1];
+    __shared__ float rows[kFlowWarps][5][kWarpCols];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t N = static_cast<int64_t>(H) * W;
+    const int64_t b2 = blockIdx.y, i0 = static_cast<int64_t>(blockIdx.x) * kWindowTokens;
+    const bool cols = b2 >= B;
+    const int n = cols ? bands : chunks, width = cols ? band_rows : kPoolCols;
+    const float *maxima = (cols ? col_max + (b2 - B) * bands * N : row_max + b2 * chunks * N) + i0;
+    const auto average = [](float sum) { return DT<T>::rnd(__fdiv_rn(sum, 25.f)); };
+    {
+        const int t = threadIdx.x % kWindowTokens, g = threadIdx.x / kWindowTokens;
+        float m = 0.f;
+        if (i0 + t < N) {
+#pragma unroll 4
+            for (int c = g; c < n; c += kGroups) m = fmaxf(m, maxima[static_cast<int64_t>(c) * N + t]);
+        }
+        top[t][g] = m;
+    }
+    __syncthreads();
+    const int64_t i = i0 + warp;
+    if (i >= N) return;
+    const T *base = prob + b2 * N * N;
+    const float least = average(warp_max(top[warp][lane]) * (1.f - kScreen));
+    float bv = -1.f;
+    int bj = 0x7fffffff;
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const float m = c0 + lane < n ? maxima[static_cast<int64_t>(c0 + lane) * N + warp] : 0.f;
+        unsigned pass = __ballot_sync(0xffffffffu, c0 + lane < n && average(m * (1.f + kScreen)) >= least);
+        for (; pass != 0; pass &= pass - 1) {
+            const int64_t first = static_cast<int64_t>(c0 + __ffs(pass) - 1) * width;
+#pragma unroll
+            for (int k = 0; k < kWarpCols / 32; ++k) {
+                const int64_t j = first - 2 + lane + 32 * k;
+                float p[5];
+#pragma unroll
+                for (int d = 0; d < 5; ++d) {
+                    const int64_t ii = i + d - 2;
+                    p[d] = (ii >= 0 && ii < N && j >= 0 && j < N && j < first + width + 2) ? load_one<T>(base + ii * N + j) : 0.f;
+                }
+#pragma unroll
+                for (int d = 0; d < 5; ++d) rows[warp][d][lane + 32 * k] = p[d];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < kWarpCols / 32; ++k) {
+                const int c = lane + 32 * k;
+                if (c < width && c + 4 < kWarpCols && first + c < N) {
+                    float sum = 0.f;
+#pragma unroll
+                    for (int d = 0; d < 5; ++d)
+#pragma unroll
+                        for (int e = 0; e < 5; ++e) sum += rows[warp][d][c + e];
+                    const float v = average(sum);
+                    if (v > bv) {
+                        bv = v;
+                        bj = static_cast<int>(first) + c;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {      // larger value wins, equal values keep the smaller index
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
+        if (ov > bv || (ov == bv && oj < bj)) {
+            bv = ov;
+            bj = oj;
+        }
+    }
+    const int cy = min(max(bj / W, 2), H - 3), cx = min(max(bj % W, 2), W - 3);
+    const float mean = DT<T>::rnd(static_cast<float>(1.0 / static_cast<double>(N)));   // the scalar is converted to T first
+    const int tx = cx + lane % 5 - 2, ty = cy + lane / 5 - 2;
+    float p = lane < 25 ? load_one<T>(base + i * N + static_cast<int64_t>(ty) * W + tx) : 0.f;
+    if (p < mean) p = 0.f;
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 25; ++k) sum += __shfl_sync(0xffffffffu, p, k);
     sum = fmaxf(DT<T>::rnd(sum), tiny);
+    const float np = DT<T>::rnd(__fdiv_rn(p, sum));
+    const float px = DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(tx))), py = DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(ty)));
     float ax = 0.f, ay = 0.f;
 #pragma unroll
     for (int k = 0; k < 25; ++k) {
-        const float np = DT<T>::rnd(__fdiv_rn(p[k], sum));
-        ax += DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(cx + k % 5 - 2)));
-        ay += DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(cy + k / 5 - 2)));
+        ax += __shfl_sync(0xffffffffu, px, k);
+        ay += __shfl_sync(0xffffffffu, py, k);
     }
-    const int qy = static_cast<int>(i / W), qx = static_cast<int>(i - static_cast<int64_t>(qy) * W);
-    store_one<T>(flow + t * 2, DT<T>::rnd(DT<T>::rnd(ax) - DT<T>::rnd(static_cast<float>(qx))));
-    store_one<T>(flow + t * 2 + 1, DT<T>::rnd(DT<T>::rnd(ay) - DT<T>::rnd(static_cast<float>(qy))));
-    if (centre_out != nullptr) centre_out[t] = cy * W + cx;
+    if (lane == 0) {
+        const int64_t at = b2 * N + i;
+        const int qy = static_cast<int>(i / W), qx = static_cast<int>(i - static_cast<int64_t>(qy) * W);
+        store_one<T>(flow + at * 2, DT<T>::rnd(DT<T>::rnd(ax) - DT<T>::rnd(static_cast<float>(qx))));
+        store_one<T>(flow + at * 2 + 1, DT<T>::rnd(DT<T>::rnd(ay) - DT<T>::rnd(static_cast<float>(qy))));
+        if (centre_out != nullptr) centre_out[at] = cy * W + cx;
+        if (blur_max != nullptr) store_one<T>(blur_max + at, bv);
+    }
+}
+
+template <typename T, bool VEC>
+cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow, T *blur, int *centre, char *scratch, int B, int H,
+                             int W, float tiny, cudaStream_t stream)
+{
+    const int64_t N = pl.N;
+    float *row_part = reinterpret_cast<float *>(scratch), *col_part = reinterpret_cast<float *>(scratch + pl.off_col);
+    float2 *stats = reinterpret_cast<float2 *>(scratch + pl.off_stats);
+    float *row_max = reinterpret_cast<float *>(scratch + pl.off_row_max), *col_max = reinterpret_cast<float *>(scratch + pl.off_col_max);
+    const int64_t units = static_cast<int64_t>(pl.row_parts) * pl.col_parts;
+    flow_max_kernel<T, VEC><<<dim3(static_cast<unsigned>((units + kFlowWarps - 1) / kFlowWarps), B), kFlowThreads, 0, stream>>>(
+        corr, row_part, col_part, N, pl.max_rows, pl.row_parts, pl.col_parts);
+    const auto launch_sums = [&](auto columns, auto batch) {
+        constexpr int kColumns = decltype(columns)::value, kThreadsHere = kColumns * kSumGroups, kRows = kThreadsHere / 32;
+        const int col_blocks = static_cast<int>((N + kColumns - 1) / kColumns);
+        flow_sum_kernel<T, VEC, kColumns, decltype(batch)::value>
+            <<<dim3(static_cast<unsigned>(col_blocks + (N + kRows - 1) / kRows), B), kThreadsHere, 0, stream>>>(
+                corr, row_part, col_part, stats, N, pl.row_parts, pl.col_parts, col_blocks);
+    };
+    // up to about 5000 tokens 64-column blocks would leave SMs without work
+    if (N >= 5000) launch_sums(std::integral_constant<int, 64>(), std::integral_constant<int, 16>());
+    else launch_sums(std::integral_constant<int, 16>(), std::integral_constant<int, 32>());
+    constexpr int smem = kPoolWarps * kPoolSmemPerWarp;
+    const cudaError_t e = cudaFuncSetAttribute(flow_prob_pool_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t regions = static_cast<int64_t>((pl.bands + kPoolWarps - 1) / kPoolWarps) * ((pl.chunks + kPoolWarps - 1) / kPoolWarps);
+    flow_prob_pool_kernel<T, VEC><<<dim3(static_cast<unsigned>(regions * 2 * kPoolWarps), B), 32 * kPoolWarps, smem, stream>>>(
+        corr, prob, PoolParams{stats, row_max, col_max, N, B, pl.band, pl.chunks, pl.bands});
+    flow_window_kernel<T><<<dim3(static_cast<unsigned>((N + kWindowTokens - 1) / kWindowTokens), 2 * B), kFlowThreads, 0, stream>>>(
+        prob, row_max, col_max, flow, blur, centre, B, H, W, pl.chunks, pl.bands, pl.band, tiny);
+    return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t run_flow_init(const void *corr_, void *prob_, void *flow_, void *blur_, int *centre, void *scratch, int B, int H,
                           int W, float tiny, cudaStream_t stream)
 {
-    const int64_t N = static_cast<int64_t>(H) * W;
+    const FlowPlan pl = flow_plan(B, H, W);
     const T *corr = static_cast<const T *>(corr_);
-    T *prob = static_cast<T *>(prob_);
-    float *cmax = static_cast<float *>(scratch), *csum = cmax + B * N;
-    int *arg = reinterpret_cast<int *>(csum + B * N);
-    flow_row_softmax_kernel<T><<<dim3(static_cast<unsigned>(N), B), kFlowThreads, 0, stream>>>(corr, prob, N);
-    flow_col_stats_kernel<T><<<dim3(static_cast<unsigned>((N + 63) / 64), B), kFlowThreads, 0, stream>>>(corr, cmax, csum, N);
-    const unsigned tiles = static_cast<unsigned>((N + 31) / 32);
-    flow_transposed_softmax_kernel<T><<<dim3(tiles, tiles, B), kFlowThreads, 0, stream>>>(corr, cmax, csum, prob + B * N * N, N);
-    flow_pool_argmax_kernel<T><<<dim3(static_cast<unsigned>((N + kPoolRows - 1) / kPoolRows), 2 * B), kFlowThreads, 0, stream>>>(
-        prob, static_cast<T *>(blur_), arg, N);
-    const int64_t total = 2 * B * N;
-    flow_window_kernel<T><<<static_cast<unsigned>((total + kFlowThreads - 1) / kFlowThreads), kFlowThreads, 0, stream>>>(
-        prob, arg, static_cast<T *>(flow_), centre, H, W, total, tiny);
-    return cudaGetLastError();
+    T *prob = static_cast<T *>(prob_), *flow = static_cast<T *>(flow_), *blur = static_cast<T *>(blur_);
+    // groups of four columns and of 16 bytes of rows: every row of corr and prob starts 16-byte aligned
+    const bool vec = pl.N % 8 == 0 && (reinterpret_cast<uintptr_t>(corr_) & 15u) == 0 && (reinterpret_cast<uintptr_t>(prob_) & 15u) == 0;
+    char *ws = static_cast<char *>(scratch);
+    return vec ? run_flow_kernels<T, true>(pl, corr, prob, flow, blur, centre, ws, B, H, W, tiny, stream)
+               : run_flow_kernels<T, false>(pl, corr, prob, flow, blur, centre, ws, B, H, W, tiny, stream);
 }
 
 }  // namespace
@@ -264,7 +794,7 @@ cudaError_t run_flow_init(const void *corr_, void *prob_, void *flow_, void *blu
 extern "C" size_t matchattn_flow_init_scratch_bytes(int B, int H, int W)
 {
     if (B <= 0 || H <= 0 || W <= 0) return 0;
-    return static_cast<size_t>(B) * H * W * (2 * sizeof(float) + 2 * sizeof(int));
+    return matchattn::flow_plan(B, H, W).bytes;
 }
 
 extern "C" int matchattn_flow_init(const void *correlation, void *prob, void *flow, void *blur_max, int *centre,

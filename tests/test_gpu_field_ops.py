@@ -140,3 +140,25 @@ def test_flow_init_kernels_match_reference_on_the_gpu(dtype, H, W):
     clear = ((top2[..., 0] - top2[..., 1]) > (1e-6 if dtype == torch.float32 else 0.0)).view(2 * B, H, W)
     assert clear.float().mean() > 0.5
     assert _close16(flow[clear], want_flow[clear], dtype, ulps=2.0)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H,W,sharpness", [(5, 5, 2.0), (8, 15, 2.0), (11, 11, 2.0), (8, 16, 2.0), (5, 51, 2.0), (16, 16, 300.0),
+                                           (72, 72, 2.0)])
+def test_flow_init_kernels_at_the_edges_of_their_tiles(H, W, sharpness, dtype):
+    """Token counts around one chunk of 120 / 128 targets and one band of rows, rows of prob that are and are not
+    16-byte aligned, the long bands of large maps, and scores spread so widely that no shared reference serves a tile."""
+    import oracle
+    g = torch.Generator().manual_seed(H * W)
+    second = torch.randn(1, H * W, 16, generator=g)
+    first = second.roll(3, 1) + 0.3 * torch.randn(1, H * W, 16, generator=g)
+    corr = (torch.matmul(first, second.transpose(1, 2)) * sharpness / 4.0).to(dtype)
+    want_flow, want_prob, want_blur, want_centre = oracle.flow_init(corr, H, W)
+    flow, prob, blur, centre = _ma().flow_init(corr.cuda(), H, W, return_debug=True)
+    steps = ((prob.float().cpu() - want_prob.float()).abs() - 2.0 ** -24).clamp_min(0)     # float16: below 2^-14 the spacing is 2^-24
+    assert _close16(want_prob.float() + steps, want_prob, dtype) and _close16(blur, want_blur, dtype)
+    same = centre.cpu() == want_centre
+    assert same.float().mean() > 0.98           # the rest: equal box averages
+    off = (flow.cpu().float().view(-1, H * W, 2)[same] - want_flow.float().view(-1, H * W, 2)[same]).abs().max().item()
+    limit = 1e-3 if dtype == torch.float32 else 2.0 * float(ulp16(torch.tensor(float(max(H, W))), dtype))
+    assert off <= limit         # the flow is a position on the map, rounded, minus the token's own
