@@ -1,15 +1,19 @@
-"""ctypes binding of libmatchattn_b200.so (the C ABI in include/matchattn.h).
+"""ctypes binding of libmatchattn_b200.so (the C ABI in include/matchattn.h), and
+the host extension _host.so that ops.py calls on its eager paths.
 
-The library is loaded from matchattention_b200/lib/.  There is no fallback: if
-it is missing, importing this module raises, and so does every op.
+Both are loaded from matchattention_b200/lib/.  There is no fallback: if one is
+missing, importing this module raises, and so does every op.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libmatchattn_b200.so")
+HOST_PATH = os.path.join(_PKG, "lib", "_host.so")
 
 # every symbol include/matchattn.h declares
 EXPORTS = ("matchattn_fused_forward", "matchattn_fused_forward_ex", "matchattn_fused_forward_ws",
@@ -74,7 +78,18 @@ def _load() -> ctypes.CDLL:
     return lib
 
 
+def _load_host():
+    if not os.path.exists(HOST_PATH):
+        raise ImportError(f"{HOST_PATH} is missing: build it first with `python -m matchattention_b200.build`")
+    import torch  # noqa: F401  (the extension's symbols come from torch's libraries)
+    loader = importlib.machinery.ExtensionFileLoader(__package__ + "._host", HOST_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+    loader.exec_module(module)
+    return module
+
+
 lib = _load()
+host = _load_host()
 
 
 def strerror(status: int) -> str:

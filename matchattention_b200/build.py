@@ -1,11 +1,12 @@
-"""Builds libmatchattn_b200.so for sm_100a, in-tree, with nvcc alone.
+"""Builds libmatchattn_b200.so for sm_100a, in-tree, with nvcc alone, and the host extension _host.so on top of it.
 
     python -m matchattention_b200.build [--force]
 
 The translation units (C ABI, one per element type, the built-in scratch area) are compiled in
 parallel and linked into matchattention_b200/lib/libmatchattn_b200.so.  The
 library carries its own static CUDA runtime and has no Python or torch
-dependency.
+dependency; _host.so (csrc/host_binding.cpp, the eager entry points of ops.py)
+is compiled with g++ against the running Python and torch and links to it.
 """
 from __future__ import annotations
 
@@ -14,12 +15,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 OBJ_DIR = os.path.join(PKG, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libmatchattn_b200.so")
+HOST_PATH = os.path.join(LIB_DIR, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host_binding.cpp")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 SOURCES = ["matchattn_api.cu", "matchattn_f32.cu", "matchattn_f16.cu", "matchattn_bf16.cu",
@@ -45,6 +49,26 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > built for d in deps)
 
 
+def _build_host() -> None:
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    include = [sysconfig.get_paths()["include"], os.path.join(root, "include"),
+               os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in include], HOST_SOURCE,
+           "-o", HOST_PATH, f"-L{LIB_DIR}", "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
+           "-L" + os.path.join(root, "lib"), "-lc10", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SOURCE}:\n{res.stdout}\n{res.stderr}")
+
+
+def _host_stale() -> bool:
+    deps = (HOST_SOURCE, os.path.join(INCLUDE, "matchattn.h"))
+    return not os.path.exists(HOST_PATH) or any(os.path.getmtime(d) > os.path.getmtime(HOST_PATH) for d in deps)
+
+
 def _compile(src: str) -> tuple[str, str]:
     obj = os.path.join(OBJ_DIR, src.replace(".cu", ".o"))
     extra = os.environ.get("MATCHATTN_NVCC_EXTRA", "").split()      # e.g. -DMATCHATTN_FAST_EXP=1 for experiments
@@ -56,8 +80,14 @@ def _compile(src: str) -> tuple[str, str]:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not _stale():
-        return LIB_PATH
+    if force or _stale():
+        _build_library(verbose)
+    if force or _host_stale():
+        _build_host()
+    return LIB_PATH
+
+
+def _build_library(verbose: bool) -> None:
     os.makedirs(LIB_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
     with concurrent.futures.ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
@@ -71,7 +101,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
-    return LIB_PATH
 
 
 if __name__ == "__main__":

@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "matchattn_kernels.cuh"
 #include "matchattn_mma.cuh"
 #include "matchattn_binned.cuh"
@@ -193,13 +195,17 @@ Plan make_plan(int h, int hd, int r, int cpl_request)
     return pl;
 }
 
-// SMs of the current device (148 when the query fails)
+// SMs of the current device (148 when the query fails); asked once per device
 inline int sm_count()
 {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return 148;
-    return sms > 0 ? sms : 148;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev < kDevices && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    if (dev < kDevices) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
 }
 
 inline bool aligned(const void *p, uintptr_t a) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -513,10 +519,7 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
             bp.TX = gmt.TX; bp.TY = gmt.TY; bp.RW = gmt.RW; bp.RH = gmt.RH; bp.region_bytes = gmt.region_bytes;
             cudaError_t err = cudaMemsetAsync(bp.counts, 0, 4 * static_cast<size_t>(gmt.nbins) + 4 * kCtrlWords, stream);
             if (err != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(err);
-            int dev = 0, sms = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            const int grid_blocks = 2 * (sms > 0 ? sms : 148);
+            const int grid_blocks = 2 * sm_count();
             const size_t smem_bytes = 2 * static_cast<size_t>(gmt.region_bytes);
             const int main_cpl = strategy == kStrategyBinned ? pl.cpl : 0;     // 0: sorting passes only
             err = dtype == MATCHATTN_F16 ? launch_binned<__half>(bp, main_cpl, grid_blocks, smem_bytes, stream)

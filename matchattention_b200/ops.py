@@ -15,6 +15,11 @@ Differences, all on the safe side: arguments are validated (shape, dtype,
 device, contiguity) and violations raise; the launch goes to PyTorch's current
 stream; nothing is allocated or synchronised inside the call; outputs need not
 be zero-filled.  Inputs must be CUDA tensors: there is no CPU path.
+
+Ordinary eager calls go through the extension in csrc/host_binding.cpp, which
+checks the arguments, allocates the outputs and launches in one step (about 6 us
+instead of 15 to 60 us in Python).  It answers None for whatever it does not
+cover; the Python code here then handles the call or words the error.
 """
 from __future__ import annotations
 
@@ -30,6 +35,8 @@ from . import _lib
 # MATCHATTN_B200_NVTX=1 wraps every operator launch in an NVTX range named after its shape, so that a
 # profiler's NVTX filter can pick the operator out of a model's timeline (off by default: two extra calls)
 _NVTX = os.environ.get("MATCHATTN_B200_NVTX", "0") not in ("", "0")
+
+_host = _lib.host
 
 _DTYPE_CODE = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
@@ -116,9 +123,12 @@ def launch(max_offset, q, k, v, output, attn_out, H: int, W: int, win_r, attn_ty
     nothing.  The tuning knobs (tile_w, force_generic, chunks_per_lane, variant) belong to the
     direct kernels and imply strategy 1.
     """
-    rx, ry = _window_radius(win_r)
     if q_row_end is None:
         q_row_end = H
+    if strategy == STRATEGY_AUTO and workspace is None and not (tile_w or force_generic or chunks_per_lane or variant or _NVTX) \
+            and _host.launch(max_offset, q, k, v, output, attn_out, H, W, win_r, attn_type, scale, q_row_begin, q_row_end):
+        return
+    rx, ry = _window_radius(win_r)
     if attn_type not in _lib.ATTN_TYPE_CODE:
         raise NotImplementedError(f"attn_type {attn_type!r}: 'l1_norm' and 'dot_product' exist")
     attn_num = (2 * rx + 2) * (2 * ry + 2)
@@ -213,6 +223,10 @@ class MF_FusedForwardOps(nn.Module):
     def forward(self, max_offset: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, H: int, W: int,
                 win_r: List[int], attn_num: int, attn_type: str = "l1_norm",
                 scale: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
+        if not torch.compiler.is_compiling() and not _NVTX:      # a compiler traces the opaque custom op below instead
+            done = _host.module_forward(max_offset, q, k, v, H, W, win_r, attn_num, attn_type, scale)
+            if done is not None:
+                return done
         if torch.is_grad_enabled() and any(t.requires_grad for t in (max_offset, q, k, v)):
             rx, ry = _window_radius(win_r)
             if attn_type != "l1_norm" or rx != ry:
@@ -248,46 +262,16 @@ def describe_dispatch(h: int, hd: int, r: int, dtype: torch.dtype, aligned32: bo
 
 # ---- training: the operator as an autograd function ------------------------------------------------
 
-class _MatchAttentionFn(torch.autograd.Function):
-    """Forward = the fused kernel; backward = matchattn_fused_backward.  Nothing but the inputs is saved:
-    the backward kernel recomputes scores and softmaxes."""
-
-    @staticmethod
-    def forward(ctx, max_offset, q, k, v, H, W, r, scale):
-        out = torch.empty_like(q)
-        attn = q.new_empty(q.size(0), q.size(1), max_offset.size(2), (2 * r + 2) ** 2)
-        launch(max_offset, q, k, v, out, attn, H, W, (r, r), "l1_norm", scale)
-        ctx.save_for_backward(max_offset, q, k, v)
-        ctx.geometry = (H, W, r, scale)
-        return out, attn
-
-    @staticmethod
-    def backward(ctx, d_out, d_attn):
-        max_offset, q, k, v = ctx.saved_tensors
-        H, W, r, scale = ctx.geometry
-        B, Nq, C = q.shape
-        h = max_offset.size(2)
-        d_q = torch.empty_like(q)
-        d_mo = torch.empty_like(max_offset) if ctx.needs_input_grad[0] else None
-        d_k = torch.zeros(k.shape, dtype=torch.float32, device=k.device)
-        d_v = torch.zeros(v.shape, dtype=torch.float32, device=v.device)
-        d_out = d_out.contiguous()
-        d_attn = d_attn.contiguous() if d_attn is not None else None
-        with torch.cuda.device(q.device):
-            status = _lib.lib.matchattn_fused_backward(
-                max_offset.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), d_out.data_ptr(),
-                d_attn.data_ptr() if d_attn is not None else None, d_q.data_ptr(), d_k.data_ptr(), d_v.data_ptr(),
-                d_mo.data_ptr() if d_mo is not None else None, B, H, W, h, C // h, r, r, _DTYPE_CODE[q.dtype],
-                _lib.L1_NORM, float(scale), 0, H, torch.cuda.current_stream().cuda_stream)
-        _lib.check(status)
-        return d_mo, d_q, d_k.to(k.dtype), d_v.to(v.dtype), None, None, None, None
-
-
 def match_attention_autograd(max_offset, q, k, v, H: int, W: int, r: int, scale: float):
     """The operator for training: (out, attn) with gradients to q, k, v and max_offset, as autograd gives them
-    for the reference's 'pytorch' path (its native path has no backward).  Contiguous CUDA tensors."""
-    return _MatchAttentionFn.apply(max_offset.contiguous(), q.contiguous(), k.contiguous(), v.contiguous(), H, W, r,
-                                   float(scale))
+    for the reference's 'pytorch' path (its native path has no backward).  CUDA tensors.  Nothing but the inputs is
+    saved: the backward kernel recomputes scores and softmaxes.  (The autograd node is in csrc/host_binding.cpp.)"""
+    tensors = tuple(t.contiguous() for t in (max_offset, q, k, v))
+    done = _host.autograd(*tensors, H, W, r, scale)
+    if done is None:
+        _check_tensors(*tensors, tensors[1], None, H, W, H, (2 * r + 2) ** 2)
+        raise NotImplementedError("match_attention_autograd does not run under functional transforms")
+    return done
 
 
 # ---- the caller's glue folded into the kernel ------------------------------------------------
@@ -326,6 +310,9 @@ def cross_attention_core(max_offset, q, k, v, gate, H: int, W: int, r: int, scal
     (b + kv_shift) mod B, so with B // 2 the caller passes K and V of the un-swapped batch.
 
     Returns a [B, N, C + h*(2r+2)^2] tensor ready for ``proj``."""
+    done = _host.cross_core(max_offset, q, k, v, gate, H, W, r, scale, clamp, kv_shift)
+    if done is not None:
+        return done
     B, N, C = q.shape
     h = max_offset.size(2)
     M = (2 * r + 2) ** 2
@@ -339,6 +326,9 @@ def cross_attention_core(max_offset, q, k, v, gate, H: int, W: int, r: int, scal
 def self_attention_core(max_offset, q, k, v, H: int, W: int, r: int, scale: float, clamp: bool = True):
     """The self branch (models/attention_blocks.py:79-93,99): clamp + operator; the attention weights,
     which that branch discards, are never written.  Returns out [B, N, C]."""
+    done = _host.self_core(max_offset, q, k, v, H, W, r, scale, clamp)
+    if done is not None:
+        return done
     out = torch.empty_like(q)
     launch_glue(max_offset, q, k, v, None, out.data_ptr(), None, H, W, r, scale, clamp=clamp)
     return out
@@ -347,6 +337,9 @@ def self_attention_core(max_offset, q, k, v, H: int, W: int, r: int, scale: floa
 def upsample_field(field: torch.Tensor, mask: torch.Tensor, factor: int) -> torch.Tensor:
     """Convex upsampling of a field, same arguments and result as ``MatchStereo.upsample_field``
     (models/match_stereo.py:73-84): field [B,H,W,D], mask [B,9*f*f,H,W] -> [B,f*H,f*W,D], one kernel."""
+    done = _host.upsample_field(field, mask, factor)
+    if done is not None:
+        return done
     if not field.is_cuda:
         raise RuntimeError("matchattn_b200 runs on CUDA tensors only (no CPU fallback); got device " + str(field.device))
     if field.dtype not in _DTYPE_CODE or mask.dtype != field.dtype or mask.device != field.device:
@@ -373,6 +366,9 @@ def stereo_volume(correlation: torch.Tensor) -> torch.Tensor:
     """The cost volume GlobalCorrelation builds from its row-wise correlation in the stereo branch
     (models/cost_volume.py:26-51): correlation [B,H,W,W] -> volume [2B,W,H,W] (softmaxed over the
     disparity axis, out-of-view columns filled), one kernel instead of the loops over disparities."""
+    done = _host.stereo_volume(correlation)
+    if done is not None:
+        return done
     if not correlation.is_cuda:
         raise RuntimeError("matchattn_b200 runs on CUDA tensors only (no CPU fallback); got device "
                            + str(correlation.device))
@@ -394,6 +390,10 @@ def consistency_mask(field: torch.Tensor, threshold: float = 2.0, return_diff: b
     """Same argument and result as ``MatchAttentionLayer.consistency_mask(field, A)``
     (models/attention_blocks.py:130-138): field [B,H,W,2] (two views stacked on the batch) ->
     noc_mask [B,H,W,1], one kernel.  ``return_diff`` also returns the thresholded quantity."""
+    if not return_diff:
+        done = _host.consistency_mask(field, threshold)
+        if done is not None:
+            return done
     if not field.is_cuda:
         raise RuntimeError("matchattn_b200 runs on CUDA tensors only (no CPU fallback); got device " + str(field.device))
     if field.dtype not in _DTYPE_CODE:
@@ -417,6 +417,10 @@ def local_disparity_estimator(volume: torch.Tensor, return_debug: bool = False):
     """Same argument and result as ``local_disparity_estimator(cv)`` (models/cost_volume.py:123-167, with
     disp_to_flow :169-178): cost volume [B,D,H,W] -> field [B,H,W,2], one kernel.  ``return_debug``
     also returns the blurred maximum [B,H,W] and the window centre [B,H,W] (int32)."""
+    if not return_debug:
+        done = _host.local_disparity(volume)
+        if done is not None:
+            return done
     if not volume.is_cuda:
         raise RuntimeError("matchattn_b200 runs on CUDA tensors only (no CPU fallback); got device " + str(volume.device))
     if volume.dtype not in _DTYPE_CODE:
@@ -441,6 +445,10 @@ def flow_init(correlation: torch.Tensor, H: int, W: int, return_debug: bool = Fa
     """What GlobalCorrelation.forward does after its matmul when ``stereo=False`` (models/cost_volume.py:61-69,
     with local_flow_estimator :71-121): correlation [B,N,N] (N = H*W) -> (flow [2B,H,W,2], prob [2B,H,W,N]).
     ``return_debug`` adds the pooled maximum [2B,N] and the clamped window centre [2B,N] (int32)."""
+    if not return_debug:
+        done = _host.flow_init(correlation, H, W)
+        if done is not None:
+            return done
     if not correlation.is_cuda:
         raise RuntimeError("matchattn_b200 runs on CUDA tensors only (no CPU fallback); got device "
                            + str(correlation.device))

@@ -122,3 +122,34 @@ def test_checked_entry_point_finds_no_stray_index():
         torch.cuda.synchronize()
         same = lambda a, b: torch.equal(torch.nan_to_num(a.float(), nan=7.0), torch.nan_to_num(b.float(), nan=7.0))
         assert same(out, want_out) and same(attn, want_attn)
+
+
+@pytest.mark.parametrize("around", ["plain", "parameter", "subclass", "device_mode", "dispatch_mode", "inference_mode", "training"])
+def test_host_extension_and_python_path_agree(case, around):
+    """Ordinary calls are served by the host extension; subclasses and dispatch modes take the Python path."""
+    import contextlib
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from matchattention_b200 import MF_FusedForwardOps, self_attention_core
+
+    class Sub(torch.Tensor):
+        pass
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    mo, q, k, v = case["gpu"]
+    if around == "parameter":
+        q = torch.nn.Parameter(q, requires_grad=False)
+    if around == "subclass":
+        q = q.as_subclass(Sub)
+    if around == "training":
+        q = q.clone().requires_grad_(True)
+    context = {"device_mode": torch.device("cuda"), "dispatch_mode": Mode(), "inference_mode": torch.inference_mode()}
+    with context.get(around, contextlib.nullcontext()):
+        out, attn = MF_FusedForwardOps()(mo, q, k, v, case["H"], case["W"], [1, 1], 16, scale=case["scale"])
+        own = self_attention_core(mo, q.detach(), k, v, case["H"], case["W"], 1, case["scale"], clamp=False)
+    assert_close(out, case["ref"][0], torch.float16)
+    assert_close(attn, case["ref"][1], torch.float16)
+    assert_close(own, case["ref"][0], torch.float16)
+    assert out.requires_grad == (around == "training")
