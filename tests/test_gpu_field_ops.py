@@ -162,3 +162,18 @@ def test_flow_init_kernels_at_the_edges_of_their_tiles(H, W, sharpness, dtype):
     off = (flow.cpu().float().view(-1, H * W, 2)[same] - want_flow.float().view(-1, H * W, 2)[same]).abs().max().item()
     limit = 1e-3 if dtype == torch.float32 else 2.0 * float(ulp16(torch.tensor(float(max(H, W))), dtype))
     assert off <= limit         # the flow is a position on the map, rounded, minus the token's own
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("D,H,W", [(5, 1, 31), (7, 3, 11), (40, 2, 33), (63, 5, 13), (159, 2, 17)])
+def test_local_disparity_kernel_at_the_edges_of_its_shares(D, H, W, dtype):
+    """Disparity counts that leave shares short or empty, and pixel counts around one warp."""
+    import oracle
+    g = torch.Generator().manual_seed(D)
+    vol = torch.softmax(torch.randn(2, D, H, W, generator=g) * 2.0, dim=1).to(dtype)
+    want_flow, want_blur, want_centre = oracle.local_disparity(vol)
+    flow, blur, centre = _ma().local_disparity_estimator(vol.cuda(), return_debug=True)
+    assert _close16(blur, want_blur, dtype)
+    same = centre.cpu() == want_centre
+    assert same.float().mean() > 0.98           # the rest: equal box averages
+    assert _close16(flow.cpu()[same], want_flow[same], dtype)

@@ -36,3 +36,12 @@ def test_too_wide_rows_are_refused():
     import matchattention_b200 as ma
     with pytest.raises(RuntimeError):
         ma.stereo_volume(torch.zeros(1, 2, 200, 200, device="cuda"))
+
+
+@pytest.mark.parametrize("W", [2, 31, 32, 64, 65, 97, 128, 129, 159])
+def test_kernel_at_the_edges_of_its_pieces(W):
+    import matchattention_b200 as ma
+    import oracle
+    g = torch.Generator().manual_seed(W)
+    corr = torch.randn(1, 2, W, W, generator=g) * 3
+    assert_close(ma.stereo_volume(corr.cuda()).cpu(), oracle.stereo_volume(corr), torch.float32)
