@@ -180,6 +180,25 @@ MATCHATTN_API int matchattn_fused_backward(const void *max_offset, const void *q
                                            int q_row_begin, int q_row_end, void *cuda_stream);
 
 /*
+ * The same gradients with scratch memory from the caller and d_k, d_v in the tensor type, WRITTEN rather than
+ * accumulated: the (query, head) items are bucketed by the token their window starts at, and every token sums the
+ * contributions of the buckets around it (no floating-point atomics).  About three times as fast as the call above
+ * plus the clearing and conversion around it.  Covered: head widths that are multiples of 8, r = 1 or 2, 16-byte
+ * aligned arrays; MATCHATTN_ERR_VARIANT otherwise.
+ *   workspace  at least matchattn_backward_workspace_bytes(...) bytes of device memory, 256-byte aligned; contents
+ *              need not be preserved between calls, but calls that overlap on the device must not share it
+ */
+MATCHATTN_API size_t matchattn_backward_workspace_bytes(int B, int H, int W, int h, int hd, int r, int dtype,
+                                                        int q_row_begin, int q_row_end);
+MATCHATTN_API int matchattn_fused_backward_ws(const void *max_offset, const void *q, const void *k, const void *v,
+                                              const void *d_out, const void *d_attn,
+                                              void *d_q, void *d_k, void *d_v, void *d_max_offset,
+                                              int B, int H, int W, int h, int hd, int rx, int ry,
+                                              int dtype, int attn_type, float scale,
+                                              int q_row_begin, int q_row_end,
+                                              void *workspace, size_t workspace_bytes, void *cuda_stream);
+
+/*
  * The same operator with scratch memory from the caller, which opens the binned
  * path: the queries are counting-sorted by the tile of the token map their window
  * falls into and each tile of K/V is staged in shared memory once for all the

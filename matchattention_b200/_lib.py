@@ -18,7 +18,8 @@ HOST_PATH = os.path.join(_PKG, "lib", "_host.so")
 # every symbol include/matchattn.h declares
 EXPORTS = ("matchattn_fused_forward", "matchattn_fused_forward_ex", "matchattn_fused_forward_ws",
            "matchattn_fused_forward_static", "matchattn_fused_forward_glue", "matchattn_fused_forward_checked",
-           "matchattn_fused_backward", "matchattn_upsample_field",
+           "matchattn_fused_backward", "matchattn_fused_backward_ws", "matchattn_backward_workspace_bytes",
+           "matchattn_upsample_field",
            "matchattn_stereo_volume", "matchattn_consistency_mask", "matchattn_local_disparity",
            "matchattn_flow_init", "matchattn_flow_init_scratch_bytes", "matchattn_copy_blocks",
            "matchattn_workspace_bytes", "matchattn_describe_dispatch", "matchattn_version", "matchattn_strerror")
@@ -50,6 +51,10 @@ def _load() -> ctypes.CDLL:
     lib.matchattn_fused_forward_checked.argtypes = [_vp] * 6 + [_i] * 9 + [_f, _i, _i, _vp, _vp]
     lib.matchattn_fused_backward.restype = _i
     lib.matchattn_fused_backward.argtypes = [_vp] * 10 + [_i] * 9 + [_f, _i, _i, _vp]
+    lib.matchattn_fused_backward_ws.restype = _i
+    lib.matchattn_fused_backward_ws.argtypes = [_vp] * 10 + [_i] * 9 + [_f, _i, _i, _vp, ctypes.c_size_t, _vp]
+    lib.matchattn_backward_workspace_bytes.restype = ctypes.c_size_t
+    lib.matchattn_backward_workspace_bytes.argtypes = [_i] * 9
     lib.matchattn_fused_forward_glue.restype = _i
     lib.matchattn_fused_forward_glue.argtypes = [_vp] * 7 + [_i] * 9 + [_f, _i, _i, _i, ctypes.c_longlong,
                                                  ctypes.c_longlong, _i, _vp]

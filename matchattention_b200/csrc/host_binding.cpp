@@ -187,13 +187,25 @@ struct MatchAttentionFn : torch::autograd::Function<MatchAttentionFn> {
         Tensor d_out = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(q);
         Tensor d_attn = grads[1].defined() ? grads[1].contiguous() : Tensor();
         Tensor d_q = at::empty_like(q), d_mo = ctx->needs_input_grad(0) ? at::empty_like(mo) : Tensor();
+        const float scale = static_cast<float>(ctx->saved_data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(q.device());
+        void *stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+        void *dattn = d_attn.defined() ? data(d_attn) : nullptr, *dmo = d_mo.defined() ? data(d_mo) : nullptr;
+        const size_t bytes = matchattn_backward_workspace_bytes(B, H, W, h, C / h, r, dtype_code(q), 0, H);
+        if (bytes != 0) {
+            Tensor d_k = at::empty_like(k), d_v = at::empty_like(v), ws = at::empty({static_cast<int64_t>(bytes)}, q.options().dtype(at::kByte));
+            const int status = matchattn_fused_backward_ws(data(mo), data(q), data(k), data(v), data(d_out), dattn, data(d_q), data(d_k), data(d_v),
+                                                           dmo, B, H, W, h, C / h, r, r, dtype_code(q), MATCHATTN_L1_NORM, scale, 0, H, data(ws),
+                                                           bytes, stream);
+            if (status != MATCHATTN_ERR_VARIANT) {       // that one: a tensor is not 16-byte aligned
+                check_status(status);
+                return {d_mo, d_q, d_k, d_v, Tensor(), Tensor(), Tensor(), Tensor()};
+            }
+        }
         Tensor d_k = at::zeros(k.sizes(), k.options().dtype(at::kFloat)), d_v = at::zeros(v.sizes(), v.options().dtype(at::kFloat));
-        check_status(matchattn_fused_backward(data(mo), data(q), data(k), data(v), data(d_out), d_attn.defined() ? data(d_attn) : nullptr,
-                                              data(d_q), static_cast<float *>(data(d_k)), static_cast<float *>(data(d_v)),
-                                              d_mo.defined() ? data(d_mo) : nullptr, B, H, W, h, C / h, r, r, dtype_code(q), MATCHATTN_L1_NORM,
-                                              static_cast<float>(ctx->saved_data["scale"].toDouble()), 0, H,
-                                              c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
+        check_status(matchattn_fused_backward(data(mo), data(q), data(k), data(v), data(d_out), dattn, data(d_q), static_cast<float *>(data(d_k)),
+                                              static_cast<float *>(data(d_v)), dmo, B, H, W, h, C / h, r, r, dtype_code(q), MATCHATTN_L1_NORM,
+                                              scale, 0, H, stream));
         return {d_mo, d_q, d_k.to(k.scalar_type()), d_v.to(v.scalar_type()), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };

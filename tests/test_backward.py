@@ -100,3 +100,31 @@ def test_backward_kernels_match_the_restatement(h, hd, r):
     ((out * g_out.cuda()).sum() + (attn * g_attn.cuda()).sum()).backward()
     for leaf, ref, key in zip(leaves, want, ("d_max_offset", "d_q", "d_k", "d_v")):
         assert _rel(leaf.grad, ref) < 1e-4, key
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("per_head", [False, True], ids=["shared", "per-head"])
+@pytest.mark.parametrize("B,H,W,h,hd,r,kind", [(1, 4, 4, 2, 8, 1, "raw"), (1, 6, 7, 1, 40, 2, "raw"), (2, 9, 17, 2, 16, 1, "flow"),
+                                               (1, 17, 9, 2, 80, 2, "raw"), (1, 8, 16, 4, 24, 1, "self"), (1, 8, 8, 4, 128, 1, "flow"),
+                                               (1, 10, 33, 2, 16, 1, "corner")])
+def test_gathered_backward_at_the_edges_of_its_tiles(B, H, W, h, hd, r, kind, per_head):
+    """Maps of one bucket, of one tile and one token more, windows that stick out of the map on every side, and all
+    queries on the corner token; with one centre per query (one list for all heads) and with one per head."""
+    import matchattention_b200 as ma
+    from oracle import matchattn_backward
+    mo, q, k, v = make_inputs(61 + hd, B, H, W, h, hd, r, torch.float32, kind="raw" if kind == "corner" else kind, spread=3.0,
+                              border_frac=0.3, per_head=per_head)
+    if kind == "corner":
+        mo = mo * 0 - 40.0 + torch.arange(h, dtype=torch.float32).view(1, 1, h, 1) * (40.0 if per_head else 0.0)
+    if not per_head:
+        mo = mo[:, :, :1].expand_as(mo).contiguous()
+    gen = torch.Generator().manual_seed(62)
+    g_out = torch.randn(q.shape, generator=gen)
+    g_attn = torch.randn(B, H * W, h, (2 * r + 2) ** 2, generator=gen)
+    want = matchattn_backward.backward(mo, q, k, v, g_out, g_attn, H, W, r, hd ** -0.5)
+    leaves = [t.cuda().requires_grad_(True) for t in (mo, q, k, v)]
+    out, attn = ma.match_attention_autograd(*leaves, H, W, r, hd ** -0.5)
+    got = torch.autograd.grad([out, attn], leaves, [g_out.cuda(), g_attn.cuda()])
+    for g, ref, key in zip(got, want, ("d_max_offset", "d_q", "d_k", "d_v")):
+        ref = torch.as_tensor(ref).double()         # on one token the score gradients cancel: d_q and d_k are zero up to rounding
+        assert (g.double().cpu() - ref).abs().max() < 1e-4 * max(ref.abs().max().item(), 0.05), key
