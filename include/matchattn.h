@@ -345,7 +345,8 @@ MATCHATTN_API int matchattn_flow_init(const void *correlation, void *prob, void 
                                       void *cuda_stream);
 
 /* Name of the kernel variant the arguments would dispatch to ("fast cpl=2 lph=1",
- * "generic", ...) or NULL if they are rejected.  Launches nothing. */
+ * "generic", ...) or NULL if they are rejected.  The split is the coarsest one; a launch may spread a
+ * head over more lanes.  Launches nothing. */
 MATCHATTN_API const char *matchattn_describe_dispatch(int h, int hd, int r, int dtype, int pointers_32B_aligned);
 
 /*

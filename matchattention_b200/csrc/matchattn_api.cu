@@ -11,6 +11,7 @@
 #include "matchattn_mma.cuh"
 #include "matchattn_binned.cuh"
 #include "matchattn_staged.cuh"
+#include "matchattn_lanes.cuh"
 
 namespace matchattn {
 namespace {
@@ -195,6 +196,22 @@ Plan make_plan(int h, int hd, int r, int cpl_request)
     return pl;
 }
 
+// The split that the direct kernel uses for heads of a power-of-two width: 32 bytes per lane and tap, so that the lanes of
+// a query read whole lines, and up to eight lanes per head, which share the softmax (matchattn_lanes.cuh).  Measured
+// best for every such width and both radii; 16-bit heads of 16 channels and narrower, and odd widths, stay as planned.
+Plan refine_plan(Plan pl, int hd, int esize)
+{
+    const int hd8 = hd / 8;
+    if (!pl.fast || !is_pow2(hd8)) return pl;
+    int cpl = esize == 4 || hd8 == 1 ? 1 : 2;
+    while (cpl < 4 && hd8 / cpl > 8) cpl *= 2;
+    if (hd8 / cpl > pl.lph) {
+        pl.cpl = cpl;
+        pl.lph = hd8 / cpl;
+    }
+    return pl;
+}
+
 // SMs of the current device (148 when the query fails); asked once per device
 inline int sm_count()
 {
@@ -294,7 +311,11 @@ int run(Params &p, const Plan &pl, int r, int tile_w_request, cudaStream_t strea
         }
         if (blocks > 2147483647LL) return MATCHATTN_ERR_TOO_LARGE;
         const dim3 grid(static_cast<unsigned>(blocks), grid_y);
-        err = launch_fast<T>(p, r, pl.cpl, pl.lph > 1, grid, threads, stream);
+        // heads shared by lanes: the kernel that shares the softmax too, except for the options only the other one knows
+        err = cudaErrorInvalidConfiguration;
+        if (pl.lph > 1 && p.guard == nullptr && p.sorted == nullptr && p.debug == nullptr)
+            err = launch_lanes<T>(p, r, pl.cpl, grid, threads, stream);
+        if (err == cudaErrorInvalidConfiguration) err = launch_fast<T>(p, r, pl.cpl, pl.lph > 1, grid, threads, stream);
     } else {
         const long long per_item = 1LL * p.Nq * p.h;
         const long long blocks = (per_item + kThreads - 1) / kThreads;
@@ -379,6 +400,10 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
         return MATCHATTN_ERR_ALIGN;
 
     Plan pl = force_generic ? Plan{false, 0, 0, false, 2} : make_plan(h, hd, r, cpl_request);
+    if (cpl_request == 0 && variant == 0 && (strategy == kStrategyAuto || strategy == kStrategyDirect)) {
+        const Plan fine = refine_plan(pl, hd, static_cast<int>(esize));
+        if (fine.lph * h <= kThreads) pl = fine;
+    }
     if (pl.fast) {
         // vector width of a lane's slice decides the alignment the specialised kernel needs
         const int slice_bytes = pl.cpl * 8 * static_cast<int>(esize);

@@ -492,22 +492,32 @@ __device__ __forceinline__ void bilinear_softmax(const float (&s)[(2 * R + 2) * 
         float e[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) e[m] = softmax_exp(s[m] - gmax);
-        float top[SIDE], bot[SIDE];
+        // sums of the rows over the left and the right SUB columns, then over the rows, in halves: the order in which
+        // lanes that share a head add them (matchattn_lanes.cuh), so that the number of lanes does not show in the result
+        constexpr int HALF = SIDE / 2;
+        float den[4];
 #pragma unroll
-        for (int i = 0; i < SIDE; ++i) {
-            float mid = e[SIDE + i];
+        for (int ox = 0; ox < 2; ++ox) {
+            float upper[2], lower[2];
 #pragma unroll
-            for (int j = 2; j < SUB; ++j) mid += e[j * SIDE + i];
-            top[i] = e[i] + mid;
-            bot[i] = mid + e[(SIDE - 1) * SIDE + i];
+            for (int hf = 0; hf < 2; ++hf) {
+                float up = 0.f, low = 0.f;
+#pragma unroll
+                for (int k = 0; k < HALF; ++k) {
+                    const int j = hf * HALF + k;
+                    float m = e[j * SIDE + 1];
+#pragma unroll
+                    for (int i = 2; i < SUB; ++i) m += e[j * SIDE + i];
+                    const float line = ox == 0 ? e[j * SIDE] + m : m + e[j * SIDE + SIDE - 1];
+                    if (j < SIDE - 1) up = k == 0 ? line : up + line;
+                    if (j > 0) low = (k == 0 || j == 1) ? line : low + line;
+                }
+                upper[hf] = up;
+                lower[hf] = low;
+            }
+            den[ox] = upper[0] + upper[1];
+            den[2 + ox] = lower[0] + lower[1];
         }
-        float mt = top[1], mb = bot[1];
-#pragma unroll
-        for (int i = 2; i < SUB; ++i) {
-            mt += top[i];
-            mb += bot[i];
-        }
-        const float den[4] = {top[0] + mt, mt + top[SIDE - 1], bot[0] + mb, mb + bot[SIDE - 1]};
 #pragma unroll
         for (int t = 0; t < 4; ++t)
             blend_subwindow<T, R>(aw, t, w[t], softmax_rcp(den[t]), [&](int m) { return e[m]; });

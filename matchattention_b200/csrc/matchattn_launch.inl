@@ -1,6 +1,7 @@
 // Included once per element type with MATCHATTN_T defined: instantiates the
 // specialised kernels for that type and the switch that picks one.
 #include "matchattn_kernels.cuh"
+#include "matchattn_lanes.cuh"
 #ifdef MATCHATTN_T_IS_16BIT
 #include "matchattn_mma.cuh"
 #include "matchattn_binned.cuh"
@@ -31,6 +32,28 @@ static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid
     MA_CASE(5, false) MA_CASE(5, true)
 #undef MA_CASE
     return cudaErrorInvalidValue;
+}
+
+template <typename T, int R>
+static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream)
+{
+#define MA_LANES(CPL_, L_)                                                                 \
+    if (cpl == CPL_ && p.lph == L_) {                                                      \
+        lanes_forward_kernel<T, R, CPL_, L_><<<grid, threads, 0, stream>>>(p);             \
+        return cudaGetLastError();                                                         \
+    }
+    MA_LANES(1, 2) MA_LANES(1, 4) MA_LANES(1, 8)
+    MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8)
+    MA_LANES(4, 4) MA_LANES(4, 8)
+    MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
+#undef MA_LANES
+    return cudaErrorInvalidConfiguration;
+}
+
+template <>
+cudaError_t launch_lanes<MATCHATTN_T>(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream)
+{
+    return r == 1 ? launch_lanes_r<MATCHATTN_T, 1>(p, cpl, grid, threads, stream) : launch_lanes_r<MATCHATTN_T, 2>(p, cpl, grid, threads, stream);
 }
 
 template <>

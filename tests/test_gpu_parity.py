@@ -190,3 +190,29 @@ def test_nan_and_huge_centres_do_not_fault():
     finite = torch.isfinite(ref_out)
     assert torch.equal(torch.isfinite(out), finite)
     assert (out[finite] - ref_out[finite]).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("r", [1, 2])
+@pytest.mark.parametrize("h,hd", [(1, 32), (3, 16), (4, 64), (2, 128), (1, 256), (3, 48), (2, 80)])
+def test_heads_shared_by_lanes(h, hd, r, dtype):
+    """Heads that two, four or eight lanes share, head counts that leave lanes without a query, and both evaluations of
+    the softmax: scores close together and (scale 6) spread so widely that sub-windows need maxima of their own."""
+    H, W = 2 * r + 3, 11
+    for scale in (hd ** -0.5, 6.0):
+        inputs = make_inputs(400 + hd + r, 2, H, W, h, hd, r, dtype, kind="raw", per_head=True)
+        out, attn = run_kernel(inputs, H, W, r, scale)
+        ref_out, ref_attn = _oracle().forward(*inputs, H, W, r, scale)
+        if scale == 6.0:
+            # scores in the hundreds: in 16 bits they are a quarter apart or more, in float32 3e-5, and one that rounds the
+            # other way moves the weights
+            off = (attn.float() - ref_attn.float()).abs()
+            assert (off > (2e-3 if dtype == torch.float32 else 4e-2)).float().mean() < 1e-3
+        else:
+            assert_close(attn, ref_attn, dtype, "attn")
+            assert_close(out, ref_out, dtype, "out")
+    mo, q, k, v = inputs
+    mo[0, 3, 0, 0] = float("nan")
+    out, attn = run_kernel((mo, q, k, v), H, W, r, hd ** -0.5)
+    ref_out, ref_attn = _oracle().forward(mo, q, k, v, H, W, r, hd ** -0.5)
+    assert torch.equal(torch.isnan(attn), torch.isnan(ref_attn)) and torch.equal(torch.isnan(out), torch.isnan(ref_out))
