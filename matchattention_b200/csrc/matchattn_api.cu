@@ -196,18 +196,25 @@ Plan make_plan(int h, int hd, int r, int cpl_request)
     return pl;
 }
 
-// The split that the direct kernel uses for heads of a power-of-two width: 32 bytes per lane and tap, so that the lanes of
-// a query read whole lines, and up to eight lanes per head, which share the softmax (matchattn_lanes.cuh).  Measured
-// best for every such width and both radii; 16-bit heads of 16 channels and narrower, and odd widths, stay as planned.
-Plan refine_plan(Plan pl, int hd, int esize)
+// The split that the direct kernel uses: 32 bytes per lane and tap, so that the lanes of a query read whole lines, and up to
+// eight lanes per head, which share the softmax (matchattn_lanes.cuh).  Measured best for every power-of-two width and
+// both radii; 16-bit heads of 16 channels and narrower stay with one lane.  `rows32`: every row of the arrays starts
+// 32-byte aligned; then 16-bit heads of 40 channels go to two lanes (one lane's 80-byte slice takes five loads that
+// touch a line per lane each).
+Plan refine_plan(Plan pl, int hd, int esize, bool rows32)
 {
     const int hd8 = hd / 8;
-    if (!pl.fast || !is_pow2(hd8)) return pl;
-    int cpl = esize == 4 || hd8 == 1 ? 1 : 2;
-    while (cpl < 4 && hd8 / cpl > 8) cpl *= 2;
-    if (hd8 / cpl > pl.lph) {
-        pl.cpl = cpl;
-        pl.lph = hd8 / cpl;
+    if (!pl.fast) return pl;
+    if (is_pow2(hd8)) {
+        int cpl = esize == 4 || hd8 == 1 ? 1 : 2;
+        while (cpl < 4 && hd8 / cpl > 8) cpl *= 2;
+        if (hd8 / cpl > pl.lph) {
+            pl.cpl = cpl;
+            pl.lph = hd8 / cpl;
+        }
+    } else if (esize == 2 && hd8 == 5 && rows32) {
+        pl.cpl = 3;
+        pl.lph = 2;
     }
     return pl;
 }
@@ -400,8 +407,11 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
         return MATCHATTN_ERR_ALIGN;
 
     Plan pl = force_generic ? Plan{false, 0, 0, false, 2} : make_plan(h, hd, r, cpl_request);
+    // (the checked entry runs on the kernel whose slices are contiguous)
+    const bool rows32 = glue.debug == nullptr && aligned(q, 32) && aligned(k, 32) && aligned(v, 32) && aligned(out, 32) &&
+                        aligned(glue.gate, 32) && C * esize % 32 == 0 && out_stride * esize % 32 == 0;
     if (cpl_request == 0 && variant == 0 && (strategy == kStrategyAuto || strategy == kStrategyDirect)) {
-        const Plan fine = refine_plan(pl, hd, static_cast<int>(esize));
+        const Plan fine = refine_plan(pl, hd, static_cast<int>(esize), rows32);
         if (fine.lph * h <= kThreads) pl = fine;
     }
     if (pl.fast) {

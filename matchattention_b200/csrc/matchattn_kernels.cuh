@@ -548,11 +548,14 @@ constexpr int min_blocks()
     return (DT<T>::kHalfPipe && CPL <= 2) ? 3 : 2;
 }
 
-// EXTRAS selects the build of the kernel that also honours the rarely used Params fields (sorted
-// query order, guard, clamp, gate, strided outputs); the plain build ignores them and keeps the
-// hot path free of their branches and registers.
+// OPTIONS selects the build: kNoOptions ignores the Params fields of the caller's glue (clamp, gate, strided outputs,
+// view swap) and keeps the hot path free of their branches and registers, kGlueOptions honours them, kAllOptions the
+// rare ones too (sorted query order, guard, index checks).  MULTI (several lanes per head, each with the whole softmax)
+// is left for those rare options and for more than eight lanes; see matchattn_lanes.cuh for the rest.
 // POW2: the host found `scale` to be a power of two that the 16-bit type T represents exactly.
-template <typename T, int R, int CPL, bool MULTI, bool EXTRAS, bool POW2 = false>
+constexpr int kNoOptions = 0, kGlueOptions = 1, kAllOptions = 2;
+
+template <typename T, int R, int CPL, bool MULTI, int OPTIONS, bool POW2 = false>
 __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forward_kernel(const Params p)
 {
     constexpr int SIDE = 2 * R + 2, M = SIDE * SIDE;
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forwa
     constexpr int EPW = DT<T>::kElemsPerWord;
     constexpr int SLICE = CPL * 8;                          // channels per lane
 
-    if constexpr (EXTRAS) {
+    if constexpr (OPTIONS == kAllOptions) {
         if (p.guard != nullptr && ((*p.guard != 0u) != (p.guard_run_if != 0))) return;
     }
 
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forwa
     bool valid;
     int b;
     int64_t bq;
-    if (EXTRAS && p.sorted != nullptr) {
+    if (OPTIONS == kAllOptions && p.sorted != nullptr) {
         // queries in the order of the sorted list: neighbours in the list look at the same tile of
         // the map, so their taps hit in L1
         const int qpb = p.tile_w * p.tile_h;
@@ -611,7 +614,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forwa
     // sampling centre -> origin, weights, clamped tap rows / columns (in elements)
     float x, y;
     DT<T>::load_xy(static_cast<const T *>(p.mo) + (bq * p.h + head) * 2, x, y);
-    if (EXTRAS && p.clamp) {
+    if (OPTIONS != kNoOptions && p.clamp) {
         x = clamp_keep_nan(x, p.clamp_lo, p.clamp_hi_x);
         y = clamp_keep_nan(y, p.clamp_lo, p.clamp_hi_y);
     }
@@ -630,12 +633,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forwa
 
     const int lane_off = head * p.hd + sl * SLICE;
     // the cross branch reads the other view's keys / values: the caller's batch roll folded into the index
-    const int b_kv = (EXTRAS && p.kv_shift != 0) ? (b + p.kv_shift >= p.B ? b + p.kv_shift - p.B : b + p.kv_shift) : b;
+    const int b_kv = (OPTIONS != kNoOptions && p.kv_shift != 0) ? (b + p.kv_shift >= p.B ? b + p.kv_shift - p.B : b + p.kv_shift) : b;
     const int64_t kv_base = static_cast<int64_t>(b_kv) * p.N * p.C + lane_off;
     const T *kb = static_cast<const T *>(p.k) + kv_base;
     const T *vb = static_cast<const T *>(p.v) + kv_base;
 
-    if (EXTRAS && p.debug != nullptr) {
+    if (OPTIONS == kAllOptions && p.debug != nullptr) {
         // checked entry point: every index this lane is about to use, against the extent of its array
         const int64_t item_elems = static_cast<int64_t>(p.N) * p.C;
 #pragma unroll
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forwa
     bilinear_softmax<T, R>(s, wgt, aw);
 
     if (p.attn != nullptr && sl == 0 && valid)
-        store_words<NWA>(static_cast<T *>(p.attn) + (EXTRAS ? bq * p.attn_stride + head * M : (bq * p.h + head) * M), aw);
+        store_words<NWA>(static_cast<T *>(p.attn) + (OPTIONS != kNoOptions ? bq * p.attn_stride + head * M : (bq * p.h + head) * M), aw);
 
     // weighted sum of the value taps
     float o[NW * EPW];
@@ -745,13 +748,13 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, R, CPL>()) fused_forwa
         uint32_t ow[NW];
 #pragma unroll
         for (int w = 0; w < NW; ++w) ow[w] = DT<T>::pack(&o[w * EPW]);
-        if (EXTRAS && p.gate != nullptr) {
+        if (OPTIONS != kNoOptions && p.gate != nullptr) {
             uint32_t gw[NW];
             load_words<NW>(gw, static_cast<const T *>(p.gate) + bq * p.C + lane_off);
 #pragma unroll
             for (int w = 0; w < NW; ++w) ow[w] = DT<T>::gate_mul(ow[w], gw[w]);
         }
-        store_words<NW>(static_cast<T *>(p.out) + bq * (EXTRAS ? p.out_stride : p.C) + lane_off, ow);
+        store_words<NW>(static_cast<T *>(p.out) + bq * (OPTIONS != kNoOptions ? p.out_stride : p.C) + lane_off, ow);
     }
 }
 

@@ -6,8 +6,14 @@
 // per window where a full exchange takes 32), every lane evaluates its rows, and the finished weights, two to a word in
 // the 16-bit types, are gathered for the sum over the value taps.
 //
-// A lane's chunks lie in 32-byte pieces (16-byte ones for odd chunk counts in the 16-bit types), piece i of lane s
-// at piece i * lanes + s of the head: the lanes of a query read whole lines of a token.
+// A lane's chunks lie in 32-byte pieces, piece i of lane s at piece i * lanes + s of the head: the lanes of a query read
+// whole lines of a token.  Odd chunk counts in the 16-bit types take 16-byte pieces (hd = 80 on two lanes: 58 us where
+// 32-byte pieces and a last one of 16 took 71: their eight neighbouring registers leave the compiler less room).
+//
+// RAGGED (16-bit types, hd = 40): a 32-byte piece per lane and a 16-byte one for lane 0; lane 1 reads that along and
+// leaves it out.  Every other head starts half way into a 32-byte piece and has its 16-byte piece in front.
+// Measured, float16, r = 2, 4 heads: 2 x 48x48 tokens 13.4 -> 11.4 us, 2 x 160x160 125 -> 112 (one lane per head:
+// five loads per tap that touch a line per lane each, L1 71 % busy, issue 29 %).
 //
 // Bound by instruction issue and the L1 path.  Measured on a B200 against one lane's full softmax in every lane and
 // 64-byte slices: float16, 2 x 272x480 tokens, 4 heads x 64, r = 1: 320 -> 225 us; 2 x 68x120, 4 x 128, r = 2:
@@ -101,13 +107,14 @@ __device__ __forceinline__ void store_run(void *p, const uint32_t *w)
 template <typename T, int R, int CPL>
 constexpr int lanes_min_blocks() { return R == 1 && CPL * DT<T>::kWordsPerChunk <= 8 ? 3 : 2; }
 
-template <typename T, int R, int CPL, int L>
+template <typename T, int R, int CPL, int L, bool RAGGED>
 __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes_forward_kernel(const Params p)
 {
     using Share = RowShare<R, L>;
     constexpr int SIDE = Share::SIDE, SUB = 2 * R + 1, ROWS = Share::ROWS;
     constexpr int NW = CPL * DT<T>::kWordsPerChunk, EPW = DT<T>::kElemsPerWord;
-    constexpr int PW = NW % 8 == 0 ? 8 : 4, PIECES = NW / PW;      // 32-bit words per piece, pieces per lane and tap
+    constexpr int PW = RAGGED || NW % 8 == 0 ? 8 : 4, PIECES = RAGGED ? 1 : NW / PW;   // 32-bit words of a piece, pieces per lane and tap
+    static_assert(!RAGGED || (NW == 12 && L == 2), "");
     constexpr int WPR = SIDE / EPW;                                // words of a row of weights
     constexpr unsigned kAll = 0xffffffffu;
 
@@ -140,8 +147,11 @@ __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes
         row[i] = min(max(y0 + i, 0), p.H - 1) * p.W * p.C;
     }
 
-    const int lane_off = head * p.hd + sl * (PW * EPW);
-    constexpr int kStep = L * PW * EPW;                            // elements between a lane's pieces
+    constexpr int kPiece = PW * EPW, kStep = L * kPiece;           // elements of a piece; from one of a lane's pieces to the next
+    const int shift = RAGGED && (head & 1) ? kPiece / 2 : 0;
+    const int lane_off = head * p.hd + sl * kPiece + shift;
+    const int tail = (shift ? -shift : kStep) - sl * kPiece;       // a ragged head's 16-byte piece, from lane_off
+    const bool full = !RAGGED || sl == 0;
     const int b_kv = b + p.kv_shift >= p.B ? b + p.kv_shift - p.B : b + p.kv_shift;
     const int64_t kv_base = static_cast<int64_t>(b_kv) * p.N * p.C + lane_off;
     const T *kb = static_cast<const T *>(p.k) + kv_base;
@@ -152,6 +162,7 @@ __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes
             if constexpr (PW == 8) ld_nc_256(&w[8 * i], at + i * kStep);
             else ld_nc_128(&w[4 * i], at + i * kStep);
         }
+        if constexpr (RAGGED) ld_nc_128(&w[8], at + tail);
     };
 
     uint32_t qw[NW];
@@ -166,7 +177,7 @@ __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes
         for (int j = 0; j < SIDE; ++j) {
             uint32_t kw[NW];
             load_slice(kw, tap_ptr(kb + row[j], col[i]));
-            float a0 = 0.f, a1 = 0.f;
+            float a0 = 0.f, a1 = 0.f, t0 = 0.f, t1 = 0.f;          // t: the last piece of a ragged head
             if constexpr (EPW == 1) {
 #pragma unroll
                 for (int w = 0; w < NW; w += 2) {
@@ -178,9 +189,13 @@ __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes
                 }
             } else {
 #pragma unroll
-                for (int w = 0; w < NW; ++w) DT<T>::absdiff(a0, a1, qw[w], kw[w]);
+                for (int w = 0; w < NW; ++w) {
+                    if (RAGGED && w >= 8) DT<T>::absdiff(t0, t1, qw[w], kw[w]);
+                    else DT<T>::absdiff(a0, a1, qw[w], kw[w]);
+                }
             }
             part[j] = a0 + a1;
+            if constexpr (RAGGED) part[j] += full ? t0 + t1 : 0.f;
         }
         Share::reduce(part, sum, sl);
 #pragma unroll
@@ -352,6 +367,7 @@ __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes
             if constexpr (PW == 8) st_256(out + i * kStep, &ow[8 * i]);
             else st_128(out + i * kStep, &ow[4 * i]);
         }
+        if (RAGGED && full) st_128(out + tail, &ow[NW - 4]);
     }
 }
 

@@ -13,17 +13,20 @@ namespace matchattn {
 template <typename T, int R>
 static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid, int threads, cudaStream_t stream)
 {
-    const bool extras = p.guard != nullptr || p.sorted != nullptr || p.gate != nullptr || p.clamp != 0 || p.debug != nullptr || p.kv_shift != 0 ||
-                        p.out_stride != p.C || p.attn_stride != p.h * (2 * R + 2) * (2 * R + 2);
-    // power-of-two scale: a build of the plain kernel that finishes two scores per packed instruction
+    const bool glue = p.gate != nullptr || p.clamp != 0 || p.kv_shift != 0 || p.out_stride != p.C ||
+                      p.attn_stride != p.h * (2 * R + 2) * (2 * R + 2);
+    const bool rare = multi || p.guard != nullptr || p.sorted != nullptr || p.debug != nullptr;
+    // power-of-two scale: builds that finish two scores per packed instruction
     constexpr bool kCanPack = sizeof(T) == 2;
-    const bool pow2 = kCanPack && p.scale_pow2 != 0 && !extras;
-#define MA_CASE(CPL_, MULTI_)                                                              \
-    if (cpl == CPL_ && multi == MULTI_) {                                                  \
-        if (extras) fused_forward_kernel<T, R, CPL_, MULTI_, true><<<grid, threads, 0, stream>>>(p);   \
-        else if (pow2) fused_forward_kernel<T, R, CPL_, MULTI_, false, kCanPack><<<grid, threads, 0, stream>>>(p);  \
-        else fused_forward_kernel<T, R, CPL_, MULTI_, false><<<grid, threads, 0, stream>>>(p);         \
-        return cudaGetLastError();                                                         \
+    const bool pow2 = kCanPack && p.scale_pow2 != 0;
+#define MA_CASE(CPL_, MULTI_)                                                                                           \
+    if (cpl == CPL_ && multi == MULTI_) {                                                                               \
+        if (MULTI_ || rare) fused_forward_kernel<T, R, CPL_, MULTI_, kAllOptions><<<grid, threads, 0, stream>>>(p);     \
+        else if (glue && pow2) fused_forward_kernel<T, R, CPL_, false, kGlueOptions, kCanPack><<<grid, threads, 0, stream>>>(p);  \
+        else if (glue) fused_forward_kernel<T, R, CPL_, false, kGlueOptions><<<grid, threads, 0, stream>>>(p);          \
+        else if (pow2) fused_forward_kernel<T, R, CPL_, false, kNoOptions, kCanPack><<<grid, threads, 0, stream>>>(p);  \
+        else fused_forward_kernel<T, R, CPL_, false, kNoOptions><<<grid, threads, 0, stream>>>(p);                      \
+        return cudaGetLastError();                                                                                      \
     }
     MA_CASE(1, false) MA_CASE(1, true)
     MA_CASE(2, false) MA_CASE(2, true)
@@ -37,15 +40,22 @@ static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid
 template <typename T, int R>
 static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream)
 {
+    const int width = p.hd / 8;      // chunks of a head
 #define MA_LANES(CPL_, L_)                                                                 \
-    if (cpl == CPL_ && p.lph == L_) {                                                      \
-        lanes_forward_kernel<T, R, CPL_, L_><<<grid, threads, 0, stream>>>(p);             \
+    if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) {                                \
+        lanes_forward_kernel<T, R, CPL_, L_, false><<<grid, threads, 0, stream>>>(p);      \
         return cudaGetLastError();                                                         \
     }
     MA_LANES(1, 2) MA_LANES(1, 4) MA_LANES(1, 8)
     MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8)
     MA_LANES(4, 4) MA_LANES(4, 8)
     MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
+    if constexpr (sizeof(T) == 2) {
+        if (cpl == 3 && p.lph == 2 && width == 5) {
+            lanes_forward_kernel<T, R, 3, 2, true><<<grid, threads, 0, stream>>>(p);
+            return cudaGetLastError();
+        }
+    }
 #undef MA_LANES
     return cudaErrorInvalidConfiguration;
 }
