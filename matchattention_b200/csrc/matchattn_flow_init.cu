@@ -18,8 +18,8 @@
 // prob and the deciding averages are formed in one fixed order (sums of exponentials in 256 interleaved partial sums
 // per row and four per column, box sums row by row) whatever the split of the work, and only the screening in step 3
 // adds in another.
-// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.22 ms = 0.09 + 0.34 +
-// 0.72 + 0.08; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
+// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.06 ms = 0.09 + 0.26 +
+// 0.63 + 0.08; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
 // the pooling took 4.1.  48x48 tokens: 56 us, before 189.
 // Rounding of the 16-bit types as eager PyTorch on the GPU: softmax, pooling and sums accumulate in float32
 // and round once, every elementwise op rounds.
@@ -40,9 +40,9 @@ constexpr int kLaneCols = 4;                          // consecutive columns of 
 constexpr int kWarpCols = 32 * kLaneCols;
 constexpr int kMaxRows = 16;                          // rows of corr that a lane holds at a time in the maximum pass
 constexpr int kPoolCols = kWarpCols - 2 * kLaneCols;  // columns a warp pools: its outer lanes are the halo
-constexpr int kPoolStep = 8;                          // rows per unrolled step of the pooling kernel (two halves of four)
-constexpr int kTransBytes = 64, kTransPitch = kTransBytes + 16;   // run of a prob row that a transposed store writes; its slot in shared memory
-constexpr int kPoolSmemPerWarp = kWarpCols * kTransPitch;
+constexpr int kPoolStep = 4;                          // rows per step of the pooling kernel, the next four on their way
+constexpr int kTransBytes = 64;                       // run of a prob row that a transposed store writes
+constexpr int kPoolSmemPerWarp = kWarpCols * (kTransBytes + 16);
 constexpr int kPoolWarps = 4;                         // warps per block of the pooling kernel
 constexpr int kSumGroups = 4;                         // interleaved partial sums per column
 constexpr int kWindowTokens = kFlowWarps;             // tokens per block of the window kernel: one per warp
@@ -441,25 +441,20 @@ __device__ __forceinline__ void pool_rows(const PoolParams &pp, const T *src, T 
         const float4 v = st[a - (a0 - 2)];
         return Softmax{v.x, v.y, v.z};
     };
-    Group<T> now[kPoolStep / 2], next[kPoolStep / 2];     // corr is read four rows ahead
+    Group<T> now[kPoolStep], next[kPoolStep];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) next[i] = load(a0 - 2 + i);
+    for (int i = 0; i < kPoolStep; ++i) now[i] = load(a0 - 2 + i);
+    const int64_t end = a0 + pp.band_rows;
+#pragma unroll 1
+    for (int64_t a = a0 - 2; a < end + 2; a += kPoolStep) {
 #pragma unroll
-    for (int i = 0; i < kPoolStep / 2; ++i) now[i] = load(a0 + i);
+        for (int i = 0; i < kPoolStep; ++i) next[i] = load(a + kPoolStep + i);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) row_step(next[i], stat(a0 - 2 + i), a0 - 2 + i, false, false);
-    for (int64_t a = a0; a < a0 + pp.band_rows; a += kPoolStep) {
-#pragma unroll
-        for (int i = 0; i < kPoolStep / 2; ++i) next[i] = load(a + kPoolStep / 2 + i);
-#pragma unroll
-        for (int i = 0; i < kPoolStep / 2; ++i) row_step(now[i], stat(a + i), a + i, true, i >= 2 || a > a0);
-#pragma unroll
-        for (int i = 0; i < kPoolStep / 2; ++i) now[i] = load(a + kPoolStep + i);
-#pragma unroll
-        for (int i = 0; i < kPoolStep / 2; ++i) row_step(next[i], stat(a + kPoolStep / 2 + i), a + kPoolStep / 2 + i, true, true);
+        for (int i = 0; i < kPoolStep; ++i) {
+            row_step(now[i], stat(a + i), a + i, i < 2 ? a >= a0 : a + i < end, i < 2 ? a > a0 : a >= a0);
+            now[i] = next[i];
+        }
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) row_step(now[i], stat(a0 + pp.band_rows + i), a0 + pp.band_rows + i, false, true);
     __syncwarp();
     for (int i = lane; i < pp.band_rows; i += 32)
         if (FULL || a0 + i < N) pp.row_max[(b * pp.chunks + chunk) * N + a0 + i] = row_max[i];
@@ -470,8 +465,9 @@ template <typename T, bool VEC, bool FULL>
 __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T *dst, char *smem, int64_t b, int64_t a0, int64_t c0,
                                           int chunk, int band, int lane)
 {
-    constexpr int kPerStore = 16 / sizeof(T);               // rows of a column in 16 bytes
     constexpr int kTransRows = kTransBytes / sizeof(T);     // rows gathered before a transposed store
+    // a column's slot in shared memory: the pitch keeps the stores of four rows (8 or 16 bytes) free of bank conflicts
+    constexpr int kPitch = kTransBytes + (sizeof(T) == 2 ? 8 : 16);
     const int64_t N = pp.N;
     const bool inner = lane != 0 && lane != 31;
     PairSums lo, hi;
@@ -519,71 +515,64 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
         return load_group<T, VEC, FULL>(src + (FULL ? min(a, N - 1) : a) * N, c0, N, a >= 0 && a < N);
     };
     uint32_t w[kLaneCols][2];
-    Group<T> now[kPoolStep / 2], next[kPoolStep / 2];     // corr is read four rows ahead
-    next[0] = load(a0 - 2);
-    next[1] = load(a0 - 1);
+    Group<T> now[kPoolStep], next[kPoolStep];
 #pragma unroll
-    for (int i = 0; i < kPoolStep / 2; ++i) now[i] = load(a0 + i);
-    two_rows(next[0], next[1], a0 - 2, false, w);
-    for (int64_t a = a0; a < a0 + pp.band_rows; a += kPoolStep) {
+    for (int i = 0; i < kPoolStep; ++i) now[i] = load(a0 - 2 + i);
+    uint32_t pend[kLaneCols][2];          // rows a - 2 and a - 1
+#pragma unroll 1
+    for (int64_t a = a0 - 2; a < a0 + pp.band_rows + 2; a += kPoolStep) {
 #pragma unroll
-        for (int i = 0; i < kPoolStep / 2; ++i) next[i] = load(a + kPoolStep / 2 + i);
-        uint32_t pend[kLaneCols][4];      // 16 bytes of rows of every column
-#pragma unroll
-        for (int i = 0; i < kPoolStep; i += 2) {
-            // the first two box sums of a band belong to the rows above it
-            if (i < kPoolStep / 2) {
-                two_rows(now[i % 4], now[i % 4 + 1], a + i, i > 0 || a > a0, w);
-            } else {
-                if (i == kPoolStep / 2) {
-#pragma unroll
-                    for (int j = 0; j < kPoolStep / 2; ++j) now[j] = load(a + kPoolStep + j);
-                }
-                two_rows(next[i % 4], next[i % 4 + 1], a + i, true, w);
-            }
+        for (int i = 0; i < kPoolStep; ++i) next[i] = load(a + kPoolStep + i);
+        two_rows(now[0], now[1], a, a > a0, w);
+        if (a > a0 - 2) {
+            const int at = static_cast<int>(a - 2 - a0) & (kTransRows - 1);
+            // column k of lane l in slot k * 32 + l
 #pragma unroll
             for (int k = 0; k < kLaneCols; ++k) {
-                if constexpr (sizeof(T) == 2) {
-                    pend[k][i / 2] = w[k][0];
-                } else {
-                    pend[k][i & 3] = w[k][0];
-                    pend[k][(i & 3) + 1] = w[k][1];
-                }
+                char *slot = smem + (k * 32 + lane) * kPitch + at * sizeof(T);
+                if constexpr (sizeof(T) == 2) *reinterpret_cast<uint2 *>(slot) = make_uint2(pend[k][0], w[k][0]);
+                else *reinterpret_cast<uint4 *>(slot) = make_uint4(pend[k][0], pend[k][1], w[k][0], w[k][1]);
             }
-            if ((i + 2) % kPerStore == 0) {
-                // column k of lane l in slot k * 32 + l: eight lanes' 16-byte pieces fall into different banks
-                const int at = static_cast<int>(a + i + 2 - kPerStore - a0) & (kTransRows - 1);
+            if (at == kTransRows - kPoolStep) {
+                __syncwarp();
+                const int64_t row0 = a + 2 - kTransRows, token0 = static_cast<int64_t>(chunk) * kPoolCols - kLaneCols;
+                if constexpr (VEC) {      // four lanes per column, eight columns per store
+                    const int64_t row = row0 + (lane & 3) * (16 / sizeof(T));
+#pragma unroll 4
+                    for (int u = 0; u < kWarpCols; u += 8) {
+                        const int l = (u + (lane >> 2)) & 31, k = u >> 5;
+                        const int64_t token = token0 + l * kLaneCols + k;
+                        const char *slot = smem + (k * 32 + l) * kPitch + (lane & 3) * 16;
+                        uint4 v;
+                        if constexpr (sizeof(T) == 2) {
+                            const uint2 v0 = *reinterpret_cast<const uint2 *>(slot), v1 = *reinterpret_cast<const uint2 *>(slot + 8);
+                            v = make_uint4(v0.x, v0.y, v1.x, v1.y);
+                        } else {
+                            v = *reinterpret_cast<const uint4 *>(slot);
+                        }
+                        if (l != 0 && l != 31 && (FULL || (token < N && row < N))) *reinterpret_cast<uint4 *>(dst + token * N + row) = v;
+                    }
+                } else {                  // 2-byte types: one column per store, float32: two
+                    const int r = lane & (kTransRows - 1);
+#pragma unroll 4
+                    for (int c = kLaneCols + lane / kTransRows; c < kWarpCols - kLaneCols; c += 32 / kTransRows) {
+                        const int64_t token = token0 + c;
+                        const T v = *reinterpret_cast<const T *>(smem + ((c & 3) * 32 + (c >> 2)) * kPitch + r * sizeof(T));
+                        if (FULL || (token < N && row0 + r < N)) dst[token * N + row0 + r] = v;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        two_rows(now[2], now[3], a + 2, a >= a0, w);
 #pragma unroll
-                for (int k = 0; k < kLaneCols; ++k)
-                    *reinterpret_cast<uint4 *>(smem + (k * 32 + lane) * kTransPitch + at * sizeof(T)) =
-                        make_uint4(pend[k][0], pend[k][1], pend[k][2], pend[k][3]);
-            }
+        for (int k = 0; k < kLaneCols; ++k) {
+            pend[k][0] = w[k][0];
+            pend[k][1] = w[k][1];
         }
-        if ((static_cast<int>(a + kPoolStep - a0) & (kTransRows - 1)) == 0) {
-            __syncwarp();
-            const int64_t row0 = a + kPoolStep - kTransRows, token0 = static_cast<int64_t>(chunk) * kPoolCols - kLaneCols;
-            if constexpr (VEC) {      // four lanes per column, eight columns per store
-                const int64_t row = row0 + (lane & 3) * kPerStore;
-#pragma unroll 4
-                for (int u = 0; u < kWarpCols; u += 8) {
-                    const int l = (u + (lane >> 2)) & 31, k = u >> 5;
-                    const int64_t token = token0 + l * kLaneCols + k;
-                    const uint4 v = *reinterpret_cast<const uint4 *>(smem + (k * 32 + l) * kTransPitch + (lane & 3) * 16);
-                    if (l != 0 && l != 31 && (FULL || (token < N && row < N))) *reinterpret_cast<uint4 *>(dst + token * N + row) = v;
-                }
-            } else {                  // 2-byte types: one column per store, float32: two
-                const int r = lane & (kTransRows - 1);
-#pragma unroll 4
-                for (int c = kLaneCols + lane / kTransRows; c < kWarpCols - kLaneCols; c += 32 / kTransRows) {
-                    const int64_t token = token0 + c;
-                    const T v = *reinterpret_cast<const T *>(smem + ((c & 3) * 32 + (c >> 2)) * kTransPitch + r * sizeof(T));
-                    if (FULL || (token < N && row0 + r < N)) dst[token * N + row0 + r] = v;
-                }
-            }
-            __syncwarp();
-        }
+#pragma unroll
+        for (int i = 0; i < kPoolStep; ++i) now[i] = next[i];
     }
-    two_rows(now[0], now[1], a0 + pp.band_rows, true, w);
     if (inner) {
 #pragma unroll
         for (int k = 0; k < kLaneCols; ++k)
@@ -598,10 +587,11 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
 // them as 16 bytes of a prob row, or, where rows of prob are not 16-byte aligned, through shared memory.
 // Eight consecutive blocks (four of either role) cover one 4-band x 4-chunk region, so the second role finds corr in L2.
 // Bound by instruction issue (about 25 per element and role, a third of them the exponential; 60 % of the slots busy).
-// Measured, float16, 16384 x 16384: 0.72 ms.  With 16-byte stores straight from the registers to 32 rows of prob the
+// Measured, float16, 16384 x 16384: 0.63 ms (0.72 with eight rows unrolled and the halo rows apart: the instruction cache
+// ran short, 2.2 of 8 stalls).  With 16-byte stores straight from the registers to 32 rows of prob the
 // second role alone took 0.67 ms; five blocks of four warps hold 20 warps per SM (0.75 ms with four blocks).
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(32 * kPoolWarps, 5) flow_prob_pool_kernel(const T *__restrict__ corr, T *__restrict__ prob, const PoolParams pp)
+__global__ void __launch_bounds__(32 * kPoolWarps, sizeof(T) == 2 ? 5 : 4) flow_prob_pool_kernel(const T *__restrict__ corr, T *__restrict__ prob, const PoolParams pp)
 {
     extern __shared__ __align__(16) char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -760,8 +750,10 @@ cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow
             <<<dim3(static_cast<unsigned>(col_blocks + (N + kRows - 1) / kRows), B), kThreadsHere, 0, stream>>>(
                 corr, row_part, col_part, stats, N, pl.row_parts, pl.col_parts, col_blocks);
     };
-    // up to about 5000 tokens 64-column blocks would leave SMs without work
-    if (N >= 5000) launch_sums(std::integral_constant<int, 64>(), std::integral_constant<int, 16>());
+    // Narrow blocks up to about 5000 tokens, where 32-column ones would leave SMs without work.  Above, 32 columns and 16
+    // (float32: 24) rows in flight measured best: 128x128 tokens float16 262 us, 337 with 64-column blocks, of which some
+    // SMs get two and some one; 88x88 float32 80 us, 102.
+    if (N >= 5000) launch_sums(std::integral_constant<int, 32>(), std::integral_constant<int, sizeof(T) == 2 ? 16 : 24>());
     else launch_sums(std::integral_constant<int, 16>(), std::integral_constant<int, 32>());
     constexpr int smem = kPoolWarps * kPoolSmemPerWarp;
     const cudaError_t e = cudaFuncSetAttribute(flow_prob_pool_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
