@@ -95,12 +95,136 @@ template <>
 __device__ __forceinline__ __nv_bfloat162 word_as_pair<__nv_bfloat16>(uint32_t w) { return *reinterpret_cast<const __nv_bfloat162 *>(&w); }
 
 
-// Vector path for the shapes the model uses (F*D <= 8, W a multiple of VW = 4): one thread owns four
-// consecutive coarse cells of one row h and ONE fine row i.  Its mask reads are 8- or 16-byte loads (four
-// cells of one channel), and the 4*f fine cells it produces are one contiguous run of 4*F*D elements of the
-// output row, stored 16 bytes at a time.  Four cells keep the thread light (about 110 registers, ~1000
-// threads resident per SM); the softmax exponentials use the fast intrinsic (the weights are rounded to the
-// tensor type right after, which hides its error in all but ~0.1 % of the 16-bit cases).
+// element-wise maximum of two pairs
+__device__ __forceinline__ __half2 pair_max(__half2 a, __half2 b) { return __hmax2(a, b); }
+__device__ __forceinline__ __nv_bfloat162 pair_max(__nv_bfloat162 a, __nv_bfloat162 b) { return __hmax2(a, b); }
+template <typename P>
+__device__ __forceinline__ uint32_t pair_word(P p) { return *reinterpret_cast<const uint32_t *>(&p); }
+
+// Reciprocals of two numbers in [1, 9]: the approximate ones and a Newton step (error below one ulp of float32)
+__device__ __forceinline__ float2 rcp_pair(float2 d)
+{
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
+    const float2 e = fma_f32x2(make_float2(-d.x, -d.y), r, make_float2(1.f, 1.f));
+    return fma_f32x2(r, e, r);
+}
+
+// 16-bit types, two-component fields (the model's), factors 2 and 4, any width.  A thread owns two cells of a row and
+// ONE fine row i and takes them through everything in pairs: a weight word holds both cells' weights, multiplied by the
+// pair of their neighbours' components, packed float32 arithmetic in between.  EVEN: the two cells are neighbours and a
+// mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous, and the exponent
+// keeps the rounding error of l * log2(e) (as expf does, which odd widths used to go through).
+// A cell's F fine cells are one aligned store of 8 or 16 bytes.
+// Bound by instruction issue.  Measured, float16: 2 x 384x384 by 4: 33 -> 29 us (four cells and five
+// blocks per SM before); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
+// fine rows per thread) -> 19.
+template <typename T, int F, bool EVEN>
+__global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
+                                                            int B, int H, int W, int segments)
+{
+    constexpr int COLS = EVEN ? 4 : 6;             // columns of neighbours: -1 .. 2 around the pair, or -1 .. 1 around either
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5);
+    const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, fine row
+    const int w0 = static_cast<int>(warp - line * segments) * 64 + (EVEN ? 2 * lane : lane);
+    const uint32_t b = line / static_cast<uint32_t>(H * F);
+    if (b >= static_cast<uint32_t>(B) || w0 >= W) return;
+    const int hi = static_cast<int>(line - b * (H * F)), h = hi / F, i = hi - h * F;
+    const int w1 = EVEN ? w0 + 1 : min(w0 + 32, W - 1);
+    const bool second = EVEN || w0 + 32 < W;
+    const int64_t plane = static_cast<int64_t>(H) * W;
+
+    // neighbours times F, rounded to T, zero outside the map: the pair of x and the pair of y components per tap
+    uint32_t nx[9], ny[9];
+    {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(field) + b * plane;
+        const uint32_t factor = DT<T>::aw_bcast(static_cast<float>(F));
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+            const int hh = h + ky - 1;
+            uint32_t v[COLS];
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                const int ww = EVEN || c < 3 ? w0 + c - 1 : w1 + c - 4;
+                const bool inside = hh >= 0 && hh < H && ww >= 0 && ww < W;
+                v[c] = inside ? DT<T>::aw_mul(__ldg(src + hh * W + ww), factor) : 0u;
+            }
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx) {
+                nx[3 * ky + kx] = __byte_perm(v[kx], v[EVEN ? kx + 1 : kx + 3], 0x5410);
+                ny[3 * ky + kx] = __byte_perm(v[kx], v[EVEN ? kx + 1 : kx + 3], 0x7632);
+            }
+        }
+    }
+
+    const T *m0 = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(i) * F * plane + static_cast<int64_t>(h) * W;
+    uint32_t o0[F], o1[F];
+#pragma unroll
+    for (int j = 0; j < F; ++j) {
+        uint32_t raw[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const T *at = m0 + static_cast<int64_t>(k * F * F + j) * plane;
+            if constexpr (EVEN) {
+                raw[k] = __ldg(reinterpret_cast<const uint32_t *>(at + w0));
+            } else {
+                const unsigned short *u = reinterpret_cast<const unsigned short *>(at);
+                raw[k] = static_cast<uint32_t>(__ldg(u + w0)) | static_cast<uint32_t>(__ldg(u + w1)) << 16;
+            }
+        }
+        typename DT<T>::Bcast top = word_as_pair<T>(raw[0]);
+#pragma unroll
+        for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(raw[k]));
+        const uint32_t tw = pair_word(top);
+        const float2 mx = make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
+        constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+        // log2(e) - kLog2e: what the float32 constant leaves out
+        constexpr float kLog2eRest = static_cast<float>(1.4426950408889634073599 - static_cast<double>(kLog2e));
+        const float2 log2e = make_float2(kLog2e, kLog2e);
+        float2 p[9], den;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
+            if constexpr (EVEN) {      // exp(l - max) as 2^(l * log2e - max * log2e)
+                const float2 t = fma_f32x2(l, log2e, make_float2(mx.x * -kLog2e, mx.y * -kLog2e));
+                p[k] = make_float2(exp2_approx(t.x), exp2_approx(t.y));
+            } else {                   // t = (l - max) * log2e rounded, r what it leaves out: 2^t * (1 + r * ln 2)
+                const float2 d = add_f32x2(l, make_float2(-mx.x, -mx.y));
+                const float2 t = mul_f32x2(d, log2e);
+                float2 r = fma_f32x2(d, log2e, make_float2(-t.x, -t.y));
+                r = fma_f32x2(d, make_float2(kLog2eRest, kLog2eRest), r);
+                const float2 e = make_float2(exp2_approx(t.x), exp2_approx(t.y));
+                p[k] = fma_f32x2(e, mul_f32x2(r, make_float2(kLn2, kLn2)), e);
+            }
+            den = k == 0 ? p[0] : add_f32x2(den, p[k]);
+        }
+        const float2 inv = rcp_pair(den);
+        float sx[2] = {0.f, 0.f}, sy[2] = {0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const float2 q = mul_f32x2(p[k], inv);
+            const typename DT<T>::Bcast w = word_as_pair<T>(DT<T>::aw_from(q.x, q.y));
+            DT<T>::wmul(w, nx[k], sx);
+            DT<T>::wmul(w, ny[k], sy);
+        }
+        o0[j] = DT<T>::aw_from(sx[0], sy[0]);
+        o1[j] = DT<T>::aw_from(sx[1], sy[1]);
+    }
+    uint32_t *row = reinterpret_cast<uint32_t *>(out) + static_cast<int64_t>(line) * W * F;
+    if constexpr (F == 4) {
+        st_128(row + static_cast<int64_t>(w0) * F, o0);
+        if (second) st_128(row + static_cast<int64_t>(w1) * F, o1);
+    } else {
+        st_64(row + static_cast<int64_t>(w0) * F, o0);
+        if (second) st_64(row + static_cast<int64_t>(w1) * F, o1);
+    }
+}
+
+// float32 for the shapes the model uses (F*D <= 8, W a multiple of VW = 4): one thread owns four consecutive coarse cells
+// of one row h and ONE fine row i.  Its mask reads are 16-byte loads (four cells of one channel), and the 4*f fine cells
+// it produces are one contiguous run of the output row, stored 16 bytes at a time.
 template <typename T, int F, int D>
 __global__ void __launch_bounds__(128) upsample_field_vec_kernel(const T *__restrict__ field, const T *__restrict__ mask,
                                                                  T *__restrict__ out, int B, int H, int W)
@@ -129,14 +253,6 @@ __global__ void __launch_bounds__(128) upsample_field_vec_kernel(const T *__rest
         }
     }
 
-    [[maybe_unused]] uint32_t nbw[3][VW + 2];
-    if constexpr (EPW == 2 && D == 2) {
-#pragma unroll
-        for (int ky = 0; ky < 3; ++ky)
-#pragma unroll
-            for (int c = 0; c < VW + 2; ++c) nbw[ky][c] = DT<T>::aw_from(nb[ky][c][0], nb[ky][c][1]);
-    }
-
     float res[VW][F][D];
     const T *mbase = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(h) * W + w0;
 #pragma unroll
@@ -144,20 +260,10 @@ __global__ void __launch_bounds__(128) upsample_field_vec_kernel(const T *__rest
         float lg[9][VW];
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-            uint32_t wds[VW / EPW];
-            const T *src = mbase + static_cast<int64_t>((k * F + i) * F + j) * plane;
-            if constexpr (EPW == 2) {
-                const uint2 t2 = __ldg(reinterpret_cast<const uint2 *>(src));
-                wds[0] = t2.x;
-                wds[1] = t2.y;
-            } else {
-                ld_nc_128(wds, src);
-            }
+            uint32_t wds[VW];
+            ld_nc_128(wds, mbase + static_cast<int64_t>((k * F + i) * F + j) * plane);
 #pragma unroll
-            for (int c = 0; c < VW; ++c) {
-                if constexpr (EPW == 2) lg[k][c] = DT<T>::unpack(wds[c >> 1], c & 1);
-                else lg[k][c] = __uint_as_float(wds[c]);
-            }
+            for (int c = 0; c < VW; ++c) lg[k][c] = __uint_as_float(wds[c]);
         }
 #pragma unroll
         for (int c = 0; c < VW; ++c) {
@@ -176,21 +282,11 @@ __global__ void __launch_bounds__(128) upsample_field_vec_kernel(const T *__rest
             const float inv = __frcp_rn(den);
 #pragma unroll
             for (int d = 0; d < D; ++d) res[c][j][d] = 0.f;
-            if constexpr (EPW == 2 && D == 2) {
-                // both components of a neighbour are one packed word: weight (rounded to T, broadcast)
-                // times word in one packed multiply, each rounded product added to its float32 sum
 #pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    const float pf = p[k] * inv;
-                    DT<T>::wmul(word_as_pair<T>(DT<T>::aw_from(pf, pf)), nbw[k / 3][c + k % 3], &res[c][j][0]);
-                }
-            } else {
+            for (int k = 0; k < 9; ++k) {
+                const float pk = DT<T>::rnd(p[k] * inv);
 #pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    const float pk = DT<T>::rnd(p[k] * inv);
-#pragma unroll
-                    for (int d = 0; d < D; ++d) res[c][j][d] += DT<T>::rnd(pk * nb[k / 3][c + k % 3][d]);
-                }
+                for (int d = 0; d < D; ++d) res[c][j][d] += DT<T>::rnd(pk * nb[k / 3][c + k % 3][d]);
             }
         }
     }
@@ -232,8 +328,23 @@ cudaError_t launch(const void *field, const void *mask, void *out, int B, int H,
     const T *f = static_cast<const T *>(field), *m = static_cast<const T *>(mask);
     T *o = static_cast<T *>(out);
     // the model's shapes: a 2-component field, factor 2 between stages and 4 at the end
-    if (D == 2 && factor == 2 && try_vec<T, 2, 2>(f, m, o, B, H, W, stream)) return cudaGetLastError();
-    if (D == 2 && factor == 4 && try_vec<T, 4, 2>(f, m, o, B, H, W, stream)) return cudaGetLastError();
+    if constexpr (sizeof(T) == 2) {
+        const int64_t segments = (W + 63) / 64, warps = segments * H * factor * B;
+        if (D == 2 && (factor == 2 || factor == 4) && (reinterpret_cast<uintptr_t>(f) & 3u) == 0 &&
+            (reinterpret_cast<uintptr_t>(o) & 15u) == 0 && static_cast<int64_t>(H) * W < (1LL << 31) && warps < (1LL << 31)) {
+            const bool even = W % 2 == 0 && (reinterpret_cast<uintptr_t>(m) & 3u) == 0;
+            const unsigned blocks = static_cast<unsigned>((warps + 3) / 4);
+            const int seg = static_cast<int>(segments);
+            if (factor == 4 && even) upsample_pair_kernel<T, 4, true><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+            else if (factor == 4) upsample_pair_kernel<T, 4, false><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+            else if (even) upsample_pair_kernel<T, 2, true><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+            else upsample_pair_kernel<T, 2, false><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+            return cudaGetLastError();
+        }
+    } else {
+        if (D == 2 && factor == 2 && try_vec<T, 2, 2>(f, m, o, B, H, W, stream)) return cudaGetLastError();
+        if (D == 2 && factor == 4 && try_vec<T, 4, 2>(f, m, o, B, H, W, stream)) return cudaGetLastError();
+    }
     switch (factor) {
     case 1: upsample_field_kernel<T, 1><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;
     case 2: upsample_field_kernel<T, 2><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;

@@ -55,3 +55,17 @@ def test_bad_arguments_raise():
         ma.upsample_field(field, torch.zeros(1, 81, 4, 4, device="cuda"), 3)        # factor 3 is not built
     with pytest.raises(RuntimeError):
         ma.upsample_field(field.cpu(), torch.zeros(1, 36, 4, 4), 2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("factor", [2, 4])
+@pytest.mark.parametrize("H,W", [(1, 1), (2, 2), (3, 31), (2, 33), (1, 63), (3, 64), (2, 65), (5, 98), (2, 129)])
+def test_pairs_of_cells_at_the_edges_of_a_warp(H, W, factor, dtype):
+    """Widths around the 32 and 64 cells of a warp, odd and even, down to a map of one cell."""
+    import matchattention_b200 as ma
+    import oracle
+    g = torch.Generator().manual_seed(H * W + factor)
+    field = (torch.randn(2, H, W, 2, generator=g) * 4).to(dtype)
+    mask = (torch.randn(2, 9 * factor * factor, H, W, generator=g) * 2).to(dtype)
+    out = ma.upsample_field(field.cuda(), mask.cuda(), factor).cpu()
+    assert_close_sum_of_products(out, oracle.upsample_field(field, mask, factor), dtype, float(field.float().abs().max()) * factor)
