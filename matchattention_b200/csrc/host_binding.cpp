@@ -192,12 +192,20 @@ struct MatchAttentionFn : torch::autograd::Function<MatchAttentionFn> {
         void *stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
         void *dattn = d_attn.defined() ? data(d_attn) : nullptr, *dmo = d_mo.defined() ? data(d_mo) : nullptr;
         const size_t bytes = matchattn_backward_workspace_bytes(B, H, W, h, C / h, r, dtype_code(q), 0, H);
+        // without room for the workspace (8 bytes per query, head and tap) the accumulating call below serves
+        Tensor ws;
         if (bytes != 0) {
-            Tensor d_k = at::empty_like(k), d_v = at::empty_like(v), ws = at::empty({static_cast<int64_t>(bytes)}, q.options().dtype(at::kByte));
+            try {
+                ws = at::empty({static_cast<int64_t>(bytes)}, q.options().dtype(at::kByte));
+            } catch (const c10::OutOfMemoryError &) {
+            }
+        }
+        if (ws.defined()) {
+            Tensor d_k = at::empty_like(k), d_v = at::empty_like(v);
             const int status = matchattn_fused_backward_ws(data(mo), data(q), data(k), data(v), data(d_out), dattn, data(d_q), data(d_k), data(d_v),
                                                            dmo, B, H, W, h, C / h, r, r, dtype_code(q), MATCHATTN_L1_NORM, scale, 0, H, data(ws),
                                                            bytes, stream);
-            if (status != MATCHATTN_ERR_VARIANT) {       // that one: a tensor is not 16-byte aligned
+            if (status != MATCHATTN_ERR_VARIANT) {       // that one: a tensor is not 32-byte aligned
                 check_status(status);
                 return {d_mo, d_q, d_k, d_v, Tensor(), Tensor(), Tensor(), Tensor()};
             }
