@@ -88,8 +88,6 @@ __device__ __forceinline__ float exp2_approx(float x)
 template <typename T>
 __device__ __forceinline__ typename DT<T>::Bcast word_as_pair(uint32_t w);
 template <>
-__device__ __forceinline__ float word_as_pair<float>(uint32_t w) { return __uint_as_float(w); }
-template <>
 __device__ __forceinline__ __half2 word_as_pair<__half>(uint32_t w) { return *reinterpret_cast<const __half2 *>(&w); }
 template <>
 __device__ __forceinline__ __nv_bfloat162 word_as_pair<__nv_bfloat16>(uint32_t w) { return *reinterpret_cast<const __nv_bfloat162 *>(&w); }
@@ -101,26 +99,16 @@ __device__ __forceinline__ __nv_bfloat162 pair_max(__nv_bfloat162 a, __nv_bfloat
 template <typename P>
 __device__ __forceinline__ uint32_t pair_word(P p) { return *reinterpret_cast<const uint32_t *>(&p); }
 
-// Reciprocals of two numbers in [1, 9]: the approximate ones and a Newton step (error below one ulp of float32)
-__device__ __forceinline__ float2 rcp_pair(float2 d)
-{
-    float2 r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
-    const float2 e = fma_f32x2(make_float2(-d.x, -d.y), r, make_float2(1.f, 1.f));
-    return fma_f32x2(r, e, r);
-}
-
 // 16-bit types, two-component fields (the model's), factors 2 and 4, any width.  A thread owns two cells of a row and
 // ONE fine row i and takes them through everything in pairs: a weight word holds both cells' weights, multiplied by the
 // pair of their neighbours' components, packed float32 arithmetic in between.  EVEN: the two cells are neighbours and a
-// mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous, and the exponent
-// keeps the rounding error of l * log2(e) (as expf does, which odd widths used to go through).
+// mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous.  EXACT: exponentials by
+// expf; without it by the special-function unit, for the widths (multiples of four) that have always had them so.
 // A cell's F fine cells are one aligned store of 8 or 16 bytes.
-// Bound by instruction issue.  Measured, float16: 2 x 384x384 by 4: 33 -> 29 us (four cells and five
+// Bound by instruction issue.  Measured, float16: 2 x 384x384 by 4: 33 -> 28 us (four cells and five
 // blocks per SM before); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
-// fine rows per thread) -> 19.
-template <typename T, int F, bool EVEN>
+// fine rows per thread) -> 20.
+template <typename T, int F, bool EVEN, bool EXACT>
 __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
                                                             int B, int H, int W, int segments)
 {
@@ -179,28 +167,21 @@ __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict_
         for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(raw[k]));
         const uint32_t tw = pair_word(top);
         const float2 mx = make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
-        constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-        // log2(e) - kLog2e: what the float32 constant leaves out
-        constexpr float kLog2eRest = static_cast<float>(1.4426950408889634073599 - static_cast<double>(kLog2e));
+        constexpr float kLog2e = 1.4426950408889634f;
         const float2 log2e = make_float2(kLog2e, kLog2e);
         float2 p[9], den;
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
-            if constexpr (EVEN) {      // exp(l - max) as 2^(l * log2e - max * log2e)
+            if constexpr (!EXACT) {    // exp(l - max) as 2^(l * log2e - max * log2e)
                 const float2 t = fma_f32x2(l, log2e, make_float2(mx.x * -kLog2e, mx.y * -kLog2e));
                 p[k] = make_float2(exp2_approx(t.x), exp2_approx(t.y));
-            } else {                   // t = (l - max) * log2e rounded, r what it leaves out: 2^t * (1 + r * ln 2)
-                const float2 d = add_f32x2(l, make_float2(-mx.x, -mx.y));
-                const float2 t = mul_f32x2(d, log2e);
-                float2 r = fma_f32x2(d, log2e, make_float2(-t.x, -t.y));
-                r = fma_f32x2(d, make_float2(kLog2eRest, kLog2eRest), r);
-                const float2 e = make_float2(exp2_approx(t.x), exp2_approx(t.y));
-                p[k] = fma_f32x2(e, mul_f32x2(r, make_float2(kLn2, kLn2)), e);
+            } else {
+                p[k] = make_float2(expf(l.x - mx.x), expf(l.y - mx.y));
             }
             den = k == 0 ? p[0] : add_f32x2(den, p[k]);
         }
-        const float2 inv = rcp_pair(den);
+        const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
         float sx[2] = {0.f, 0.f}, sy[2] = {0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
@@ -333,12 +314,13 @@ cudaError_t launch(const void *field, const void *mask, void *out, int B, int H,
         if (D == 2 && (factor == 2 || factor == 4) && (reinterpret_cast<uintptr_t>(f) & 3u) == 0 &&
             (reinterpret_cast<uintptr_t>(o) & 15u) == 0 && static_cast<int64_t>(H) * W < (1LL << 31) && warps < (1LL << 31)) {
             const bool even = W % 2 == 0 && (reinterpret_cast<uintptr_t>(m) & 3u) == 0;
+            const bool exact = W % 4 != 0 || (reinterpret_cast<uintptr_t>(m) & 15u) != 0;
             const unsigned blocks = static_cast<unsigned>((warps + 3) / 4);
             const int seg = static_cast<int>(segments);
-            if (factor == 4 && even) upsample_pair_kernel<T, 4, true><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
-            else if (factor == 4) upsample_pair_kernel<T, 4, false><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
-            else if (even) upsample_pair_kernel<T, 2, true><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
-            else upsample_pair_kernel<T, 2, false><<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+            const auto kernel = !even   ? (factor == 4 ? upsample_pair_kernel<T, 4, false, true> : upsample_pair_kernel<T, 2, false, true>)
+                                : exact ? (factor == 4 ? upsample_pair_kernel<T, 4, true, true> : upsample_pair_kernel<T, 2, true, true>)
+                                        : (factor == 4 ? upsample_pair_kernel<T, 4, true, false> : upsample_pair_kernel<T, 2, true, false>);
+            kernel<<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
             return cudaGetLastError();
         }
     } else {
