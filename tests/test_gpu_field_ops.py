@@ -177,3 +177,15 @@ def test_local_disparity_kernel_at_the_edges_of_its_shares(D, H, W, dtype):
     same = centre.cpu() == want_centre
     assert same.float().mean() > 0.98           # the rest: equal box averages
     assert _close16(flow.cpu()[same], want_flow[same], dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H,W", [(5, 6), (10, 13), (6, 22), (12, 21), (71, 74), (68, 77)])
+def test_flow_init_rows_aligned_to_two_and_four_elements(H, W, dtype):
+    """Token counts that are multiples of 2 or 4 but not of 8, around a chunk, below and above 5000: the same bits as the
+    any-alignment kernels, which an operand that starts one element off takes."""
+    g = torch.Generator().manual_seed(H * W)
+    corr = (torch.randn(2, H * W, H * W, generator=g) * 2.0).to(dtype).cuda()
+    odd = torch.empty(corr.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(corr).copy_(corr)
+    for got, want in zip(_ma().flow_init(corr, H, W, return_debug=True), _ma().flow_init(odd, H, W, return_debug=True)):
+        assert torch.equal(got, want)
