@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict_
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
-            if constexpr (!EXACT) {    // exp(l - max) as 2^(l * log2e - max * log2e)
-                const float2 t = fma_f32x2(l, log2e, make_float2(mx.x * -kLog2e, mx.y * -kLog2e));
+            if constexpr (!EXACT) {    // the difference first: log2e times a logit near the largest of the type overflows
+                const float2 t = mul_f32x2(add_f32x2(l, make_float2(-mx.x, -mx.y)), log2e);
                 p[k] = make_float2(exp2_approx(t.x), exp2_approx(t.y));
             } else {
                 p[k] = make_float2(expf(l.x - mx.x), expf(l.y - mx.y));
@@ -251,13 +251,12 @@ __global__ void __launch_bounds__(128) upsample_field_vec_kernel(const T *__rest
             float mx = lg[0][c];
 #pragma unroll
             for (int k = 1; k < 9; ++k) mx = fmaxf(mx, lg[k][c]);
-            // exp(l - mx) as 2^(l * log2e - mx * log2e), one fused multiply-add and one special-function op
+            // exp(l - mx) as 2^((l - mx) * log2e); the difference first, log2e times a logit near the largest float overflows
             constexpr float kLog2e = 1.4426950408889634f;
-            const float shift = -mx * kLog2e;
             float p[9], den = 0.f;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
-                p[k] = exp2_approx(fmaf(lg[k][c], kLog2e, shift));
+                p[k] = exp2_approx((lg[k][c] - mx) * kLog2e);
                 den += p[k];
             }
             const float inv = __frcp_rn(den);

@@ -69,3 +69,22 @@ def test_pairs_of_cells_at_the_edges_of_a_warp(H, W, factor, dtype):
     mask = (torch.randn(2, 9 * factor * factor, H, W, generator=g) * 2).to(dtype)
     out = ma.upsample_field(field.cuda(), mask.cuda(), factor).cpu()
     assert_close_sum_of_products(out, oracle.upsample_field(field, mask, factor), dtype, float(field.float().abs().max()) * factor)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("factor,W", [(2, 8), (4, 8), (4, 6), (2, 7)])
+def test_logits_at_the_ends_of_the_type(factor, W, dtype):
+    """Logits at the type's lowest and largest value (a caller's mask) are ordinary numbers to a softmax: nine equal
+    ones weigh 1/9 each, one that stands out takes all."""
+    import matchattention_b200 as ma
+    H, low, top = 3, torch.finfo(dtype).min, torch.finfo(dtype).max
+    field = torch.ones(1, H, W, 2, dtype=dtype)
+    for fill, pick in ((low, None), (top, None), (low, top), (low, 0.0)):
+        mask = torch.full((1, 9, factor * factor, H, W), fill, dtype=dtype)
+        if pick is not None:
+            mask[:, 4] = pick                        # the cell itself
+        out = ma.upsample_field(field.cuda(), mask.view(1, -1, H, W).cuda(), factor).float().cpu()
+        if pick is None:                             # cells inside the map's border see nine ones
+            out = out[:, factor:-factor, factor:-factor]
+        # nine weights and nine products, each rounded to the type, then the sum
+        assert (out - factor).abs().max() <= 4 * torch.finfo(dtype).eps * factor
