@@ -15,12 +15,49 @@
 
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "matchattn_kernels.cuh"
 
 namespace matchattn {
 namespace {
 
 constexpr int kMaxD = 8;
+constexpr float kLog2e = 1.4426950408889634f;
+
+__device__ __forceinline__ float exp2_approx(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// exp(l - top), top the largest logit: one way per type, whatever the width, the address or the kernel.  float32: expf.  The
+// 16-bit types round the weight to the type right after and take the special-function unit alone; bfloat16 takes the
+// difference first, since log2e times a logit near its largest value overflows, which float16 is far from (the rounding of
+// top * log2e is a factor common to the nine weights).  Relative error of the result against 64 bits, 2 x 384x384 by 4:
+// float16 3.597e-4 and bfloat16 2.875e-3, with expf the same; float32 8.55e-8 (8.71e-8 with the special-function unit).
+template <typename T>
+__device__ __forceinline__ float weight_exp(float l, float top)
+{
+    if constexpr (sizeof(T) == 4) return expf(l - top);
+    else if constexpr (std::is_same_v<T, __half>) return exp2_approx(fmaf(l, kLog2e, top * -kLog2e));
+    else return exp2_approx((l - top) * kLog2e);
+}
+template <typename T>
+__device__ __forceinline__ float2 weight_exp(float2 l, float2 top)
+{
+    const float2 log2e = make_float2(kLog2e, kLog2e);
+    float2 t;
+    if constexpr (std::is_same_v<T, __half>) {
+        t = fma_f32x2(l, log2e, make_float2(top.x * -kLog2e, top.y * -kLog2e));
+    } else {
+        t = add_f32x2(l, make_float2(-top.x, -top.y));
+        if constexpr (sizeof(T) == 4) return make_float2(expf(t.x), expf(t.y));
+        t = mul_f32x2(t, log2e);
+    }
+    return make_float2(exp2_approx(t.x), exp2_approx(t.y));
+}
 
 template <typename T, int F>
 __global__ void __launch_bounds__(128) upsample_field_kernel(const T *__restrict__ field, const T *__restrict__ mask,
@@ -58,7 +95,7 @@ __global__ void __launch_bounds__(128) upsample_field_kernel(const T *__restrict
             float den = 0.f;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
-                p[k] = expf(p[k] - mx);
+                p[k] = weight_exp<T>(p[k], mx);
                 den += p[k];
             }
             const float inv = __frcp_rn(den);
@@ -74,14 +111,6 @@ __global__ void __launch_bounds__(128) upsample_field_kernel(const T *__restrict
             }
         }
     }
-}
-
-// 2^x by the special-function unit (the weights are rounded to the tensor type right after)
-__device__ __forceinline__ float exp2_approx(float x)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 
 // a packed 32-bit word of two 16-bit values as the pair type of the element-wise helpers
@@ -102,13 +131,11 @@ __device__ __forceinline__ uint32_t pair_word(P p) { return *reinterpret_cast<co
 // 16-bit types, two-component fields (the model's), factors 2 and 4, any width.  A thread owns two cells of a row and
 // ONE fine row i and takes them through everything in pairs: a weight word holds both cells' weights, multiplied by the
 // pair of their neighbours' components, packed float32 arithmetic in between.  EVEN: the two cells are neighbours and a
-// mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous.  EXACT: exponentials by
-// expf; without it by the special-function unit, for the widths (multiples of four) that have always had them so.
-// A cell's F fine cells are one aligned store of 8 or 16 bytes.
+// mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous.  A cell's F fine cells are one aligned store of 8 or 16 bytes.
 // Bound by instruction issue.  Measured, float16: 2 x 384x384 by 4: 33 -> 28 us (four cells and five
 // blocks per SM before); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
-// fine rows per thread) -> 20.
-template <typename T, int F, bool EVEN, bool EXACT>
+// fine rows per thread) -> 17.7.
+template <typename T, int F, bool EVEN>
 __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
                                                             int B, int H, int W, int segments)
 {
@@ -167,18 +194,11 @@ __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict_
         for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(raw[k]));
         const uint32_t tw = pair_word(top);
         const float2 mx = make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
-        constexpr float kLog2e = 1.4426950408889634f;
-        const float2 log2e = make_float2(kLog2e, kLog2e);
         float2 p[9], den;
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
-            if constexpr (!EXACT) {    // the difference first: log2e times a logit near the largest of the type overflows
-                const float2 t = mul_f32x2(add_f32x2(l, make_float2(-mx.x, -mx.y)), log2e);
-                p[k] = make_float2(exp2_approx(t.x), exp2_approx(t.y));
-            } else {
-                p[k] = make_float2(expf(l.x - mx.x), expf(l.y - mx.y));
-            }
+            p[k] = weight_exp<T>(l, mx);
             den = k == 0 ? p[0] : add_f32x2(den, p[k]);
         }
         const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
@@ -203,101 +223,67 @@ __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict_
     }
 }
 
-// float32 for the shapes the model uses (F*D <= 8, W a multiple of VW = 4): one thread owns four consecutive coarse cells
-// of one row h and ONE fine row i.  Its mask reads are 16-byte loads (four cells of one channel), and the 4*f fine cells
-// it produces are one contiguous run of the output row, stored 16 bytes at a time.
-template <typename T, int F, int D>
-__global__ void __launch_bounds__(128) upsample_field_vec_kernel(const T *__restrict__ field, const T *__restrict__ mask,
-                                                                 T *__restrict__ out, int B, int H, int W)
+// float32, two-component fields, factors 2 and 4, even widths: a thread owns two neighbouring cells of a row and ONE fine
+// row i, as above; the cells go through the softmax and the components through the sums in pairs (packed float32
+// arithmetic), and its 2*F fine cells are one contiguous run of the output row, stored 16 bytes at a time.
+// Measured, 2 x 384x384 by 4: 43.8 us (four cells per thread, exponentials by the special-function unit alone: 47.7; with
+// expf 50.7, in pairs 64.2 at 137 registers); 2 x 201x302 by 4: 22.7 (one cell and all its fine rows per thread: 55.5).
+template <int F>
+__global__ void __launch_bounds__(128) upsample_f32_kernel(const float *__restrict__ field, const float *__restrict__ mask,
+                                                           float *__restrict__ out, int B, int H, int W, int segments)
 {
-    constexpr int VW = 4;                           // cells per thread
-    constexpr int EPW = DT<T>::kElemsPerWord;
-    const int wq = blockIdx.x * blockDim.x + threadIdx.x;        // group of VW cells
-    const int w0 = wq * VW;
-    if (w0 >= W) return;
-    const int hi = blockIdx.y, b = blockIdx.z;
-    const int h = hi / F, i = hi - h * F;
+    const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5);
+    const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, fine row
+    const int w0 = static_cast<int>(warp - line * segments) * 64 + 2 * (threadIdx.x & 31);
+    const uint32_t b = line / static_cast<uint32_t>(H * F);
+    if (b >= static_cast<uint32_t>(B) || w0 >= W) return;
+    const int hi = static_cast<int>(line - b * (H * F)), h = hi / F, i = hi - h * F;
     const int64_t plane = static_cast<int64_t>(H) * W;
 
-    // field * f for rows h-1..h+1, columns w0-1..w0+VW, rounded to T; zero outside the map
-    float nb[3][VW + 2][D];
+    // neighbours times F in columns w0 - 1 .. w0 + 2, zero outside the map
+    float2 nb[3][4];
 #pragma unroll
     for (int ky = 0; ky < 3; ++ky) {
         const int hh = h + ky - 1;
 #pragma unroll
-        for (int c = 0; c < VW + 2; ++c) {
+        for (int c = 0; c < 4; ++c) {
             const int ww = w0 + c - 1;
             const bool inside = hh >= 0 && hh < H && ww >= 0 && ww < W;
-            const T *src = field + ((static_cast<int64_t>(b) * H + (inside ? hh : h)) * W + (inside ? ww : w0)) * D;
-#pragma unroll
-            for (int d = 0; d < D; ++d) nb[ky][c][d] = inside ? DT<T>::rnd(load_one<T>(src + d) * static_cast<float>(F)) : 0.f;
+            const float *src = field + (b * plane + (inside ? static_cast<int64_t>(hh) * W + ww : 0)) * 2;
+            nb[ky][c] = inside ? make_float2(load_one<float>(src) * F, load_one<float>(src + 1) * F) : make_float2(0.f, 0.f);
         }
     }
 
-    float res[VW][F][D];
-    const T *mbase = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(h) * W + w0;
+    const float *m0 = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(i) * F * plane + static_cast<int64_t>(h) * W + w0;
+    float2 first[F], second[F];
 #pragma unroll
     for (int j = 0; j < F; ++j) {
-        float lg[9][VW];
+        float2 p[9], den;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) p[k] = __ldg(reinterpret_cast<const float2 *>(m0 + static_cast<int64_t>(k * F * F + j) * plane));
+        float2 mx = p[0];
+#pragma unroll
+        for (int k = 1; k < 9; ++k) mx = make_float2(fmaxf(mx.x, p[k].x), fmaxf(mx.y, p[k].y));
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-            uint32_t wds[VW];
-            ld_nc_128(wds, mbase + static_cast<int64_t>((k * F + i) * F + j) * plane);
-#pragma unroll
-            for (int c = 0; c < VW; ++c) lg[k][c] = __uint_as_float(wds[c]);
+            p[k] = weight_exp<float>(p[k], mx);
+            den = k == 0 ? p[0] : add_f32x2(den, p[k]);
         }
+        const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
+        first[j] = second[j] = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < VW; ++c) {
-            float mx = lg[0][c];
-#pragma unroll
-            for (int k = 1; k < 9; ++k) mx = fmaxf(mx, lg[k][c]);
-            // exp(l - mx) as 2^((l - mx) * log2e); the difference first, log2e times a logit near the largest float overflows
-            constexpr float kLog2e = 1.4426950408889634f;
-            float p[9], den = 0.f;
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                p[k] = exp2_approx((lg[k][c] - mx) * kLog2e);
-                den += p[k];
-            }
-            const float inv = __frcp_rn(den);
-#pragma unroll
-            for (int d = 0; d < D; ++d) res[c][j][d] = 0.f;
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                const float pk = DT<T>::rnd(p[k] * inv);
-#pragma unroll
-                for (int d = 0; d < D; ++d) res[c][j][d] += DT<T>::rnd(pk * nb[k / 3][c + k % 3][d]);
-            }
+        for (int k = 0; k < 9; ++k) {
+            const float2 q = mul_f32x2(p[k], inv);
+            first[j] = fma_f32x2(make_float2(q.x, q.x), nb[k / 3][k % 3], first[j]);
+            second[j] = fma_f32x2(make_float2(q.y, q.y), nb[k / 3][k % 3 + 1], second[j]);
         }
     }
-
-    // VW*F*D consecutive elements of the fine row h*F+i
-    T *orow = out + ((static_cast<int64_t>(b) * H * F + hi) * W * F + static_cast<int64_t>(w0) * F) * D;
-    constexpr int NEL = VW * F * D;
-    const float *flat = &res[0][0][0];
-    if constexpr ((NEL * sizeof(T)) % 16 == 0) {
-        constexpr int NWORDS = NEL / EPW;
-        uint32_t ow[NWORDS];
+    float4 *row = reinterpret_cast<float4 *>(out + (static_cast<int64_t>(line) * W + w0) * F * 2);
 #pragma unroll
-        for (int x = 0; x < NWORDS; ++x) ow[x] = DT<T>::pack(&flat[x * EPW]);
-#pragma unroll
-        for (int x = 0; x < NWORDS / 4; ++x) st_128(reinterpret_cast<char *>(orow) + 16 * x, &ow[4 * x]);
-    } else {
-#pragma unroll
-        for (int x = 0; x < NEL; ++x) store_one<T>(orow + x, flat[x]);
+    for (int j = 0; j < F / 2; ++j) {
+        row[j] = make_float4(first[2 * j].x, first[2 * j].y, first[2 * j + 1].x, first[2 * j + 1].y);
+        row[F / 2 + j] = make_float4(second[2 * j].x, second[2 * j].y, second[2 * j + 1].x, second[2 * j + 1].y);
     }
-}
-
-template <typename T, int F, int D>
-bool try_vec(const T *f, const T *m, T *o, int B, int H, int W, cudaStream_t stream)
-{
-    constexpr int VW = 4;
-    if (W % VW != 0 || (reinterpret_cast<uintptr_t>(m) % 16) != 0 || (reinterpret_cast<uintptr_t>(o) % 16) != 0 ||
-        1LL * H * F > 65535)
-        return false;
-    const dim3 grid((W / VW + 127) / 128, H * F, B), block(128);
-    upsample_field_vec_kernel<T, F, D><<<grid, block, 0, stream>>>(f, m, o, B, H, W);
-    return true;
 }
 
 template <typename T>
@@ -308,23 +294,24 @@ cudaError_t launch(const void *field, const void *mask, void *out, int B, int H,
     const T *f = static_cast<const T *>(field), *m = static_cast<const T *>(mask);
     T *o = static_cast<T *>(out);
     // the model's shapes: a 2-component field, factor 2 between stages and 4 at the end
-    if constexpr (sizeof(T) == 2) {
-        const int64_t segments = (W + 63) / 64, warps = segments * H * factor * B;
-        if (D == 2 && (factor == 2 || factor == 4) && (reinterpret_cast<uintptr_t>(f) & 3u) == 0 &&
-            (reinterpret_cast<uintptr_t>(o) & 15u) == 0 && static_cast<int64_t>(H) * W < (1LL << 31) && warps < (1LL << 31)) {
-            const bool even = W % 2 == 0 && (reinterpret_cast<uintptr_t>(m) & 3u) == 0;
-            const bool exact = W % 4 != 0 || (reinterpret_cast<uintptr_t>(m) & 15u) != 0;
-            const unsigned blocks = static_cast<unsigned>((warps + 3) / 4);
-            const int seg = static_cast<int>(segments);
-            const auto kernel = !even   ? (factor == 4 ? upsample_pair_kernel<T, 4, false, true> : upsample_pair_kernel<T, 2, false, true>)
-                                : exact ? (factor == 4 ? upsample_pair_kernel<T, 4, true, true> : upsample_pair_kernel<T, 2, true, true>)
-                                        : (factor == 4 ? upsample_pair_kernel<T, 4, true, false> : upsample_pair_kernel<T, 2, true, false>);
+    const int64_t segments = (W + 63) / 64, warps = segments * H * factor * B;
+    const unsigned blocks = static_cast<unsigned>((warps + 3) / 4);
+    const int seg = static_cast<int>(segments);
+    const bool even = W % 2 == 0 && reinterpret_cast<uintptr_t>(m) % (2 * sizeof(T)) == 0;
+    if (D == 2 && (factor == 2 || factor == 4) && (reinterpret_cast<uintptr_t>(o) & 15u) == 0 &&
+        static_cast<int64_t>(H) * W < (1LL << 31) && warps < (1LL << 31)) {
+        if constexpr (sizeof(T) == 2) {
+            if ((reinterpret_cast<uintptr_t>(f) & 3u) == 0) {
+                const auto kernel = even ? (factor == 4 ? upsample_pair_kernel<T, 4, true> : upsample_pair_kernel<T, 2, true>)
+                                         : (factor == 4 ? upsample_pair_kernel<T, 4, false> : upsample_pair_kernel<T, 2, false>);
+                kernel<<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+                return cudaGetLastError();
+            }
+        } else if (even) {
+            const auto kernel = factor == 4 ? upsample_f32_kernel<4> : upsample_f32_kernel<2>;
             kernel<<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
             return cudaGetLastError();
         }
-    } else {
-        if (D == 2 && factor == 2 && try_vec<T, 2, 2>(f, m, o, B, H, W, stream)) return cudaGetLastError();
-        if (D == 2 && factor == 4 && try_vec<T, 4, 2>(f, m, o, B, H, W, stream)) return cudaGetLastError();
     }
     switch (factor) {
     case 1: upsample_field_kernel<T, 1><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;

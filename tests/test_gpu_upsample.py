@@ -88,3 +88,30 @@ def test_logits_at_the_ends_of_the_type(factor, W, dtype):
             out = out[:, factor:-factor, factor:-factor]
         # nine weights and nine products, each rounded to the type, then the sum
         assert (out - factor).abs().max() <= 4 * torch.finfo(dtype).eps * factor
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,factor,W", [(2, 2, 64), (2, 4, 36), (2, 4, 62), (2, 2, 33), (3, 4, 32)])
+def test_the_address_does_not_change_the_bits(D, factor, W, dtype):
+    """The same mask one, two, four or eight elements into a buffer reaches other kernels and loads; the result is the same."""
+    import matchattention_b200 as ma
+    g = torch.Generator().manual_seed(W)
+    field = (torch.randn(2, 5, W, D, generator=g) * 4).to(dtype).cuda()
+    mask = (torch.randn(2, 9 * factor * factor, 5, W, generator=g) * 3).to(dtype).cuda()
+    want = ma.upsample_field(field, mask, factor)
+    for shift in (1, 2, 4, 8):
+        moved = torch.empty(mask.numel() + shift, dtype=dtype, device="cuda")[shift:].view(mask.shape).copy_(mask)
+        assert torch.equal(ma.upsample_field(field, moved, factor), want), shift
+
+
+@pytest.mark.parametrize("factor", [2, 4])
+@pytest.mark.parametrize("H,W", [(1, 2), (2, 4), (1, 62), (3, 64), (2, 66), (5, 98), (2, 130)])
+def test_float32_pairs_at_the_edges_of_a_warp(H, W, factor):
+    """Even widths around the 64 cells of a warp, down to a map of two cells."""
+    import matchattention_b200 as ma
+    import oracle
+    g = torch.Generator().manual_seed(H * W + factor)
+    field = torch.randn(2, H, W, 2, generator=g) * 4
+    mask = torch.randn(2, 9 * factor * factor, H, W, generator=g) * 2
+    out = ma.upsample_field(field.cuda(), mask.cuda(), factor).cpu()
+    assert_close_sum_of_products(out, oracle.upsample_field(field, mask, factor), torch.float32, float(field.abs().max()) * factor)
