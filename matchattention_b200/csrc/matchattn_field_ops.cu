@@ -62,11 +62,13 @@ __global__ void __launch_bounds__(256) consistency_mask_kernel(const T *__restri
 // Measured, float16, 2 x 120 x 68 x 120: 5.8 us, before 41.4.
 constexpr int kDispGroups = 8, kDispBatch = 8;
 
-// x / 5 to the last bit: one Newton step on the product with the rounded reciprocal (Markstein, IBM J. Res. Dev. 34, 1990)
+// x / 5: 1/5 as the sum of two floats of one sign, so that an infinite x stays infinite (multiplication by a constant of
+// two words: Brisebarre and Muller, IEEE Trans. Computers 57, 2008).  The quotient of every |x| >= 2^-120 to the last bit
+// (all 2^23 significands tried); below, the first product underflows and the last bit may differ.
 __device__ __forceinline__ float fifth(float x)
 {
-    const float q = x * 0.2f;
-    return fmaf(fmaf(-q, 5.f, x), 0.2f, q);
+    constexpr float kHigh = 0.19999998807907104f, kLow = 0.2 - static_cast<double>(kHigh);
+    return fmaf(x, kHigh, x * kLow);
 }
 
 template <typename T>

@@ -189,3 +189,14 @@ def test_flow_init_rows_aligned_to_two_and_four_elements(H, W, dtype):
     odd = torch.empty(corr.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(corr).copy_(corr)
     for got, want in zip(_ma().flow_init(corr, H, W, return_debug=True), _ma().flow_init(odd, H, W, return_debug=True)):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_local_disparity_of_an_infinite_value(dtype):
+    """A window that holds an infinity has an infinite average: the first such window is the arg max, and its flow is
+    infinity over infinity."""
+    vol = torch.rand(2, 40, 3, 5).to(dtype)
+    vol[:, 17, 1, 2] = float("inf")
+    flow, blur, centre = _ma().local_disparity_estimator(vol.cuda(), return_debug=True)
+    assert (blur[:, 1, 2] == float("inf")).all() and (centre[:, 1, 2] == 15).all() and flow[:, 1, 2, 0].isnan().all()
+    assert torch.isfinite(flow).sum() == flow.numel() - 2
