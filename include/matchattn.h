@@ -184,7 +184,7 @@ MATCHATTN_API int matchattn_fused_backward(const void *max_offset, const void *q
  * accumulated: the (query, head) items are bucketed by the token their window starts at, and every token sums the
  * contributions of the buckets around it (no floating-point atomics).  About three times as fast as the call above
  * plus the clearing and conversion around it.  Covered: head widths that are multiples of 8, r = 1 or 2, 32-byte
- * aligned arrays; MATCHATTN_ERR_VARIANT otherwise.
+ * aligned arrays (max_offset: aligned to its pair); MATCHATTN_ERR_VARIANT otherwise.
  *   workspace  at least matchattn_backward_workspace_bytes(...) bytes of device memory, 256-byte aligned; contents
  *              need not be preserved between calls, but calls that overlap on the device must not share it
  */

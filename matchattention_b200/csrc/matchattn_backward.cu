@@ -32,6 +32,7 @@
 
 #include <stdint.h>
 
+#include <initializer_list>
 #include <type_traits>
 
 #include "matchattn_kernels.cuh"
@@ -1235,6 +1236,10 @@ int backward_params(BwdParams &p, const void *max_offset, const void *q, const v
     if (2 * rx + 2 > W || 2 * ry + 2 > H) return MATCHATTN_ERR_WINDOW_FIT;
     const long long C = 1LL * h * hd, N = 1LL * H * W, Nq = 1LL * (q_row_end - q_row_begin) * W;
     if (C > 65536 || N * C >= 2147483647LL || Nq * h >= 2147483647LL || B > 65535) return MATCHATTN_ERR_TOO_LARGE;
+    const uintptr_t esize = dtype == MATCHATTN_F32 ? 4 : 2;
+    const std::initializer_list<const void *> arrays = {max_offset, q, k, v, d_out, d_attn, d_q, d_max_offset};
+    for (const void *ptr : arrays)
+        if (reinterpret_cast<uintptr_t>(ptr) % esize != 0) return MATCHATTN_ERR_ALIGN;
     p.mo = max_offset; p.q = q; p.k = k; p.v = v; p.dout = d_out; p.dattn = d_attn;
     p.dq = d_q; p.dmo = d_max_offset;
     p.B = B; p.H = H; p.W = W; p.h = h; p.hd = hd; p.C = static_cast<int>(C); p.r = rx;
@@ -1259,6 +1264,7 @@ extern "C" int matchattn_fused_backward(const void *max_offset, const void *q, c
     const int status = backward_params(p, max_offset, q, k, v, d_out, d_attn, d_q, d_max_offset, B, H, W, h, hd, rx, ry, dtype,
                                        attn_type, scale, q_row_begin, q_row_end);
     if (status != MATCHATTN_OK) return status;
+    if (((reinterpret_cast<uintptr_t>(d_k) | reinterpret_cast<uintptr_t>(d_v)) & 3u) != 0) return MATCHATTN_ERR_ALIGN;
     p.dk = d_k; p.dv = d_v;
     const dim3 grid(static_cast<unsigned>((1LL * p.Nq * h + 127) / 128), B);
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
@@ -1294,7 +1300,9 @@ extern "C" int matchattn_fused_backward_ws(const void *max_offset, const void *q
     if (status != MATCHATTN_OK) return status;
     const GatherPlan pl = gather_plan(B, H, W, h, hd, rx, dtype, g.b.Nq);
     const auto aligned32 = [](const void *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 31u) == 0; };
-    if (pl.bytes == 0 || workspace_bytes < pl.bytes || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0 || !aligned32(q) ||
+    // (a centre is read as one word of two elements)
+    if (pl.bytes == 0 || workspace_bytes < pl.bytes || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0 ||
+        reinterpret_cast<uintptr_t>(max_offset) % (dtype == MATCHATTN_F32 ? 8 : 4) != 0 || !aligned32(q) ||
         !aligned32(k) || !aligned32(v) || !aligned32(d_out) || !aligned32(d_attn) || !aligned32(d_q) || !aligned32(d_k) || !aligned32(d_v))
         return MATCHATTN_ERR_VARIANT;
     char *ws = static_cast<char *>(workspace);

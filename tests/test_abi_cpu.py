@@ -66,6 +66,30 @@ def test_block_copy_arguments_are_checked_on_the_host():
     assert f(dst, src, sizes, 2, 0, None) == 1
 
 
+def test_backward_alignment_is_checked_on_the_host():
+    """Both backward entry points refuse arrays that their kernels cannot read, before any CUDA call: an element that
+    straddles its size (7), and for the one with a workspace a centre that straddles its pair (9: the other one serves)."""
+    from matchattention_b200 import _lib
+    at = ctypes.c_void_p
+    sizes = (1, 8, 8, 2, 16, 1, 1)
+
+    def ws(dtype, mo=4096, **moved):
+        a = [moved.get(n, 4096) for n in ("q", "k", "v", "d_out", "d_attn", "d_q", "d_k", "d_v", "d_mo")]
+        return _lib.lib.matchattn_fused_backward_ws(at(mo), *map(at, a), *sizes, dtype, 0, 0.25, 0, 8, at(4096), 1 << 30, None)
+
+    def scattered(dtype, mo=4096, **moved):
+        a = [moved.get(n, 4096) for n in ("q", "k", "v", "d_out", "d_attn", "d_q", "d_k", "d_v", "d_mo")]
+        return _lib.lib.matchattn_fused_backward(at(mo), *map(at, a), *sizes, dtype, 0, 0.25, 0, 8, None)
+
+    for dtype, esize in ((_lib.F32, 4), (_lib.F16, 2), (_lib.BF16, 2)):
+        assert ws(dtype, mo=4096 + esize) == 9
+        assert ws(dtype, q=4096 + 16) == 9
+        for call in (ws, scattered):
+            assert call(dtype, mo=4097) == 7 and call(dtype, d_attn=4096 + esize // 2) == 7 and call(dtype, d_mo=4097) == 7
+        assert scattered(dtype, d_k=4098) == 7
+    assert "not aligned" in _lib.strerror(7) and "variant" in _lib.strerror(9)
+
+
 def test_dispatch_table():
     from matchattention_b200 import describe_dispatch
     assert describe_dispatch(8, 16, 1, torch.float16) == "fast cpl=2 lph=1"
