@@ -344,9 +344,9 @@ MATCHATTN_API int matchattn_flow_init(const void *correlation, void *prob, void 
                                       void *scratch, size_t scratch_bytes, int B, int H, int W, int dtype,
                                       void *cuda_stream);
 
-/* Name of the kernel variant the arguments would dispatch to ("fast cpl=2 lph=1",
- * "generic", ...) or NULL if they are rejected.  The split is the coarsest one; a launch may spread a
- * head over more lanes.  Launches nothing. */
+/* Name of the kernel variant that matchattn_fused_forward runs for these sizes ("fast cpl=2 lph=1": chunks of
+ * eight channels per lane, lanes per head; "generic") or NULL if they are rejected.  pointers_32B_aligned: q, k, v
+ * and out are (else 16-byte aligned); attn_out is taken to be aligned as its kernel needs.  Launches nothing. */
 MATCHATTN_API const char *matchattn_describe_dispatch(int h, int hd, int r, int dtype, int pointers_32B_aligned);
 
 /*

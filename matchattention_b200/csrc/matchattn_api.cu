@@ -219,6 +219,18 @@ Plan refine_plan(Plan pl, int hd, int esize, bool rows32)
     return pl;
 }
 
+// The split of a call.  `refine`: no knob asks for another one.
+Plan direct_plan(int h, int hd, int r, int esize, int cpl_request, bool refine, bool rows32)
+{
+    const Plan pl = make_plan(h, hd, r, cpl_request);
+    if (!refine) return pl;
+    const Plan fine = refine_plan(pl, hd, esize, rows32);
+    return fine.lph * h <= kThreads ? fine : pl;
+}
+
+// Alignment the specialised kernels need for q, k, v, out and the gate: the vector width of a lane's slice.
+uintptr_t slice_alignment(const Plan &pl, int esize) { return (pl.cpl * 8 * esize) % 32 == 0 ? 32 : 16; }
+
 // SMs of the current device (148 when the query fails); asked once per device
 inline int sm_count()
 {
@@ -406,18 +418,13 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
         !aligned(out, esize) || !aligned(attn_out, esize))
         return MATCHATTN_ERR_ALIGN;
 
-    Plan pl = force_generic ? Plan{false, 0, 0, false, 2} : make_plan(h, hd, r, cpl_request);
     // (the checked entry runs on the kernel whose slices are contiguous)
     const bool rows32 = glue.debug == nullptr && aligned(q, 32) && aligned(k, 32) && aligned(v, 32) && aligned(out, 32) &&
                         aligned(glue.gate, 32) && C * esize % 32 == 0 && out_stride * esize % 32 == 0;
-    if (cpl_request == 0 && variant == 0 && (strategy == kStrategyAuto || strategy == kStrategyDirect)) {
-        const Plan fine = refine_plan(pl, hd, static_cast<int>(esize), rows32);
-        if (fine.lph * h <= kThreads) pl = fine;
-    }
+    const bool refine = cpl_request == 0 && variant == 0 && (strategy == kStrategyAuto || strategy == kStrategyDirect);
+    Plan pl = force_generic ? Plan{false, 0, 0, false, 2} : direct_plan(h, hd, r, static_cast<int>(esize), cpl_request, refine, rows32);
     if (pl.fast) {
-        // vector width of a lane's slice decides the alignment the specialised kernel needs
-        const int slice_bytes = pl.cpl * 8 * static_cast<int>(esize);
-        const uintptr_t need = (slice_bytes % 32 == 0) ? 32 : 16;
+        const uintptr_t need = slice_alignment(pl, static_cast<int>(esize));
         const uintptr_t need_attn = (M * esize) % 32 == 0 ? 32 : ((M * esize) % 16 == 0 ? 16 : 8);
         if (!aligned(q, need) || !aligned(k, need) || !aligned(v, need) || !aligned(out, need) ||
             !aligned(attn_out, need_attn) || !aligned(glue.gate, need) || (out_stride * esize) % need != 0 ||
@@ -659,11 +666,10 @@ const char *matchattn_describe_dispatch(int h, int hd, int r, int dtype, int poi
     static thread_local char text[64];
     if (dtype != MATCHATTN_F32 && dtype != MATCHATTN_F16 && dtype != MATCHATTN_BF16) return nullptr;
     if (h <= 0 || hd <= 0 || r < 0 || r > MATCHATTN_MAX_R) return nullptr;
-    matchattn::Plan pl = matchattn::make_plan(h, hd, r, 0);
-    if (pl.fast && !pointers_32B_aligned) {
-        const int esize = dtype == MATCHATTN_F32 ? 4 : 2;
-        if ((pl.cpl * 8 * esize) % 32 == 0) pl.fast = false;
-    }
+    const int esize = dtype == MATCHATTN_F32 ? 4 : 2;
+    const bool aligned = pointers_32B_aligned != 0;
+    matchattn::Plan pl = matchattn::direct_plan(h, hd, r, esize, 0, true, aligned && 1LL * h * hd * esize % 32 == 0);
+    if (pl.fast && !aligned && matchattn::slice_alignment(pl, esize) == 32) pl.fast = false;
     if (!pl.fast) return "generic";
     snprintf(text, sizeof(text), "fast cpl=%d lph=%d", pl.cpl, pl.lph);
     return text;

@@ -95,8 +95,14 @@ def test_dispatch_table():
     assert describe_dispatch(8, 16, 1, torch.float16) == "fast cpl=2 lph=1"
     assert describe_dispatch(8, 16, 1, torch.float16, aligned32=False) == "generic"
     assert describe_dispatch(4, 8, 1, torch.float16, aligned32=False) == "fast cpl=1 lph=1"
-    assert describe_dispatch(4, 40, 2, torch.bfloat16) == "fast cpl=5 lph=1"
-    assert describe_dispatch(4, 128, 1, torch.float32) == "fast cpl=4 lph=4"
+    assert describe_dispatch(8, 16, 1, torch.float32) == "fast cpl=1 lph=2"
+    assert describe_dispatch(4, 64, 1, torch.float16) == "fast cpl=2 lph=4"
+    assert describe_dispatch(4, 128, 1, torch.float32) == "fast cpl=2 lph=8"
+    # 40 channels: two lanes (a 32-byte piece each and one of 16 bytes) where every row starts 32-byte aligned
+    assert describe_dispatch(4, 40, 2, torch.bfloat16) == "fast cpl=3 lph=2"
+    assert describe_dispatch(4, 40, 2, torch.bfloat16, aligned32=False) == "fast cpl=5 lph=1"
+    assert describe_dispatch(3, 40, 2, torch.bfloat16) == "fast cpl=5 lph=1"
+    assert describe_dispatch(40, 64, 2, torch.float32) == "fast cpl=2 lph=4"          # 320 lanes of the finer split do not fit a block
     assert describe_dispatch(4, 12, 1, torch.float32) == "generic"
     assert describe_dispatch(4, 16, 3, torch.float32) == "generic"
 
