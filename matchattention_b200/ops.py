@@ -23,18 +23,30 @@ cover; the Python code here then handles the call or words the error.
 """
 from __future__ import annotations
 
+import contextlib
+import os
 from typing import List, Optional, Tuple
 
 import torch
 import torch.nn as nn
 
-import os
-
 from . import _lib
 
-# MATCHATTN_B200_NVTX=1 wraps every operator launch in an NVTX range named after its shape, so that a
-# profiler's NVTX filter can pick the operator out of a model's timeline (off by default: two extra calls)
+# MATCHATTN_B200_NVTX=1 wraps every call of the operator (also the forward of a training step) in an NVTX range named
+# after its shape, so that a profiler's NVTX filter can pick it out of a model's timeline (off by default: two extra calls)
 _NVTX = os.environ.get("MATCHATTN_B200_NVTX", "0") not in ("", "0")
+
+
+@contextlib.contextmanager
+def _nvtx_range(max_offset, q, H, W, r):
+    # (shapes may still be unchecked here)
+    B, h, C = (q.size(0), max_offset.size(2), q.size(2)) if q.dim() == 3 and max_offset.dim() == 4 else (0, 0, 0)
+    torch.cuda.nvtx.range_push(f"matchattn_b200 B{B} {H}x{W} h{h}x{C // max(h, 1)} r{r} {str(q.dtype)[6:]}")
+    try:
+        yield
+    finally:
+        torch.cuda.nvtx.range_pop()
+
 
 _host = _lib.host
 
@@ -136,9 +148,7 @@ def launch(max_offset, q, k, v, output, attn_out, H: int, W: int, win_r, attn_ty
     knobs = tile_w or force_generic or chunks_per_lane or variant
     if knobs and strategy == STRATEGY_BINNED:
         raise ValueError("the direct-kernel knobs cannot be combined with strategy=2")
-    if _NVTX:
-        torch.cuda.nvtx.range_push(f"matchattn_b200 B{B} {H}x{W} h{h}x{hd} r{rx} {str(q.dtype)[6:]}")
-    with torch.cuda.device(q.device):
+    with _nvtx_range(max_offset, q, H, W, rx) if _NVTX else contextlib.nullcontext(), torch.cuda.device(q.device):
         stream = torch.cuda.current_stream().cuda_stream
         args = (max_offset.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), output.data_ptr(),
                 attn_out.data_ptr() if attn_out is not None else None,
@@ -165,8 +175,6 @@ def launch(max_offset, q, k, v, output, attn_out, H: int, W: int, win_r, attn_ty
                     raise ValueError("workspace must be a contiguous uint8 tensor on q's device")
                 ws_ptr, ws_len = workspace.data_ptr(), workspace.numel()
             status = _lib.lib.matchattn_fused_forward_ws(*args, ws_ptr, ws_len, int(strategy))
-    if _NVTX:
-        torch.cuda.nvtx.range_pop()
     _lib.check(status)
 
 
@@ -267,7 +275,8 @@ def match_attention_autograd(max_offset, q, k, v, H: int, W: int, r: int, scale:
     for the reference's 'pytorch' path (its native path has no backward).  CUDA tensors.  Nothing but the inputs is
     saved: the backward kernel recomputes scores and softmaxes.  (The autograd node is in csrc/host_binding.cpp.)"""
     tensors = tuple(t.contiguous() for t in (max_offset, q, k, v))
-    done = _host.autograd(*tensors, H, W, r, scale)
+    with _nvtx_range(tensors[0], tensors[1], H, W, r) if _NVTX else contextlib.nullcontext():
+        done = _host.autograd(*tensors, H, W, r, scale)
     if done is None:
         _check_tensors(*tensors, tensors[1], None, H, W, H, (2 * r + 2) ** 2)
         raise NotImplementedError("match_attention_autograd does not run under functional transforms")

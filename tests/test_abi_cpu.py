@@ -112,3 +112,28 @@ def test_cpu_tensors_are_refused():
     t = torch.zeros(1, 64, 16)
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         match_attention(torch.zeros(1, 64, 2, 2), t, t, t, 8, 8, 1, 1.0)
+
+
+def test_a_training_step_has_its_profiler_range(monkeypatch):
+    """MATCHATTN_B200_NVTX: the autograd entry point opens and closes a range around the native call, also when it raises."""
+    import types
+
+    from matchattention_b200 import ops
+    seen = []
+    mo, t = torch.zeros(1, 64, 2, 2), torch.zeros(1, 64, 16)
+
+    def native(*args):
+        seen.append("call")
+        if len(seen) > 3:
+            raise RuntimeError("refused")
+        return t, t
+
+    monkeypatch.setattr(ops, "_NVTX", True)
+    monkeypatch.setattr(ops, "_host", types.SimpleNamespace(autograd=native))
+    monkeypatch.setattr(torch.cuda.nvtx, "range_push", seen.append)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: seen.append("end"))
+    ops.match_attention_autograd(mo, t, t, t, 8, 8, 1, 0.25)
+    assert seen == ["matchattn_b200 B1 8x8 h2x8 r1 float32", "call", "end"]
+    with pytest.raises(RuntimeError, match="refused"):
+        ops.match_attention_autograd(mo, t, t, t, 8, 8, 1, 0.25)
+    assert seen[-1] == "end"
