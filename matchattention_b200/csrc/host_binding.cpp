@@ -12,9 +12,11 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
@@ -40,12 +42,23 @@ bool untransformed()
     return !c10::impl::tls_local_dispatch_key_set().included_.has_any(modes);
 }
 
-// ... nor any mode that has to see the operators of this call (dispatch modes, tracing).
+// A torch function mode that has to see the calls.  (The one behind torch.set_default_device only places new tensors.)
+bool function_mode()
+{
+    if (!at::impl::torch_function_mode_enabled()) return false;
+    for (int64_t i = 0; i < at::impl::PythonTorchFunctionTLS::stack_len(); ++i) {
+        PyObject *mode = at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter());
+        if (std::strcmp(Py_TYPE(mode)->tp_name, "DeviceContext") != 0) return true;
+    }
+    return false;
+}
+
+// ... nor any mode that has to see the operators of this call (function and dispatch modes, tracing).
 bool eager()
 {
     using c10::DispatchKey;
     static const c10::DispatchKeySet modes({DispatchKey::Python, DispatchKey::PythonDispatcher, DispatchKey::PreDispatch});
-    return untransformed() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+    return untransformed() && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !function_mode() &&
            !c10::impl::tls_local_dispatch_key_set().included_.has_any(modes) && !torch::jit::tracer::isTracing();
 }
 

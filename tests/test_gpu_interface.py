@@ -153,3 +153,31 @@ def test_host_extension_and_python_path_agree(case, around):
     assert_close(attn, case["ref"][1], torch.float16)
     assert_close(own, case["ref"][0], torch.float16)
     assert out.requires_grad == (around == "training")
+
+
+def test_a_torch_function_mode_sees_the_operator(case):
+    """A mode (a tracer, a logger) is shown the custom op, as it is for any other operator; the one behind
+    torch.set_default_device is not in the way."""
+    from torch.overrides import TorchFunctionMode
+
+    from matchattention_b200 import MF_FusedForwardOps
+
+    class Log(TorchFunctionMode):
+        seen = []
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            Log.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    def call():
+        return MF_FusedForwardOps()(*case["gpu"], case["H"], case["W"], [case["r"]] * 2, case["M"], attn_type="l1_norm",
+                                    scale=case["scale"])
+
+    want = call()
+    with Log():
+        got = call()
+    assert any("fused_forward_ops" in name for name in Log.seen), Log.seen
+    with torch.device("cuda"):
+        placed = call()
+    for a, b, c in zip(want, got, placed):
+        assert torch.equal(a, b) and torch.equal(a, c)
