@@ -13,6 +13,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/record_function.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -167,6 +168,9 @@ PyObject *not_covered() { Py_RETURN_NONE; }
 // ---- training: the operator as an autograd function ------------------------------------------------------
 // Only the inputs are saved: the backward recomputes scores and softmaxes.
 
+// the name under which torch.profiler shows the operator: that of the custom op
+constexpr const char *kOpName = "matchattn_b200::fused_forward_ops";
+
 void check_status(int status)
 {
     TORCH_CHECK(status == MATCHATTN_OK, "matchattn_b200: ", matchattn_strerror(status), " (status ", status, ")");
@@ -178,7 +182,8 @@ struct MatchAttentionFn : torch::autograd::Function<MatchAttentionFn> {
     {
         const int64_t B = q.size(0), Nq = q.size(1), C = q.size(2), h = mo.size(2), M = (2 * r + 2) * (2 * r + 2);
         Tensor out = at::empty({B, Nq, C}, q.options()), attn = at::empty({B, Nq, h, M}, q.options());
-        const c10::cuda::CUDAGuard guard(q.device());
+        const c10::cuda::CUDAGuard device(q.device());
+        RECORD_FUNCTION(kOpName, std::vector<c10::IValue>({mo, q, k, v}));
         check_status(matchattn_fused_forward(data(mo), data(q), data(k), data(v), data(out), data(attn), B, H, W, h, C / h, r, r,
                                              dtype_code(q), MATCHATTN_L1_NORM, static_cast<float>(scale), 0, H,
                                              c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
@@ -272,6 +277,7 @@ PyObject *module_forward(PyObject *const *a, Py_ssize_t n)
         return Py_BuildValue("(NN)", THPVariable_Wrap(out[0]), THPVariable_Wrap(out[1]));
     }
     Tensor out = at::empty({o.B, o.Nq, o.C}, o.q.options()), attn = at::empty({o.B, o.Nq, o.h, M}, o.q.options());
+    RECORD_FUNCTION(kOpName, std::vector<c10::IValue>({o.mo, o.q, o.k, o.v}));
     if (!enqueue(o.q, [&](void *stream) {
             return matchattn_fused_forward(data(o.mo), data(o.q), data(o.k), data(o.v), data(out), data(attn), o.B, H, W, o.h, o.C / o.h, rx, ry,
                                            o.dtype, type, static_cast<float>(scale), 0, H, stream);

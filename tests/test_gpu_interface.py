@@ -181,3 +181,15 @@ def test_a_torch_function_mode_sees_the_operator(case):
         placed = call()
     for a, b, c in zip(want, got, placed):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_the_profiler_shows_the_operator(case, train):
+    """torch.profiler lists the operator by the custom op's name, with its inputs, in inference and in training."""
+    from matchattention_b200 import MF_FusedForwardOps
+    inputs = [t.detach().requires_grad_(train) for t in case["gpu"]]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU], record_shapes=True,
+                                acc_events=True) as prof:
+        MF_FusedForwardOps()(*inputs, case["H"], case["W"], [case["r"]] * 2, case["M"], attn_type="l1_norm", scale=case["scale"])
+    events = [e for e in prof.events() if e.name == "matchattn_b200::fused_forward_ops"]
+    assert len(events) == 1 and list(events[0].input_shapes[1]) == list(case["gpu"][1].shape)
