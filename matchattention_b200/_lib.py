@@ -1,5 +1,5 @@
 """ctypes binding of libmatchattn_b200.so (the C ABI in include/matchattn.h), and
-the host extension _host.so that ops.py calls on its eager paths.
+the host extension that ops.py calls on its eager paths.
 
 Both are loaded from matchattention_b200/lib/.  There is no fallback: if one is
 missing, importing this module raises, and so does every op.
@@ -11,9 +11,7 @@ import importlib.machinery
 import importlib.util
 import os
 
-_PKG = os.path.dirname(os.path.abspath(__file__))
-LIB_PATH = os.path.join(_PKG, "lib", "libmatchattn_b200.so")
-HOST_PATH = os.path.join(_PKG, "lib", "_host.so")
+from .build import LIB_PATH, host_path
 
 # every symbol include/matchattn.h declares
 EXPORTS = ("matchattn_fused_forward", "matchattn_fused_forward_ex", "matchattn_fused_forward_ws",
@@ -84,10 +82,12 @@ def _load() -> ctypes.CDLL:
 
 
 def _load_host():
-    if not os.path.exists(HOST_PATH):
-        raise ImportError(f"{HOST_PATH} is missing: build it first with `python -m matchattention_b200.build`")
     import torch  # noqa: F401  (the extension's symbols come from torch's libraries)
-    loader = importlib.machinery.ExtensionFileLoader(__package__ + "._host", HOST_PATH)
+    path = host_path()
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing: the host extension is built for one Python and torch; build it for these "
+                          "with `python -m matchattention_b200.build` (needs nvcc, g++ and the Python headers)")
+    loader = importlib.machinery.ExtensionFileLoader(__package__ + "._host", path)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
     loader.exec_module(module)
     return module

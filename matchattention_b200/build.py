@@ -1,12 +1,14 @@
-"""Builds libmatchattn_b200.so for sm_100a, in-tree, with nvcc alone, and the host extension _host.so on top of it.
+"""Builds libmatchattn_b200.so for sm_100a, in-tree, with nvcc alone, and the host extension on top of it with g++.
 
     python -m matchattention_b200.build [--force]
 
 The translation units (C ABI, one per element type, the built-in scratch area) are compiled in
 parallel and linked into matchattention_b200/lib/libmatchattn_b200.so.  The
 library carries its own static CUDA runtime and has no Python or torch
-dependency; _host.so (csrc/host_binding.cpp, the eager entry points of ops.py)
-is compiled with g++ against the running Python and torch and links to it.
+dependency; the host extension (csrc/host_binding.cpp, the eager entry points of
+ops.py) is compiled against the headers of the running Python and torch and links
+to it.  Its file name carries both versions: another Python or torch needs, and
+finds missing, a build of its own.
 """
 from __future__ import annotations
 
@@ -22,7 +24,6 @@ CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 OBJ_DIR = os.path.join(PKG, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libmatchattn_b200.so")
-HOST_PATH = os.path.join(LIB_DIR, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host_binding.cpp")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
@@ -41,6 +42,12 @@ def _nvcc() -> str:
     return exe
 
 
+def host_path() -> str:
+    """Where the host extension for the running Python and torch lies."""
+    import torch
+    return os.path.join(LIB_DIR, f"_host.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
+
+
 def _stale() -> bool:
     if not os.path.exists(LIB_PATH):
         return True
@@ -57,7 +64,7 @@ def _build_host() -> None:
                os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in include], HOST_SOURCE,
-           "-o", HOST_PATH, f"-L{LIB_DIR}", "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
+           "-o", host_path(), f"-L{LIB_DIR}", "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
            "-L" + os.path.join(root, "lib"), "-lc10", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10_cuda"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
@@ -66,7 +73,8 @@ def _build_host() -> None:
 
 def _host_stale() -> bool:
     deps = (HOST_SOURCE, os.path.join(INCLUDE, "matchattn.h"))
-    return not os.path.exists(HOST_PATH) or any(os.path.getmtime(d) > os.path.getmtime(HOST_PATH) for d in deps)
+    path = host_path()
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
 
 
 def _compile(src: str) -> tuple[str, str]:

@@ -137,3 +137,16 @@ def test_a_training_step_has_its_profiler_range(monkeypatch):
     with pytest.raises(RuntimeError, match="refused"):
         ops.match_attention_autograd(mo, t, t, t, 8, 8, 1, 0.25)
     assert seen[-1] == "end"
+
+
+def test_the_host_extension_belongs_to_one_python_and_torch(monkeypatch):
+    """After an upgrade of torch (or Python) the old extension is neither taken for current by the build nor loaded."""
+    from matchattention_b200 import _lib, build
+    assert _lib.host.__file__ == build.host_path()
+    monkeypatch.setattr(torch, "__version__", "99.0.0")
+    assert build._host_stale()
+    with pytest.raises(ImportError, match="99.0.0.*build it"):
+        _lib._load_host()
+    monkeypatch.undo()
+    monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name: "cpython-399")
+    assert build._host_stale()
