@@ -84,8 +84,8 @@ def test_inference_path_is_untouched_by_autograd_support():
 @pytest.mark.parametrize("h,hd,r", [(3, 12, 1), (2, 8, 3), (2, 24, 2), (8, 16, 1)],
                          ids=["scalar-hd12", "scalar-r3", "vector-hd24-r2", "vector-hd16-r1"])
 def test_backward_kernels_match_the_restatement(h, hd, r):
-    """Both CUDA kernels (one element at a time for any head width and radius; eight channels at a time
-    for head widths that are multiples of 8 and r <= 2) against the float64 plain-loop restatement."""
+    """Autograd against the float64 plain-loop restatement, on either way it takes: gathered sums for head widths that are
+    multiples of 8 and r <= 2 (the ids say "vector"), the accumulating kernel one element at a time otherwise."""
     import matchattention_b200 as ma
     from oracle import matchattn_backward
     B, H, W = 1, 9, 10
@@ -128,3 +128,100 @@ def test_gathered_backward_at_the_edges_of_its_tiles(B, H, W, h, hd, r, kind, pe
     for g, ref, key in zip(got, want, ("d_max_offset", "d_q", "d_k", "d_v")):
         ref = torch.as_tensor(ref).double()         # on one token the score gradients cancel: d_q and d_k are zero up to rounding
         assert (g.double().cpu() - ref).abs().max() < 1e-4 * max(ref.abs().max().item(), 0.05), key
+
+
+def _accumulate(mo, q, k, v, g_out, g_attn, H, W, r, scale, dk, dv):
+    """matchattn_fused_backward through the C ABI: d_max_offset and d_q; dk and dv (float32) are added to."""
+    from matchattention_b200 import _lib
+    B, N, C = q.shape
+    h = mo.size(2)
+    d_q, d_mo = torch.empty_like(q), torch.empty_like(mo)
+    code = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}[q.dtype]
+    _lib.check(_lib.lib.matchattn_fused_backward(
+        mo.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), g_out.data_ptr(), g_attn.data_ptr() if g_attn is not None else None,
+        d_q.data_ptr(), dk.data_ptr(), dv.data_ptr(), d_mo.data_ptr(), B, H, W, h, C // h, r, r, code, _lib.L1_NORM, scale, 0, H,
+        torch.cuda.current_stream().cuda_stream))
+    return d_mo, d_q
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.float16, 2e-3), (torch.bfloat16, 1.6e-2)], ids=["f32", "f16", "bf16"])
+@pytest.mark.parametrize("need_attn_grad", [True, False])
+@pytest.mark.parametrize("h,hd,r", [(3, 12, 1), (2, 8, 3), (2, 24, 2), (8, 16, 1)],
+                         ids=["scalar-hd12", "scalar-r3", "vector-hd24-r2", "vector-hd16-r1"])
+def test_accumulating_backward_kernels_match_the_restatement(h, hd, r, need_attn_grad, dtype, tol):
+    """Both kernels of the accumulating entry point (one element at a time; eight channels at a time), on top of what dk
+    and dv hold.  16-bit types: float32 arithmetic on the rounded inputs, one rounding of d_q and d_max_offset (2^-11,
+    2^-8), four times that."""
+    from oracle import matchattn_backward
+    B, H, W = 2, 9, 10
+    mo, q, k, v = make_inputs(57, B, H, W, h, hd, r, dtype, kind="flow", spread=3.0, border_frac=0.2, per_head=True)
+    gen = torch.Generator().manual_seed(58)
+    g_out = torch.randn(q.shape, generator=gen).to(dtype)
+    g_attn = torch.randn(B, H * W, h, (2 * r + 2) ** 2, generator=gen).to(dtype)
+    want = matchattn_backward.backward(*(t.float() for t in (mo, q, k, v, g_out)), (g_attn if need_attn_grad else g_attn * 0).float(),
+                                       H, W, r, hd ** -0.5)
+    dk, dv = torch.full(k.shape, 0.5, device="cuda"), torch.full(v.shape, -2.0, device="cuda")
+    d_mo, d_q = _accumulate(*(t.cuda() for t in (mo, q, k, v, g_out)), g_attn.cuda() if need_attn_grad else None, H, W, r, hd ** -0.5, dk, dv)
+    for got, ref, key in zip((d_mo, d_q, dk - 0.5, dv + 2.0), want, ("d_max_offset", "d_q", "d_k", "d_v")):
+        assert _rel(got, ref) < tol, key
+
+
+def _step(inputs, g_out, g_attn, H, W, r, scale):
+    import matchattention_b200 as ma
+    out, attn = ma.match_attention_autograd(*inputs, H, W, r, scale)
+    return lambda: torch.autograd.grad([out, attn], inputs, [g_out, g_attn])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float16, 2e-3)], ids=["f32", "f16"])
+@pytest.mark.parametrize("offset", [16, 4])
+def test_training_on_arrays_that_are_not_32_byte_aligned(offset, dtype, tol):
+    """Views some bytes into a buffer: the backward with a workspace declines and the accumulating one serves, with the
+    gradients of the aligned arrays (float32 sums in another order; 16 bits: one rounding apart)."""
+    B, H, W, h, hd, r = 1, 20, 33, 4, 16, 1
+    inputs = [t.cuda() for t in make_inputs(63, B, H, W, h, hd, r, dtype, kind="flow", spread=3.0, per_head=True)]
+    gen = torch.Generator(device="cuda").manual_seed(64)
+    g_out = torch.randn(inputs[1].shape, generator=gen, device="cuda").to(dtype)
+    g_attn = torch.randn(B, H * W, h, 16, generator=gen, device="cuda").to(dtype)
+
+    def moved(t):
+        skip = offset // t.element_size()
+        return torch.empty(t.numel() + skip, dtype=dtype, device="cuda")[skip:].view(t.shape).copy_(t)
+
+    want = _step([t.requires_grad_(True) for t in inputs], g_out, g_attn, H, W, r, hd ** -0.5)()
+    views = [inputs[0].detach().requires_grad_(True)] + [moved(t.detach()).requires_grad_(True) for t in inputs[1:]]
+    assert views[1].data_ptr() % 32 == offset % 32
+    got = _step(views, g_out, g_attn, H, W, r, hd ** -0.5)()
+    for g, w, key in zip(got, want, ("d_max_offset", "d_q", "d_k", "d_v")):
+        assert _rel(g, w) < tol, key
+
+
+@pytest.mark.gpu
+def test_training_without_room_for_the_workspace():
+    """When the workspace (44 MB here) finds no room the accumulating call serves: the same gradients, no workspace.  The limit
+    is the caching allocator's own, far below what the device holds."""
+    from matchattention_b200 import _lib
+    B, H, W, h, hd, r = 1, 192, 192, 4, 8, 2
+    inputs = [t.cuda().requires_grad_(True) for t in make_inputs(65, B, H, W, h, hd, r, torch.float32, kind="self")]
+    gen = torch.Generator(device="cuda").manual_seed(66)
+    g_out = torch.randn(inputs[1].shape, generator=gen, device="cuda")
+    g_attn = torch.randn(B, H * W, h, 36, generator=gen, device="cuda")
+    want = _step(inputs, g_out, g_attn, H, W, r, 0.25)()
+    nbytes = _lib.lib.matchattn_backward_workspace_bytes(B, H, W, h, hd, r, _lib.F32, 0, H)
+    assert nbytes > 40 << 20
+    backward = _step(inputs, g_out, g_attn, H, W, r, 0.25)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    try:        # room for the gradients (16 MB, in one 20 MB segment), not for the workspace
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) /
+                                                   torch.cuda.get_device_properties(0).total_memory)
+        got = backward()
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.cuda.max_memory_allocated() - held < nbytes
+    for g, w, key in zip(got, want, ("d_max_offset", "d_q", "d_k", "d_v")):
+        assert _rel(g, w) < 1e-5, key
