@@ -880,9 +880,10 @@ def run_volume_mode(args):
 
 def run_backward_mode(args):
     """Training step of the operator alone: forward + backward through autograd on one batch item of the
-    chosen workload (gradients of both outputs given), the backward kernel by itself, and, where the
-    reference's code is present, autograd over the reference's 'pytorch' path on the same GPU (its native
-    path has no backward).  One JSON line; the value is the forward + backward time."""
+    chosen workload (gradients of both outputs given), the backward by itself (the six kernels that autograd runs, and
+    the accumulating kernel that it falls back to), and, where the reference's code is present, autograd over the
+    reference's 'pytorch' path on the same GPU (its native path has no backward).  One JSON line; the value is the
+    forward + backward time."""
     import matchattention_b200 as ma
     from matchattention_b200 import _lib
     from matchattention_b200.ops import _DTYPE_CODE
@@ -895,15 +896,21 @@ def run_backward_mode(args):
     g = torch.Generator(device=dev).manual_seed(5)
     g_out = torch.randn(q.shape, generator=g, device=dev).to(q.dtype)
     g_attn = torch.randn(B, H * W, h, (2 * r + 2) ** 2, generator=g, device=dev).to(q.dtype)
-    d_q, d_mo = torch.empty_like(q), torch.empty_like(mo)
-    d_k, d_v = (torch.zeros(k.shape, dtype=torch.float32, device=dev) for _ in range(2))
+    d_q, d_mo, d_k, d_v = (torch.empty_like(t) for t in (q, mo, k, v))
+    sum_k, sum_v = (torch.zeros(k.shape, dtype=torch.float32, device=dev) for _ in range(2))
+    code = _DTYPE_CODE[q.dtype]
+    ws = torch.empty(_lib.lib.matchattn_backward_workspace_bytes(B, H, W, h, hd, r, code, 0, H), dtype=torch.uint8, device=dev)
     stream = torch.cuda.current_stream().cuda_stream
+    inputs = [t.data_ptr() for t in (mo, q, k, v, g_out, g_attn)]
+    sizes = (B, H, W, h, hd, r, r, code, _lib.L1_NORM, float(scale), 0, H)
 
-    def kernel_only():
-        _lib.check(_lib.lib.matchattn_fused_backward(
-            mo.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), g_out.data_ptr(), g_attn.data_ptr(), d_q.data_ptr(),
-            d_k.data_ptr(), d_v.data_ptr(), d_mo.data_ptr(), B, H, W, h, hd, r, r, _DTYPE_CODE[q.dtype], _lib.L1_NORM,
-            float(scale), 0, H, stream))
+    def gathered_only():          # what autograd runs; it keeps no workspace, this timing does
+        _lib.check(_lib.lib.matchattn_fused_backward_ws(*inputs, d_q.data_ptr(), d_k.data_ptr(), d_v.data_ptr(), d_mo.data_ptr(),
+                                                        *sizes, ws.data_ptr(), ws.numel(), stream))
+
+    def accumulating_only():      # what it falls back to
+        _lib.check(_lib.lib.matchattn_fused_backward(*inputs, d_q.data_ptr(), sum_k.data_ptr(), sum_v.data_ptr(), d_mo.data_ptr(),
+                                                     *sizes, stream))
 
     def autograd_step(op):
         def step():
@@ -926,7 +933,8 @@ def run_backward_mode(args):
 
     n = max(10, min(args.steps, 50))
     ours = timed(autograd_step(lambda a, b, c, d: ma.match_attention_autograd(a, b, c, d, H, W, r, scale)), n)
-    kern = timed(kernel_only, n)
+    kern = timed(gathered_only, n) if ws.numel() else None          # head widths and radii without it accumulate
+    accumulating = timed(accumulating_only, n)
     fwd = timed(lambda: ma.match_attention(mo, q, k, v, H, W, r, scale), n)
     ref = None
     if ref_loader.available():
@@ -935,9 +943,9 @@ def run_backward_mode(args):
     print(json.dumps({"metric": "matchattention_forward_backward_ms", "value": ours, "unit": "ms", "n_gpus": 1, "steps": n,
                       "higher_is_better": False, "dtype": str(q.dtype)[6:], "data": "synthetic",
                       "config": {"workload": args.workload + " (one batch item)", "queries": H * W},
-                      "backward_kernel_ms": kern, "forward_kernel_ms": fwd,
+                      "backward_kernel_ms": kern, "backward_accumulating_kernel_ms": accumulating, "forward_kernel_ms": fwd,
                       "reference_pytorch_autograd_ms": ref,
-                      "gpu_launches": 2 * n + n + n}), flush=True)
+                      "gpu_launches": (n * (1 + 6) + n * 6 if ws.numel() else 2 * n) + n + n}), flush=True)
 
 
 SHAPE_WORKLOADS = ("op_384x384_b4_h8x16_r1_f32_flow", "op_384x384_b4_h8x16_r1_bf16_flow",
