@@ -46,6 +46,18 @@ constexpr int kPoolSmemPerWarp = kWarpCols * (kTransBytes + 16);
 constexpr int kPoolWarps = 4;                         // warps per block of the pooling kernel
 constexpr int kSumGroups = 4;                         // interleaved partial sums per column
 constexpr int kWindowTokens = kFlowWarps;             // tokens per block of the window kernel: one per warp
+// Rows per warp of the maximum and the pooling kernel: long columns amortise the start of a warp (the halo rows, the
+// merges of the partials), from so many tokens on; below there are not enough warps to fill the chip with long ones, and
+// the single-element accesses of odd token counts want more of them.  Measured, float16, long against short: 64x64 tokens
+// 117.4 / 113.1 us, 68x72 145.9 / 148.3, 76x76 181.9 / 189.5, 128x128 1142 / 1231; odd: 67x71 208 / 186, 79x83 352 / 331,
+// 97x101 692 / 691; float32: 60x60 105.3 / 103.9, 68x72 167.9 / 173.0, 79x83 356 / 333.
+constexpr int64_t kLongBands = 5000, kLongBandsOdd = 10000;
+// Column sums: 32-column blocks with 16 (float32: 24) rows in flight from so many tokens on, 16-column blocks with 32 below,
+// where the wider ones leave SMs without work.  Measured, the whole call, wide against narrow, long bands: float16 72x72
+// tokens 168.1 / 156.6 us, 96x96 418.2 / 407.9, 96x100 433.3 / 445.5, 128x128 1069 / 1142; float32 72x72 192.7 / 185.8,
+// 76x80 239.9 / 246.2, 88x88 352.9 / 375.3.
+template <typename T>
+constexpr int64_t kWideSums = sizeof(T) == 2 ? 9400 : 6000;
 
 // Sizes and scratch areas of one call, computed alike by the size query and the launcher.
 struct FlowPlan {
@@ -63,10 +75,9 @@ FlowPlan flow_plan(int B, int H, int W)
     FlowPlan pl{};
     pl.N = static_cast<int64_t>(H) * W;
     const auto parts = [&](int64_t of) { return static_cast<int>((pl.N + of - 1) / of); };
-    // Rows per warp: long columns amortise the start of a warp (the halo rows, the merges of the partials); below
-    // about 5000 tokens there are not enough warps to fill the chip with long ones.
-    pl.max_rows = pl.N >= 5000 ? 128 : 32;
-    pl.band = pl.N >= 5000 ? 64 : 32;
+    const bool long_bands = pl.N >= (pl.N % 2 == 0 ? kLongBands : kLongBandsOdd);
+    pl.max_rows = long_bands ? 128 : 32;
+    pl.band = long_bands ? 64 : 32;
     pl.row_parts = parts(kWarpCols);
     pl.col_parts = parts(pl.max_rows);
     pl.chunks = parts(kPoolCols);
@@ -763,10 +774,7 @@ cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow
             <<<dim3(static_cast<unsigned>(col_blocks + (N + kRows - 1) / kRows), B), kThreadsHere, 0, stream>>>(
                 corr, row_part, col_part, stats, N, pl.row_parts, pl.col_parts, col_blocks);
     };
-    // Narrow blocks up to about 5000 tokens, where 32-column ones would leave SMs without work.  Above, 32 columns and 16
-    // (float32: 24) rows in flight measured best: 128x128 tokens float16 262 us, 337 with 64-column blocks, of which some
-    // SMs get two and some one; 88x88 float32 80 us, 102.
-    if (N >= 5000) launch_sums(std::integral_constant<int, 32>(), std::integral_constant<int, sizeof(T) == 2 ? 16 : 24>());
+    if (N >= kWideSums<T>) launch_sums(std::integral_constant<int, 32>(), std::integral_constant<int, sizeof(T) == 2 ? 16 : 24>());
     else launch_sums(std::integral_constant<int, 16>(), std::integral_constant<int, 32>());
     constexpr int smem = kPoolWarps * kPoolSmemPerWarp;
     const cudaError_t e = cudaFuncSetAttribute(flow_prob_pool_kernel<T, ALIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

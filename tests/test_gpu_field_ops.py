@@ -200,3 +200,22 @@ def test_local_disparity_of_an_infinite_value(dtype):
     flow, blur, centre = _ma().local_disparity_estimator(vol.cuda(), return_debug=True)
     assert (blur[:, 1, 2] == float("inf")).all() and (centre[:, 1, 2] == 15).all() and flow[:, 1, 2, 0].isnan().all()
     assert torch.isfinite(flow).sum() == flow.numel() - 2
+
+
+@pytest.mark.parametrize("H,W,dtype", [(71, 73, torch.float16), (84, 72, torch.float32), (98, 96, torch.float16), (97, 97, torch.bfloat16)])
+def test_flow_init_kernels_beyond_their_thresholds(H, W, dtype):
+    """Short bands of an odd token count, and the wide column sums of either type's large maps."""
+    import oracle
+    g = torch.Generator().manual_seed(H * W)
+    second = torch.randn(1, H * W, 16, generator=g)
+    first = second.roll(3, 1) + 0.3 * torch.randn(1, H * W, 16, generator=g)
+    corr = (torch.matmul(first, second.transpose(1, 2)) / 2.0).to(dtype)
+    want_flow, want_prob, want_blur, want_centre = oracle.flow_init(corr, H, W)
+    flow, prob, blur, centre = _ma().flow_init(corr.cuda(), H, W, return_debug=True)
+    steps = ((prob.float().cpu() - want_prob.float()).abs() - 2.0 ** -24).clamp_min(0)     # float16: below 2^-14 the spacing is 2^-24
+    assert _close16(want_prob.float() + steps, want_prob, dtype)
+    # 16 bits: an average of probabilities that are one step off, a relative 2^-10 (2^-7) at most, is less than two of its own
+    # steps off, and rounding adds less than one
+    assert _close16(blur, want_blur, dtype, ulps=3.0)
+    same = centre.cpu() == want_centre
+    assert same.float().mean() > 0.98           # the rest: equal box averages
