@@ -198,9 +198,10 @@ Plan make_plan(int h, int hd, int r, int cpl_request)
 
 // The split that the direct kernel uses: 32 bytes per lane and tap, so that the lanes of a query read whole lines, and up to
 // eight lanes per head, which share the softmax (matchattn_lanes.cuh).  Measured best for every power-of-two width and
-// both radii; 16-bit heads of 16 channels and narrower stay with one lane.  `rows32`: every row of the arrays starts
-// 32-byte aligned; then 16-bit heads of 40 channels go to two lanes (one lane's 80-byte slice takes five loads that
-// touch a line per lane each).
+// both radii; 16-bit heads of 16 channels and narrower stay with one lane (two lanes of 16 bytes each, 8 heads x 16, r = 1:
+// float16 4 x 384x384 tokens 411 us against 290, 104x208 16.4 against 13.5; bfloat16 459 against 332).  `rows32`: every row
+// of the arrays starts 32-byte aligned; then 16-bit heads of 40 channels go to two lanes (one lane's 80-byte slice takes
+// five loads that touch a line per lane each).
 Plan refine_plan(Plan pl, int hd, int esize, bool rows32)
 {
     const int hd8 = hd / 8;
