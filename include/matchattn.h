@@ -182,8 +182,8 @@ MATCHATTN_API int matchattn_fused_backward(const void *max_offset, const void *q
 /*
  * The same gradients with scratch memory from the caller and d_k, d_v in the tensor type, WRITTEN rather than
  * accumulated: the (query, head) items are bucketed by the token their window starts at, and every token sums the
- * contributions of the buckets around it (no floating-point atomics).  About three times as fast as the call above
- * plus the clearing and conversion around it.  Covered: head widths that are multiples of 8, r = 1 or 2, 32-byte
+ * contributions of the buckets around it (no floating-point atomics).  About twice as fast as the call above plus
+ * the clearing and conversion around it (384x384 tokens, 8 heads x 16, float16: 396 against 785 us).  Covered: head widths that are multiples of 8, r = 1 or 2, 32-byte
  * aligned arrays (max_offset: aligned to its pair); MATCHATTN_ERR_VARIANT otherwise.
  *   workspace  at least matchattn_backward_workspace_bytes(...) bytes of device memory, 256-byte aligned; contents
  *              need not be preserved between calls, but calls that overlap on the device must not share it

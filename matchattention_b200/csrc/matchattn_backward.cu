@@ -603,7 +603,8 @@ struct QueryGradient {           // dq -= ds * sign(q - k)
 // With e_m the exponentials around the largest score, den_t and v_t the sums of e_m and e_m da_m over sub-window t and
 // c_t = w_t / den_t:   a_m = e_m C_m,  ds_m = e_m (da_m C_m - U_m),  C_m = sum of c_t, U_m = sum of c_t v_t / den_t
 // over the sub-windows t that hold m, so one exponential per tap serves all four.
-// Bound by the L1 path and the bytes in flight: the window of V once, of K twice, 128 bytes of coefficients out.
+// Bound by the latency of the taps at four blocks of 128 threads per SM (issue 59 %, L1 49 %; with a centre per head the
+// slots' stores bring L1 to 79 %): the window of V once, of K twice, 128 bytes of coefficients out.
 // Measured, float16, 384x384 tokens, 8 heads x 16, r = 1: 163 us (207 us with per-head slots, whose stores touch a line
 // per lane), at 128 registers; the rows of the second walk over K as a loop, or the compiler moves all its loads up and
 // spills (266 us).
@@ -913,8 +914,8 @@ __device__ __forceinline__ void copy16_async(void *smem, const void *global)
 // dk and dv of a tile of tokens, one head, one slice of its channels: a thread per (token, eight channels).  The items
 // of all buckets that the tile needs are staged in shared memory, `batch` at a time: coefficients, q and dout.
 // A slot of coefficients is padded by 16 bytes: neighbouring tokens read the same tap of neighbouring slots.
-// Bound by instruction issue (about 57 per token, item and eight channels; two thirds of the lanes busy, lists differ in
-// length).  Measured, same sizes as above: 276 us; walking a token's four ranges as one list costs as much as it saves.
+// Bound by instruction issue (69 % of the slots; about 57 per token, item and eight channels; two thirds of the lanes busy,
+// lists differ in length).  Measured, same sizes as above: 276 us; walking a token's four ranges as one list costs as much as it saves.
 template <typename T, int R>
 __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
 {
@@ -1011,6 +1012,7 @@ __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
 // The same with shared centres: `lanes` lanes per token, each with CPT chunks of eight channels (chunk = lane + s * lanes),
 // `per_warp` tokens per warp.  A query's row of q and dout is read as a whole, a tap's coefficients of all heads lie
 // side by side, and the lanes of a token walk the same list.  The rows are shared by the tokens of a block through L1.
+// Bound by the latency of those loads at 75 registers, three blocks per SM (issue 59 %).
 // Measured, same sizes: 208 us (300 us range by range: too few loads under way, and the border rows started last).
 template <typename T, int R, int CPT>
 __global__ void __launch_bounds__(256) gather_sum_shared_kernel(const GatherParams g)

@@ -20,7 +20,7 @@
 // adds in another.
 // Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.06 ms = 0.09 + 0.26 +
 // 0.63 + 0.08; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
-// the pooling took 4.1.  48x48 tokens: 56 us, before 189.
+// the pooling took 4.1.  48x48 tokens: 51 us, before 189 (as a CUDA graph).
 // Rounding of the 16-bit types as eager PyTorch on the GPU: softmax, pooling and sums accumulate in float32
 // and round once, every elementwise op rounds.
 #include "../../include/matchattn.h"
@@ -348,8 +348,9 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T 
     if (lane == 0) stats[b * N + row] = make_float2(mx, total);
 }
 
-// Softmax of an element: the quotient exp(x - max) / sum, to the last bit, by one Newton step on the product with the
-// rounded reciprocal (Markstein, IBM J. Res. Dev. 34, 1990).
+// Softmax of an element: the quotient exp(x - max) / sum by one Newton step on the product with the rounded reciprocal
+// (Markstein, IBM J. Res. Dev. 34, 1990): to the last bit as long as the residual does not underflow, which it does for
+// float32 quotients below 2^-102; there the last bit may differ.
 struct Softmax {
     float max, sum, inv;
     __device__ __forceinline__ float operator()(float x) const
@@ -610,7 +611,7 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
 // the softmax runs over (pool_rows, pool_cols); a lane of the second gathers eight rows of its columns and stores
 // them as 16 bytes of a prob row, or, where rows of prob are not 16-byte aligned, through shared memory.
 // Eight consecutive blocks (four of either role) cover one 4-band x 4-chunk region, so the second role finds corr in L2.
-// Bound by instruction issue (about 25 per element and role, a third of them the exponential; 60 % of the slots busy).
+// Bound by instruction issue (about 25 per element and role, a third of them the exponential; 81 % of the slots busy).
 // Measured, float16, 16384 x 16384: 0.63 ms (0.72 with eight rows unrolled and the halo rows apart: the instruction cache
 // ran short, 2.2 of 8 stalls).  With 16-byte stores straight from the registers to 32 rows of prob the
 // second role alone took 0.67 ms; five blocks of four warps hold 20 warps per SM (0.75 ms with four blocks).

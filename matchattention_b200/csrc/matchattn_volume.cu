@@ -14,7 +14,7 @@
 // exponentials are taken in place: maxima by a warp per column, exponentials by all threads over the triangle in
 // view, sums by a thread per column (in the order of d), then the W rows of W outputs, coalesced along w.
 // HBM traffic: corr once per view, vol once.  Latency-bound (136 blocks at 68 x 120): everything but the W additions
-// of a column's sum is spread over the whole block.  Measured, float16, 68 x 120: 9.0 us; one thread per column for
+// of a column's sum is spread over the whole block.  Measured, float16, 68 x 120: 8.8 us; one thread per column for
 // all three steps took 29.5 us.
 #include "../../include/matchattn.h"
 
