@@ -202,8 +202,8 @@ struct MatchAttentionFn : torch::autograd::Function<MatchAttentionFn> {
         const Tensor &mo = saved[0], &q = saved[1], &k = saved[2], &v = saved[3];
         const int64_t H = ctx->saved_data["H"].toInt(), W = ctx->saved_data["W"].toInt(), r = ctx->saved_data["r"].toInt();
         const int64_t B = q.size(0), C = q.size(2), h = mo.size(2);
-        Tensor d_out = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(q);
-        Tensor d_attn = grads[1].defined() ? grads[1].contiguous() : Tensor();
+        Tensor d_out = grads[0].defined() ? grads[0].contiguous().resolve_neg() : at::zeros_like(q);
+        Tensor d_attn = grads[1].defined() ? grads[1].contiguous().resolve_neg() : Tensor();
         Tensor d_q = at::empty_like(q), d_mo = ctx->needs_input_grad(0) ? at::empty_like(mo) : Tensor();
         const float scale = static_cast<float>(ctx->saved_data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(q.device());

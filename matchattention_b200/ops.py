@@ -140,6 +140,7 @@ def launch(max_offset, q, k, v, output, attn_out, H: int, W: int, win_r, attn_ty
     if strategy == STRATEGY_AUTO and workspace is None and not (tile_w or force_generic or chunks_per_lane or variant or _NVTX) \
             and _host.launch(max_offset, q, k, v, output, attn_out, H, W, win_r, attn_type, scale, q_row_begin, q_row_end):
         return
+    max_offset, q, k, v = (t.resolve_neg() for t in (max_offset, q, k, v))
     rx, ry = _window_radius(win_r)
     if attn_type not in _lib.ATTN_TYPE_CODE:
         raise NotImplementedError(f"attn_type {attn_type!r}: 'l1_norm' and 'dot_product' exist")
@@ -274,7 +275,7 @@ def match_attention_autograd(max_offset, q, k, v, H: int, W: int, r: int, scale:
     """The operator for training: (out, attn) with gradients to q, k, v and max_offset, as autograd gives them
     for the reference's 'pytorch' path (its native path has no backward).  CUDA tensors.  Nothing but the inputs is
     saved: the backward kernel recomputes scores and softmaxes.  (The autograd node is in csrc/host_binding.cpp.)"""
-    tensors = tuple(t.contiguous() for t in (max_offset, q, k, v))
+    tensors = tuple(t.contiguous().resolve_neg() for t in (max_offset, q, k, v))
     with _nvtx_range(tensors[0], tensors[1], H, W, r) if _NVTX else contextlib.nullcontext():
         done = _host.autograd(*tensors, H, W, r, scale)
     if done is None:
@@ -288,6 +289,7 @@ def match_attention_autograd(max_offset, q, k, v, H: int, W: int, r: int, scale:
 def launch_glue(max_offset, q, k, v, gate, out_base, attn_base, H: int, W: int, r: int, scale: float, *,
                 clamp: bool, out_stride: int = 0, attn_stride: int = 0, kv_shift: int = 0) -> None:
     """Enqueue the direct kernel with clamp / gate / strided outputs (see matchattn_fused_forward_glue)."""
+    max_offset, q, k, v, gate = (t if t is None else t.resolve_neg() for t in (max_offset, q, k, v, gate))
     B, Nq, C = q.shape
     h = max_offset.size(2)
     M = (2 * r + 2) ** 2
@@ -358,7 +360,7 @@ def upsample_field(field: torch.Tensor, mask: torch.Tensor, factor: int) -> torc
     B, H, W, D = field.shape
     if tuple(mask.shape) != (B, 9 * factor * factor, H, W):
         raise ValueError(f"mask has shape {tuple(mask.shape)}, expected {(B, 9 * factor * factor, H, W)}")
-    field, mask = field.contiguous(), mask.contiguous()
+    field, mask = field.contiguous().resolve_neg(), mask.contiguous().resolve_neg()
     out = field.new_empty(B, H * factor, W * factor, D)
     with torch.cuda.device(field.device):
         status = _lib.lib.matchattn_upsample_field(field.data_ptr(), mask.data_ptr(), out.data_ptr(), B, H, W, D,
@@ -385,7 +387,7 @@ def stereo_volume(correlation: torch.Tensor) -> torch.Tensor:
         raise TypeError(f"unsupported dtype {correlation.dtype}")
     if correlation.dim() != 4 or correlation.size(2) != correlation.size(3):
         raise ValueError("expected correlation [B,H,W,W]")
-    corr = correlation.contiguous()
+    corr = correlation.contiguous().resolve_neg()
     B, H, W, _ = corr.shape
     vol = corr.new_empty(2 * B, W, H, W)
     with torch.cuda.device(corr.device):
@@ -409,7 +411,7 @@ def consistency_mask(field: torch.Tensor, threshold: float = 2.0, return_diff: b
         raise TypeError(f"unsupported dtype {field.dtype}")
     if field.dim() != 4 or field.size(-1) != 2 or field.size(0) % 2:
         raise ValueError("expected field [B,H,W,2] with an even batch (two views)")
-    field = field.contiguous()
+    field = field.contiguous().resolve_neg()
     B, H, W, _ = field.shape
     mask = field.new_empty(B, H, W, 1)
     diff = field.new_empty(B, H, W, 1) if return_diff else None
@@ -436,7 +438,7 @@ def local_disparity_estimator(volume: torch.Tensor, return_debug: bool = False):
         raise TypeError(f"unsupported dtype {volume.dtype}")
     if volume.dim() != 4 or volume.size(0) % 2 or volume.size(1) < 5:
         raise ValueError("expected volume [B,D,H,W] with an even batch (two views) and D >= 5")
-    vol = volume.contiguous()
+    vol = volume.contiguous().resolve_neg()
     B, D, H, W = vol.shape
     flow = vol.new_empty(B, H, W, 2)
     blur = vol.new_empty(B, H, W) if return_debug else None
@@ -465,7 +467,7 @@ def flow_init(correlation: torch.Tensor, H: int, W: int, return_debug: bool = Fa
         raise TypeError(f"unsupported dtype {correlation.dtype}")
     if correlation.dim() != 3 or correlation.size(1) != H * W or correlation.size(2) != H * W:
         raise ValueError("expected correlation [B, H*W, H*W]")
-    corr = correlation.contiguous()
+    corr = correlation.contiguous().resolve_neg()
     B, N, _ = corr.shape
     prob = corr.new_empty(2 * B, H, W, N)
     flow = corr.new_empty(2 * B, H, W, 2)

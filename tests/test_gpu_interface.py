@@ -193,3 +193,32 @@ def test_the_profiler_shows_the_operator(case, train):
         MF_FusedForwardOps()(*inputs, case["H"], case["W"], [case["r"]] * 2, case["M"], attn_type="l1_norm", scale=case["scale"])
     events = [e for e in prof.events() if e.name == "matchattn_b200::fused_forward_ops"]
     assert len(events) == 1 and list(events[0].input_shapes[1]) == list(case["gpu"][1].shape)
+
+
+def test_a_tensor_with_the_negative_bit_stands_for_its_values(case):
+    """A lazily negated view (torch keeps a bit instead of new values) gives what the values give, through every entry
+    point that takes tensors."""
+    import matchattention_b200 as ma
+    mo, q, k, v = case["gpu"]
+    H, W, r, scale = case["H"], case["W"], case["r"], case["scale"]
+    g = torch.Generator(device="cuda").manual_seed(5)
+
+    def normal(*shape):
+        return torch.randn(*shape, generator=g, device="cuda")
+
+    field, mask, corr, flow = normal(2, 4, 6, 2), normal(2, 36, 4, 6), normal(1, 3, 24, 24), normal(1, 48, 48)
+    volume = normal(2, 24, 3, 5).abs()
+    for call in (lambda s: ma.match_attention_autograd(mo, s(q), k, v, H, W, r, scale),
+                 lambda s: ma.match_attention(mo, q, s(k), v, H, W, r, scale),
+                 lambda s: ma.cross_attention_core(mo, q, k, v, s(q), H, W, r, scale),
+                 lambda s: ma.self_attention_core(mo, q, k, s(v), H, W, r, scale),
+                 lambda s: ma.upsample_field(s(field), s(mask), 2), lambda s: ma.stereo_volume(s(corr)),
+                 lambda s: ma.consistency_mask(s(field)), lambda s: ma.local_disparity_estimator(s(volume)),
+                 lambda s: ma.flow_init(s(flow), 6, 8)):
+        want, got = call(lambda t: -t), call(torch._neg_view)
+        for a, b in zip(*((x if isinstance(x, tuple) else (x,)) for x in (want, got))):
+            assert torch.equal(a, b)
+    leaf = q.detach().requires_grad_(True)
+    out, _ = ma.match_attention_autograd(mo, leaf, k, v, H, W, r, scale)
+    want, got = (torch.autograd.grad(out, leaf, f(q), retain_graph=True)[0] for f in (torch.neg, torch._neg_view))
+    assert torch.equal(want, got)
