@@ -23,6 +23,7 @@ EXPORTS = ("matchattn_fused_forward", "matchattn_fused_forward_ex", "matchattn_f
            "matchattn_workspace_bytes", "matchattn_describe_dispatch", "matchattn_version", "matchattn_strerror")
 
 F32, F16, BF16 = 0, 1, 2
+ERR_WINDOW = 6
 L1_NORM = 0
 DOT_PRODUCT = 1
 ATTN_TYPE_CODE = {"l1_norm": L1_NORM, "dot_product": DOT_PRODUCT}

@@ -276,6 +276,7 @@ PyObject *module_forward(PyObject *const *a, Py_ssize_t n)
         }
         return Py_BuildValue("(NN)", THPVariable_Wrap(out[0]), THPVariable_Wrap(out[1]));
     }
+    if (PyLong_Check(a[6])) return not_covered();      // the custom op wants a list
     Tensor out = at::empty({o.B, o.Nq, o.C}, o.q.options()), attn = at::empty({o.B, o.Nq, o.h, M}, o.q.options());
     RECORD_FUNCTION(kOpName, std::vector<c10::IValue>({o.mo, o.q, o.k, o.v}));
     if (!enqueue(o.q, [&](void *stream) {

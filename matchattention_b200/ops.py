@@ -275,11 +275,14 @@ def match_attention_autograd(max_offset, q, k, v, H: int, W: int, r: int, scale:
     """The operator for training: (out, attn) with gradients to q, k, v and max_offset, as autograd gives them
     for the reference's 'pytorch' path (its native path has no backward).  CUDA tensors.  Nothing but the inputs is
     saved: the backward kernel recomputes scores and softmaxes.  (The autograd node is in csrc/host_binding.cpp.)"""
+    scale = float(scale)
     tensors = tuple(t.contiguous().resolve_neg() for t in (max_offset, q, k, v))
     with _nvtx_range(tensors[0], tensors[1], H, W, r) if _NVTX else contextlib.nullcontext():
         done = _host.autograd(*tensors, H, W, r, scale)
     if done is None:
         _check_tensors(*tensors, tensors[1], None, H, W, H, (2 * r + 2) ** 2)
+        if r < 0:
+            _lib.check(_lib.ERR_WINDOW)
         raise NotImplementedError("match_attention_autograd does not run under functional transforms")
     return done
 

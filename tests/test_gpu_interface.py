@@ -222,3 +222,30 @@ def test_a_tensor_with_the_negative_bit_stands_for_its_values(case):
     out, _ = ma.match_attention_autograd(mo, leaf, k, v, H, W, r, scale)
     want, got = (torch.autograd.grad(out, leaf, f(q), retain_graph=True)[0] for f in (torch.neg, torch._neg_view))
     assert torch.equal(want, got)
+
+
+def test_wrong_arguments_raise_alike_on_every_path(case):
+    """What a refused argument raises is the same with and without the native entry (in inference the custom op words it)."""
+    from torch.overrides import TorchFunctionMode
+
+    from matchattention_b200 import MF_FusedForwardOps
+
+    class Python(TorchFunctionMode):                # takes calls off the native entry
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    def call(train, win_r=(1, 1), M=16, scale=0.25):
+        inputs = [t.detach().requires_grad_(train) for t in case["gpu"]]
+        return MF_FusedForwardOps()(*inputs, case["H"], case["W"], win_r, M, attn_type="l1_norm", scale=scale)
+
+    for train in (False, True):
+        for error, kwargs in ((ValueError if train else RuntimeError, dict(scale="x")), (TypeError if train else RuntimeError, dict(scale=None)),
+                              (RuntimeError, dict(win_r=[-1, -1], M=0))):
+            with pytest.raises(error) as native:
+                call(train, **kwargs)
+            assert not isinstance(native.value, NotImplementedError)
+            with Python(), pytest.raises(error):
+                call(train, **kwargs)
+    with pytest.raises(TypeError):                  # an int is no list of two; the training path takes it
+        call(False, win_r=1)
+    assert call(True, win_r=1)[0].shape == case["gpu"][1].shape
