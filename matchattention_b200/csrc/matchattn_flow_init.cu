@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
     if (i >= N) return;
     const T *base = prob + b2 * N * N;
     const float least = average(warp_max(top[warp][lane]) * (1.f - kScreen));
-    float bv = -1.f;
+    float bv = -INFINITY;
     int bj = 0x7fffffff;
     for (int c0 = 0; c0 < n; c0 += 32) {
         const float m = c0 + lane < n ? maxima[static_cast<int64_t>(c0 + lane) * N + warp] : 0.f;

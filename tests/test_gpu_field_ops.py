@@ -219,3 +219,18 @@ def test_flow_init_kernels_beyond_their_thresholds(H, W, dtype):
     assert _close16(blur, want_blur, dtype, ulps=3.0)
     same = centre.cpu() == want_centre
     assert same.float().mean() > 0.98           # the rest: equal box averages
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_flow_init_of_a_row_without_numbers(dtype):
+    """A token whose scores are not numbers has no arg max: its pooled maximum stays at minus infinity, its window at the
+    far end of the map; the tokens two and more away do not see it."""
+    H, W = 12, 14
+    corr = torch.randn(1, H * W, H * W).to(dtype)
+    corr[0, 70] = float("nan")
+    flow, prob, blur, centre = _ma().flow_init(corr.cuda(), H, W, return_debug=True)
+    assert (blur[0, 68:73] == -float("inf")).all() and prob[0].view(H * W, -1)[70].isnan().all()
+    away = torch.ones(H * W, dtype=torch.bool)
+    away[68:73] = False
+    assert (blur[0].cpu()[away] > 0).all() and torch.isfinite(flow[0].cpu().view(-1, 2)[away]).all()
+    assert ((centre >= 0) & (centre < H * W)).all()
