@@ -51,7 +51,8 @@ static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid
     return cudaErrorInvalidValue;
 }
 
-// The splits that a call of up to 32 heads gets without knobs; any other runs on the kernel above.
+// The splits that calls get without knobs (float32 on (2, 2) and (2, 4): from 33 heads on, r = 2); any other runs on the
+// kernel above, so do 33 to 64 heads of 128 channels at r = 1.
 template <typename T, int R>
 static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream)
 {
@@ -61,10 +62,9 @@ static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threa
         lanes_forward_kernel<T, R, CPL_, L_, false><<<grid, threads, 0, stream>>>(p);      \
         return cudaGetLastError();                                                         \
     }
-    MA_LANES(2, 8) MA_LANES(4, 8)
+    MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8) MA_LANES(4, 8)
     MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
     if constexpr (sizeof(T) == 2) {
-        MA_LANES(2, 2) MA_LANES(2, 4)
         if (cpl == 3 && p.lph == 2 && width == 5) {
             lanes_forward_kernel<T, R, 3, 2, true><<<grid, threads, 0, stream>>>(p);
             return cudaGetLastError();
