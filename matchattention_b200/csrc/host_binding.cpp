@@ -5,8 +5,8 @@
 // Python, a torch custom-op dispatch and a ctypes call with 19 arguments took about 60 us on the host.  Here it is
 // about 6 us, most of it the launch itself and two tensor allocations.
 //
-// Every function returns None when it does not cover its arguments (a tensor subclass or wrapper, a tracing or
-// dispatch mode, a wrong type, shape, device or layout); the caller then takes the Python path, which handles the rest
+// Every function returns None when it does not cover its arguments (a tensor subclass or wrapper, a tracing,
+// function or dispatch mode, a wrong type, shape, device or layout); the caller then takes the Python path, which handles the rest
 // and words the errors.  Nothing is kept between calls.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
