@@ -390,7 +390,7 @@ struct GatherParams {
     int *counts, *cursor, *differ;   // [B * h * cells_y][cells_x]; one word each: next free slot, heads differ
     int *starts;                 // [B * h * cells_y][cells_x + 1]: first slot of a bucket
     int *rank;                   // [items]: place of an item within its bucket
-    int2 *meta;                  // [slot]: (b * Nq + query, x0)
+    int2 *meta;                  // [slot]: (b * Nq + query, x0) -- shared centres: row of q in its batch item (elements), first tap - x0
     float2 *coef;                // (scale * ds, a) per slot, tap -- shared centres: slot, tap, head
     // summing kernel, per head
     int tile_x, tile_y, tiles_x, slice_chunks, batch;
@@ -789,7 +789,8 @@ __global__ void __launch_bounds__(128, R == 1 && CPL <= 2 ? 4 : 3) gather_coef_k
     float2 *coef = g.coef + (shared ? slot * M * p.h + head : slot * M);     // tap m at coef[m * coef_step]
     const int coef_step = shared ? p.h : 1;
     if (valid) {
-        if (sl == 0 && (!shared || head == 0)) g.meta[slot] = make_int2(static_cast<int>(bq), x_in);
+        if (sl == 0 && !shared) g.meta[slot] = make_int2(static_cast<int>(bq), x_in);
+        else if (sl == 0 && head == 0) g.meta[slot] = make_int2(static_cast<int>((bq - b * p.Nq) * p.C), static_cast<int>(slot * M - x_in));
         if (shared) {
 #pragma unroll
             for (int m = 0; m < M; ++m)
@@ -911,6 +912,14 @@ __device__ __forceinline__ void copy16_async(void *smem, const void *global)
                  : "memory");
 }
 
+// Has L2 fetch `count` pieces of `bytes` (a multiple of 16, from an address aligned to 16) that lie one after another.
+__device__ __forceinline__ void prefetch_l2(const void *global, int count, uint32_t bytes)
+{
+    // (one request holds a 32-bit size: what does not fit in is left to the loads)
+    const uint32_t most = 0x7ffffff0u / bytes, n = min(static_cast<uint32_t>(count), most);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(global), "r"(n * bytes) : "memory");
+}
+
 // dk and dv of a tile of tokens, one head, one slice of its channels: a thread per (token, eight channels).  The items
 // of all buckets that the tile needs are staged in shared memory, `batch` at a time: coefficients, q and dout.
 // A slot of coefficients is padded by 16 bytes: neighbouring tokens read the same tap of neighbouring slots.
@@ -1009,38 +1018,59 @@ __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
     }
 }
 
+// resident blocks of the kernel below per SM: as many as the registers of its chunks allow (0: no limit asked for)
+// (float16, 384x384 tokens, 8 heads x 16: 183 us with three, 173 with four; float32, r = 1: 126 with four, 79 with three)
+template <typename T, int R, int CPT>
+constexpr int sum_min_blocks() { return CPT == 4 ? 0 : CPT == 2 ? 2 : sizeof(T) == 2 && R == 1 ? 4 : 3; }
+// blocks ahead whose coefficients a block asks L2 for (600: 173 us, 300: 171, 1000: 176)
+constexpr unsigned kPrefetchAhead = 300;
+
 // The same with shared centres: `lanes` lanes per token, each with CPT chunks of eight channels (chunk = lane + s * lanes),
 // `per_warp` tokens per warp.  A query's row of q and dout is read as a whole, a tap's coefficients of all heads lie
 // side by side, and the lanes of a token walk the same list.  The rows are shared by the tokens of a block through L1.
-// Bound by the latency of those loads at 75 registers, three blocks per SM (issue 59 %).
-// Measured, same sizes: 208 us (300 us range by range: too few loads under way, and the border rows started last).
+// The coefficients are read once and come from memory: every block has L2 fetch those of the buckets that a block some
+// way ahead starts with, whole runs of slots in one request each.
+// Bound by the latency of the loads (issue 59 % at three blocks per SM without the prefetch, and more lanes or items side
+// by side add their own start: 230 to 265 us).
+// Measured, same sizes: 171 us (209 without the prefetch at three blocks).
 template <typename T, int R, int CPT>
-__global__ void __launch_bounds__(256) gather_sum_shared_kernel(const GatherParams g)
+__global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_shared_kernel(const GatherParams g)
 {
     constexpr int SIDE = 2 * R + 2, M = SIDE * SIDE;
     if (*g.differ != 0) return;
     const BwdParams &p = g.b;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane / g.lanes, own = lane - sub * g.lanes;
+    const int b = blockIdx.y, tile_rows = gridDim.x / g.shared_tiles_x;
     const int order = blockIdx.x / g.shared_tiles_x, tile_x = blockIdx.x - order * g.shared_tiles_x;
+    if (blockIdx.x + kPrefetchAhead < gridDim.x && threadIdx.x < g.shared_y) {
+        const int then = blockIdx.x + kPrefetchAhead, then_row = then / g.shared_tiles_x;
+        const int cy = tile_row(then_row, tile_rows) * g.shared_y + threadIdx.x, cx = (then - then_row * g.shared_tiles_x) * g.shared_x;
+        if (cy < g.cells_y && cx < g.cells_x) {
+            const int *start = g.starts + (static_cast<int64_t>(b) * g.cells_y + cy) * (g.cells_x + 1);
+            const int from = __ldg(start + cx), slots = __ldg(start + min(cx + g.shared_x, g.cells_x)) - from;
+            if (slots > 0) prefetch_l2(g.coef + static_cast<int64_t>(from) * M * p.h, slots, M * p.h * static_cast<uint32_t>(sizeof(float2)));
+        }
+    }
     const int t = warp * g.per_warp + sub, ty_in = t / g.shared_x;
-    const int tx = tile_x * g.shared_x + t - ty_in * g.shared_x, ty = tile_row(order, gridDim.x / g.shared_tiles_x) * g.shared_y + ty_in;
+    const int tx = tile_x * g.shared_x + t - ty_in * g.shared_x, ty = tile_row(order, tile_rows) * g.shared_y + ty_in;
     if (sub >= g.per_warp || tx >= p.W || ty >= p.H) return;
-    const int b = blockIdx.y, hd8 = p.hd >> 3;
+    const int hd8 = p.hd >> 3;
     const int64_t token_off = (static_cast<int64_t>(b) * p.N + static_cast<int64_t>(ty) * p.W + tx) * p.C;
 
-    const T *q = static_cast<const T *>(p.q) + own * 8, *go = static_cast<const T *>(p.dout) + own * 8, *k = static_cast<const T *>(p.k) + token_off + own * 8;
+    const int64_t query_off = static_cast<int64_t>(b) * p.Nq * p.C + own * 8;
+    const T *q = static_cast<const T *>(p.q) + query_off, *go = static_cast<const T *>(p.dout) + query_off;
     const int step = g.lanes * 8;                       // channels between the chunks of a lane
     Accumulate<T> acc[CPT];
 #pragma unroll
-    for (int s = 0; s < CPT; ++s) acc[s].start(k + s * step);
+    for (int s = 0; s < CPT; ++s) acc[s].start(static_cast<const T *>(p.k) + token_off + own * 8 + s * step);
     int head[CPT];
 #pragma unroll
     for (int s = 0; s < CPT; ++s) head[s] = (own + s * g.lanes) / hd8;
 
     // the token's items, one range of slots per row of buckets, numbered through: item f of row j lies in slot
-    // base[j] + f, its coefficients start at tap_base[j] + f * M + tx - x0
-    int until[SIDE], base[SIDE], tap_base[SIDE], total = 0;
+    // base[j] + f
+    int until[SIDE], base[SIDE], total = 0;
     {
         const int c_lo = max(tx - (SIDE - 1), 0), c_hi = min(tx + 1, g.cells_x);
         int lo[SIDE], hi[SIDE];
@@ -1055,39 +1085,38 @@ __global__ void __launch_bounds__(256) gather_sum_shared_kernel(const GatherPara
 #pragma unroll
         for (int j = 0; j < SIDE; ++j) {
             base[j] = lo[j] - total;
-            tap_base[j] = base[j] * M + j * SIDE + tx;
             total += hi[j] - lo[j];
             until[j] = total;
         }
     }
     const auto locate = [&](int f, int &slot, int &tap) {
         slot = base[0];
-        tap = tap_base[0];
+        tap = tx;
 #pragma unroll
         for (int j = 1; j < SIDE; ++j)
             if (f >= until[j - 1]) {
                 slot = base[j];
-                tap = tap_base[j];
+                tap = tx + j * SIDE;
             }
         slot += f;
-        tap += f * M;
     };
-    // two items at a time, so that their loads are under way together; their (query, x0) are read one step ahead
-    int2 meta[2] = {make_int2(0, 0), make_int2(0, 0)};
-    int tap[2];
+    // two items at a time, so that their loads are under way together; their places are read one step ahead
+    uint32_t row[2] = {0u, 0u}, tap[2] = {0u, 0u};
     const auto fetch = [&](int f) {
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-            int slot;
-            locate(min(f + n, total - 1), slot, tap[n]);
-            meta[n] = __ldg(g.meta + slot);
+            int slot, at;
+            locate(min(f + n, total - 1), slot, at);
+            const int2 m = __ldg(g.meta + slot);
+            row[n] = static_cast<uint32_t>(m.x);
+            tap[n] = static_cast<uint32_t>(at + m.y);
         }
     };
     if (total > 0) fetch(0);
     for (int f = 0; f < total; f += 2) {
         const bool second = f + 1 < total;
-        const float2 *c0 = g.coef + static_cast<int64_t>(tap[0] - meta[0].y) * p.h, *c1 = g.coef + static_cast<int64_t>(tap[1] - meta[1].y) * p.h;
-        const int64_t r0 = static_cast<int64_t>(meta[0].x) * p.C, r1 = static_cast<int64_t>(meta[1].x) * p.C;
+        const uint32_t r0 = row[0], r1 = row[1];
+        const float2 *c0 = g.coef + static_cast<uint64_t>(tap[0]) * static_cast<uint32_t>(p.h), *c1 = g.coef + static_cast<uint64_t>(tap[1]) * static_cast<uint32_t>(p.h);
 #pragma unroll
         for (int s = 0; s < CPT; ++s) {
             Piece<T> first, other;
