@@ -51,6 +51,7 @@ struct BwdParams {
 template <typename T>
 __global__ void __launch_bounds__(128) backward_kernel(const BwdParams p)
 {
+    chain_begin();
     const int64_t per_item = static_cast<int64_t>(p.Nq) * p.h;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= per_item) return;
@@ -226,6 +227,7 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16 *p, const fl
 template <typename T, int R>
 __global__ void __launch_bounds__(128, R == 2 ? 4 : 3) backward_vec_kernel(const BwdParams p)
 {
+    chain_begin();
     constexpr int SIDE = 2 * R + 2, SUB = 2 * R + 1, M = SIDE * SIDE;
     const int64_t per_item = static_cast<int64_t>(p.Nq) * p.h;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -425,6 +427,7 @@ struct ItemIndex {
 template <typename T>
 __global__ void __launch_bounds__(256) gather_check_kernel(const GatherParams g, uint32_t queries)
 {
+    chain_begin();
     using Pair = typename std::conditional<sizeof(T) == 4, uint2, uint32_t>::type;       // one (x, y)
     const uint32_t bq = blockIdx.x * 256u + threadIdx.x;
     if (bq >= queries) return;
@@ -444,6 +447,7 @@ __global__ void __launch_bounds__(256) gather_check_kernel(const GatherParams g,
 template <typename T, int R>
 __global__ void __launch_bounds__(256) gather_count_kernel(const GatherParams g)
 {
+    chain_begin();
     constexpr int SIDE = 2 * R + 2;
     const uint32_t item = blockIdx.x * 256u + threadIdx.x;
     if (item >= g.items) return;
@@ -461,6 +465,7 @@ __global__ void __launch_bounds__(256) gather_count_kernel(const GatherParams g)
 // A warp per row of buckets: the buckets' first slots, the row's place from the cursor.
 __global__ void __launch_bounds__(256) gather_starts_kernel(const GatherParams g, int64_t rows)
 {
+    chain_begin();
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= (*g.differ == 0 ? rows / g.b.h : rows)) return;
@@ -611,6 +616,7 @@ struct QueryGradient {           // dq -= ds * sign(q - k)
 template <typename T, int R, int CPL>
 __global__ void __launch_bounds__(128, R == 1 && CPL <= 2 ? 4 : 3) gather_coef_kernel(const GatherParams g)
 {
+    chain_begin();
     constexpr int SIDE = 2 * R + 2, SUB = 2 * R + 1, M = SIDE * SIDE;
     constexpr int NW = CPL * DT<T>::kWordsPerChunk;
     const BwdParams &p = g.b;
@@ -928,6 +934,7 @@ __device__ __forceinline__ void prefetch_l2(const void *global, int count, uint3
 template <typename T, int R>
 __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
 {
+    chain_begin();
     constexpr int SIDE = 2 * R + 2, M = SIDE * SIDE, kCoefPitch = M * 8 + 16;
     extern __shared__ __align__(16) char smem[];
     if (*g.differ == 0) return;
@@ -1036,6 +1043,7 @@ constexpr unsigned kPrefetchAhead = 300;
 template <typename T, int R, int CPT>
 __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_shared_kernel(const GatherParams g)
 {
+    chain_begin();
     constexpr int SIDE = 2 * R + 2, M = SIDE * SIDE;
     if (*g.differ != 0) return;
     const BwdParams &p = g.b;
@@ -1214,27 +1222,27 @@ cudaError_t launch_gather(const GatherParams &g, const GatherPlan &pl, cudaStrea
     cudaError_t e = cudaMemsetAsync(g.counts, 0, pl.off_cursor + 2 * sizeof(int), stream);
     if (e != cudaSuccess) return e;
     const uint32_t queries = static_cast<uint32_t>(g.items / g.b.h);
-    gather_check_kernel<T><<<(queries + 255) / 256, 256, 0, stream>>>(g, queries);
-    gather_count_kernel<T, R><<<static_cast<unsigned>((g.items + 255) / 256), 256, 0, stream>>>(g);
-    gather_starts_kernel<<<static_cast<unsigned>((pl.bucket_rows + 7) / 8), 256, 0, stream>>>(g, pl.bucket_rows);
+    launch_chained(gather_check_kernel<T>, (queries + 255) / 256, 256, 0, stream, g, queries);
+    launch_chained(gather_count_kernel<T, R>, static_cast<unsigned>((g.items + 255) / 256), 256, 0, stream, g);
+    launch_chained(gather_starts_kernel, static_cast<unsigned>((pl.bucket_rows + 7) / 8), 256, 0, stream, g, pl.bucket_rows);
     const unsigned coef_blocks = static_cast<unsigned>((g.items * pl.lph + 127) / 128);
     switch (pl.cpl) {
-    case 1: gather_coef_kernel<T, R, 1><<<coef_blocks, 128, 0, stream>>>(g); break;
-    case 2: gather_coef_kernel<T, R, 2><<<coef_blocks, 128, 0, stream>>>(g); break;
-    case 3: gather_coef_kernel<T, R, 3><<<coef_blocks, 128, 0, stream>>>(g); break;
-    default: gather_coef_kernel<T, R, 5><<<coef_blocks, 128, 0, stream>>>(g); break;
+    case 1: launch_chained(gather_coef_kernel<T, R, 1>, coef_blocks, 128, 0, stream, g); break;
+    case 2: launch_chained(gather_coef_kernel<T, R, 2>, coef_blocks, 128, 0, stream, g); break;
+    case 3: launch_chained(gather_coef_kernel<T, R, 3>, coef_blocks, 128, 0, stream, g); break;
+    default: launch_chained(gather_coef_kernel<T, R, 5>, coef_blocks, 128, 0, stream, g); break;
     }
     if (pl.smem > 48 * 1024) {     // per-device attribute of the kernel: set on every launch (cheap, idempotent, thread-safe)
         e = cudaFuncSetAttribute(gather_sum_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
         if (e != cudaSuccess) return e;
     }
     const unsigned tiles = static_cast<unsigned>(g.tiles_x) * ((g.b.H + pl.tile_y - 1) / pl.tile_y);
-    gather_sum_kernel<T, R><<<dim3(tiles, g.b.B * g.b.h, pl.slices), pl.threads, pl.smem, stream>>>(g);
+    launch_chained(gather_sum_kernel<T, R>, dim3(tiles, g.b.B * g.b.h, pl.slices), pl.threads, pl.smem, stream, g);
     const dim3 shared_grid(static_cast<unsigned>(g.shared_tiles_x) * ((g.b.H + pl.shared_y - 1) / pl.shared_y), g.b.B);
     switch (pl.cpt) {
-    case 1: gather_sum_shared_kernel<T, R, 1><<<shared_grid, 256, 0, stream>>>(g); break;
-    case 2: gather_sum_shared_kernel<T, R, 2><<<shared_grid, 256, 0, stream>>>(g); break;
-    default: gather_sum_shared_kernel<T, R, 4><<<shared_grid, 256, 0, stream>>>(g); break;
+    case 1: launch_chained(gather_sum_shared_kernel<T, R, 1>, shared_grid, 256, 0, stream, g); break;
+    case 2: launch_chained(gather_sum_shared_kernel<T, R, 2>, shared_grid, 256, 0, stream, g); break;
+    default: launch_chained(gather_sum_shared_kernel<T, R, 4>, shared_grid, 256, 0, stream, g); break;
     }
     return cudaGetLastError();
 }
@@ -1242,9 +1250,9 @@ cudaError_t launch_gather(const GatherParams &g, const GatherPlan &pl, cudaStrea
 template <typename T>
 void launch_backward(const BwdParams &p, bool vec, dim3 grid, cudaStream_t stream)
 {
-    if (vec && p.r == 1) backward_vec_kernel<T, 1><<<grid, 128, 0, stream>>>(p);
-    else if (vec && p.r == 2) backward_vec_kernel<T, 2><<<grid, 128, 0, stream>>>(p);
-    else backward_kernel<T><<<grid, 128, 0, stream>>>(p);
+    if (vec && p.r == 1) launch_chained(backward_vec_kernel<T, 1>, grid, 128, 0, stream, p);
+    else if (vec && p.r == 2) launch_chained(backward_vec_kernel<T, 2>, grid, 128, 0, stream, p);
+    else launch_chained(backward_kernel<T>, grid, 128, 0, stream, p);
 }
 
 }  // namespace

@@ -21,6 +21,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) consistency_mask_kernel(const T *__restrict__ field, T *__restrict__ mask,
                                                                 T *__restrict__ diff_out, int B, int H, int W, float A)
 {
+    chain_begin();
     const int64_t px = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t plane = static_cast<int64_t>(H) * W;
     if (px >= B * plane) return;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(32 * kDispGroups) local_disparity_kernel(const
                                                                            T *__restrict__ blur_out, int *__restrict__ centre_out,
                                                                            int B, int D, int H, int W, float tiny)
 {
+    chain_begin();
     __shared__ float best_of[kDispGroups][32];
     __shared__ int arg_of[kDispGroups][32];
     const int64_t plane = static_cast<int64_t>(H) * W;
@@ -147,7 +149,7 @@ cudaError_t run_mask(const void *field, void *mask, void *diff, int B, int H, in
 {
     const int64_t total = static_cast<int64_t>(B) * H * W;
     const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-    consistency_mask_kernel<T><<<blocks, 256, 0, stream>>>(static_cast<const T *>(field), static_cast<T *>(mask),
+    launch_chained(consistency_mask_kernel<T>, blocks, 256, 0, stream, static_cast<const T *>(field), static_cast<T *>(mask),
                                                           static_cast<T *>(diff), B, H, W, A);
     return cudaGetLastError();
 }
@@ -158,7 +160,7 @@ cudaError_t run_disparity(const void *cv, void *flow, void *blur, int *centre, i
 {
     const int64_t plane = static_cast<int64_t>(H) * W;
     const dim3 grid(static_cast<unsigned>((plane + 31) / 32), B);
-    local_disparity_kernel<T><<<grid, 32 * kDispGroups, 0, stream>>>(static_cast<const T *>(cv), static_cast<T *>(flow),
+    launch_chained(local_disparity_kernel<T>, grid, 32 * kDispGroups, 0, stream, static_cast<const T *>(cv), static_cast<T *>(flow),
                                                        static_cast<T *>(blur), centre, B, D, H, W, tiny);
     return cudaGetLastError();
 }

@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_max_kernel(const T *__restr
                                                                 float *__restrict__ col_part, int64_t N, int rows_per_warp,
                                                                 int row_parts, int col_parts)
 {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int64_t unit = static_cast<int64_t>(blockIdx.x) * kFlowWarps + (threadIdx.x >> 5);
     const int band = static_cast<int>(unit / row_parts), chunk = static_cast<int>(unit - static_cast<int64_t>(band) * row_parts);
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T 
                                                                 const float *__restrict__ col_part, float2 *__restrict__ stats,
                                                                 int64_t N, int row_parts, int col_parts, int col_blocks)
 {
+    chain_begin();
     const int64_t b = blockIdx.y;
     const T *src = corr + b * N * N;
     if (static_cast<int>(blockIdx.x) < col_blocks) {
@@ -618,6 +620,7 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
 template <typename T, int ALIGN>
 __global__ void __launch_bounds__(32 * kPoolWarps, sizeof(T) == 2 ? 5 : 4) flow_prob_pool_kernel(const T *__restrict__ corr, T *__restrict__ prob, const PoolParams pp)
 {
+    chain_begin();
     extern __shared__ __align__(16) char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int chunk_groups = (pp.chunks + kPoolWarps - 1) / kPoolWarps;
@@ -658,6 +661,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
                                                                    T *__restrict__ blur_max, int *__restrict__ centre_out, int B, int H,
                                                                    int W, int chunks, int bands, int band_rows, float tiny)
 {
+    chain_begin();
     constexpr int kGroups = kFlowThreads / kWindowTokens;
     __shared__ float top[kWindowTokens][kGroups + 1];
     __shared__ float rows[kFlowWarps][5][kWarpCols];
@@ -766,13 +770,12 @@ cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow
     float2 *stats = reinterpret_cast<float2 *>(scratch + pl.off_stats);
     float *row_max = reinterpret_cast<float *>(scratch + pl.off_row_max), *col_max = reinterpret_cast<float *>(scratch + pl.off_col_max);
     const int64_t units = static_cast<int64_t>(pl.row_parts) * pl.col_parts;
-    flow_max_kernel<T, ALIGN><<<dim3(static_cast<unsigned>((units + kFlowWarps - 1) / kFlowWarps), B), kFlowThreads, 0, stream>>>(
+    launch_chained(flow_max_kernel<T, ALIGN>, dim3(static_cast<unsigned>((units + kFlowWarps - 1) / kFlowWarps), B), kFlowThreads, 0, stream, 
         corr, row_part, col_part, N, pl.max_rows, pl.row_parts, pl.col_parts);
     const auto launch_sums = [&](auto columns, auto batch) {
         constexpr int kColumns = decltype(columns)::value, kThreadsHere = kColumns * kSumGroups, kRows = kThreadsHere / 32;
         const int col_blocks = static_cast<int>((N + kColumns - 1) / kColumns);
-        flow_sum_kernel<T, ALIGN, kColumns, decltype(batch)::value>
-            <<<dim3(static_cast<unsigned>(col_blocks + (N + kRows - 1) / kRows), B), kThreadsHere, 0, stream>>>(
+        launch_chained(flow_sum_kernel<T, ALIGN, kColumns, decltype(batch)::value>, dim3(static_cast<unsigned>(col_blocks + (N + kRows - 1) / kRows), B), kThreadsHere, 0, stream, 
                 corr, row_part, col_part, stats, N, pl.row_parts, pl.col_parts, col_blocks);
     };
     if (N >= kWideSums<T>) launch_sums(std::integral_constant<int, 32>(), std::integral_constant<int, sizeof(T) == 2 ? 16 : 24>());
@@ -781,9 +784,9 @@ cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow
     const cudaError_t e = cudaFuncSetAttribute(flow_prob_pool_kernel<T, ALIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int64_t regions = static_cast<int64_t>((pl.bands + kPoolWarps - 1) / kPoolWarps) * ((pl.chunks + kPoolWarps - 1) / kPoolWarps);
-    flow_prob_pool_kernel<T, ALIGN><<<dim3(static_cast<unsigned>(regions * 2 * kPoolWarps), B), 32 * kPoolWarps, smem, stream>>>(
+    launch_chained(flow_prob_pool_kernel<T, ALIGN>, dim3(static_cast<unsigned>(regions * 2 * kPoolWarps), B), 32 * kPoolWarps, smem, stream, 
         corr, prob, PoolParams{stats, row_max, col_max, N, B, pl.band, pl.chunks, pl.bands});
-    flow_window_kernel<T><<<dim3(static_cast<unsigned>((N + kWindowTokens - 1) / kWindowTokens), 2 * B), kFlowThreads, 0, stream>>>(
+    launch_chained(flow_window_kernel<T>, dim3(static_cast<unsigned>((N + kWindowTokens - 1) / kWindowTokens), 2 * B), kFlowThreads, 0, stream, 
         prob, row_max, col_max, flow, blur, centre, B, H, W, pl.chunks, pl.bands, pl.band, tiny);
     return cudaGetLastError();
 }

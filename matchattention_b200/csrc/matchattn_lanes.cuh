@@ -111,6 +111,7 @@ constexpr int lanes_min_blocks() { return R == 1 && CPL * DT<T>::kWordsPerChunk 
 template <typename T, int R, int CPL, int L, bool RAGGED>
 __global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes_forward_kernel(const Params p)
 {
+    chain_begin();
     using Share = RowShare<R, L>;
     constexpr int SIDE = Share::SIDE, SUB = 2 * R + 1, ROWS = Share::ROWS;
     constexpr int NW = CPL * DT<T>::kWordsPerChunk, EPW = DT<T>::kElemsPerWord;

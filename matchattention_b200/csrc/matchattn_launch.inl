@@ -30,20 +30,20 @@ static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid
         constexpr int CPL = decltype(chunks)::value;
         if constexpr (kPlainBuilds<T, CPL>) {
             if (!rare) {
-                if (glue && pow2) fused_forward_kernel<T, R, CPL, false, kGlueOptions, kCanPack><<<grid, threads, 0, stream>>>(p);
-                else if (glue) fused_forward_kernel<T, R, CPL, false, kGlueOptions><<<grid, threads, 0, stream>>>(p);
-                else if (pow2) fused_forward_kernel<T, R, CPL, false, kNoOptions, kCanPack><<<grid, threads, 0, stream>>>(p);
-                else fused_forward_kernel<T, R, CPL, false, kNoOptions><<<grid, threads, 0, stream>>>(p);
+                if (glue && pow2) launch_chained(fused_forward_kernel<T, R, CPL, false, kGlueOptions, kCanPack>, grid, threads, 0, stream, p);
+                else if (glue) launch_chained(fused_forward_kernel<T, R, CPL, false, kGlueOptions>, grid, threads, 0, stream, p);
+                else if (pow2) launch_chained(fused_forward_kernel<T, R, CPL, false, kNoOptions, kCanPack>, grid, threads, 0, stream, p);
+                else launch_chained(fused_forward_kernel<T, R, CPL, false, kNoOptions>, grid, threads, 0, stream, p);
                 return cudaGetLastError();
             }
         }
-        fused_forward_kernel<T, R, CPL, false, kAllOptions><<<grid, threads, 0, stream>>>(p);
+        launch_chained(fused_forward_kernel<T, R, CPL, false, kAllOptions>, grid, threads, 0, stream, p);
         return cudaGetLastError();
     };
 #define MA_CASE(CPL_)                                                                            \
     if (cpl == CPL_) {                                                                           \
         if (!multi) return one_lane(std::integral_constant<int, CPL_>());                        \
-        fused_forward_kernel<T, R, CPL_, true, kAllOptions><<<grid, threads, 0, stream>>>(p);    \
+        launch_chained(fused_forward_kernel<T, R, CPL_, true, kAllOptions>, grid, threads, 0, stream, p);    \
         return cudaGetLastError();                                                               \
     }
     MA_CASE(1) MA_CASE(2) MA_CASE(3) MA_CASE(4) MA_CASE(5)
@@ -59,14 +59,14 @@ static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threa
     const int width = p.hd / 8;      // chunks of a head
 #define MA_LANES(CPL_, L_)                                                                 \
     if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) {                                \
-        lanes_forward_kernel<T, R, CPL_, L_, false><<<grid, threads, 0, stream>>>(p);      \
+        launch_chained(lanes_forward_kernel<T, R, CPL_, L_, false>, grid, threads, 0, stream, p);      \
         return cudaGetLastError();                                                         \
     }
     MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8) MA_LANES(4, 8)
     MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
     if constexpr (sizeof(T) == 2) {
         if (cpl == 3 && p.lph == 2 && width == 5) {
-            lanes_forward_kernel<T, R, 3, 2, true><<<grid, threads, 0, stream>>>(p);
+            launch_chained(lanes_forward_kernel<T, R, 3, 2, true>, grid, threads, 0, stream, p);
             return cudaGetLastError();
         }
     } else {
@@ -212,7 +212,7 @@ cudaError_t launch_staged<MATCHATTN_T>(const StagedParams &sp, int cpl, const CU
 template <>
 cudaError_t launch_generic<MATCHATTN_T>(const Params &p, dim3 grid, cudaStream_t stream)
 {
-    generic_forward_kernel<MATCHATTN_T><<<grid, kThreads, 0, stream>>>(p);
+    launch_chained(generic_forward_kernel<MATCHATTN_T>, grid, kThreads, 0, stream, p);
     return cudaGetLastError();
 }
 

@@ -63,6 +63,7 @@ template <typename T, int F>
 __global__ void __launch_bounds__(128) upsample_field_kernel(const T *__restrict__ field, const T *__restrict__ mask,
                                                              T *__restrict__ out, int B, int H, int W, int D)
 {
+    chain_begin();
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     const int h = blockIdx.y, b = blockIdx.z;
     if (w >= W) return;
@@ -139,6 +140,7 @@ template <typename T, int F, bool EVEN>
 __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
                                                             int B, int H, int W, int segments)
 {
+    chain_begin();
     constexpr int COLS = EVEN ? 4 : 6;             // columns of neighbours: -1 .. 2 around the pair, or -1 .. 1 around either
     const int lane = threadIdx.x & 31;
     const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5);
@@ -232,6 +234,7 @@ template <int F>
 __global__ void __launch_bounds__(128) upsample_f32_kernel(const float *__restrict__ field, const float *__restrict__ mask,
                                                            float *__restrict__ out, int B, int H, int W, int segments)
 {
+    chain_begin();
     const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5);
     const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, fine row
     const int w0 = static_cast<int>(warp - line * segments) * 64 + 2 * (threadIdx.x & 31);
@@ -304,20 +307,20 @@ cudaError_t launch(const void *field, const void *mask, void *out, int B, int H,
             if ((reinterpret_cast<uintptr_t>(f) & 3u) == 0) {
                 const auto kernel = even ? (factor == 4 ? upsample_pair_kernel<T, 4, true> : upsample_pair_kernel<T, 2, true>)
                                          : (factor == 4 ? upsample_pair_kernel<T, 4, false> : upsample_pair_kernel<T, 2, false>);
-                kernel<<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+                launch_chained(kernel, blocks, 128, 0, stream, f, m, o, B, H, W, seg);
                 return cudaGetLastError();
             }
         } else if (even) {
             const auto kernel = factor == 4 ? upsample_f32_kernel<4> : upsample_f32_kernel<2>;
-            kernel<<<blocks, 128, 0, stream>>>(f, m, o, B, H, W, seg);
+            launch_chained(kernel, blocks, 128, 0, stream, f, m, o, B, H, W, seg);
             return cudaGetLastError();
         }
     }
     switch (factor) {
-    case 1: upsample_field_kernel<T, 1><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;
-    case 2: upsample_field_kernel<T, 2><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;
-    case 4: upsample_field_kernel<T, 4><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;
-    case 8: upsample_field_kernel<T, 8><<<grid, block, 0, stream>>>(f, m, o, B, H, W, D); break;
+    case 1: launch_chained(upsample_field_kernel<T, 1>, grid, block, 0, stream, f, m, o, B, H, W, D); break;
+    case 2: launch_chained(upsample_field_kernel<T, 2>, grid, block, 0, stream, f, m, o, B, H, W, D); break;
+    case 4: launch_chained(upsample_field_kernel<T, 4>, grid, block, 0, stream, f, m, o, B, H, W, D); break;
+    case 8: launch_chained(upsample_field_kernel<T, 8>, grid, block, 0, stream, f, m, o, B, H, W, D); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -36,6 +36,7 @@ __host__ __device__ constexpr int volume_pitch(int W) { return (W + 3) / 4 * 4 +
 template <typename T, int PIECES>
 __global__ void __launch_bounds__(1024) stereo_volume_kernel(const T *__restrict__ corr, T *__restrict__ vol, int B, int H, int W)
 {
+    chain_begin();
     extern __shared__ float slice[];              // [W][P]: corr[w][j], then exp(corr - maximum of its column of vol)
     const int P = volume_pitch(W);
     float *top = slice + W * P, *inv = top + W;   // per column w: maximum, reciprocal of the sum
@@ -126,7 +127,7 @@ cudaError_t launch(const void *corr, void *vol, int B, int H, int W, cudaStream_
         }
         // as many warps as there are rows to share out, within what two blocks per SM can hold
         const int threads = W > 64 ? 1024 : 512;
-        stereo_volume_kernel<T, kPieces><<<dim3(H, 2 * B), threads, smem, stream>>>(static_cast<const T *>(corr), static_cast<T *>(vol), B, H, W);
+        launch_chained(stereo_volume_kernel<T, kPieces>, dim3(H, 2 * B), threads, smem, stream, static_cast<const T *>(corr), static_cast<T *>(vol), B, H, W);
         return cudaGetLastError();
     };
     switch ((W + 31) / 32) {
