@@ -18,9 +18,9 @@
 // prob and the deciding averages are formed in one fixed order (sums of exponentials in 256 interleaved partial sums
 // per row and four per column, box sums row by row) whatever the split of the work, and only the screening in step 3
 // adds in another.
-// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.06 ms = 0.09 + 0.26 +
-// 0.63 + 0.08; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
-// the pooling took 4.1.  48x48 tokens: 51 us, before 189 (as a CUDA graph).
+// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.03 ms = 0.09 + 0.26 +
+// 0.63 + 0.05; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
+// the pooling took 4.1.  48x48 tokens: 47 us, before 196.
 // Rounding of the 16-bit types as eager PyTorch on the GPU: softmax, pooling and sums accumulate in float32
 // and round once, every elementwise op rounds.
 #include "../../include/matchattn.h"
@@ -650,9 +650,15 @@ __global__ void __launch_bounds__(32 * kPoolWarps, sizeof(T) == 2 ? 5 : 4) flow_
 // Per token (b2, i): the first target j whose 5x5 box average, rounded to T, is the largest, and the expected target
 // position within the 5x5 window of probabilities around it (clamped to the map) minus the token's own position.
 // The box maxima per chunk of targets screen the chunks: the average is monotone in the box sum, and the screening
-// sums are within kScreen of the ones that decide.  A block takes eight tokens: its threads scan the chunk maxima of
-// all of them, then every warp serves one: it sums the boxes of the chunks that pass (as a rule one) from prob, row by
-// row, lanes = targets, then takes the window, lanes = its 25 elements.  Latency-bound: a few dependent reads.
+// sums are within kScreen of the ones that decide.  A block takes eight tokens: its threads read the chunk maxima of
+// all of them at once, then every warp serves one: it sums the boxes of the chunks that pass (as a rule one) from prob, one,
+// two or four neighbouring targets per lane, then takes the window, lanes = its 25 elements.  Bound by instruction issue and
+// a few dependent reads.  Measured, float16: 128x128 tokens 78.7 -> 48.5 us, 48x48 10.3 -> 7.8 (a second walk over the
+// maxima with a division per chunk, every box on its own, the 25 terms handed round by shuffles before).
+// A chunk maximum below kCoarse * top - kCoarseStep cannot round to the top average: the 16-bit types are at most 2^-7 of a
+// value and 2^-24 apart, a box sum is 25 averages.
+constexpr float kCoarse = 1.f - 0x1p-6f, kCoarseStep = 25.f * 0x1p-23f;
+constexpr int kKeptChunks = 256;      // chunk maxima per token that a block of the window kernel keeps in shared memory
 constexpr float kScreen = 4e-6f;      // 24 float32 additions of positive terms in two different orders
 
 template <typename T>
@@ -663,8 +669,8 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
 {
     chain_begin();
     constexpr int kGroups = kFlowThreads / kWindowTokens;
-    __shared__ float top[kWindowTokens][kGroups + 1];
-    __shared__ float rows[kFlowWarps][5][kWarpCols];
+    __shared__ float kept[kWindowTokens][kKeptChunks + 1];
+    __shared__ __align__(16) float rows[kFlowWarps][5][kWarpCols];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t N = static_cast<int64_t>(H) * W;
     const int64_t b2 = blockIdx.y, i0 = static_cast<int64_t>(blockIdx.x) * kWindowTokens;
@@ -672,56 +678,82 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
     const int n = cols ? bands : chunks, width = cols ? band_rows : kPoolCols;
     const float *maxima = (cols ? col_max + (b2 - B) * bands * N : row_max + b2 * chunks * N) + i0;
     const auto average = [](float sum) { return DT<T>::rnd(__fdiv_rn(sum, 25.f)); };
-    {
+    {       // eight tokens' maxima of a chunk lie side by side: a thread reads every 32nd chunk of one token, all under way at once
         const int t = threadIdx.x % kWindowTokens, g = threadIdx.x / kWindowTokens;
-        float m = 0.f;
         if (i0 + t < N) {
-#pragma unroll 4
-            for (int c = g; c < n; c += kGroups) m = fmaxf(m, maxima[static_cast<int64_t>(c) * N + t]);
+#pragma unroll 8
+            for (int c = g; c < min(n, kKeptChunks); c += kGroups) kept[t][c] = __ldg(maxima + static_cast<int64_t>(c) * N + t);
         }
-        top[t][g] = m;
     }
     __syncthreads();
     const int64_t i = i0 + warp;
     if (i >= N) return;
     const T *base = prob + b2 * N * N;
-    const float least = average(warp_max(top[warp][lane]) * (1.f - kScreen));
+    const auto chunk_max = [&](int c) {
+        return c >= n ? 0.f : c < kKeptChunks ? kept[warp][c] : __ldg(maxima + static_cast<int64_t>(c) * N + warp);
+    };
+    float top = 0.f;
+    for (int c = lane; c < n; c += 32) top = fmaxf(top, chunk_max(c));
+    top = warp_max(top);
+    const float least = average(top * (1.f - kScreen));
+    const float far = top * kCoarse - kCoarseStep;      // below: rounds to less than `least` whatever the type
+    float(*const mine)[kWarpCols] = rows[warp];
     float bv = -INFINITY;
     int bj = 0x7fffffff;
+    // boxes of PER neighbouring targets per lane, each summed in the deciding order
+    const auto pool = [&](auto per, int64_t first) {
+        constexpr int PER = decltype(per)::value;
+        if (lane * PER >= width) return;
+        float sum[PER];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) {
+            float p[PER + 4];
+            if constexpr (PER == 4) {
+                const float4 a = *reinterpret_cast<const float4 *>(&mine[d][4 * lane]), c = *reinterpret_cast<const float4 *>(&mine[d][4 * lane + 4]);
+                p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w; p[4] = c.x; p[5] = c.y; p[6] = c.z; p[7] = c.w;
+            } else if constexpr (PER == 2) {
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {
+                    const float2 a = *reinterpret_cast<const float2 *>(&mine[d][2 * lane + 2 * e]);
+                    p[2 * e] = a.x;
+                    p[2 * e + 1] = a.y;
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 5; ++e) p[e] = mine[d][lane + e];
+            }
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+#pragma unroll
+                for (int e = 0; e < 5; ++e) sum[k] = d == 0 && e == 0 ? p[k] : sum[k] + p[k + e];
+        }
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int c = lane * PER + k;
+            const float v = average(sum[k]);
+            if (c < width && first + c < N && v > bv) {
+                bv = v;
+                bj = static_cast<int>(first) + c;
+            }
+        }
+    };
     for (int c0 = 0; c0 < n; c0 += 32) {
-        const float m = c0 + lane < n ? maxima[static_cast<int64_t>(c0 + lane) * N + warp] : 0.f;
+        const float m = chunk_max(c0 + lane);
+        if (!__any_sync(0xffffffffu, !(m < far))) continue;
         unsigned pass = __ballot_sync(0xffffffffu, c0 + lane < n && average(m * (1.f + kScreen)) >= least);
         for (; pass != 0; pass &= pass - 1) {
-            const int64_t first = static_cast<int64_t>(c0 + __ffs(pass) - 1) * width;
+            const int64_t first = static_cast<int64_t>(c0 + __ffs(pass) - 1) * width, j0 = first - 2 + lane;
+            const T *at = base + (i - 2) * N + j0;
+            for (int c = lane; c < width + 4; c += 32, at += 32) {
+                const int64_t j = first - 2 + c;
+                const bool in = j >= 0 && j < N;
 #pragma unroll
-            for (int k = 0; k < kWarpCols / 32; ++k) {
-                const int64_t j = first - 2 + lane + 32 * k;
-                float p[5];
-#pragma unroll
-                for (int d = 0; d < 5; ++d) {
-                    const int64_t ii = i + d - 2;
-                    p[d] = (ii >= 0 && ii < N && j >= 0 && j < N && j < first + width + 2) ? load_one<T>(base + ii * N + j) : 0.f;
-                }
-#pragma unroll
-                for (int d = 0; d < 5; ++d) rows[warp][d][lane + 32 * k] = p[d];
+                for (int d = 0; d < 5; ++d) mine[d][c] = in && i + d >= 2 && i + d - 2 < N ? load_one<T>(at + d * N) : 0.f;
             }
             __syncwarp();
-#pragma unroll
-            for (int k = 0; k < kWarpCols / 32; ++k) {
-                const int c = lane + 32 * k;
-                if (c < width && c + 4 < kWarpCols && first + c < N) {
-                    float sum = 0.f;
-#pragma unroll
-                    for (int d = 0; d < 5; ++d)
-#pragma unroll
-                        for (int e = 0; e < 5; ++e) sum += rows[warp][d][c + e];
-                    const float v = average(sum);
-                    if (v > bv) {
-                        bv = v;
-                        bj = static_cast<int>(first) + c;
-                    }
-                }
-            }
+            if (width <= 32) pool(std::integral_constant<int, 1>(), first);
+            else if (width <= 64) pool(std::integral_constant<int, 2>(), first);
+            else pool(std::integral_constant<int, 4>(), first);
             __syncwarp();
         }
     }
@@ -739,23 +771,28 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
     const int tx = cx + lane % 5 - 2, ty = cy + lane / 5 - 2;
     float p = lane < 25 ? load_one<T>(base + i * N + static_cast<int64_t>(ty) * W + tx) : 0.f;
     if (p < mean) p = 0.f;
-    float sum = 0.f;
+    // sums of 25 in order, the terms read back four at a time
+    const auto sum_25 = [](const float *v) {
+        float sum = 0.f;
 #pragma unroll
-    for (int k = 0; k < 25; ++k) sum += __shfl_sync(0xffffffffu, p, k);
-    sum = fmaxf(DT<T>::rnd(sum), tiny);
+        for (int k = 0; k < 24; k += 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(v + k);
+            sum += q.x; sum += q.y; sum += q.z; sum += q.w;
+        }
+        return sum + v[24];
+    };
+    mine[0][lane] = p;
+    __syncwarp();
+    const float sum = fmaxf(DT<T>::rnd(sum_25(mine[0])), tiny);
     const float np = DT<T>::rnd(__fdiv_rn(p, sum));
-    const float px = DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(tx))), py = DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(ty)));
-    float ax = 0.f, ay = 0.f;
-#pragma unroll
-    for (int k = 0; k < 25; ++k) {
-        ax += __shfl_sync(0xffffffffu, px, k);
-        ay += __shfl_sync(0xffffffffu, py, k);
-    }
+    mine[1][lane] = DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(tx)));
+    mine[2][lane] = DT<T>::rnd(np * DT<T>::rnd(static_cast<float>(ty)));
+    __syncwarp();
+    const int64_t at = b2 * N + i;
+    const int qy = static_cast<int>(i / W), qx = static_cast<int>(i - static_cast<int64_t>(qy) * W);
+    if (lane < 2)       // x, y
+        store_one<T>(flow + at * 2 + lane, DT<T>::rnd(DT<T>::rnd(sum_25(mine[1 + lane])) - DT<T>::rnd(static_cast<float>(lane == 0 ? qx : qy))));
     if (lane == 0) {
-        const int64_t at = b2 * N + i;
-        const int qy = static_cast<int>(i / W), qx = static_cast<int>(i - static_cast<int64_t>(qy) * W);
-        store_one<T>(flow + at * 2, DT<T>::rnd(DT<T>::rnd(ax) - DT<T>::rnd(static_cast<float>(qx))));
-        store_one<T>(flow + at * 2 + 1, DT<T>::rnd(DT<T>::rnd(ay) - DT<T>::rnd(static_cast<float>(qy))));
         if (centre_out != nullptr) centre_out[at] = cy * W + cx;
         if (blur_max != nullptr) store_one<T>(blur_max + at, bv);
     }
