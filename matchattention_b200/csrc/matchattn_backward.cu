@@ -383,6 +383,14 @@ __global__ void __launch_bounds__(128, R == 2 ? 4 : 3) backward_vec_kernel(const
 // Where all heads of every query share one centre (the cross branch, whose field has no head axis) one list of queries
 // serves all heads and a warp sums whole token rows; a first kernel finds out, the others read its verdict.
 
+// Tile of a block of the staged sums and chunks of eight channels of a head: a thread per token and chunk.
+constexpr int kStagedX = 16, kStagedY = 8, kStagedChunks = 2;
+
+// Split of the direct sums: chunks per lane, lanes per token, tokens per warp, tile of a block.
+struct SumTiles {
+    int cpt, lanes, per_warp, x, y, tiles_x;
+};
+
 struct GatherParams {
     BwdParams b;                 // b.dk, b.dv unused
     void *dk, *dv;               // tensor type, written
@@ -392,12 +400,10 @@ struct GatherParams {
     int *counts, *cursor, *differ;   // [B * h * cells_y][cells_x]; one word each: next free slot, heads differ
     int *starts;                 // [B * h * cells_y][cells_x + 1]: first slot of a bucket
     int *rank;                   // [items]: place of an item within its bucket
-    int2 *meta;                  // [slot]: (b * Nq + query, x0) -- shared centres: row of q in its batch item (elements), first tap - x0
+    int2 *meta;                  // [slot]: row of q in its batch item (elements), x0 -- shared centres: slot * taps - x0
     float2 *coef;                // (scale * ds, a) per slot, tap -- shared centres: slot, tap, head
-    // summing kernel, per head
-    int tile_x, tile_y, tiles_x, slice_chunks, batch;
-    // summing kernel, shared centres: lanes per token, tokens per warp, tile of a block
-    int lanes, per_warp, shared_x, shared_y, shared_tiles_x;
+    int batch;                                          // staged sums: items at a time
+    SumTiles all_heads, one_head;                       // direct sums: shared centres, one head
 };
 
 template <typename T, int R>
@@ -524,6 +530,14 @@ __device__ __forceinline__ float2 sign_pair(uint32_t a, uint32_t b)
     return make_float2(DT<T>::unpack(w, 0), DT<T>::unpack(w, 1));
 }
 
+__device__ __forceinline__ float sign_of(float a, float b)      // sign(a - b), 0 where one of them is no number
+{
+    float gt, lt;
+    asm("set.gt.f32.f32 %0, %1, %2;" : "=f"(gt) : "f"(a), "f"(b));
+    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(lt) : "f"(a), "f"(b));
+    return gt - lt;
+}
+
 // A lane's slice (NW words) of q or dout against one tap's words of K or V.
 template <typename T, int NW>
 struct Distance {                // sum of |q - k|, exact differences
@@ -587,9 +601,7 @@ struct QueryGradient {           // dq -= ds * sign(q - k)
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             if constexpr (EPW == 1) {
-                const float d = __uint_as_float(k[w]) - __uint_as_float(q[w]);
-                const float signed_ds = __uint_as_float(__float_as_uint(ds) ^ (__float_as_uint(d) & 0x80000000u));
-                dq[w] += d != 0.f ? signed_ds : 0.f;
+                dq[w] = fmaf(ds, sign_of(__uint_as_float(k[w]), __uint_as_float(q[w])), dq[w]);
             } else {
                 const float2 s = sign_pair<T>(k[w], q[w]);
                 dq[2 * w] = fmaf(ds, s.x, dq[2 * w]);
@@ -795,8 +807,7 @@ __global__ void __launch_bounds__(128, R == 1 && CPL <= 2 ? 4 : 3) gather_coef_k
     float2 *coef = g.coef + (shared ? slot * M * p.h + head : slot * M);     // tap m at coef[m * coef_step]
     const int coef_step = shared ? p.h : 1;
     if (valid) {
-        if (sl == 0 && !shared) g.meta[slot] = make_int2(static_cast<int>(bq), x_in);
-        else if (sl == 0 && head == 0) g.meta[slot] = make_int2(static_cast<int>((bq - b * p.Nq) * p.C), static_cast<int>(slot * M - x_in));
+        if (sl == 0 && (!shared || head == 0)) g.meta[slot] = make_int2(static_cast<int>((bq - b * p.Nq) * p.C), shared ? static_cast<int>(slot * M) - x_in : x_in);
         if (shared) {
 #pragma unroll
             for (int m = 0; m < M; ++m)
@@ -855,16 +866,32 @@ __global__ void __launch_bounds__(128, R == 1 && CPL <= 2 ? 4 : 3) gather_coef_k
         for (int i = 0; i < SIDE; ++i) fold(coef + i * coef_step, SIDE * coef_step, y0 - y_in);
 }
 
-// Eight channels of q and dout as loaded.
+// Eight channels of q and dout as loaded: 16 bytes, or 32 in one piece (float32, 192x192 tokens, 4 heads x 16: 77 -> 71 us).
 template <typename T>
 struct Piece {
-    uint4 q[sizeof(T) / 2], go[sizeof(T) / 2];
-    __device__ __forceinline__ void load(const T *qp, const T *gp)
+    static constexpr int NW = DT<T>::kWordsPerChunk;
+    uint32_t q[NW], go[NW];
+    static __device__ __forceinline__ void load(uint32_t (&w)[NW], const T *at)      // (the 32-byte form takes global addresses only)
+    {
+        if constexpr (NW == 8) {
+            ld_nc_256(w, at);
+        } else {
+            const uint4 u = *reinterpret_cast<const uint4 *>(at);
+            w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+        }
+    }
+    __device__ __forceinline__ void load(const T *qp, const T *gp)         // from global memory
+    {
+        load(q, qp);
+        load(go, gp);
+    }
+    __device__ __forceinline__ void load_staged(const char *qp, const char *gp)      // from shared memory
     {
 #pragma unroll
-        for (int i = 0; i < static_cast<int>(sizeof(T)) / 2; ++i) {
-            q[i] = reinterpret_cast<const uint4 *>(qp)[i];
-            go[i] = reinterpret_cast<const uint4 *>(gp)[i];
+        for (int i = 0; i < NW / 4; ++i) {
+            const uint4 u = reinterpret_cast<const uint4 *>(qp)[i], v = reinterpret_cast<const uint4 *>(gp)[i];
+            q[4 * i] = u.x; q[4 * i + 1] = u.y; q[4 * i + 2] = u.z; q[4 * i + 3] = u.w;
+            go[4 * i] = v.x; go[4 * i + 1] = v.y; go[4 * i + 2] = v.z; go[4 * i + 3] = v.w;
         }
     }
 };
@@ -887,22 +914,16 @@ struct Accumulate {
     __device__ __forceinline__ void add(const Piece<T> &pc, float ds, float a)
     {
 #pragma unroll
-        for (int i = 0; i < static_cast<int>(sizeof(T)) / 2; ++i) {
-            const uint32_t qw[4] = {pc.q[i].x, pc.q[i].y, pc.q[i].z, pc.q[i].w}, gw[4] = {pc.go[i].x, pc.go[i].y, pc.go[i].z, pc.go[i].w};
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                if constexpr (sizeof(T) == 4) {
-                    const int c = 4 * i + w;
-                    const float qv = __uint_as_float(qw[w]), kv = __uint_as_float(k[c]);
-                    dk[c] += qv > kv ? ds : (qv < kv ? -ds : 0.f);
-                    dv[c] = fmaf(a, __uint_as_float(gw[w]), dv[c]);
-                } else {
-                    const float2 s = sign_pair<T>(qw[w], k[w]);
-                    dk[2 * w] = fmaf(ds, s.x, dk[2 * w]);
-                    dk[2 * w + 1] = fmaf(ds, s.y, dk[2 * w + 1]);
-                    dv[2 * w] = fmaf(a, DT<T>::unpack(gw[w], 0), dv[2 * w]);
-                    dv[2 * w + 1] = fmaf(a, DT<T>::unpack(gw[w], 1), dv[2 * w + 1]);
-                }
+        for (int w = 0; w < Piece<T>::NW; ++w) {
+            if constexpr (sizeof(T) == 4) {
+                dk[w] = fmaf(ds, sign_of(__uint_as_float(pc.q[w]), __uint_as_float(k[w])), dk[w]);
+                dv[w] = fmaf(a, __uint_as_float(pc.go[w]), dv[w]);
+            } else {
+                const float2 s = sign_pair<T>(pc.q[w], k[w]);
+                dk[2 * w] = fmaf(ds, s.x, dk[2 * w]);
+                dk[2 * w + 1] = fmaf(ds, s.y, dk[2 * w + 1]);
+                dv[2 * w] = fmaf(a, DT<T>::unpack(pc.go[w], 0), dv[2 * w]);
+                dv[2 * w + 1] = fmaf(a, DT<T>::unpack(pc.go[w], 1), dv[2 * w + 1]);
             }
         }
     }
@@ -926,30 +947,33 @@ __device__ __forceinline__ void prefetch_l2(const void *global, int count, uint3
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(global), "r"(n * bytes) : "memory");
 }
 
-// dk and dv of a tile of tokens, one head, one slice of its channels: a thread per (token, eight channels).  The items
+// dk and dv of a tile of tokens, one head of two chunks of channels: a thread per (token, eight channels).  The items
 // of all buckets that the tile needs are staged in shared memory, `batch` at a time: coefficients, q and dout.
 // A slot of coefficients is padded by 16 bytes: neighbouring tokens read the same tap of neighbouring slots.
+// Such narrow heads alone: read straight from global memory, every item of a list is a line of its own for as few bytes
+// (float16, 384x384 tokens, 8 heads x 16, a centre per head: 219 us, the kernel below 260; float32, 2 x 192x192, 4 x 16: 79
+// and 105; 4 x 8 channels: 54 and 50, 4 x 64: 190 and 160).
 // Bound by instruction issue (69 % of the slots; about 57 per token, item and eight channels; two thirds of the lanes busy,
-// lists differ in length).  Measured, same sizes as above: 276 us; walking a token's four ranges as one list costs as much as it saves.
+// lists differ in length); walking a token's four ranges as one list costs as much as it saves.
 template <typename T, int R>
-__global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
+__global__ void __launch_bounds__(kStagedX * kStagedY * kStagedChunks) gather_sum_staged_kernel(const GatherParams g)
 {
     chain_begin();
     constexpr int SIDE = 2 * R + 2, M = SIDE * SIDE, kCoefPitch = M * 8 + 16;
     extern __shared__ __align__(16) char smem[];
     if (*g.differ == 0) return;
     const BwdParams &p = g.b;
-    const int tid = threadIdx.x, threads = blockDim.x;
-    const int order = blockIdx.x / g.tiles_x, tile_x = blockIdx.x - order * g.tiles_x;
-    const int tx0 = tile_x * g.tile_x, ty0 = tile_row(order, gridDim.x / g.tiles_x) * g.tile_y;
+    constexpr int threads = kStagedX * kStagedY * kStagedChunks, row_bytes = kStagedChunks * 8 * static_cast<int>(sizeof(T));
+    constexpr int rows = kStagedY + SIDE - 1, cols = kStagedX + SIDE;         // bucket rows, bucket starts per row
+    const int tid = threadIdx.x, tiles_x = (p.W + kStagedX - 1) / kStagedX;
+    const int order = blockIdx.x / tiles_x, tile_x = blockIdx.x - order * tiles_x;
+    const int tx0 = tile_x * kStagedX, ty0 = tile_row(order, gridDim.x / tiles_x) * kStagedY;
     const int bh = blockIdx.y, b = bh / p.h, head = bh - b * p.h;
-    const int slice_off = head * p.hd + blockIdx.z * g.slice_chunks * 8;      // channels of this block
-    const int rows = g.tile_y + SIDE - 1, cols = g.tile_x + SIDE;             // bucket rows, bucket starts per row
-    const int row_bytes = g.slice_chunks * 8 * static_cast<int>(sizeof(T));
+    const int head_off = head * p.hd;
 
     char *coef_s = smem;
     char *q_s = coef_s + g.batch * kCoefPitch, *go_s = q_s + g.batch * row_bytes;
-    int2 *meta_s = reinterpret_cast<int2 *>(go_s + g.batch * row_bytes);      // (query, x0) of a staged item
+    int2 *meta_s = reinterpret_cast<int2 *>(go_s + g.batch * row_bytes);      // (row of q, x0) of a staged item
     int *slot_s = reinterpret_cast<int *>(meta_s + g.batch);
     int *start_s = slot_s + g.batch, *base_s = start_s + rows * cols;         // base_s[r]: items of the tile before row r
 
@@ -972,11 +996,11 @@ __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
     __syncthreads();
     const int total = base_s[rows];
 
-    const int chunk = tid % g.slice_chunks, token = tid / g.slice_chunks;
-    const int txl = token % g.tile_x, tyl = token / g.tile_x;
+    const int chunk = tid % kStagedChunks, token = tid / kStagedChunks;
+    const int txl = token % kStagedX, tyl = token / kStagedX;
     const int tx = tx0 + txl, ty = ty0 + tyl;
-    const bool mine = tyl < g.tile_y && tx < p.W && ty < p.H;
-    const int64_t token_off = (static_cast<int64_t>(b) * p.N + static_cast<int64_t>(ty) * p.W + tx) * p.C + slice_off + chunk * 8;
+    const bool mine = tx < p.W && ty < p.H;
+    const int64_t token_off = (static_cast<int64_t>(b) * p.N + static_cast<int64_t>(ty) * p.W + tx) * p.C + head_off + chunk * 8;
     Accumulate<T> acc;
     acc.start(static_cast<const T *>(p.k) + (mine ? token_off : 0));
 
@@ -994,10 +1018,10 @@ __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
             const int i = e / (M / 2), k = e - i * (M / 2);
             copy16_async(coef_s + i * kCoefPitch + k * 16, reinterpret_cast<const char *>(g.coef + static_cast<int64_t>(slot_s[i]) * M) + k * 16);
         }
-        const int pieces = row_bytes / 16;
+        constexpr int pieces = row_bytes / 16;
         for (int e = tid; e < n * pieces; e += threads) {
             const int i = e / pieces, k = e - i * pieces;
-            const int64_t off = static_cast<int64_t>(meta_s[i].x) * p.C + slice_off;
+            const int64_t off = static_cast<int64_t>(b) * p.Nq * p.C + meta_s[i].x + head_off;
             copy16_async(q_s + i * row_bytes + k * 16, reinterpret_cast<const char *>(static_cast<const T *>(p.q) + off) + k * 16);
             copy16_async(go_s + i * row_bytes + k * 16, reinterpret_cast<const char *>(static_cast<const T *>(p.dout) + off) + k * 16);
         }
@@ -1011,8 +1035,7 @@ __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
                 for (int i = lo; i < hi; ++i) {
                     const float2 co = *reinterpret_cast<const float2 *>(coef_s + i * kCoefPitch + (j * SIDE + tx - meta_s[i].y) * 8);
                     Piece<T> piece;
-                    piece.load(reinterpret_cast<const T *>(q_s + i * row_bytes) + chunk * 8,
-                               reinterpret_cast<const T *>(go_s + i * row_bytes) + chunk * 8);
+                    piece.load_staged(q_s + i * row_bytes + chunk * 8 * sizeof(T), go_s + i * row_bytes + chunk * 8 * sizeof(T));
                     acc.add(piece, co.x, co.y);
                 }
             }
@@ -1026,55 +1049,60 @@ __global__ void __launch_bounds__(512) gather_sum_kernel(const GatherParams g)
 }
 
 // resident blocks of the kernel below per SM: as many as the registers of its chunks allow (0: no limit asked for)
-// (float16, 384x384 tokens, 8 heads x 16: 183 us with three, 173 with four; float32, r = 1: 126 with four, 79 with three)
+// (float16, 384x384 tokens, 8 heads x 16: 183 us with three, 173 with four; float32, r = 1: 126 with four, 79 with three;
+// float32, 2 x 45x79, 4 x 32, r = 2: 41 to 48 with three, 34 with two)
 template <typename T, int R, int CPT>
-constexpr int sum_min_blocks() { return CPT == 4 ? 0 : CPT == 2 ? 2 : sizeof(T) == 2 && R == 1 ? 4 : 3; }
+constexpr int sum_min_blocks() { return CPT == 4 ? 0 : CPT == 2 ? 2 : sizeof(T) == 2 && R == 1 ? 4 : sizeof(T) == 4 && R == 2 ? 2 : 3; }
 // blocks ahead whose coefficients a block asks L2 for (600: 173 us, 300: 171, 1000: 176)
 constexpr unsigned kPrefetchAhead = 300;
 
-// The same with shared centres: `lanes` lanes per token, each with CPT chunks of eight channels (chunk = lane + s * lanes),
-// `per_warp` tokens per warp.  A query's row of q and dout is read as a whole, a tap's coefficients of all heads lie
-// side by side, and the lanes of a token walk the same list.  The rows are shared by the tokens of a block through L1.
+// The same without staging: `lanes` lanes per token, each with CPT chunks of eight channels (chunk = lane + s * lanes),
+// `per_warp` tokens per warp; the lanes of a token walk the same list.  SHARED: one list for all heads, a query's row of
+// q and dout is read as a whole, a tap's coefficients of all heads lie side by side; otherwise one head.  The rows are
+// shared by the tokens of a block through L1.
 // The coefficients are read once and come from memory: every block has L2 fetch those of the buckets that a block some
 // way ahead starts with, whole runs of slots in one request each.
 // Bound by the latency of the loads (issue 59 % at three blocks per SM without the prefetch, and more lanes or items side
 // by side add their own start: 230 to 265 us).
-// Measured, same sizes: 171 us (209 without the prefetch at three blocks).
-template <typename T, int R, int CPT>
-__global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_shared_kernel(const GatherParams g)
+// Measured, float16, 384x384 tokens, 8 heads x 16, r = 1, shared: 171 us (209 without the prefetch at three blocks).  One
+// head: float16, 2 x 192x192, 4 x 64: 160 us (staged 190); float32, 2 x 45x79, 4 x 32, r = 2: 34 us (staged 38).
+template <typename T, int R, int CPT, bool SHARED>
+__global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_direct_kernel(const GatherParams g)
 {
     chain_begin();
     constexpr int SIDE = 2 * R + 2, M = SIDE * SIDE;
-    if (*g.differ != 0) return;
+    if ((*g.differ == 0) != SHARED) return;
     const BwdParams &p = g.b;
+    const SumTiles &tl = SHARED ? g.all_heads : g.one_head;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int sub = lane / g.lanes, own = lane - sub * g.lanes;
-    const int b = blockIdx.y, tile_rows = gridDim.x / g.shared_tiles_x;
-    const int order = blockIdx.x / g.shared_tiles_x, tile_x = blockIdx.x - order * g.shared_tiles_x;
-    if (blockIdx.x + kPrefetchAhead < gridDim.x && threadIdx.x < g.shared_y) {
-        const int then = blockIdx.x + kPrefetchAhead, then_row = then / g.shared_tiles_x;
-        const int cy = tile_row(then_row, tile_rows) * g.shared_y + threadIdx.x, cx = (then - then_row * g.shared_tiles_x) * g.shared_x;
+    const int sub = lane / tl.lanes, own = lane - sub * tl.lanes;
+    const int list = blockIdx.y, b = SHARED ? list : list / p.h, tile_rows = gridDim.x / tl.tiles_x;
+    const uint32_t coef_step = SHARED ? p.h : 1;         // heads whose coefficients of a tap lie side by side
+    const int order = blockIdx.x / tl.tiles_x, tile_x = blockIdx.x - order * tl.tiles_x;
+    if (blockIdx.x + kPrefetchAhead < gridDim.x && threadIdx.x < tl.y) {
+        const int then = blockIdx.x + kPrefetchAhead, then_row = then / tl.tiles_x;
+        const int cy = tile_row(then_row, tile_rows) * tl.y + threadIdx.x, cx = (then - then_row * tl.tiles_x) * tl.x;
         if (cy < g.cells_y && cx < g.cells_x) {
-            const int *start = g.starts + (static_cast<int64_t>(b) * g.cells_y + cy) * (g.cells_x + 1);
-            const int from = __ldg(start + cx), slots = __ldg(start + min(cx + g.shared_x, g.cells_x)) - from;
-            if (slots > 0) prefetch_l2(g.coef + static_cast<int64_t>(from) * M * p.h, slots, M * p.h * static_cast<uint32_t>(sizeof(float2)));
+            const int *start = g.starts + (static_cast<int64_t>(list) * g.cells_y + cy) * (g.cells_x + 1);
+            const int from = __ldg(start + cx), slots = __ldg(start + min(cx + tl.x, g.cells_x)) - from;
+            if (slots > 0) prefetch_l2(g.coef + static_cast<int64_t>(from) * M * coef_step, slots, M * coef_step * static_cast<uint32_t>(sizeof(float2)));
         }
     }
-    const int t = warp * g.per_warp + sub, ty_in = t / g.shared_x;
-    const int tx = tile_x * g.shared_x + t - ty_in * g.shared_x, ty = tile_row(order, tile_rows) * g.shared_y + ty_in;
-    if (sub >= g.per_warp || tx >= p.W || ty >= p.H) return;
+    const int t = warp * tl.per_warp + sub, ty_in = t / tl.x;
+    const int tx = tile_x * tl.x + t - ty_in * tl.x, ty = tile_row(order, tile_rows) * tl.y + ty_in;
+    if (sub >= tl.per_warp || tx >= p.W || ty >= p.H) return;
     const int hd8 = p.hd >> 3;
-    const int64_t token_off = (static_cast<int64_t>(b) * p.N + static_cast<int64_t>(ty) * p.W + tx) * p.C;
+    const int64_t token_off = (static_cast<int64_t>(b) * p.N + static_cast<int64_t>(ty) * p.W + tx) * p.C + (SHARED ? 0 : (list - b * p.h) * p.hd);
 
-    const int64_t query_off = static_cast<int64_t>(b) * p.Nq * p.C + own * 8;
+    const int64_t query_off = static_cast<int64_t>(b) * p.Nq * p.C + (SHARED ? 0 : (list - b * p.h) * p.hd) + own * 8;
     const T *q = static_cast<const T *>(p.q) + query_off, *go = static_cast<const T *>(p.dout) + query_off;
-    const int step = g.lanes * 8;                       // channels between the chunks of a lane
+    const int step = tl.lanes * 8;                       // channels between the chunks of a lane
     Accumulate<T> acc[CPT];
 #pragma unroll
     for (int s = 0; s < CPT; ++s) acc[s].start(static_cast<const T *>(p.k) + token_off + own * 8 + s * step);
     int head[CPT];
 #pragma unroll
-    for (int s = 0; s < CPT; ++s) head[s] = (own + s * g.lanes) / hd8;
+    for (int s = 0; s < CPT; ++s) head[s] = SHARED ? (own + s * tl.lanes) / hd8 : 0;
 
     // the token's items, one range of slots per row of buckets, numbered through: item f of row j lies in slot
     // base[j] + f
@@ -1085,7 +1113,7 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_s
 #pragma unroll
         for (int j = 0; j < SIDE; ++j) {
             const int cy = ty - j;
-            const int *start = g.starts + (static_cast<int64_t>(b) * g.cells_y + cy) * (g.cells_x + 1);
+            const int *start = g.starts + (static_cast<int64_t>(list) * g.cells_y + cy) * (g.cells_x + 1);
             const bool ok = cy >= 0 && cy < g.cells_y;
             lo[j] = ok ? __ldg(start + c_lo) : 0;
             hi[j] = ok ? __ldg(start + c_hi) : 0;
@@ -1109,7 +1137,9 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_s
         slot += f;
     };
     // two items at a time, so that their loads are under way together; their places are read one step ahead
-    uint32_t row[2] = {0u, 0u}, tap[2] = {0u, 0u};
+    using Tap = std::conditional_t<SHARED, uint32_t, uint64_t>;       // fewer than 2^31 (query, tap), or not
+    uint32_t row[2] = {0u, 0u};
+    Tap tap[2] = {0u, 0u};
     const auto fetch = [&](int f) {
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
@@ -1117,14 +1147,14 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_s
             locate(min(f + n, total - 1), slot, at);
             const int2 m = __ldg(g.meta + slot);
             row[n] = static_cast<uint32_t>(m.x);
-            tap[n] = static_cast<uint32_t>(at + m.y);
+            tap[n] = SHARED ? static_cast<Tap>(at + m.y) : static_cast<Tap>(slot) * M + static_cast<Tap>(at - m.y);
         }
     };
     if (total > 0) fetch(0);
     for (int f = 0; f < total; f += 2) {
         const bool second = f + 1 < total;
         const uint32_t r0 = row[0], r1 = row[1];
-        const float2 *c0 = g.coef + static_cast<uint64_t>(tap[0]) * static_cast<uint32_t>(p.h), *c1 = g.coef + static_cast<uint64_t>(tap[1]) * static_cast<uint32_t>(p.h);
+        const float2 *c0 = g.coef + static_cast<uint64_t>(tap[0]) * coef_step, *c1 = g.coef + static_cast<uint64_t>(tap[1]) * coef_step;
 #pragma unroll
         for (int s = 0; s < CPT; ++s) {
             Piece<T> first, other;
@@ -1147,8 +1177,10 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_s
 struct GatherPlan {
     size_t off_cursor, off_starts, off_rank, off_meta, off_coef, bytes;
     int64_t bucket_rows;
-    int cells_x, cells_y, lph, cpl, tile_x, tile_y, slice_chunks, slices, batch, threads, smem;
-    int cpt, lanes, per_warp, shared_x, shared_y;
+    int cells_x, cells_y, lph, cpl;
+    bool staged;
+    int batch, smem;
+    SumTiles all_heads, one_head;
 };
 
 GatherPlan gather_plan(int B, int H, int W, int h, int hd, int r, int dtype, int64_t Nq)
@@ -1172,39 +1204,34 @@ GatherPlan gather_plan(int B, int H, int W, int h, int hd, int r, int dtype, int
     }
     if (pl.lph > 32) return pl;
     if (pl.cpl > 3 && pl.cpl != 5) return pl;
-    // summing kernel: at most 64 channels per block, 16 x 8 tokens for narrow heads and 8 x 8 for wide ones
-    pl.slices = 1;
-    while (chunks % pl.slices != 0 || chunks / pl.slices > 8) {
-        if (++pl.slices > chunks) return pl;
-    }
-    pl.slice_chunks = chunks / pl.slices;
-    pl.tile_x = pl.slice_chunks <= 2 ? 16 : 8;
-    pl.tile_y = 8;
-    pl.threads = (pl.tile_x * pl.tile_y * pl.slice_chunks + 31) / 32 * 32;
-    const int per_item = M * 8 + 16 + 2 * pl.slice_chunks * 8 * esize + 12;
-    // room for one and a half items per bucket of the tile (one is the mean), at most 72 KB: three blocks per SM
-    const int cells = (pl.tile_x + side - 1) * (pl.tile_y + side - 1);
+    // staged sums: room for one and a half items per bucket of the tile (one is the mean), at most four blocks per SM
+    // (float16, 384x384 tokens, 8 heads x 16: 219 us, three 238), or the three that float32 has registers for
+    pl.staged = chunks == kStagedChunks;
+    const int per_item = M * 8 + 16 + 2 * kStagedChunks * 8 * esize + 12;
+    const int cells = (kStagedX + side - 1) * (kStagedY + side - 1), room = (esize == 2 ? 54 : 72) * 1024;
     pl.batch = cells * 3 / 2;
-    if (pl.batch * per_item > 72 * 1024) pl.batch = 72 * 1024 / per_item;
+    if (pl.batch * per_item > room) pl.batch = room / per_item;
     pl.batch &= ~3;
-    pl.smem = pl.batch * per_item + ((pl.tile_y + side - 1) * (pl.tile_x + side + 1) + 1) * 4;
-    // shared centres: one, two or four chunks per lane, whichever leaves the fewest lanes idle
-    const int row_chunks = chunks * h;
-    int best = 0;
-    for (int cpt = 1; cpt <= 4; cpt *= 2) {
-        if (row_chunks % cpt != 0 || row_chunks / cpt > 32) continue;
-        const int lanes = row_chunks / cpt, used = 32 / lanes * lanes;
-        if (used > best) {
-            best = used;
-            pl.cpt = cpt;
-            pl.lanes = lanes;
-            pl.per_warp = 32 / lanes;
+    pl.smem = pl.batch * per_item + ((kStagedY + side - 1) * (kStagedX + side + 1) + 1) * 4;
+    const auto split = [&](int row_chunks, SumTiles &tl) {     // one, two or four chunks per lane, whichever leaves the fewest lanes idle
+        int best = 0;
+        for (int cpt = 1; cpt <= 4; cpt *= 2) {
+            if (row_chunks % cpt != 0 || row_chunks / cpt > 32) continue;
+            const int lanes = row_chunks / cpt, used = 32 / lanes * lanes;
+            if (used > best) {
+                best = used;
+                tl.cpt = cpt;
+                tl.lanes = lanes;
+                tl.per_warp = 32 / lanes;
+            }
         }
-    }
-    if (best == 0) return pl;
-    const int tokens = 8 * pl.per_warp;
-    pl.shared_x = tokens >= 32 ? 8 : tokens >= 16 && tokens % 4 == 0 ? 4 : tokens % 3 == 0 ? 6 : 4;
-    pl.shared_y = tokens / pl.shared_x;
+        const int tokens = 8 * tl.per_warp;
+        tl.x = tokens >= 32 ? 8 : tokens >= 16 && tokens % 4 == 0 ? 4 : tokens % 3 == 0 ? 6 : 4;
+        tl.y = tokens / tl.x;
+        tl.tiles_x = (W + tl.x - 1) / tl.x;
+        return best != 0;
+    };
+    if (!split(chunks * h, pl.all_heads) || !split(chunks, pl.one_head)) return pl;
     const auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
     size_t off = static_cast<size_t>(pl.bucket_rows) * pl.cells_x * sizeof(int);    // counts and the two words are cleared together
     pl.off_cursor = off; off = up(off + 2 * sizeof(int));
@@ -1232,18 +1259,26 @@ cudaError_t launch_gather(const GatherParams &g, const GatherPlan &pl, cudaStrea
     case 3: launch_chained(gather_coef_kernel<T, R, 3>, coef_blocks, 128, 0, stream, g); break;
     default: launch_chained(gather_coef_kernel<T, R, 5>, coef_blocks, 128, 0, stream, g); break;
     }
-    if (pl.smem > 48 * 1024) {     // per-device attribute of the kernel: set on every launch (cheap, idempotent, thread-safe)
-        e = cudaFuncSetAttribute(gather_sum_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
-        if (e != cudaSuccess) return e;
+    const auto sums = [&](auto shared, const SumTiles &tl, int lists) {
+        constexpr bool SHARED = decltype(shared)::value;
+        const dim3 grid(static_cast<unsigned>(tl.tiles_x) * ((g.b.H + tl.y - 1) / tl.y), lists);
+        switch (tl.cpt) {
+        case 1: launch_chained(gather_sum_direct_kernel<T, R, 1, SHARED>, grid, 256, 0, stream, g); break;
+        case 2: launch_chained(gather_sum_direct_kernel<T, R, 2, SHARED>, grid, 256, 0, stream, g); break;
+        default: launch_chained(gather_sum_direct_kernel<T, R, 4, SHARED>, grid, 256, 0, stream, g); break;
+        }
+    };
+    if (pl.staged) {
+        if (pl.smem > 48 * 1024) {     // per-device attribute of the kernel: set on every launch (cheap, idempotent, thread-safe)
+            e = cudaFuncSetAttribute(gather_sum_staged_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
+            if (e != cudaSuccess) return e;
+        }
+        const unsigned tiles = static_cast<unsigned>((g.b.W + kStagedX - 1) / kStagedX) * ((g.b.H + kStagedY - 1) / kStagedY);
+        launch_chained(gather_sum_staged_kernel<T, R>, dim3(tiles, g.b.B * g.b.h), kStagedX * kStagedY * kStagedChunks, pl.smem, stream, g);
+    } else {
+        sums(std::false_type(), pl.one_head, g.b.B * g.b.h);
     }
-    const unsigned tiles = static_cast<unsigned>(g.tiles_x) * ((g.b.H + pl.tile_y - 1) / pl.tile_y);
-    launch_chained(gather_sum_kernel<T, R>, dim3(tiles, g.b.B * g.b.h, pl.slices), pl.threads, pl.smem, stream, g);
-    const dim3 shared_grid(static_cast<unsigned>(g.shared_tiles_x) * ((g.b.H + pl.shared_y - 1) / pl.shared_y), g.b.B);
-    switch (pl.cpt) {
-    case 1: launch_chained(gather_sum_shared_kernel<T, R, 1>, shared_grid, 256, 0, stream, g); break;
-    case 2: launch_chained(gather_sum_shared_kernel<T, R, 2>, shared_grid, 256, 0, stream, g); break;
-    default: launch_chained(gather_sum_shared_kernel<T, R, 4>, shared_grid, 256, 0, stream, g); break;
-    }
+    sums(std::true_type(), pl.all_heads, g.b.B);
     return cudaGetLastError();
 }
 
@@ -1353,14 +1388,12 @@ extern "C" int matchattn_fused_backward_ws(const void *max_offset, const void *q
     g.counts = reinterpret_cast<int *>(ws);
     g.cursor = reinterpret_cast<int *>(ws + pl.off_cursor);
     g.differ = g.cursor + 1;
-    g.lanes = pl.lanes; g.per_warp = pl.per_warp;
-    g.shared_x = pl.shared_x; g.shared_y = pl.shared_y; g.shared_tiles_x = (W + pl.shared_x - 1) / pl.shared_x;
+    g.all_heads = pl.all_heads; g.one_head = pl.one_head;
     g.starts = reinterpret_cast<int *>(ws + pl.off_starts);
     g.rank = reinterpret_cast<int *>(ws + pl.off_rank);
     g.meta = reinterpret_cast<int2 *>(ws + pl.off_meta);
     g.coef = reinterpret_cast<float2 *>(ws + pl.off_coef);
-    g.tile_x = pl.tile_x; g.tile_y = pl.tile_y; g.tiles_x = (W + pl.tile_x - 1) / pl.tile_x;
-    g.slice_chunks = pl.slice_chunks; g.batch = pl.batch;
+    g.batch = pl.batch;
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
     const auto run = [&](auto tag) {
         using T = decltype(tag);

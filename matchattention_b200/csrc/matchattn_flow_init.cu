@@ -122,6 +122,16 @@ template <typename T>
 struct Group {
     uint32_t w[kLaneCols / DT<T>::kElemsPerWord];
     __device__ __forceinline__ float get(int k) const { return DT<T>::unpack(w[k / DT<T>::kElemsPerWord], k % DT<T>::kElemsPerWord); }
+    // element k + x, the element converted in the addition
+    __device__ __forceinline__ float plus(int k, float x) const
+    {
+        if constexpr (sizeof(T) == 4) return __uint_as_float(w[k]) + x;
+        else {
+            const unsigned short h = static_cast<unsigned short>(k % 2 ? w[k / 2] >> 16 : w[k / 2] & 0xffffu);
+            if constexpr (std::is_same_v<T, __half>) return add_f32_f16(x, h);
+            else return add_f32_bf16(x, h);
+        }
+    }
     __device__ __forceinline__ void max_with(const Group &o)      // element by element
     {
 #pragma unroll
@@ -141,9 +151,9 @@ struct Group {
     }
 };
 
-__device__ __forceinline__ float to_float(float x) { return x; }
-__device__ __forceinline__ float to_float(__half x) { return __half2float(x); }
-__device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
+__device__ __forceinline__ float plus_float(float a, float x) { return a + x; }
+__device__ __forceinline__ float plus_float(__half a, float x) { return add_f32_f16(x, __half_as_ushort(a)); }
+__device__ __forceinline__ float plus_float(__nv_bfloat16 a, float x) { return add_f32_bf16(x, __bfloat16_as_ushort(a)); }
 
 template <typename T>
 __device__ __forceinline__ uint32_t raw_bits(const T *p)
@@ -285,7 +295,7 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T 
                         for (int i = 0; i < BATCH; ++i) next[i] = p[i * step];
                     }
 #pragma unroll
-                    for (int i = 0; i < BATCH; ++i) den += expf(to_float(now[i]) - mx);
+                    for (int i = 0; i < BATCH; ++i) den += expf(plus_float(now[i], -mx));
                     if (more) {
 #pragma unroll
                         for (int i = 0; i < BATCH; ++i) now[i] = next[i];
@@ -316,8 +326,8 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T 
             const Group<T> g0 = load_group<T, ALIGN, kWhole>(p, j, N, true), g1 = load_group<T, ALIGN, kWhole>(p, j + 4, N, true);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                s[k] += expf(g0.get(k) - mx);
-                s[k + 4] += expf(g1.get(k) - mx);
+                s[k] += expf(g0.plus(k, -mx));
+                s[k + 4] += expf(g1.plus(k, -mx));
             }
         }
 #pragma unroll
@@ -354,16 +364,17 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T 
 // (Markstein, IBM J. Res. Dev. 34, 1990): to the last bit as long as the residual does not underflow, which it does for
 // float32 quotients below 2^-102; there the last bit may differ.
 struct Softmax {
-    float max, sum, inv;
-    __device__ __forceinline__ float operator()(float x) const
+    float neg_max, sum, inv;
+    template <typename T>
+    __device__ __forceinline__ float operator()(const Group<T> &g, int k) const
     {
-        const float e = expf(x - max), q = e * inv;
+        const float e = expf(g.plus(k, neg_max)), q = e * inv;
         return fmaf(fmaf(-q, sum, e), inv, q);
     }
 };
 
 template <typename T>
-__device__ __forceinline__ Softmax softmax_of(float2 st) { return Softmax{st.x, st.y, __frcp_rn(st.y)}; }
+__device__ __forceinline__ Softmax softmax_of(float2 st) { return Softmax{-st.x, st.y, __frcp_rn(st.y)}; }
 
 // Sliding 5-sum down the rows of a pair of columns: push(p) returns p(a-4) + .. + p(a), from the pair sums it keeps.
 struct PairSums {
@@ -410,7 +421,7 @@ __device__ __forceinline__ void pool_rows(const PoolParams &pp, const T *src, T 
     for (int i = lane; i < pp.band_rows + 4; i += 32) {
         const int64_t a = a0 - 2 + i;
         const Softmax s = softmax_of<T>(FULL || (a >= 0 && a < N) ? __ldg(pp.stats + b * N + a) : make_float2(0.f, 1.f));
-        st[i] = make_float4(s.max, s.sum, s.inv, 0.f);
+        st[i] = make_float4(s.neg_max, s.sum, s.inv, 0.f);
     }
     __syncwarp();
     const bool inner = lane != 0 && lane != 31;
@@ -419,7 +430,7 @@ __device__ __forceinline__ void pool_rows(const PoolParams &pp, const T *src, T 
     hi.reset();
     // one row: probabilities, store, box sums of the row two above, their maximum over the warp
     const auto row_step = [&](const Group<T> &g, const Softmax &sm, int64_t a, bool store, bool pool) {
-        float2 p01 = make_float2(sm(g.get(0)), sm(g.get(1))), p23 = make_float2(sm(g.get(2)), sm(g.get(3)));
+        float2 p01 = make_float2(sm(g, 0), sm(g, 1)), p23 = make_float2(sm(g, 2), sm(g, 3));
         uint32_t w[kLaneCols / DT<T>::kElemsPerWord];
         if constexpr (sizeof(T) == 2) {
             w[0] = DT<T>::aw_from(p01.x, p01.y);
@@ -510,8 +521,8 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
         float2 p[2][2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            p[0][k] = make_float2(sm[2 * k](g0.get(2 * k)), sm[2 * k + 1](g0.get(2 * k + 1)));
-            p[1][k] = make_float2(sm[2 * k](g1.get(2 * k)), sm[2 * k + 1](g1.get(2 * k + 1)));
+            p[0][k] = make_float2(sm[2 * k](g0, 2 * k), sm[2 * k + 1](g0, 2 * k + 1));
+            p[1][k] = make_float2(sm[2 * k](g1, 2 * k), sm[2 * k + 1](g1, 2 * k + 1));
             if constexpr (sizeof(T) == 2) {
                 const uint32_t wx = DT<T>::aw_from(p[0][k].x, p[1][k].x), wy = DT<T>::aw_from(p[0][k].y, p[1][k].y);
                 w[2 * k][0] = wx;
