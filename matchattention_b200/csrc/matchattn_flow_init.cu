@@ -52,12 +52,22 @@ constexpr int kWindowTokens = kFlowWarps;             // tokens per block of the
 // 117.4 / 113.1 us, 68x72 145.9 / 148.3, 76x76 181.9 / 189.5, 128x128 1142 / 1231; odd: 67x71 208 / 186, 79x83 352 / 331,
 // 97x101 692 / 691; float32: 60x60 105.3 / 103.9, 68x72 167.9 / 173.0, 79x83 356 / 333.
 constexpr int64_t kLongBands = 5000, kLongBandsOdd = 10000;
-// Column sums: 32-column blocks with 16 (float32: 24) rows in flight from so many tokens on, 16-column blocks with 32 below,
-// where the wider ones leave SMs without work.  Measured, the whole call, wide against narrow, long bands: float16 72x72
-// tokens 168.1 / 156.6 us, 96x96 418.2 / 407.9, 96x100 433.3 / 445.5, 128x128 1069 / 1142; float32 72x72 192.7 / 185.8,
-// 76x80 239.9 / 246.2, 88x88 352.9 / 375.3.
+// Column sums: 32-column blocks from so many tokens on, 16-column blocks below, where the wider ones leave SMs without work.
+// Measured, the whole call, wide against narrow: float16 48x48 tokens 45.8 / 45.0 us, 64x64 103.6 / 102.4, 72x72 145.8 / 144.8,
+// 80x80 200.4 / 208.0, 96x96 365.2 / 387.6; float32 64x64 119.9 / 119.5, 76x76 206.3 / 201.8, 88x88 343.4 / 356.2.  Single
+// elements (strided): the narrow blocks read 32 rows ahead, the wide ones 16; float16 96x96 418.2 / 407.9, 96x100 433.3 / 445.5.
 template <typename T>
-constexpr int64_t kWideSums = sizeof(T) == 2 ? 9400 : 6000;
+constexpr int64_t kWideSums = sizeof(T) == 2 ? 5800 : 6600;
+constexpr int64_t kWideStrided = 9400;
+
+// Column sums of a block: batches of exponentials, two of them in shared memory.
+template <int COLUMNS>
+struct SumTile {
+    static constexpr int kPieces = COLUMNS / 8;                    // threads per row of a batch, eight columns each
+    static constexpr int kPasses = 2, kPassRows = kFlowThreads / kPieces, kRows = kPasses * kPassRows;
+    static constexpr int kPitch = COLUMNS + 4;                     // floats: keeps the 16-byte stores of neighbouring rows apart
+    static constexpr int kBytes = 2 * kRows * kPitch * static_cast<int>(sizeof(float));
+};
 
 // Sizes and scratch areas of one call, computed alike by the size query and the launcher.
 struct FlowPlan {
@@ -249,14 +259,153 @@ __global__ void __launch_bounds__(kFlowThreads) flow_max_kernel(const T *__restr
         if (col + k < N) col_part[(b * col_parts + band) * N + col + k] = cm.get(k);
 }
 
+// Maximum and sum of a row of corr by a warp: 256 partial sums (element j goes to sum j mod 256), then a tree over each 32
+// of them and a running sum over the eight results.
+template <typename T, int ALIGN>
+__device__ __forceinline__ void row_sum(const T *src, const float *row_part, float2 *stats, int64_t row, int64_t N, int row_parts)
+{
+    const int lane = threadIdx.x & 31;
+    if (row >= N) return;
+    float mx = -INFINITY;
+    for (int i = lane; i < row_parts; i += 32) mx = fmaxf(mx, row_part[i * N + row]);
+    mx = warp_max(mx);
+    const T *p = src + row * N;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float total = 0.f;
+    if constexpr (ALIGN >= 4) {     // lane l holds the partial sums 8 l .. 8 l + 7; elements past the end add exp(-inf)
+        constexpr bool kWhole = ALIGN >= 8;
+#pragma unroll 4
+        for (int64_t j = lane * 8; j < N; j += 256) {
+            const Group<T> g0 = load_group<T, ALIGN, kWhole>(p, j, N, true), g1 = load_group<T, ALIGN, kWhole>(p, j + 4, N, true);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s[k] += expf(g0.plus(k, -mx));
+                s[k + 4] += expf(g1.plus(k, -mx));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            s[k] += __shfl_xor_sync(0xffffffffu, s[k], 2);
+            s[k] += __shfl_xor_sync(0xffffffffu, s[k], 1);
+        }
+        const float sum = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+#pragma unroll
+        for (int w = 0; w < 8; ++w) total += __shfl_sync(0xffffffffu, sum, 4 * w);
+    } else {                  // lane l holds the partial sums l, l + 32, .. l + 224
+        int64_t j = lane;
+        for (; j + 224 < N; j += 256) {
+            float x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = load_one<T>(p + j + 32 * k);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s[k] += expf(x[k] - mx);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (j + 32 * k < N) s[k] += expf(load_one<T>(p + j + 32 * k) - mx);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+            total += s[k];
+        }
+    }
+    if (lane == 0) stats[row] = make_float2(mx, total);
+}
+
 // stats[half, b, token] = (maximum, sum of exp(x - maximum)) of row `token` of corr[b] (half 0) or of column `token`
-// (half 1).  The first blocks serve COLUMNS columns each, four threads per column, every fourth row per thread, BATCH
-// rows read ahead; the others serve one row per warp: 256 partial sums (element j goes to sum j mod 256), then a tree
-// over each 32 of them and a running sum over the eight results.
-// Bound by instruction issue on large maps (one exponential per element and half; the column blocks, few and long,
-// start first), on small ones by the latency of a column's chain of reads: narrower blocks with more rows in flight.
-template <typename T, int ALIGN, int COLUMNS, int BATCH>
-__global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T *__restrict__ corr, const float *__restrict__ row_part,
+// (half 1).  The first blocks serve COLUMNS columns each: all threads take the exponentials of a batch of rows into shared
+// memory, eight columns of a row at a time, then a thread per column and remainder of the row by four adds them up in order
+// while the others are at the next batch.  The other blocks serve one row per warp: 256 partial sums (element j goes to sum
+// j mod 256), then a tree over each 32 of them and a running sum over the eight results.
+// Bound by instruction issue (one exponential per element and half), on small maps by the chain of batches.  Measured, float16,
+// the sums alone: 96x96 tokens 106 -> 91 us, 128x128 259 -> 249, 82x79 81 -> 60; 48x48 14.4 -> 13.2 (a thread per column and
+// remainder that read, exponentiated and added one column, at 156 registers).
+template <typename T, int ALIGN, int COLUMNS>
+__global__ void __launch_bounds__(kFlowThreads, 4) flow_sum_kernel(const T *__restrict__ corr, const float *__restrict__ row_part,
+                                                                const float *__restrict__ col_part, float2 *__restrict__ stats,
+                                                                int64_t N, int row_parts, int col_parts, int col_blocks)
+{
+    chain_begin();
+    const int64_t b = blockIdx.y;
+    const T *src = corr + b * N * N;
+    if (static_cast<int>(blockIdx.x) < col_blocks) {
+        using Tile = SumTile<COLUMNS>;
+        extern __shared__ __align__(16) float e_s[];
+        __shared__ float part[kFlowThreads / COLUMNS][COLUMNS];
+        const int tid = threadIdx.x, c = tid % COLUMNS, g = tid / COLUMNS;
+        const int64_t c0 = static_cast<int64_t>(blockIdx.x) * COLUMNS, col = c0 + c;
+        float mx = -INFINITY;
+        if (col < N) {
+#pragma unroll 4
+            for (int i = g; i < col_parts; i += kFlowThreads / COLUMNS) mx = fmaxf(mx, __ldg(col_part + (b * col_parts + i) * N + col));
+        }
+        part[g][c] = mx;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kFlowThreads / COLUMNS; ++i) mx = fmaxf(mx, part[i][c]);
+        __syncthreads();
+        if (g == 0) part[0][c] = mx;
+        __syncthreads();
+        const int piece = tid % Tile::kPieces, first = tid / Tile::kPieces;        // eight columns, first row of a batch
+        float neg_max[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) neg_max[k] = -part[0][8 * piece + k];
+        const int64_t at = c0 + 8 * piece;
+        Group<T> raw[Tile::kPasses][2];
+        const auto load = [&](int64_t r0) {
+            const bool full = c0 + COLUMNS <= N && r0 + Tile::kRows <= N;
+#pragma unroll
+            for (int p = 0; p < Tile::kPasses; ++p) {
+                const int64_t row = r0 + first + p * Tile::kPassRows;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if (full) raw[p][i] = load_group<T, ALIGN, true>(src + row * N, at + 4 * i, N, true);
+                    else raw[p][i] = load_group<T, ALIGN, false>(src + row * N, at + 4 * i, N, row < N);
+                }
+            }
+        };
+        float den = 0.f;
+        load(0);
+        float *buffer = e_s;
+        for (int64_t r0 = 0; r0 < N; r0 += Tile::kRows) {
+#pragma unroll
+            for (int p = 0; p < Tile::kPasses; ++p) {
+                float *out = buffer + (first + p * Tile::kPassRows) * Tile::kPitch + 8 * piece;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const Group<T> &v = raw[p][i];
+                    *reinterpret_cast<float4 *>(out + 4 * i) = make_float4(expf(v.plus(0, neg_max[4 * i])), expf(v.plus(1, neg_max[4 * i + 1])),
+                                                                           expf(v.plus(2, neg_max[4 * i + 2])), expf(v.plus(3, neg_max[4 * i + 3])));
+                }
+            }
+            if (r0 + Tile::kRows < N) load(r0 + Tile::kRows);
+            __syncthreads();
+            if (g < kSumGroups) {
+                const float *in = buffer + g * Tile::kPitch + c;
+                if (r0 + Tile::kRows <= N) {
+#pragma unroll 16
+                    for (int r = 0; r < Tile::kRows; r += kSumGroups) den += in[r * Tile::kPitch];
+                } else {
+                    for (int r = 0; r0 + g + r < N; r += kSumGroups) den += in[r * Tile::kPitch];
+                }
+            }
+            buffer = buffer == e_s ? e_s + Tile::kRows * Tile::kPitch : e_s;      // the barrier of the next batch guards this one
+        }
+        if (g < kSumGroups) part[g][c] = den;
+        __syncthreads();
+        if (g == 0 && col < N)
+            stats[(gridDim.y + b) * N + col] = make_float2(mx, (part[0][c] + part[1][c]) + (part[2][c] + part[3][c]));
+        return;
+    }
+    row_sum<T, ALIGN>(src, row_part + b * row_parts * N, stats + b * N, (static_cast<int64_t>(blockIdx.x) - col_blocks) * kFlowWarps + (threadIdx.x >> 5), N, row_parts);
+}
+
+// The same where rows of 16-bit elements are aligned to single elements only: a thread per column and remainder of the row by
+// four reads, exponentiates and adds, BATCH rows ahead.  Measured, float16, the sums alone, this / the one above: 67x71 tokens
+// 40 / 55 us, 79x83 85 / 89, 97x101 141 / 166, bfloat16 111x113 204 / 240.
+template <typename T, int COLUMNS, int BATCH>
+__global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_strided_kernel(const T *__restrict__ corr, const float *__restrict__ row_part,
                                                                 const float *__restrict__ col_part, float2 *__restrict__ stats,
                                                                 int64_t N, int row_parts, int col_parts, int col_blocks)
 {
@@ -310,54 +459,8 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_kernel(const T 
             stats[(gridDim.y + b) * N + col] = make_float2(mx, (sm[0][c] + sm[1][c]) + (sm[2][c] + sm[3][c]));
         return;
     }
-    const int lane = threadIdx.x & 31;
-    const int64_t row = static_cast<int64_t>(blockIdx.x - col_blocks) * (COLUMNS * kSumGroups / 32) + (threadIdx.x >> 5);
-    if (row >= N) return;
-    float mx = -INFINITY;
-    for (int i = lane; i < row_parts; i += 32) mx = fmaxf(mx, row_part[(b * row_parts + i) * N + row]);
-    mx = warp_max(mx);
-    const T *p = src + row * N;
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float total = 0.f;
-    if constexpr (ALIGN >= 4) {     // lane l holds the partial sums 8 l .. 8 l + 7; elements past the end add exp(-inf)
-        constexpr bool kWhole = ALIGN >= 8;
-#pragma unroll 4
-        for (int64_t j = lane * 8; j < N; j += 256) {
-            const Group<T> g0 = load_group<T, ALIGN, kWhole>(p, j, N, true), g1 = load_group<T, ALIGN, kWhole>(p, j + 4, N, true);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                s[k] += expf(g0.plus(k, -mx));
-                s[k + 4] += expf(g1.plus(k, -mx));
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            s[k] += __shfl_xor_sync(0xffffffffu, s[k], 2);
-            s[k] += __shfl_xor_sync(0xffffffffu, s[k], 1);
-        }
-        const float sum = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
-#pragma unroll
-        for (int w = 0; w < 8; ++w) total += __shfl_sync(0xffffffffu, sum, 4 * w);
-    } else {                  // lane l holds the partial sums l, l + 32, .. l + 224
-        int64_t j = lane;
-        for (; j + 224 < N; j += 256) {
-            float x[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = load_one<T>(p + j + 32 * k);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) s[k] += expf(x[k] - mx);
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (j + 32 * k < N) s[k] += expf(load_one<T>(p + j + 32 * k) - mx);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-            total += s[k];
-        }
-    }
-    if (lane == 0) stats[b * N + row] = make_float2(mx, total);
+    row_sum<T, 1>(src, row_part + b * row_parts * N, stats + b * N,
+                  (static_cast<int64_t>(blockIdx.x) - col_blocks) * (COLUMNS * kSumGroups / 32) + (threadIdx.x >> 5), N, row_parts);
 }
 
 // Softmax of an element: the quotient exp(x - max) / sum by one Newton step on the product with the rounded reciprocal
@@ -820,14 +923,18 @@ cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow
     const int64_t units = static_cast<int64_t>(pl.row_parts) * pl.col_parts;
     launch_chained(flow_max_kernel<T, ALIGN>, dim3(static_cast<unsigned>((units + kFlowWarps - 1) / kFlowWarps), B), kFlowThreads, 0, stream, 
         corr, row_part, col_part, N, pl.max_rows, pl.row_parts, pl.col_parts);
-    const auto launch_sums = [&](auto columns, auto batch) {
-        constexpr int kColumns = decltype(columns)::value, kThreadsHere = kColumns * kSumGroups, kRows = kThreadsHere / 32;
-        const int col_blocks = static_cast<int>((N + kColumns - 1) / kColumns);
-        launch_chained(flow_sum_kernel<T, ALIGN, kColumns, decltype(batch)::value>, dim3(static_cast<unsigned>(col_blocks + (N + kRows - 1) / kRows), B), kThreadsHere, 0, stream, 
-                corr, row_part, col_part, stats, N, pl.row_parts, pl.col_parts, col_blocks);
+    const auto launch_sums = [&](auto kernel, int columns, int threads, int bytes) {
+        const int col_blocks = static_cast<int>((N + columns - 1) / columns), rows = threads / 32;
+        launch_chained(kernel, dim3(static_cast<unsigned>(col_blocks + (N + rows - 1) / rows), B), threads, bytes, stream, corr, row_part, col_part, stats, N,
+                       pl.row_parts, pl.col_parts, col_blocks);
     };
-    if (N >= kWideSums<T>) launch_sums(std::integral_constant<int, 32>(), std::integral_constant<int, sizeof(T) == 2 ? 16 : 24>());
-    else launch_sums(std::integral_constant<int, 16>(), std::integral_constant<int, 32>());
+    if constexpr (ALIGN == 1 && sizeof(T) == 2) {
+        if (N >= kWideStrided) launch_sums(flow_sum_strided_kernel<T, 32, 16>, 32, 32 * kSumGroups, 0);
+        else launch_sums(flow_sum_strided_kernel<T, 16, 32>, 16, 16 * kSumGroups, 0);
+    } else {
+        if (N >= kWideSums<T>) launch_sums(flow_sum_kernel<T, ALIGN, 32>, 32, kFlowThreads, SumTile<32>::kBytes);
+        else launch_sums(flow_sum_kernel<T, ALIGN, 16>, 16, kFlowThreads, SumTile<16>::kBytes);
+    }
     constexpr int smem = kPoolWarps * kPoolSmemPerWarp;
     const cudaError_t e = cudaFuncSetAttribute(flow_prob_pool_kernel<T, ALIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
