@@ -18,9 +18,9 @@
 // prob and the deciding averages are formed in one fixed order (sums of exponentials in 256 interleaved partial sums
 // per row and four per column, box sums row by row) whatever the split of the work, and only the screening in step 3
 // adds in another.
-// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.03 ms = 0.09 + 0.26 +
-// 0.63 + 0.05; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
-// the pooling took 4.1.  48x48 tokens: 47 us, before 196.
+// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 0.99 ms = 0.09 + 0.25 +
+// 0.61 + 0.05; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
+// the pooling took 4.1.  48x48 tokens: 44 us, before 196.
 // Rounding of the 16-bit types as eager PyTorch on the GPU: softmax, pooling and sums accumulate in float32
 // and round once, every elementwise op rounds.
 #include "../../include/matchattn.h"
@@ -468,13 +468,15 @@ __global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_strided_kernel(
 // float32 quotients below 2^-102; there the last bit may differ.
 struct Softmax {
     float neg_max, sum, inv;
-    template <typename T>
-    __device__ __forceinline__ float operator()(const Group<T> &g, int k) const
-    {
-        const float e = expf(g.plus(k, neg_max)), q = e * inv;
-        return fmaf(fmaf(-q, sum, e), inv, q);
-    }
 };
+// Elements k and k + 1, each by its own statistics, in packed arithmetic (the pooling kernel at 128x128 tokens 621 -> 615 us).
+template <typename T>
+__device__ __forceinline__ float2 softmax_pair(const Group<T> &g, int k, const Softmax &a, const Softmax &b)
+{
+    const float2 e = make_float2(expf(g.plus(k, a.neg_max)), expf(g.plus(k + 1, b.neg_max))), inv = make_float2(a.inv, b.inv);
+    const float2 q = mul_f32x2(e, inv);
+    return fma_f32x2(fma_f32x2(q, make_float2(-a.sum, -b.sum), e), inv, q);
+}
 
 template <typename T>
 __device__ __forceinline__ Softmax softmax_of(float2 st) { return Softmax{-st.x, st.y, __frcp_rn(st.y)}; }
@@ -533,7 +535,7 @@ __device__ __forceinline__ void pool_rows(const PoolParams &pp, const T *src, T 
     hi.reset();
     // one row: probabilities, store, box sums of the row two above, their maximum over the warp
     const auto row_step = [&](const Group<T> &g, const Softmax &sm, int64_t a, bool store, bool pool) {
-        float2 p01 = make_float2(sm(g, 0), sm(g, 1)), p23 = make_float2(sm(g, 2), sm(g, 3));
+        float2 p01 = softmax_pair(g, 0, sm, sm), p23 = softmax_pair(g, 2, sm, sm);
         uint32_t w[kLaneCols / DT<T>::kElemsPerWord];
         if constexpr (sizeof(T) == 2) {
             w[0] = DT<T>::aw_from(p01.x, p01.y);
@@ -624,8 +626,8 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
         float2 p[2][2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            p[0][k] = make_float2(sm[2 * k](g0, 2 * k), sm[2 * k + 1](g0, 2 * k + 1));
-            p[1][k] = make_float2(sm[2 * k](g1, 2 * k), sm[2 * k + 1](g1, 2 * k + 1));
+            p[0][k] = softmax_pair(g0, 2 * k, sm[2 * k], sm[2 * k + 1]);
+            p[1][k] = softmax_pair(g1, 2 * k, sm[2 * k], sm[2 * k + 1]);
             if constexpr (sizeof(T) == 2) {
                 const uint32_t wx = DT<T>::aw_from(p[0][k].x, p[1][k].x), wy = DT<T>::aw_from(p[0][k].y, p[1][k].y);
                 w[2 * k][0] = wx;
@@ -728,7 +730,7 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
 // them as 16 bytes of a prob row, or, where rows of prob are not 16-byte aligned, through shared memory.
 // Eight consecutive blocks (four of either role) cover one 4-band x 4-chunk region, so the second role finds corr in L2.
 // Bound by instruction issue (about 25 per element and role, a third of them the exponential; 81 % of the slots busy).
-// Measured, float16, 16384 x 16384: 0.63 ms (0.72 with eight rows unrolled and the halo rows apart: the instruction cache
+// Measured, float16, 16384 x 16384: 0.61 ms (0.72 with eight rows unrolled and the halo rows apart: the instruction cache
 // ran short, 2.2 of 8 stalls).  With 16-byte stores straight from the registers to 32 rows of prob the
 // second role alone took 0.67 ms; five blocks of four warps hold 20 warps per SM (0.75 ms with four blocks).
 template <typename T, int ALIGN>
