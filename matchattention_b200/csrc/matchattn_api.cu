@@ -319,8 +319,12 @@ int run(Params &p, const Plan &pl, int r, int tile_w_request, cudaStream_t strea
             blocks = 1LL * p.tiles_x * tiles_y;
             // A launch too small to give every SM two blocks is bound by the latency of one warp's
             // chain of taps: narrower blocks (the kernels only bound their size from above) spread
-            // the same queries over more SMs.
-            if (threads <= 64 || threads / 2 < p.G || blocks * p.B >= fill) break;
+            // the same queries over more SMs.  With 4 x 4 windows blocks of half the size already pay below ten
+            // per SM: an SM holds three of the large ones, and a last round of few costs as much as a full one (104x208
+            // tokens, 8 heads x 16, float32 23.2 -> 22.2 us, two maps in float16 24.4 -> 22.9; at 24 per SM smooth centres
+            // lose up to 11 % of the taps' reuse, at two all of this).  6 x 6 windows share more taps within a block and keep
+            // the large ones (96x96 tokens, a layer: 44.4 us, with half of them 47.1).
+            if (threads <= 64 || threads / 2 < p.G || blocks * p.B >= (r == 1 && threads == kThreads ? 5 * fill : fill)) break;
             threads /= 2;
         }
         unsigned grid_y = p.B;
