@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) consistency_mask_kernel(const T *__restri
 // The disparities of a pixel are split over kDispGroups threads (a warp = 32 neighbouring pixels, one share of the
 // disparities each), which read their share eight values at a time; the shares' maxima meet in shared memory.
 // Latency-bound: one thread per pixel walked its column of D dependent reads on a quarter of the warps an SM can hold.
-// Measured, float16, 2 x 120 x 68 x 120: 5.2 us, before 41.4.
+// Measured, float16, 2 x 120 x 68 x 120: 5.2 us, before 41.4; 8 x 159 x 128 x 159: 31.0, with a bounds check per read 38.4.
 constexpr int kDispGroups = 8, kDispBatch = 8;
 
 // x / 5: 1/5 as the sum of two floats of one sign, so that an infinite x stays infinite (multiplication by a constant of
@@ -84,19 +84,25 @@ __global__ void __launch_bounds__(32 * kDispGroups) local_disparity_kernel(const
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int64_t px = static_cast<int64_t>(blockIdx.x) * 32 + lane;
     const int b = blockIdx.y;
-    const T *col = cv + static_cast<int64_t>(b) * D * plane + px;      // this pixel's D values, `plane` apart
     const bool inside = px < plane;
-    const auto at = [&](int d) { return inside && d >= 0 && d < D ? load_one<T>(col + d * plane) : 0.f; };
+    const T *col = cv + static_cast<int64_t>(b) * D * plane + (inside ? px : plane - 1);      // this pixel's D values, `plane` apart
 
     // 5-tap box average over D (zero padded, divided by 5), first arg max of this share
     const int share = (D + kDispGroups - 1) / kDispGroups, first = g * share, last = min(first + share, D);
+    const auto at = [&](int d) { return d >= 0 && d < D ? load_one<T>(col + d * plane) : 0.f; };
     float best = -INFINITY;
     int arg = first;
     float w0 = at(first - 2), w1 = at(first - 1), w2 = at(first), w3 = at(first + 1);
-    for (int d0 = first; d0 < last; d0 += kDispBatch) {
+    const T *ahead = col + (first + 2) * plane;
+    for (int d0 = first; d0 < last; d0 += kDispBatch, ahead += kDispBatch * plane) {
         float next[kDispBatch];
+        if (d0 + kDispBatch + 2 <= D) {
 #pragma unroll
-        for (int i = 0; i < kDispBatch; ++i) next[i] = at(d0 + i + 2);
+            for (int i = 0; i < kDispBatch; ++i) next[i] = load_one<T>(ahead + i * plane);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kDispBatch; ++i) next[i] = d0 + i + 2 < D ? load_one<T>(ahead + i * plane) : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < kDispBatch; ++i) {
             // the sum runs over the taps in ascending order, as the pooling kernel adds them (those outside [0, D) are 0)

@@ -9,13 +9,13 @@
 //
 // The reference builds this with two Python loops over the W disparities (2 x W slice assignments,
 // W more for the fill: about 300 tiny launches at W = 48) around a softmax.  Here one block owns one
-// (view, batch item, row) and keeps the row's W x W correlation slice in shared memory.  Every pair (d, w) in view is
-// one element of the slice, the pairs out of view all score 0 and are never written (the fill replaces them), so the
-// exponentials are taken in place: maxima by a warp per column, exponentials by all threads over the triangle in
-// view, sums by a thread per column (in the order of d), then the W rows of W outputs, coalesced along w.
-// HBM traffic: corr once per view, vol once.  Latency-bound (136 blocks at 68 x 120): everything but the W additions
-// of a column's sum is spread over the whole block.  Measured, float16, 68 x 120: 8.8 us; one thread per column for
-// all three steps took 29.5 us.
+// (view, batch item, row) and keeps the row's scores in shared memory, column by column of vol: scores[w][d], as either
+// view sees them.  A warp takes the maximum and the exponentials of a column (the pairs out of view score 0), a thread
+// their sum in the order of d, then the W rows of W outputs leave coalesced along w.
+// HBM traffic: corr once per view, vol once.  Latency-bound (136 blocks at 68 x 120): three steps between barriers, every
+// load of a warp under way at once, everything but the W additions of a column's sum spread over the whole block.
+// Measured, float16, 68 x 120: 6.6 us (the maxima, the exponentials and their places in five steps 9.0; one thread per
+// column for all of it 29.5); 8 x 159 x 128 x 159 63.8 -> 51.1.
 #include "../../include/matchattn.h"
 
 #include <stdint.h>
@@ -29,113 +29,121 @@ namespace {
 
 constexpr int kVolumeMaxW = 159;
 
-// pitch of the slice in shared memory: P + 1 odd (columns walk the diagonals of the slice), P = 2 mod 4 (and its columns)
-__host__ __device__ constexpr int volume_pitch(int W) { return (W + 3) / 4 * 4 + 2; }
+// pitch of a column of scores in shared memory: odd (a row of vol walks the columns), P - 1 = 2 mod 4 (the right view's scores
+// of a row of corr arrive on a diagonal)
+__host__ __device__ constexpr int volume_pitch(int W) { return W / 4 * 4 + 3; }
 
-// PIECES: W / 32 rounded up (a warp takes a row of the slice, or a column of vol, in that many pieces at once)
-template <typename T, int PIECES>
-__global__ void __launch_bounds__(1024) stereo_volume_kernel(const T *__restrict__ corr, T *__restrict__ vol, int B, int H, int W)
+// maximum over a warp in one instruction (PTX ISA 8.6, sm_100a)
+__device__ __forceinline__ float warp_max(float v)
+{
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// PIECES: W / 32 rounded up (a warp takes a row of corr, a column or a row of vol in that many pieces at once)
+// WARPS: of a block, ROWS: W / WARPS rounded up, rows or columns per warp
+template <typename T, int PIECES, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 2) stereo_volume_kernel(const T *__restrict__ corr, T *__restrict__ vol, int B, int H, int W)
 {
     chain_begin();
-    extern __shared__ float slice[];              // [W][P]: corr[w][j], then exp(corr - maximum of its column of vol)
+    constexpr int ROWS = (32 * PIECES + WARPS - 1) / WARPS;
+    extern __shared__ float scores[];             // [W][P]: scores[w][d], then exp(score - maximum of its column)
     const int P = volume_pitch(W);
-    float *top = slice + W * P, *inv = top + W;   // per column w: maximum, reciprocal of the sum
-    const int h = blockIdx.x, b2 = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    float *inv = scores + W * P;                  // per column: reciprocal of the sum
+    const int h = blockIdx.x, b2 = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool right = b2 >= B;
     const int b = right ? b2 - B : b2;
     const T *src = corr + (static_cast<int64_t>(b) * H + h) * W * W;
-    // element (w, j) of the slice: the left view sees it at column w, disparity w - j, the right one at column j
-    for (int r0 = warp; r0 < W; r0 += 2 * warps) {        // two rows of a warp in flight
-        float x[2][PIECES];
+    // element (r, j) of the row's correlation, j <= r: disparity r - j at column r of the left view, column j of the right one
+    float x[ROWS][PIECES];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-            for (int k = 0; k < PIECES; ++k) {
-                const int r = r0 + i * warps, j = lane + 32 * k;
-                x[i][k] = r < W && j <= r ? load_one<T>(src + r * W + j) : 0.f;
-            }
+        for (int k = 0; k < PIECES; ++k) {
+            const int r = warp + i * WARPS, j = lane + 32 * k;
+            if (r < W && j <= r) x[i][k] = load_one<T>(src + r * W + j);
+        }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-            for (int k = 0; k < PIECES; ++k) {
-                const int r = r0 + i * warps, j = lane + 32 * k;
-                if (r < W && j <= r) slice[r * P + j] = x[i][k];
-            }
-    }
+        for (int k = 0; k < PIECES; ++k) {
+            const int r = warp + i * WARPS, j = lane + 32 * k;
+            if (r < W && j <= r) scores[(right ? j : r) * P + r - j] = x[i][k];
+        }
     __syncthreads();
-    for (int w = warp; w < W; w += warps) {
-        const int seen = right ? W - w : w + 1;   // disparities in view
-        float m = seen < W ? 0.f : -INFINITY;     // those out of view score 0
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int w = warp + i * WARPS;
+        if (w >= W) break;
+        const int seen = right ? W - w : w + 1;   // disparities in view; the others score 0
+        float *column = scores + w * P + lane;
+        float m = seen < W ? 0.f : -INFINITY;
 #pragma unroll
         for (int k = 0; k < PIECES; ++k) {
             const int d = lane + 32 * k;
-            if (d < seen) m = fmaxf(m, right ? slice[(w + d) * P + w] : slice[w * P + w - d]);
+            x[i][k] = d < seen ? column[32 * k] : 0.f;
+            if (d < seen) m = fmaxf(m, x[i][k]);
         }
+        m = warp_max(m);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) top[w] = m;
+        for (int k = 0; k < PIECES; ++k)
+            if (lane + 32 * k < W) column[32 * k] = expf(x[i][k] - m);
     }
     __syncthreads();
-    for (int r = warp; r < W; r += warps) {
-        float x[PIECES];
-#pragma unroll
-        for (int k = 0; k < PIECES; ++k) {
-            const int j = lane + 32 * k;
-            x[k] = j <= r ? slice[r * P + j] - top[right ? j : r] : 0.f;
-        }
-#pragma unroll
-        for (int k = 0; k < PIECES; ++k) {
-            const int j = lane + 32 * k;
-            if (j <= r) slice[r * P + j] = expf(x[k]);
-        }
-    }
-    __syncthreads();
-    for (int w = tid; w < W; w += blockDim.x) {
-        const int seen = right ? W - w : w + 1;
-        const float *p = slice + w * P + w;
-        const int step = right ? P : -1;
+    for (int w = tid; w < W; w += 32 * WARPS) {
+        const float *column = scores + w * P;
         float den = 0.f;
-#pragma unroll 8
-        for (int d = 0; d < seen; ++d) den += p[d * step];
-        const float none = expf(0.f - top[w]);
-#pragma unroll 8
-        for (int d = seen; d < W; ++d) den += none;
+        int d = 0;
+        for (; d + 8 <= W; d += 8) {
+            float e[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) e[k] = column[d + k];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) den += e[k];
+        }
+        for (; d < W; ++d) den += column[d];
         inv[w] = __frcp_rn(den);
     }
     __syncthreads();
     T *dst = vol + (static_cast<int64_t>(b2) * W * H + h) * W;
-    for (int d = warp; d < W; d += warps)
+    const int64_t step = static_cast<int64_t>(H) * W;
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int d = warp + i * WARPS;
+        if (d >= W) break;
 #pragma unroll
         for (int k = 0; k < PIECES; ++k) {
             const int w = lane + 32 * k;
             if (w >= W) break;
             const int from = right ? min(w, W - 1 - d) : max(w, d);       // the fill: columns out of view repeat the last one in view
-            const float e = right ? slice[(from + d) * P + from] : slice[from * P + from - d];
-            store_one<T>(dst + static_cast<int64_t>(d) * H * W + w, e * inv[from]);
+            store_one<T>(dst + d * step + w, scores[from * P + d] * inv[from]);
         }
+    }
 }
 
 template <typename T>
 cudaError_t launch(const void *corr, void *vol, int B, int H, int W, cudaStream_t stream)
 {
-    const int smem = static_cast<int>(sizeof(float)) * (W * volume_pitch(W) + 2 * W);
-    const auto go = [&](auto pieces) {
-        constexpr int kPieces = decltype(pieces)::value;
+    const int smem = static_cast<int>(sizeof(float)) * (W * volume_pitch(W) + W);
+    const auto go = [&](auto pieces, auto warps) {
+        const auto kernel = stereo_volume_kernel<T, decltype(pieces)::value, decltype(warps)::value>;
         if (smem > 48 * 1024) {     // per-device attribute of the kernel: set on every launch (cheap, idempotent, thread-safe)
-            const cudaError_t e = cudaFuncSetAttribute(stereo_volume_kernel<T, kPieces>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
         }
-        // as many warps as there are rows to share out, within what two blocks per SM can hold
-        const int threads = W > 64 ? 1024 : 512;
-        launch_chained(stereo_volume_kernel<T, kPieces>, dim3(H, 2 * B), threads, smem, stream, static_cast<const T *>(corr), static_cast<T *>(vol), B, H, W);
+        launch_chained(kernel, dim3(H, 2 * B), 32 * decltype(warps)::value, smem, stream, static_cast<const T *>(corr), static_cast<T *>(vol), B, H, W);
         return cudaGetLastError();
     };
+    // as many warps as there are rows to share out, within what two blocks per SM can hold
+    using Few = std::integral_constant<int, 16>;
+    using Many = std::integral_constant<int, 32>;
     switch ((W + 31) / 32) {
-    case 1: return go(std::integral_constant<int, 1>());
-    case 2: return go(std::integral_constant<int, 2>());
-    case 3: return go(std::integral_constant<int, 3>());
-    case 4: return go(std::integral_constant<int, 4>());
-    default: return go(std::integral_constant<int, 5>());
+    case 1: return go(std::integral_constant<int, 1>(), Few());
+    case 2: return go(std::integral_constant<int, 2>(), Few());
+    case 3: return go(std::integral_constant<int, 3>(), Many());
+    case 4: return go(std::integral_constant<int, 4>(), Many());
+    default: return go(std::integral_constant<int, 5>(), Many());
     }
 }
 
