@@ -178,9 +178,12 @@ __device__ __forceinline__ float add_f32_f16(float acc, unsigned short h)
     return acc;
 }
 
+// The same for bfloat16, as 1 * addend + accumulator: the product is exact, so it is the sum rounded once.  The mixed addition
+// itself takes the integer pipe as well (63 % busy in the forward, two lanes per head): r = 2, 2 x 160x160 tokens, 4 heads x
+// 32, 68.5 -> 60.9 us; 187x313, 4 x 64 142.8 -> 136.9.  In float16 the addition is the faster one (295 us, 305 as a product).
 __device__ __forceinline__ float add_f32_bf16(float acc, unsigned short h)
 {
-    asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(acc) : "h"(h));
+    asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(acc) : "h"(h), "h"(static_cast<unsigned short>(0x3f80)));
     return acc;
 }
 
@@ -368,11 +371,9 @@ struct DT<__nv_bfloat16> {
     }
     static __device__ __forceinline__ void absdiff(float &a0, float &a1, uint32_t qw, uint32_t kw)
     {
-        const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&qw),
-                                         *reinterpret_cast<const __nv_bfloat162 *>(&kw));
-        const uint32_t u = *reinterpret_cast<const uint32_t *>(&d) & 0x7fff7fffu;
-        a0 = add_f32_bf16(a0, static_cast<unsigned short>(u & 0xffffu));
-        a1 = add_f32_bf16(a1, static_cast<unsigned short>(u >> 16));
+        const __nv_bfloat162 d = __habs2(__hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&qw), *reinterpret_cast<const __nv_bfloat162 *>(&kw)));
+        a0 = add_f32_bf16(a0, __bfloat16_as_ushort(__low2bfloat16(d)));
+        a1 = add_f32_bf16(a1, __bfloat16_as_ushort(__high2bfloat16(d)));
     }
     using Bcast = __nv_bfloat162;
     static __device__ __forceinline__ Bcast bcast(__nv_bfloat16 a) { return __bfloat162bfloat162(a); }
