@@ -129,26 +129,29 @@ __device__ __forceinline__ __nv_bfloat162 pair_max(__nv_bfloat162 a, __nv_bfloat
 template <typename P>
 __device__ __forceinline__ uint32_t pair_word(P p) { return *reinterpret_cast<const uint32_t *>(&p); }
 
+constexpr int kPairRows = 2;
+
 // 16-bit types, two-component fields (the model's), factors 2 and 4, any width.  A thread owns two cells of a row and
-// ONE fine row i and takes them through everything in pairs: a weight word holds both cells' weights, multiplied by the
+// kPairRows fine rows, one after the other, and takes them through everything in pairs: a weight word holds both cells' weights, multiplied by the
 // pair of their neighbours' components, packed float32 arithmetic in between.  EVEN: the two cells are neighbours and a
 // mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous.  A cell's F fine cells are one aligned store of 8 or 16 bytes.
-// Bound by instruction issue.  Measured, float16: 2 x 384x384 by 4: 33 -> 28 us (four cells and five
-// blocks per SM before); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
+// Bound by instruction issue (70 %; integer pipe 55 %).  Measured, float16: 2 x 384x384 by 4: 33 -> 27.9 us (four cells and
+// five blocks per SM before; one fine row per thread 28.5, two without the limit of 64 registers 54); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
 // fine rows per thread) -> 17.7.
 template <typename T, int F, bool EVEN>
-__global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
+__global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
                                                             int B, int H, int W, int segments)
 {
     chain_begin();
+    constexpr int G = F / kPairRows;               // threads' shares of a cell
     constexpr int COLS = EVEN ? 4 : 6;             // columns of neighbours: -1 .. 2 around the pair, or -1 .. 1 around either
     const int lane = threadIdx.x & 31;
     const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5);
-    const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, fine row
+    const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, pair of fine rows
     const int w0 = static_cast<int>(warp - line * segments) * 64 + (EVEN ? 2 * lane : lane);
-    const uint32_t b = line / static_cast<uint32_t>(H * F);
+    const uint32_t b = line / static_cast<uint32_t>(H * G);
     if (b >= static_cast<uint32_t>(B) || w0 >= W) return;
-    const int hi = static_cast<int>(line - b * (H * F)), h = hi / F, i = hi - h * F;
+    const int hi = static_cast<int>(line - b * (H * G)), h = hi / G, i0 = (hi - h * G) * kPairRows;
     const int w1 = EVEN ? w0 + 1 : min(w0 + 32, W - 1);
     const bool second = EVEN || w0 + 32 < W;
     const int64_t plane = static_cast<int64_t>(H) * W;
@@ -176,52 +179,55 @@ __global__ void __launch_bounds__(128) upsample_pair_kernel(const T *__restrict_
         }
     }
 
-    const T *m0 = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(i) * F * plane + static_cast<int64_t>(h) * W;
-    uint32_t o0[F], o1[F];
+    const T *m0 = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(i0) * F * plane + static_cast<int64_t>(h) * W;
+    uint32_t *row = reinterpret_cast<uint32_t *>(out) + static_cast<int64_t>(line) * kPairRows * W * F;
+#pragma unroll 1
+    for (int i = 0; i < kPairRows; ++i, m0 += F * plane, row += static_cast<int64_t>(W) * F) {
+        uint32_t o0[F], o1[F];
 #pragma unroll
-    for (int j = 0; j < F; ++j) {
-        uint32_t raw[9];
+        for (int j = 0; j < F; ++j) {
+            uint32_t raw[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const T *at = m0 + static_cast<int64_t>(k * F * F + j) * plane;
-            if constexpr (EVEN) {
-                raw[k] = __ldg(reinterpret_cast<const uint32_t *>(at + w0));
-            } else {
-                const unsigned short *u = reinterpret_cast<const unsigned short *>(at);
-                raw[k] = static_cast<uint32_t>(__ldg(u + w0)) | static_cast<uint32_t>(__ldg(u + w1)) << 16;
+            for (int k = 0; k < 9; ++k) {
+                const T *at = m0 + static_cast<int64_t>(k * F * F + j) * plane;
+                if constexpr (EVEN) {
+                    raw[k] = __ldg(reinterpret_cast<const uint32_t *>(at + w0));
+                } else {
+                    const unsigned short *u = reinterpret_cast<const unsigned short *>(at);
+                    raw[k] = static_cast<uint32_t>(__ldg(u + w0)) | static_cast<uint32_t>(__ldg(u + w1)) << 16;
+                }
             }
-        }
-        typename DT<T>::Bcast top = word_as_pair<T>(raw[0]);
+            typename DT<T>::Bcast top = word_as_pair<T>(raw[0]);
 #pragma unroll
-        for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(raw[k]));
-        const uint32_t tw = pair_word(top);
-        const float2 mx = make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
-        float2 p[9], den;
+            for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(raw[k]));
+            const uint32_t tw = pair_word(top);
+            const float2 mx = make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
+            float2 p[9], den;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
-            p[k] = weight_exp<T>(l, mx);
-            den = k == 0 ? p[0] : add_f32x2(den, p[k]);
-        }
-        const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
-        float sx[2] = {0.f, 0.f}, sy[2] = {0.f, 0.f};
+            for (int k = 0; k < 9; ++k) {
+                const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
+                p[k] = weight_exp<T>(l, mx);
+                den = k == 0 ? p[0] : add_f32x2(den, p[k]);
+            }
+            const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
+            float sx[2] = {0.f, 0.f}, sy[2] = {0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const float2 q = mul_f32x2(p[k], inv);
-            const typename DT<T>::Bcast w = word_as_pair<T>(DT<T>::aw_from(q.x, q.y));
-            DT<T>::wmul(w, nx[k], sx);
-            DT<T>::wmul(w, ny[k], sy);
+            for (int k = 0; k < 9; ++k) {
+                const float2 q = mul_f32x2(p[k], inv);
+                const typename DT<T>::Bcast w = word_as_pair<T>(DT<T>::aw_from(q.x, q.y));
+                DT<T>::wmul(w, nx[k], sx);
+                DT<T>::wmul(w, ny[k], sy);
+            }
+            o0[j] = DT<T>::aw_from(sx[0], sy[0]);
+            o1[j] = DT<T>::aw_from(sx[1], sy[1]);
         }
-        o0[j] = DT<T>::aw_from(sx[0], sy[0]);
-        o1[j] = DT<T>::aw_from(sx[1], sy[1]);
-    }
-    uint32_t *row = reinterpret_cast<uint32_t *>(out) + static_cast<int64_t>(line) * W * F;
-    if constexpr (F == 4) {
-        st_128(row + static_cast<int64_t>(w0) * F, o0);
-        if (second) st_128(row + static_cast<int64_t>(w1) * F, o1);
-    } else {
-        st_64(row + static_cast<int64_t>(w0) * F, o0);
-        if (second) st_64(row + static_cast<int64_t>(w1) * F, o1);
+        if constexpr (F == 4) {
+            st_128(row + static_cast<int64_t>(w0) * F, o0);
+            if (second) st_128(row + static_cast<int64_t>(w1) * F, o1);
+        } else {
+            st_64(row + static_cast<int64_t>(w0) * F, o0);
+            if (second) st_64(row + static_cast<int64_t>(w1) * F, o1);
+        }
     }
 }
 
@@ -307,7 +313,7 @@ cudaError_t launch(const void *field, const void *mask, void *out, int B, int H,
             if ((reinterpret_cast<uintptr_t>(f) & 3u) == 0) {
                 const auto kernel = even ? (factor == 4 ? upsample_pair_kernel<T, 4, true> : upsample_pair_kernel<T, 2, true>)
                                          : (factor == 4 ? upsample_pair_kernel<T, 4, false> : upsample_pair_kernel<T, 2, false>);
-                launch_chained(kernel, blocks, 128, 0, stream, f, m, o, B, H, W, seg);
+                launch_chained(kernel, (blocks + kPairRows - 1) / kPairRows, 128, 0, stream, f, m, o, B, H, W, seg);
                 return cudaGetLastError();
             }
         } else if (even) {
