@@ -108,8 +108,8 @@ __device__ __forceinline__ void store_run(void *p, const uint32_t *w)
 template <typename T, int R, int CPL>
 constexpr int lanes_min_blocks() { return R == 1 && CPL * DT<T>::kWordsPerChunk <= 8 ? 3 : 2; }
 
-template <typename T, int R, int CPL, int L, bool RAGGED>
-__global__ void __launch_bounds__(kThreads, lanes_min_blocks<T, R, CPL>()) lanes_forward_kernel(const Params p)
+template <typename T, int R, int CPL, int L, bool RAGGED, int BLOCKS = lanes_min_blocks<T, R, CPL>()>
+__global__ void __launch_bounds__(kThreads, BLOCKS) lanes_forward_kernel(const Params p)
 {
     chain_begin();
     using Share = RowShare<R, L>;

@@ -51,24 +51,31 @@ static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid
     return cudaErrorInvalidValue;
 }
 
+// Calls whose blocks the host has cut in half (fewer than ten of them per SM) wait for their taps more than they fill the
+// chip: the build with more registers per thread keeps more of them on their way.  104x208 tokens, 8 heads x 16, float32 22.2 ->
+// 21.0 us, a centre per head 29.5 -> 27.3; float16, 2 x 64x64, 4 x 64 10.7 -> 10.2; full blocks lose (2 x 192x192, 4 x 64, float32
+// 128 -> 144).
+template <typename T, int R, int CPL, int L, bool RAGGED>
+static cudaError_t launch_lanes_one(const Params &p, dim3 grid, int threads, cudaStream_t stream)
+{
+    if constexpr (lanes_min_blocks<T, R, CPL>() > 2) {
+        if (threads < kThreads) return launch_chained(lanes_forward_kernel<T, R, CPL, L, RAGGED, 2>, grid, threads, 0, stream, p);
+    }
+    return launch_chained(lanes_forward_kernel<T, R, CPL, L, RAGGED>, grid, threads, 0, stream, p);
+}
+
 // The splits that calls get without knobs (float32 on (2, 2) and (2, 4): from 33 heads on, r = 2); any other runs on the
 // kernel above, so do 33 to 64 heads of 128 channels at r = 1.
 template <typename T, int R>
 static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream)
 {
     const int width = p.hd / 8;      // chunks of a head
-#define MA_LANES(CPL_, L_)                                                                 \
-    if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) {                                \
-        launch_chained(lanes_forward_kernel<T, R, CPL_, L_, false>, grid, threads, 0, stream, p);      \
-        return cudaGetLastError();                                                         \
-    }
+#define MA_LANES(CPL_, L_) \
+    if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) return launch_lanes_one<T, R, CPL_, L_, false>(p, grid, threads, stream);
     MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8) MA_LANES(4, 8)
     MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
     if constexpr (sizeof(T) == 2) {
-        if (cpl == 3 && p.lph == 2 && width == 5) {
-            launch_chained(lanes_forward_kernel<T, R, 3, 2, true>, grid, threads, 0, stream, p);
-            return cudaGetLastError();
-        }
+        if (cpl == 3 && p.lph == 2 && width == 5) return launch_lanes_one<T, R, 3, 2, true>(p, grid, threads, stream);
     } else {
         MA_LANES(1, 2) MA_LANES(1, 4) MA_LANES(1, 8)
     }
