@@ -21,7 +21,7 @@
 //     The (query, head) items are bucketed by the origin of their window; one kernel computes dq, d(max_offset) and the
 //     coefficients (scale * ds_m, a_m) of every item, another sums them up per token, which finds its contributions in
 //     the (2r+2)^2 buckets whose windows cover it.  dk and dv are written once, in the tensor type.
-//     Measured on a B200, float16, 384x384 tokens, 8 heads x 16, r = 1, centres spread over +-24 tokens: 396 us in all,
+//     Measured on a B200, float16, 384x384 tokens, 8 heads x 16, r = 1, centres spread over +-24 tokens: 353 us in all,
 //     against 785 us for the scattered kernel with its clearing and conversion passes (bound by the rate of the
 //     reductions at L2).
 //   scattered (matchattn_fused_backward; any head width and radius)
@@ -1062,8 +1062,8 @@ constexpr unsigned kPrefetchAhead = 300;
 // shared by the tokens of a block through L1.
 // The coefficients are read once and come from memory: every block has L2 fetch those of the buckets that a block some
 // way ahead starts with, whole runs of slots in one request each.
-// Bound by the latency of the loads (issue 59 % at three blocks per SM without the prefetch, and more lanes or items side
-// by side add their own start: 230 to 265 us).
+// Bound by instruction issue with shared centres (73 %; 59 % and the latency of the loads at three blocks per SM without the
+// prefetch; more lanes or items side by side add their own start: 230 to 265 us), by the longest lists in small calls.
 // Measured, float16, 384x384 tokens, 8 heads x 16, r = 1, shared: 171 us (209 without the prefetch at three blocks).  One
 // head: float16, 2 x 192x192, 4 x 64: 160 us (staged 190); float32, 2 x 45x79, 4 x 32, r = 2: 34 us (staged 38).
 template <typename T, int R, int CPT, bool SHARED>

@@ -15,7 +15,7 @@
 // Measured, float16, r = 2, 4 heads: 2 x 48x48 tokens 13.4 -> 11.4 us, 2 x 160x160 125 -> 112 (one lane per head:
 // five loads per tap that touch a line per lane each, L1 71 % busy, issue 29 %).
 //
-// Bound by instruction issue and the L1 path (73 and 64 % at 16-bit heads of 64, r = 1); r = 2 by the latency of the taps at
+// Bound by instruction issue and the L1 path (61 and 67 % at bfloat16 heads of 64, r = 1); r = 2 by the latency of the taps at
 // two blocks per SM (issue 60 %, L1 54 to 63 %).  Measured on a B200 against one lane's full softmax in every lane and
 // 64-byte slices: float16, 2 x 272x480 tokens, 4 heads x 64, r = 1: 320 -> 225 us; 2 x 68x120, 4 x 128, r = 2:
 // 101 -> 78; float32, 2 x 192x192, 4 x 64, r = 1: 399 -> 160.
