@@ -78,7 +78,7 @@ EncodeTiledFn encode_tiled()
     static const EncodeTiledFn fn = [] {
         void *f = nullptr;
         cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        if (status_of(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q)) != MATCHATTN_OK ||
             q != cudaDriverEntryPointSuccess)
             return static_cast<EncodeTiledFn>(nullptr);
         return reinterpret_cast<EncodeTiledFn>(f);
@@ -238,9 +238,12 @@ inline int sm_count()
     constexpr int kDevices = 64;
     static std::atomic<int> known[kDevices];
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-    if (dev < kDevices && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) {
+        if (dev < kDevices && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+        err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    if (status_of(err) != MATCHATTN_OK || sms <= 0) return 148;
     if (dev < kDevices) known[dev].store(sms, std::memory_order_relaxed);
     return sms;
 }
@@ -292,7 +295,7 @@ int run(Params &p, const Plan &pl, int r, int tile_w_request, cudaStream_t strea
         p.G = p.h * pl.lph;
         if (pl.mma) {
             err = run_mma<T>(p, pl.cpl, p.sorted != nullptr ? p.guard : nullptr, pl.mma_nch, stream);
-            return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+            return status_of(err);
         }
         int threads = kThreads;
         long long blocks = 0;
@@ -336,17 +339,16 @@ int run(Params &p, const Plan &pl, int r, int tile_w_request, cudaStream_t strea
         if (blocks > 2147483647LL) return MATCHATTN_ERR_TOO_LARGE;
         const dim3 grid(static_cast<unsigned>(blocks), grid_y);
         // heads shared by lanes: the kernel that shares the softmax too, except for the options only the other one knows
-        err = cudaErrorInvalidConfiguration;
-        if (pl.lph > 1 && p.guard == nullptr && p.sorted == nullptr && p.debug == nullptr)
-            err = launch_lanes<T>(p, r, pl.cpl, grid, threads, stream);
-        if (err == cudaErrorInvalidConfiguration) err = launch_fast<T>(p, r, pl.cpl, pl.lph > 1, grid, threads, stream);
+        const bool shared = pl.lph > 1 && p.guard == nullptr && p.sorted == nullptr && p.debug == nullptr &&
+                            launch_lanes<T>(p, r, pl.cpl, grid, threads, stream, err);
+        if (!shared) err = launch_fast<T>(p, r, pl.cpl, pl.lph > 1, grid, threads, stream);
     } else {
         const long long per_item = 1LL * p.Nq * p.h;
         const long long blocks = (per_item + kThreads - 1) / kThreads;
         if (blocks > 2147483647LL) return MATCHATTN_ERR_TOO_LARGE;
         err = launch_generic<T>(p, dim3(static_cast<unsigned>(blocks), p.B), stream);
     }
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return status_of(err);
 }
 
 // Up to sixteen block copies in one launch (matchattn_copy_blocks): grid.y picks the block, the grid.x
@@ -504,13 +506,13 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
         if (workspace != nullptr && workspace_bytes >= 8 && aligned(workspace, 8)) {
             sp.status = static_cast<unsigned long long *>(workspace);
             cudaError_t e = cudaMemsetAsync(workspace, 0, 8, stream);
-            if (e != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(e);
+            if (e != cudaSuccess) return status_of(e);
         }
         const long long sms = sm_count();
         const int grid_blocks = static_cast<int>(sp.total_tiles < sms ? sp.total_tiles : sms);
         cudaError_t err = dtype == MATCHATTN_F16 ? launch_staged_persistent<__half>(sp, pl.cpl, map_k, map_v, grid_blocks, stream)
                                                  : launch_staged_persistent<__nv_bfloat16>(sp, pl.cpl, map_k, map_v, grid_blocks, stream);
-        return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+        return status_of(err);
     }
 
     // staged path, one block per tile (two blocks per SM; kept for comparison, strategy 6)
@@ -531,7 +533,7 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
         if (workspace != nullptr && workspace_bytes >= 8 && aligned(workspace, 8)) {
             sp.fallback_tiles = static_cast<unsigned long long *>(workspace);
             cudaError_t e = cudaMemsetAsync(workspace, 0, 8, stream);
-            if (e != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(e);
+            if (e != cudaSuccess) return status_of(e);
         }
         const long long tiles = 1LL * sp.tiles_x * ((p.rows + sg.QH - 1) / sg.QH);
         if (tiles > 2147483647LL) return MATCHATTN_ERR_TOO_LARGE;
@@ -539,7 +541,7 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
         const size_t smem = sp.region_bytes + 128;
         cudaError_t err = dtype == MATCHATTN_F16 ? launch_staged<__half>(sp, pl.cpl, map_k, map_v, grid, smem, stream)
                                                  : launch_staged<__nv_bfloat16>(sp, pl.cpl, map_k, map_v, grid, smem, stream);
-        return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+        return status_of(err);
     }
 
     // binned path: sort the queries by target tile, serve each tile from shared memory
@@ -565,13 +567,13 @@ int forward_impl(const void *max_offset, const void *q, const void *k, const voi
             bp.bins_x = gmt.bins_x; bp.bins_y = gmt.bins_y; bp.nbins = gmt.nbins;
             bp.TX = gmt.TX; bp.TY = gmt.TY; bp.RW = gmt.RW; bp.RH = gmt.RH; bp.region_bytes = gmt.region_bytes;
             cudaError_t err = cudaMemsetAsync(bp.counts, 0, 4 * static_cast<size_t>(gmt.nbins) + 4 * kCtrlWords, stream);
-            if (err != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+            if (err != cudaSuccess) return status_of(err);
             const int grid_blocks = 2 * sm_count();
             const size_t smem_bytes = 2 * static_cast<size_t>(gmt.region_bytes);
             const int main_cpl = strategy == kStrategyBinned ? pl.cpl : 0;     // 0: sorting passes only
             err = dtype == MATCHATTN_F16 ? launch_binned<__half>(bp, main_cpl, grid_blocks, smem_bytes, stream)
                                          : launch_binned<__nv_bfloat16>(bp, main_cpl, grid_blocks, smem_bytes, stream);
-            if (err != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+            if (err != cudaSuccess) return status_of(err);
             if (strategy == kStrategySorted) {
                 // the direct kernel below walks the queries in sorted order; correct whatever the heads do
                 p.sorted = bp.sorted;
@@ -640,7 +642,7 @@ int matchattn_fused_forward_checked(const void *max_offset, const void *q, const
 {
     if (status == nullptr || (reinterpret_cast<uintptr_t>(status) & 7)) return MATCHATTN_ERR_NULL;
     cudaError_t e = cudaMemsetAsync(status, 0, 16, static_cast<cudaStream_t>(cuda_stream));
-    if (e != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(e);
+    if (e != cudaSuccess) return matchattn::status_of(e);
     matchattn::Glue glue;
     glue.debug = static_cast<unsigned long long *>(status);
     return matchattn::forward_impl(max_offset, q, k, v, out, attn_out, B, H, W, h, hd, rx, ry, dtype, attn_type,
@@ -707,10 +709,10 @@ int matchattn_copy_blocks(void *const *dst, const void *const *src, const size_t
         } else {
             err = cudaMemcpyAsync(dst[i], src[i], bytes[i], cudaMemcpyDefault, stream);
         }
-        if (err != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+        if (err != cudaSuccess) return status_of(err);
     }
     const cudaError_t err = flush();
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return status_of(err);
 }
 
 int matchattn_version(void) { return 102; }

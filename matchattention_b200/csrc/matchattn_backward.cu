@@ -1351,7 +1351,7 @@ extern "C" int matchattn_fused_backward(const void *max_offset, const void *q, c
     default: launch_backward<__nv_bfloat16>(p, vec, grid, stream); break;
     }
     const cudaError_t err = cudaGetLastError();
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return status_of(err);
 }
 
 extern "C" size_t matchattn_backward_workspace_bytes(int B, int H, int W, int h, int hd, int r, int dtype, int q_row_begin, int q_row_end)
@@ -1400,5 +1400,5 @@ extern "C" int matchattn_fused_backward_ws(const void *max_offset, const void *q
         return rx == 1 ? launch_gather<T, 1>(g, pl, stream) : launch_gather<T, 2>(g, pl, stream);
     };
     const cudaError_t err = dtype == MATCHATTN_F32 ? run(float()) : dtype == MATCHATTN_F16 ? run(__half()) : run(__nv_bfloat16());
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return status_of(err);
 }

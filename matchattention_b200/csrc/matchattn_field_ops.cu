@@ -188,7 +188,7 @@ extern "C" int matchattn_consistency_mask(const void *field, void *noc_mask, voi
     case MATCHATTN_BF16: err = matchattn::run_mask<__nv_bfloat16>(field, noc_mask, field_diff, B, H, W, threshold, stream); break;
     default: return MATCHATTN_ERR_DTYPE;
     }
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return matchattn::status_of(err);
 }
 
 extern "C" int matchattn_local_disparity(const void *volume, void *flow, void *blur_max, int *centre, int B, int D,
@@ -205,5 +205,5 @@ extern "C" int matchattn_local_disparity(const void *volume, void *flow, void *b
     case MATCHATTN_BF16: err = matchattn::run_disparity<__nv_bfloat16>(volume, flow, blur_max, centre, B, D, H, W, 1.17549435e-38f, stream); break;
     default: return MATCHATTN_ERR_DTYPE;
     }
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return matchattn::status_of(err);
 }

@@ -1002,5 +1002,5 @@ extern "C" int matchattn_flow_init(const void *correlation, void *prob, void *fl
     case MATCHATTN_BF16: err = matchattn::run_flow_init<__nv_bfloat16>(correlation, prob, flow, blur_max, centre, scratch, B, H, W, 1.17549435e-38f, stream); break;
     default: return MATCHATTN_ERR_DTYPE;
     }
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return matchattn::status_of(err);
 }

@@ -27,9 +27,20 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/matchattn.h"
+
 namespace matchattn {
 
 constexpr int kThreads = 256;
+
+// The status that an entry point returns.  The runtime keeps the error of a failed call until it is read; it is read here, or
+// the next entry point of this thread, which asks for the errors of its launches, would find it and report it once more.
+inline int status_of(cudaError_t err)
+{
+    if (err == cudaSuccess) return MATCHATTN_OK;
+    static_cast<void>(cudaGetLastError());
+    return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+}
 
 // Kernels that follow one another in a stream (programmatic dependent launch): a kernel launched by launch_chained is set
 // up while the last blocks of the one before it in the stream end, and begins with chain_begin(), which waits until that

@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) lanes_forward_kernel(const P
     }
 }
 
-// Runs the kernel above if it is built for these lanes; cudaErrorInvalidConfiguration if it is not.
+// Runs the kernel above if it is built for these lanes, `err` what the launch returned; false, nothing launched, if it is not.
 template <typename T>
-cudaError_t launch_lanes(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream);
+bool launch_lanes(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream, cudaError_t &err);
 
 }  // namespace matchattn

@@ -67,26 +67,33 @@ static cudaError_t launch_lanes_one(const Params &p, dim3 grid, int threads, cud
 // The splits that calls get without knobs (float32 on (2, 2) and (2, 4): from 33 heads on, r = 2); any other runs on the
 // kernel above, so do 33 to 64 heads of 128 channels at r = 1.
 template <typename T, int R>
-static cudaError_t launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream)
+static bool launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream, cudaError_t &err)
 {
     const int width = p.hd / 8;      // chunks of a head
-#define MA_LANES(CPL_, L_) \
-    if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) return launch_lanes_one<T, R, CPL_, L_, false>(p, grid, threads, stream);
+#define MA_LANES(CPL_, L_)                                                         \
+    if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) {                        \
+        err = launch_lanes_one<T, R, CPL_, L_, false>(p, grid, threads, stream);   \
+        return true;                                                               \
+    }
     MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8) MA_LANES(4, 8)
     MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
     if constexpr (sizeof(T) == 2) {
-        if (cpl == 3 && p.lph == 2 && width == 5) return launch_lanes_one<T, R, 3, 2, true>(p, grid, threads, stream);
+        if (cpl == 3 && p.lph == 2 && width == 5) {
+            err = launch_lanes_one<T, R, 3, 2, true>(p, grid, threads, stream);
+            return true;
+        }
     } else {
         MA_LANES(1, 2) MA_LANES(1, 4) MA_LANES(1, 8)
     }
 #undef MA_LANES
-    return cudaErrorInvalidConfiguration;
+    return false;
 }
 
 template <>
-cudaError_t launch_lanes<MATCHATTN_T>(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream)
+bool launch_lanes<MATCHATTN_T>(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream, cudaError_t &err)
 {
-    return r == 1 ? launch_lanes_r<MATCHATTN_T, 1>(p, cpl, grid, threads, stream) : launch_lanes_r<MATCHATTN_T, 2>(p, cpl, grid, threads, stream);
+    return r == 1 ? launch_lanes_r<MATCHATTN_T, 1>(p, cpl, grid, threads, stream, err)
+                  : launch_lanes_r<MATCHATTN_T, 2>(p, cpl, grid, threads, stream, err);
 }
 
 template <>

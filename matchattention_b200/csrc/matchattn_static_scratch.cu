@@ -15,8 +15,9 @@
 // loaded until the process exits, and the problem size is limited by it.
 #include "../../include/matchattn.h"
 
-#include <cuda_runtime.h>
 #include <mutex>
+
+#include "matchattn_kernels.cuh"
 
 namespace {
 
@@ -35,13 +36,13 @@ int scratch_on_current_device(void **address)
 {
     int dev = -1;
     cudaError_t err = cudaGetDevice(&dev);
-    if (err != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    if (err != cudaSuccess) return matchattn::status_of(err);
     if (dev < 0 || dev >= kMaxDevices) return MATCHATTN_ERR_TOO_LARGE;
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     if (!g_scratch_ready[dev]) {
         void *ptr = nullptr;
         err = cudaGetSymbolAddress(&ptr, g_static_scratch);      // with device `dev` current
-        if (err != cudaSuccess) return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+        if (err != cudaSuccess) return matchattn::status_of(err);
         if (ptr == nullptr) return MATCHATTN_ERR_NULL;
         g_scratch_address[dev] = ptr;
         g_scratch_ready[dev] = true;

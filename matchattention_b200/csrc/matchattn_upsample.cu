@@ -350,5 +350,5 @@ extern "C" int matchattn_upsample_field(const void *field, const void *mask, voi
     case MATCHATTN_BF16: err = matchattn::launch<__nv_bfloat16>(field, mask, out, B, H, W, D, factor, stream); break;
     default: return MATCHATTN_ERR_DTYPE;
     }
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return matchattn::status_of(err);
 }

@@ -164,5 +164,5 @@ extern "C" int matchattn_stereo_volume(const void *correlation, void *volume, in
     case MATCHATTN_BF16: err = matchattn::launch<__nv_bfloat16>(correlation, volume, B, H, W, stream); break;
     default: return MATCHATTN_ERR_DTYPE;
     }
-    return err == cudaSuccess ? MATCHATTN_OK : MATCHATTN_ERR_CUDA + static_cast<int>(err);
+    return matchattn::status_of(err);
 }
