@@ -164,13 +164,13 @@ __device__ __forceinline__ void load8(const T *p, float (&f)[8]);
 template <>
 __device__ __forceinline__ void load8<float>(const float *p, float (&f)[8])
 {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+    const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 template <>
 __device__ __forceinline__ void load8<__half>(const __half *p, float (&f)[8])
 {
-    const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p));
+    const uint4 u = *reinterpret_cast<const uint4 *>(p);
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -182,7 +182,7 @@ __device__ __forceinline__ void load8<__half>(const __half *p, float (&f)[8])
 template <>
 __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16 *p, float (&f)[8])
 {
-    const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p));
+    const uint4 u = *reinterpret_cast<const uint4 *>(p);
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -438,11 +438,11 @@ __global__ void __launch_bounds__(256) gather_check_kernel(const GatherParams g,
     const uint32_t bq = blockIdx.x * 256u + threadIdx.x;
     if (bq >= queries) return;
     const Pair *mo = static_cast<const Pair *>(g.b.mo) + static_cast<int64_t>(bq) * g.b.h;
-    const Pair first = __ldg(mo);
+    const Pair first = *mo;
     bool same = true;
 #pragma unroll 4
     for (int i = 1; i < g.b.h; ++i) {
-        const Pair v = __ldg(mo + i);
+        const Pair v = mo[i];
         if constexpr (sizeof(T) == 4) same = same && v.x == first.x && v.y == first.y;
         else same = same && v == first;
     }
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(128, R == 1 && CPL <= 2 ? 4 : 3) gather_coef_k
         const uint2 *gap = reinterpret_cast<const uint2 *>(static_cast<const T *>(p.dattn) + static_cast<int64_t>(item) * M);
 #pragma unroll
         for (int w = 0; w < M / EPW / 2; ++w) {
-            const uint2 u = __ldg(gap + w);
+            const uint2 u = gap[w];
 #pragma unroll
             for (int e = 0; e < 2 * EPW; ++e) da[2 * EPW * w + e] += DT<T>::unpack(e < EPW ? u.x : u.y, e % EPW);
         }
@@ -874,7 +874,7 @@ struct Piece {
     static __device__ __forceinline__ void load(uint32_t (&w)[NW], const T *at)      // (the 32-byte form takes global addresses only)
     {
         if constexpr (NW == 8) {
-            ld_nc_256(w, at);
+            ld_256(w, at);
         } else {
             const uint4 u = *reinterpret_cast<const uint4 *>(at);
             w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
@@ -905,7 +905,7 @@ struct Accumulate {
     {
 #pragma unroll
         for (int i = 0; i < static_cast<int>(sizeof(T)) / 2; ++i) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4 *>(kp) + i);
+            const uint4 u = reinterpret_cast<const uint4 *>(kp)[i];
             k[4 * i] = u.x; k[4 * i + 1] = u.y; k[4 * i + 2] = u.z; k[4 * i + 3] = u.w;
         }
 #pragma unroll
@@ -1084,7 +1084,7 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_d
         const int cy = tile_row(then_row, tile_rows) * tl.y + threadIdx.x, cx = (then - then_row * tl.tiles_x) * tl.x;
         if (cy < g.cells_y && cx < g.cells_x) {
             const int *start = g.starts + (static_cast<int64_t>(list) * g.cells_y + cy) * (g.cells_x + 1);
-            const int from = __ldg(start + cx), slots = __ldg(start + min(cx + tl.x, g.cells_x)) - from;
+            const int from = start[cx], slots = start[min(cx + tl.x, g.cells_x)] - from;
             if (slots > 0) prefetch_l2(g.coef + static_cast<int64_t>(from) * M * coef_step, slots, M * coef_step * static_cast<uint32_t>(sizeof(float2)));
         }
     }
@@ -1115,8 +1115,8 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_d
             const int cy = ty - j;
             const int *start = g.starts + (static_cast<int64_t>(list) * g.cells_y + cy) * (g.cells_x + 1);
             const bool ok = cy >= 0 && cy < g.cells_y;
-            lo[j] = ok ? __ldg(start + c_lo) : 0;
-            hi[j] = ok ? __ldg(start + c_hi) : 0;
+            lo[j] = ok ? start[c_lo] : 0;
+            hi[j] = ok ? start[c_hi] : 0;
         }
 #pragma unroll
         for (int j = 0; j < SIDE; ++j) {
@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_d
         for (int n = 0; n < 2; ++n) {
             int slot, at;
             locate(min(f + n, total - 1), slot, at);
-            const int2 m = __ldg(g.meta + slot);
+            const int2 m = g.meta[slot];
             row[n] = static_cast<uint32_t>(m.x);
             tap[n] = SHARED ? static_cast<Tap>(at + m.y) : static_cast<Tap>(slot) * M + static_cast<Tap>(at - m.y);
         }
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(256, sum_min_blocks<T, R, CPT>()) gather_sum_d
             Piece<T> first, other;
             first.load(q + r0 + s * step, go + r0 + s * step);
             other.load(q + r1 + s * step, go + r1 + s * step);
-            const float2 ca = __ldg(c0 + head[s]), cb = __ldg(c1 + head[s]);
+            const float2 ca = c0[head[s]], cb = c1[head[s]];
             if (s == CPT - 1 && f + 2 < total) fetch(f + 2);
             acc[s].add(first, ca.x, ca.y);
             if (second) acc[s].add(other, cb.x, cb.y);

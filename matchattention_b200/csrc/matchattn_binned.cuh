@@ -178,7 +178,7 @@ template <int NW>
 __device__ __forceinline__ void ldg_item(uint32_t (&w)[NW], const char *ptr, uint32_t swz)
 {
 #pragma unroll
-    for (int c = 0; c < NW / 4; ++c) ld_nc_128(&w[4 * c], ptr + ((16u * c) ^ swz));
+    for (int c = 0; c < NW / 4; ++c) ld_128(&w[4 * c], ptr + ((16u * c) ^ swz));
 }
 template <int NW>
 __device__ __forceinline__ void stg_item(char *ptr, const uint32_t (&w)[NW], uint32_t swz)

@@ -18,7 +18,7 @@ namespace matchattn {
 namespace {
 
 template <typename T>
-__global__ void __launch_bounds__(256) consistency_mask_kernel(const T *__restrict__ field, T *__restrict__ mask,
+__global__ void __launch_bounds__(256) consistency_mask_kernel(const T *field, T *__restrict__ mask,
                                                                 T *__restrict__ diff_out, int B, int H, int W, float A)
 {
     chain_begin();
@@ -73,7 +73,7 @@ __device__ __forceinline__ float fifth(float x)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(32 * kDispGroups) local_disparity_kernel(const T *__restrict__ cv, T *__restrict__ flow,
+__global__ void __launch_bounds__(32 * kDispGroups) local_disparity_kernel(const T *cv, T *__restrict__ flow,
                                                                            T *__restrict__ blur_out, int *__restrict__ centre_out,
                                                                            int B, int D, int H, int W, float tiny)
 {

@@ -168,8 +168,8 @@ __device__ __forceinline__ float plus_float(__nv_bfloat16 a, float x) { return a
 template <typename T>
 __device__ __forceinline__ uint32_t raw_bits(const T *p)
 {
-    if constexpr (sizeof(T) == 4) return __ldg(reinterpret_cast<const uint32_t *>(p));
-    else return __ldg(reinterpret_cast<const unsigned short *>(p));
+    if constexpr (sizeof(T) == 4) return *reinterpret_cast<const uint32_t *>(p);
+    else return *reinterpret_cast<const unsigned short *>(p);
 }
 
 template <typename T, int ALIGN, bool FULL>
@@ -181,7 +181,7 @@ __device__ __forceinline__ Group<T> load_group(const T *row, int64_t col, int64_
         g.mask();
 #pragma unroll
         for (int k = 0; k < kLaneCols; k += 2)
-            if (FULL || (row_ok && col + k >= 0 && col + k < N)) g.w[k / 2] = __ldg(reinterpret_cast<const uint32_t *>(row + col + k));
+            if (FULL || (row_ok && col + k >= 0 && col + k < N)) g.w[k / 2] = *reinterpret_cast<const uint32_t *>(row + col + k);
     } else if constexpr (FULL || ALIGN >= kLaneCols) {
         if (!FULL && (!row_ok || col < 0 || col >= N)) {
             g.mask();
@@ -195,10 +195,10 @@ __device__ __forceinline__ Group<T> load_group(const T *row, int64_t col, int64_
                 g.w[k / EPW] = w;
             }
         } else if constexpr (EPW == 1) {
-            const uint4 t = __ldg(reinterpret_cast<const uint4 *>(row + col));
+            const uint4 t = *reinterpret_cast<const uint4 *>(row + col);
             g.w[0] = t.x; g.w[1] = t.y; g.w[2] = t.z; g.w[3] = t.w;
         } else {
-            const uint2 t = __ldg(reinterpret_cast<const uint2 *>(row + col));
+            const uint2 t = *reinterpret_cast<const uint2 *>(row + col);
             g.w[0] = t.x; g.w[1] = t.y;
         }
     } else {
@@ -234,7 +234,7 @@ __device__ __forceinline__ void max_tile(const T *src, int64_t col, int64_t r0, 
 }
 
 template <typename T, int ALIGN>
-__global__ void __launch_bounds__(kFlowThreads) flow_max_kernel(const T *__restrict__ corr, float *__restrict__ row_part,
+__global__ void __launch_bounds__(kFlowThreads) flow_max_kernel(const T *corr, float *__restrict__ row_part,
                                                                 float *__restrict__ col_part, int64_t N, int rows_per_warp,
                                                                 int row_parts, int col_parts)
 {
@@ -322,8 +322,8 @@ __device__ __forceinline__ void row_sum(const T *src, const float *row_part, flo
 // the sums alone: 96x96 tokens 106 -> 91 us, 128x128 259 -> 249, 82x79 81 -> 60; 48x48 14.4 -> 13.2 (a thread per column and
 // remainder that read, exponentiated and added one column, at 156 registers).
 template <typename T, int ALIGN, int COLUMNS>
-__global__ void __launch_bounds__(kFlowThreads, 4) flow_sum_kernel(const T *__restrict__ corr, const float *__restrict__ row_part,
-                                                                const float *__restrict__ col_part, float2 *__restrict__ stats,
+__global__ void __launch_bounds__(kFlowThreads, 4) flow_sum_kernel(const T *corr, const float *row_part,
+                                                                const float *col_part, float2 *__restrict__ stats,
                                                                 int64_t N, int row_parts, int col_parts, int col_blocks)
 {
     chain_begin();
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kFlowThreads, 4) flow_sum_kernel(const T *__re
         float mx = -INFINITY;
         if (col < N) {
 #pragma unroll 4
-            for (int i = g; i < col_parts; i += kFlowThreads / COLUMNS) mx = fmaxf(mx, __ldg(col_part + (b * col_parts + i) * N + col));
+            for (int i = g; i < col_parts; i += kFlowThreads / COLUMNS) mx = fmaxf(mx, col_part[(b * col_parts + i) * N + col]);
         }
         part[g][c] = mx;
         __syncthreads();
@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(kFlowThreads, 4) flow_sum_kernel(const T *__re
 // four reads, exponentiates and adds, BATCH rows ahead.  Measured, float16, the sums alone, this / the one above: 67x71 tokens
 // 40 / 55 us, 79x83 85 / 89, 97x101 141 / 166, bfloat16 111x113 204 / 240.
 template <typename T, int COLUMNS, int BATCH>
-__global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_strided_kernel(const T *__restrict__ corr, const float *__restrict__ row_part,
-                                                                const float *__restrict__ col_part, float2 *__restrict__ stats,
+__global__ void __launch_bounds__(COLUMNS * kSumGroups) flow_sum_strided_kernel(const T *corr, const float *row_part,
+                                                                const float *col_part, float2 *__restrict__ stats,
                                                                 int64_t N, int row_parts, int col_parts, int col_blocks)
 {
     chain_begin();
@@ -525,7 +525,7 @@ __device__ __forceinline__ void pool_rows(const PoolParams &pp, const T *src, T 
     float *row_max = reinterpret_cast<float *>(st + pp.band_rows + 4);
     for (int i = lane; i < pp.band_rows + 4; i += 32) {
         const int64_t a = a0 - 2 + i;
-        const Softmax s = softmax_of<T>(FULL || (a >= 0 && a < N) ? __ldg(pp.stats + b * N + a) : make_float2(0.f, 1.f));
+        const Softmax s = softmax_of<T>(FULL || (a >= 0 && a < N) ? pp.stats[b * N + a] : make_float2(0.f, 1.f));
         st[i] = make_float4(s.neg_max, s.sum, s.inv, 0.f);
     }
     __syncwarp();
@@ -618,7 +618,7 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
     float best[kLaneCols];
 #pragma unroll
     for (int k = 0; k < kLaneCols; ++k) {
-        sm[k] = softmax_of<T>(FULL || (c0 + k >= 0 && c0 + k < N) ? __ldg(pp.stats + (pp.B + b) * N + c0 + k) : make_float2(0.f, 1.f));
+        sm[k] = softmax_of<T>(FULL || (c0 + k >= 0 && c0 + k < N) ? pp.stats[(pp.B + b) * N + c0 + k] : make_float2(0.f, 1.f));
         best[k] = 0.f;
     }
     // probabilities of two rows (16-bit types: a word per column, first row low), then the box sums two rows above each
@@ -734,7 +734,7 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
 // ran short, 2.2 of 8 stalls).  With 16-byte stores straight from the registers to 32 rows of prob the
 // second role alone took 0.67 ms; five blocks of four warps hold 20 warps per SM (0.75 ms with four blocks).
 template <typename T, int ALIGN>
-__global__ void __launch_bounds__(32 * kPoolWarps, sizeof(T) == 2 ? 5 : 4) flow_prob_pool_kernel(const T *__restrict__ corr, T *__restrict__ prob, const PoolParams pp)
+__global__ void __launch_bounds__(32 * kPoolWarps, sizeof(T) == 2 ? 5 : 4) flow_prob_pool_kernel(const T *corr, T *__restrict__ prob, const PoolParams pp)
 {
     chain_begin();
     extern __shared__ __align__(16) char smem_raw[];
@@ -778,8 +778,8 @@ constexpr int kKeptChunks = 256;      // chunk maxima per token that a block of 
 constexpr float kScreen = 4e-6f;      // 24 float32 additions of positive terms in two different orders
 
 template <typename T>
-__global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__restrict__ prob, const float *__restrict__ row_max,
-                                                                   const float *__restrict__ col_max, T *__restrict__ flow,
+__global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *prob, const float *row_max,
+                                                                   const float *col_max, T *__restrict__ flow,
                                                                    T *__restrict__ blur_max, int *__restrict__ centre_out, int B, int H,
                                                                    int W, int chunks, int bands, int band_rows, float tiny)
 {
@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
         const int t = threadIdx.x % kWindowTokens, g = threadIdx.x / kWindowTokens;
         if (i0 + t < N) {
 #pragma unroll 8
-            for (int c = g; c < min(n, kKeptChunks); c += kGroups) kept[t][c] = __ldg(maxima + static_cast<int64_t>(c) * N + t);
+            for (int c = g; c < min(n, kKeptChunks); c += kGroups) kept[t][c] = maxima[static_cast<int64_t>(c) * N + t];
         }
     }
     __syncthreads();
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_window_kernel(const T *__re
     if (i >= N) return;
     const T *base = prob + b2 * N * N;
     const auto chunk_max = [&](int c) {
-        return c >= n ? 0.f : c < kKeptChunks ? kept[warp][c] : __ldg(maxima + static_cast<int64_t>(c) * N + warp);
+        return c >= n ? 0.f : c < kKeptChunks ? kept[warp][c] : maxima[static_cast<int64_t>(c) * N + warp];
     };
     float top = 0.f;
     for (int c = lane; c < n; c += 32) top = fmaxf(top, chunk_max(c));

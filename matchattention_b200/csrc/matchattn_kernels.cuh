@@ -45,9 +45,12 @@ inline int status_of(cudaError_t err)
 // Kernels that follow one another in a stream (programmatic dependent launch): a kernel launched by launch_chained is set
 // up while the last blocks of the one before it in the stream end, and begins with chain_begin(), which waits until that
 // one has ended altogether and its writes are visible.  Every thread calls it before anything else: a grid that ended
-// without waiting would let the one after it run beside the one before it.  Each launch keeps the stream's order all the
-// same, whatever comes before or after it, and so does a captured one.  No kernel lets the next one in before its blocks
-// end (griddepcontrol.launch_dependents): blocks placed between running ones crowd some SMs and leave others short.
+// without waiting would let the one after it run beside the one before it.  What it reads may have been written while it was
+// set up, so it is not constant over the kernel's life: chained kernels read by ordinary loads, never by the non-coherent
+// ones (ld.global.nc, __ldg, parameters declared const __restrict__), which promise that and may move ahead of the wait.
+// Each launch keeps the stream's order all the same, whatever comes before or after it, and so does a captured one.  No
+// kernel lets the next one in before its blocks end (griddepcontrol.launch_dependents): blocks placed between running ones
+// crowd some SMs and leave others short.
 // Measured, us per call in a row of calls, before / now / with the next kernel let in at the start: 2 x 48x48 tokens, 4 heads
 // x 40, r = 2, float16 12.3 / 10.6 / 14.7; stereo volume and disparity at 68x120 17.5 / 13.6 / 19.9; flow_init at 48x48
 // 59.4 / 50.1 / 57.9 and at 128x128 1069 / 1058 / 1106; forward and backward, float32, 2 x 45x79 tokens, r = 2 121.7 / 107.5 / 111.
@@ -116,15 +119,15 @@ __device__ __forceinline__ float clamp_keep_nan(float v, float lo, float hi) { r
 
 // ------------------------------------------------------------------ loads / stores
 
-__device__ __forceinline__ void ld_nc_256(uint32_t *w, const void *p)
+__device__ __forceinline__ void ld_256(uint32_t *w, const void *p)
 {
-    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                  : "l"(p));
 }
-__device__ __forceinline__ void ld_nc_128(uint32_t *w, const void *p)
+__device__ __forceinline__ void ld_128(uint32_t *w, const void *p)
 {
-    asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
                  : "l"(p));
 }
@@ -151,10 +154,10 @@ __device__ __forceinline__ void load_words(uint32_t (&w)[NW], const void *p)
     static_assert(NW % 4 == 0, "a lane's slice is a multiple of 16 bytes");
     if constexpr (NW % 8 == 0) {
 #pragma unroll
-        for (int i = 0; i < NW / 8; ++i) ld_nc_256(&w[8 * i], static_cast<const char *>(p) + 32 * i);
+        for (int i = 0; i < NW / 8; ++i) ld_256(&w[8 * i], static_cast<const char *>(p) + 32 * i);
     } else {
 #pragma unroll
-        for (int i = 0; i < NW / 4; ++i) ld_nc_128(&w[4 * i], static_cast<const char *>(p) + 16 * i);
+        for (int i = 0; i < NW / 4; ++i) ld_128(&w[4 * i], static_cast<const char *>(p) + 16 * i);
     }
 }
 
@@ -273,7 +276,7 @@ struct DT<float> {
     static __device__ __forceinline__ float rnd(float x) { return x; }
     static __device__ __forceinline__ void load_xy(const void *p, float &x, float &y)
     {
-        const float2 t = __ldg(static_cast<const float2 *>(p));
+        const float2 t = *static_cast<const float2 *>(p);
         x = t.x;
         y = t.y;
     }
@@ -306,7 +309,7 @@ struct DT<__half> {
     static __device__ __forceinline__ float rnd(float x) { return __half2float(__float2half_rn(x)); }
     static __device__ __forceinline__ void load_xy(const void *p, float &x, float &y)
     {
-        const uint32_t u = __ldg(static_cast<const uint32_t *>(p));
+        const uint32_t u = *static_cast<const uint32_t *>(p);
         const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u));
         x = f.x;
         y = f.y;
@@ -376,7 +379,7 @@ struct DT<__nv_bfloat16> {
     static __device__ __forceinline__ float rnd(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
     static __device__ __forceinline__ void load_xy(const void *p, float &x, float &y)
     {
-        const uint32_t u = __ldg(static_cast<const uint32_t *>(p));
+        const uint32_t u = *static_cast<const uint32_t *>(p);
         x = __uint_as_float(u << 16);
         y = __uint_as_float(u & 0xffff0000u);
     }
@@ -839,11 +842,11 @@ constexpr int kMaxTaps = (2 * kMaxR + 2) * (2 * kMaxR + 2);
 template <typename T>
 __device__ __forceinline__ float load_one(const T *p);
 template <>
-__device__ __forceinline__ float load_one<float>(const float *p) { return __ldg(p); }
+__device__ __forceinline__ float load_one<float>(const float *p) { return *p; }
 template <>
-__device__ __forceinline__ float load_one<__half>(const __half *p) { return __half2float(__ldg(p)); }
+__device__ __forceinline__ float load_one<__half>(const __half *p) { return __half2float(*p); }
 template <>
-__device__ __forceinline__ float load_one<__nv_bfloat16>(const __nv_bfloat16 *p) { return __bfloat162float(__ldg(p)); }
+__device__ __forceinline__ float load_one<__nv_bfloat16>(const __nv_bfloat16 *p) { return __bfloat162float(*p); }
 
 template <typename T>
 __device__ __forceinline__ void store_one(T *p, float x);

@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) lanes_forward_kernel(const P
     const auto load_slice = [&](uint32_t (&w)[NW], const T *at) {
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
-            if constexpr (PW == 8) ld_nc_256(&w[8 * i], at + i * kStep);
-            else ld_nc_128(&w[4 * i], at + i * kStep);
+            if constexpr (PW == 8) ld_256(&w[8 * i], at + i * kStep);
+            else ld_128(&w[4 * i], at + i * kStep);
         }
-        if constexpr (RAGGED) ld_nc_128(&w[8], at + tail);
+        if constexpr (RAGGED) ld_128(&w[8], at + tail);
     };
 
     uint32_t qw[NW];

@@ -60,7 +60,7 @@ __device__ __forceinline__ float2 weight_exp(float2 l, float2 top)
 }
 
 template <typename T, int F>
-__global__ void __launch_bounds__(128) upsample_field_kernel(const T *__restrict__ field, const T *__restrict__ mask,
+__global__ void __launch_bounds__(128) upsample_field_kernel(const T *field, const T *mask,
                                                              T *__restrict__ out, int B, int H, int W, int D)
 {
     chain_begin();
@@ -139,7 +139,7 @@ constexpr int kPairRows = 2;
 // five blocks per SM before; one fine row per thread 28.5, two without the limit of 64 registers 54); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
 // fine rows per thread) -> 17.7.
 template <typename T, int F, bool EVEN>
-__global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *__restrict__ field, const T *__restrict__ mask, T *__restrict__ out,
+__global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *field, const T *mask, T *__restrict__ out,
                                                             int B, int H, int W, int segments)
 {
     chain_begin();
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *__restri
             for (int c = 0; c < COLS; ++c) {
                 const int ww = EVEN || c < 3 ? w0 + c - 1 : w1 + c - 4;
                 const bool inside = hh >= 0 && hh < H && ww >= 0 && ww < W;
-                v[c] = inside ? DT<T>::aw_mul(__ldg(src + hh * W + ww), factor) : 0u;
+                v[c] = inside ? DT<T>::aw_mul(src[hh * W + ww], factor) : 0u;
             }
 #pragma unroll
             for (int kx = 0; kx < 3; ++kx) {
@@ -191,10 +191,10 @@ __global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *__restri
             for (int k = 0; k < 9; ++k) {
                 const T *at = m0 + static_cast<int64_t>(k * F * F + j) * plane;
                 if constexpr (EVEN) {
-                    raw[k] = __ldg(reinterpret_cast<const uint32_t *>(at + w0));
+                    raw[k] = *reinterpret_cast<const uint32_t *>(at + w0);
                 } else {
                     const unsigned short *u = reinterpret_cast<const unsigned short *>(at);
-                    raw[k] = static_cast<uint32_t>(__ldg(u + w0)) | static_cast<uint32_t>(__ldg(u + w1)) << 16;
+                    raw[k] = static_cast<uint32_t>(u[w0]) | static_cast<uint32_t>(u[w1]) << 16;
                 }
             }
             typename DT<T>::Bcast top = word_as_pair<T>(raw[0]);
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *__restri
 // Measured, 2 x 384x384 by 4: 43.8 us (four cells per thread, exponentials by the special-function unit alone: 47.7; with
 // expf 50.7, in pairs 64.2 at 137 registers); 2 x 201x302 by 4: 22.7 (one cell and all its fine rows per thread: 55.5).
 template <int F>
-__global__ void __launch_bounds__(128) upsample_f32_kernel(const float *__restrict__ field, const float *__restrict__ mask,
+__global__ void __launch_bounds__(128) upsample_f32_kernel(const float *field, const float *mask,
                                                            float *__restrict__ out, int B, int H, int W, int segments)
 {
     chain_begin();
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(128) upsample_f32_kernel(const float *__restri
     for (int j = 0; j < F; ++j) {
         float2 p[9], den;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) p[k] = __ldg(reinterpret_cast<const float2 *>(m0 + static_cast<int64_t>(k * F * F + j) * plane));
+        for (int k = 0; k < 9; ++k) p[k] = *reinterpret_cast<const float2 *>(m0 + static_cast<int64_t>(k * F * F + j) * plane);
         float2 mx = p[0];
 #pragma unroll
         for (int k = 1; k < 9; ++k) mx = make_float2(fmaxf(mx.x, p[k].x), fmaxf(mx.y, p[k].y));

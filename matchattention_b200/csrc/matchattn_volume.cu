@@ -44,7 +44,7 @@ __device__ __forceinline__ float warp_max(float v)
 // PIECES: W / 32 rounded up (a warp takes a row of corr, a column or a row of vol in that many pieces at once)
 // WARPS: of a block, ROWS: W / WARPS rounded up, rows or columns per warp
 template <typename T, int PIECES, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, 2) stereo_volume_kernel(const T *__restrict__ corr, T *__restrict__ vol, int B, int H, int W)
+__global__ void __launch_bounds__(32 * WARPS, 2) stereo_volume_kernel(const T *corr, T *__restrict__ vol, int B, int H, int W)
 {
     chain_begin();
     constexpr int ROWS = (32 * PIECES + WARPS - 1) / WARPS;
