@@ -202,9 +202,18 @@ def test_local_disparity_of_an_infinite_value(dtype):
     assert torch.isfinite(flow).sum() == flow.numel() - 2
 
 
-@pytest.mark.parametrize("H,W,dtype", [(71, 73, torch.float16), (84, 72, torch.float32), (98, 96, torch.float16), (97, 97, torch.bfloat16)])
+# Token counts on either side of the thresholds: column sums 32 columns wide from 5800 tokens on in 16 bits (rows aligned to 2,
+# 4 and 8 elements) and from 6600 on in float32 (to 1 and 4), 16-bit rows of an odd count from 9400 on; short bands at odd
+# counts below 10000, long ones from 5000 (odd: 10000) on.
+BEYOND_THRESHOLDS = [(71, 73, torch.float16), (84, 72, torch.float32), (98, 96, torch.float16), (97, 97, torch.bfloat16),
+                     (76, 76, torch.bfloat16), (80, 73, torch.bfloat16), (78, 75, torch.float16), (78, 75, torch.bfloat16),
+                     (77, 76, torch.float16), (77, 76, torch.bfloat16), (75, 77, torch.float16), (88, 76, torch.float32),
+                     (83, 83, torch.float32), (79, 83, torch.float32), (101, 101, torch.float16)]
+
+
+@pytest.mark.parametrize("H,W,dtype", BEYOND_THRESHOLDS)
 def test_flow_init_kernels_beyond_their_thresholds(H, W, dtype):
-    """Short bands of an odd token count, and the wide column sums of either type's large maps."""
+    """Short and long bands, narrow and wide column sums of every alignment, remainders of their batches of rows."""
     import oracle
     g = torch.Generator().manual_seed(H * W)
     second = torch.randn(1, H * W, 16, generator=g)
