@@ -153,6 +153,13 @@ __global__ void __launch_bounds__(128) backward_kernel(const BwdParams p)
     }
 }
 
+__device__ __forceinline__ float sign_of(float a, float b)      // sign(a - b), 0 where one of them is no number
+{
+    float gt, lt;
+    asm("set.gt.f32.f32 %0, %1, %2;" : "=f"(gt) : "f"(a), "f"(b));
+    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(lt) : "f"(a), "f"(b));
+    return gt - lt;
+}
 
 // ---- the same computation for head widths that are multiples of 8 and r = 1 or 2 -----------------------
 // Eight channels at a time through 16- or 32-byte loads, the window in registers (R is a template
@@ -353,8 +360,7 @@ __global__ void __launch_bounds__(128, R == 2 ? 4 : 3) backward_vec_kernel(const
                 load8<T>(kb + off, kv);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    const float d = qv[c] - kv[c];
-                    gk[c] = d > 0.f ? ds[m] : (d < 0.f ? -ds[m] : 0.f);
+                    gk[c] = ds[m] * sign_of(qv[c], kv[c]);       // not finite where ds is not, as the product is in every other kernel
                     acc[c] -= gk[c];
                 }
                 if (ds[m] != 0.f) {
@@ -528,14 +534,6 @@ __device__ __forceinline__ float2 sign_pair(uint32_t a, uint32_t b)
         w = *reinterpret_cast<const uint32_t *>(&d);
     }
     return make_float2(DT<T>::unpack(w, 0), DT<T>::unpack(w, 1));
-}
-
-__device__ __forceinline__ float sign_of(float a, float b)      // sign(a - b), 0 where one of them is no number
-{
-    float gt, lt;
-    asm("set.gt.f32.f32 %0, %1, %2;" : "=f"(gt) : "f"(a), "f"(b));
-    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(lt) : "f"(a), "f"(b));
-    return gt - lt;
 }
 
 // A lane's slice (NW words) of q or dout against one tap's words of K or V.

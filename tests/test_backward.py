@@ -4,6 +4,7 @@ CPU: the plain-loop restatement of the gradient formulas (oracle/matchattn_backw
 autograd gives over the reference's own functions (tests/golden/backward_*.npz).
 GPU: the CUDA backward, through the autograd function and the reference-compatible module, against the same
 vectors, and against autograd over the reference's functions run on the same GPU (float32 and float16)."""
+import numpy as np
 import pytest
 import torch
 
@@ -165,6 +166,40 @@ def test_accumulating_backward_kernels_match_the_restatement(h, hd, r, need_attn
     d_mo, d_q = _accumulate(*(t.cuda() for t in (mo, q, k, v, g_out)), g_attn.cuda() if need_attn_grad else None, H, W, r, hd ** -0.5, dk, dv)
     for got, ref, key in zip((d_mo, d_q, dk - 0.5, dv + 2.0), want, ("d_max_offset", "d_q", "d_k", "d_v")):
         assert _rel(got, ref) < tol, key
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16], ids=["f32", "f16", "bf16"])
+@pytest.mark.parametrize("h,hd,r,gathered", [(2, 16, 1, True), (2, 24, 1, True), (2, 16, 1, False), (2, 24, 2, True), (2, 24, 2, False),
+                                             (2, 12, 1, False)])
+def test_an_infinite_gradient_of_a_weight(h, hd, r, gathered, dtype):
+    """Every route gives the values of the definition, sign(q - k) times the gradient of the score: not finite where that is
+    not, a channel with q = k (0 times infinity) included."""
+    from oracle import matchattn_backward
+    from test_gpu_backward_sums import _both
+    B, H, W = 1, 9, 10
+    mo, q, k, v = make_inputs(67, B, H, W, h, hd, r, dtype, kind="flow", spread=3.0, per_head=True)
+    q[..., 3] = k[..., 3] = 0.5
+    mo[0, 37, 0] = torch.tensor([4.53125, 4.28125])         # all four windows count
+    gen = torch.Generator().manual_seed(68)
+    g_out = torch.randn(q.shape, generator=gen).to(dtype)
+    g_attn = torch.randn(B, H * W, h, (2 * r + 2) ** 2, generator=gen).to(dtype)
+    g_attn[0, 37, 0, (2 * r + 2) + 1] = float("inf")
+    with np.errstate(invalid="ignore"):
+        want = matchattn_backward.backward(*(t.float() for t in (mo, q, k, v, g_out, g_attn)), H, W, r, hd ** -0.5)
+    assert np.isfinite(want[2]).sum() < want[2].size
+    args = [t.cuda() for t in (mo, q, k, v, g_out, g_attn)]
+    if gathered:
+        got, _ = _both(*args, H, W, h, r, hd ** -0.5, (0, H))
+    else:
+        dk, dv = torch.zeros(k.shape, device="cuda"), torch.zeros(v.shape, device="cuda")
+        got = (*_accumulate(*args, H, W, r, hd ** -0.5, dk, dv), dk, dv)
+    tol = {torch.float32: 1e-4, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}[dtype]        # those of the tests above
+    for g, ref, key in zip(got, want, ("d_max_offset", "d_q", "d_k", "d_v")):
+        g, ref = g.double().cpu(), torch.as_tensor(ref).double()
+        finite = ref.isfinite()
+        assert torch.equal(g.isfinite(), finite), key
+        assert (g[finite] - ref[finite]).abs().max() <= tol * ref[finite].abs().max(), key
 
 
 def _step(inputs, g_out, g_attn, H, W, r, scale):
