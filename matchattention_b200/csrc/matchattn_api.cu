@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "matchattn_kernels.cuh"
@@ -338,9 +339,11 @@ int run(Params &p, const Plan &pl, int r, int tile_w_request, cudaStream_t strea
         }
         if (blocks > 2147483647LL) return MATCHATTN_ERR_TOO_LARGE;
         const dim3 grid(static_cast<unsigned>(blocks), grid_y);
+        const long long whole = 1LL * kThreads * sm_count();
+        const int load = static_cast<int>(std::min((blocks * grid_y * threads + whole - 1) / whole, 1000LL));
         // heads shared by lanes: the kernel that shares the softmax too, except for the options only the other one knows
         const bool shared = pl.lph > 1 && p.guard == nullptr && p.sorted == nullptr && p.debug == nullptr &&
-                            launch_lanes<T>(p, r, pl.cpl, grid, threads, stream, err);
+                            launch_lanes<T>(p, r, pl.cpl, grid, threads, load, stream, err);
         if (!shared) err = launch_fast<T>(p, r, pl.cpl, pl.lph > 1, grid, threads, stream);
     } else {
         const long long per_item = 1LL * p.Nq * p.h;

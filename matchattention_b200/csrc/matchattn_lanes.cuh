@@ -374,7 +374,8 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) lanes_forward_kernel(const P
 }
 
 // Runs the kernel above if it is built for these lanes, `err` what the launch returned; false, nothing launched, if it is not.
+// load: blocks of 256 threads per SM, rounded up, as many as the launch has threads for.
 template <typename T>
-bool launch_lanes(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream, cudaError_t &err);
+bool launch_lanes(const Params &p, int r, int cpl, dim3 grid, int threads, int load, cudaStream_t stream, cudaError_t &err);
 
 }  // namespace matchattn

@@ -51,15 +51,19 @@ static cudaError_t launch_fast_r(const Params &p, int cpl, bool multi, dim3 grid
     return cudaErrorInvalidValue;
 }
 
-// Calls whose blocks the host has cut in half (fewer than ten of them per SM) wait for their taps more than they fill the
-// chip: the build with more registers per thread keeps more of them on their way.  104x208 tokens, 8 heads x 16, float32 22.2 ->
-// 21.0 us, a centre per head 29.5 -> 27.3; float16, 2 x 64x64, 4 x 64 10.7 -> 10.2; full blocks lose (2 x 192x192, 4 x 64, float32
-// 128 -> 144).
+// load: blocks of 256 threads per SM, rounded up.  Calls whose blocks the host has cut in half (fewer than ten per SM) wait for
+// their taps more than they fill the chip.  A build for two blocks per SM has the registers to keep more of them on their way,
+// and pays where it goes through no more rounds than the one for three, at a load of 1, 2 or 4.  Three blocks / two: float16, 4
+// heads x 64, 64x64 tokens 5.9 / 5.8 us, 72x72 (load 3) 6.8 / 7.5, 2 x 64x64 11.7 / 10.7, 104x104 (load 5) 14.1 / 14.3; 4 x 32,
+// 104x104 (load 3) 7.3 / 7.9; float32, 8 x 16, 72x72 6.7 / 7.3, 2 x 64x64 12.8 / 10.7.  Two lanes per float32 head gain by the
+// registers at higher loads too (8 x 16, 104x208 23.8 / 23.1, a centre per head 30.2 / 29.4); full blocks lose (2 x 192x192, 4 x 64,
+// float32 128 / 144).
 template <typename T, int R, int CPL, int L, bool RAGGED>
-static cudaError_t launch_lanes_one(const Params &p, dim3 grid, int threads, cudaStream_t stream)
+static cudaError_t launch_lanes_one(const Params &p, dim3 grid, int threads, int load, cudaStream_t stream)
 {
     if constexpr (lanes_min_blocks<T, R, CPL>() > 2) {
-        if (threads < kThreads) return launch_chained(lanes_forward_kernel<T, R, CPL, L, RAGGED, 2>, grid, threads, 0, stream, p);
+        if (threads < kThreads && ((load + 1) / 2 == (load + 2) / 3 || (sizeof(T) == 4 && L == 2 && load > 4)))
+            return launch_chained(lanes_forward_kernel<T, R, CPL, L, RAGGED, 2>, grid, threads, 0, stream, p);
     }
     return launch_chained(lanes_forward_kernel<T, R, CPL, L, RAGGED>, grid, threads, 0, stream, p);
 }
@@ -67,19 +71,19 @@ static cudaError_t launch_lanes_one(const Params &p, dim3 grid, int threads, cud
 // The splits that calls get without knobs (float32 on (2, 2) and (2, 4): from 33 heads on, r = 2); any other runs on the
 // kernel above, so do 33 to 64 heads of 128 channels at r = 1.
 template <typename T, int R>
-static bool launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cudaStream_t stream, cudaError_t &err)
+static bool launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, int load, cudaStream_t stream, cudaError_t &err)
 {
     const int width = p.hd / 8;      // chunks of a head
 #define MA_LANES(CPL_, L_)                                                         \
     if (cpl == CPL_ && p.lph == L_ && width == CPL_ * L_) {                        \
-        err = launch_lanes_one<T, R, CPL_, L_, false>(p, grid, threads, stream);   \
+        err = launch_lanes_one<T, R, CPL_, L_, false>(p, grid, threads, load, stream); \
         return true;                                                               \
     }
     MA_LANES(2, 2) MA_LANES(2, 4) MA_LANES(2, 8) MA_LANES(4, 8)
     MA_LANES(3, 2) MA_LANES(3, 4) MA_LANES(5, 2)
     if constexpr (sizeof(T) == 2) {
         if (cpl == 3 && p.lph == 2 && width == 5) {
-            err = launch_lanes_one<T, R, 3, 2, true>(p, grid, threads, stream);
+            err = launch_lanes_one<T, R, 3, 2, true>(p, grid, threads, load, stream);
             return true;
         }
     } else {
@@ -90,10 +94,10 @@ static bool launch_lanes_r(const Params &p, int cpl, dim3 grid, int threads, cud
 }
 
 template <>
-bool launch_lanes<MATCHATTN_T>(const Params &p, int r, int cpl, dim3 grid, int threads, cudaStream_t stream, cudaError_t &err)
+bool launch_lanes<MATCHATTN_T>(const Params &p, int r, int cpl, dim3 grid, int threads, int load, cudaStream_t stream, cudaError_t &err)
 {
-    return r == 1 ? launch_lanes_r<MATCHATTN_T, 1>(p, cpl, grid, threads, stream, err)
-                  : launch_lanes_r<MATCHATTN_T, 2>(p, cpl, grid, threads, stream, err);
+    return r == 1 ? launch_lanes_r<MATCHATTN_T, 1>(p, cpl, grid, threads, load, stream, err)
+                  : launch_lanes_r<MATCHATTN_T, 2>(p, cpl, grid, threads, load, stream, err);
 }
 
 template <>

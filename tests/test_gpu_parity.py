@@ -84,6 +84,18 @@ def test_kernel_matches_oracle(shape, dtype):
     assert_close(out, ref_out, dtype, "out", ties=ties)
 
 
+@pytest.mark.parametrize("B,H,W", [(1, 47, 49), (1, 72, 72), (2, 64, 64), (1, 97, 103)])
+@pytest.mark.parametrize("h,hd,dtype", [(4, 64, torch.float16), (4, 64, torch.bfloat16), (8, 16, torch.float32), (4, 32, torch.float32)])
+def test_either_build_of_half_size_blocks(B, H, W, h, hd, dtype):
+    """Launches of one, three, four and five blocks of 256 threads per SM (148): two and three resident blocks by turns."""
+    inputs = make_inputs(31 + H, B, H, W, h, hd, 1, dtype, kind="flow", spread=12.0, per_head=True, border_frac=0.2)
+    ref_out, ref_attn = _oracle().forward(*inputs, H, W, 1, hd ** -0.5)
+    out, attn = run_kernel(inputs, H, W, 1, hd ** -0.5)
+    ties = hd > 16          # see _cases.py: rounding ties of wide-head score sums
+    assert_close(attn, ref_attn, dtype, "attn", ties=ties)
+    assert_close(out, ref_out, dtype, "out", ties=ties)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("per_head", [False, True])
 def test_headline_config_full_size(dtype, per_head):
