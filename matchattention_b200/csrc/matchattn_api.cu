@@ -233,22 +233,6 @@ Plan direct_plan(int h, int hd, int r, int esize, int cpl_request, bool refine, 
 // Alignment the specialised kernels need for q, k, v, out and the gate: the vector width of a lane's slice.
 uintptr_t slice_alignment(const Plan &pl, int esize) { return (pl.cpl * 8 * esize) % 32 == 0 ? 32 : 16; }
 
-// SMs of the current device (148 when the query fails); asked once per device
-inline int sm_count()
-{
-    constexpr int kDevices = 64;
-    static std::atomic<int> known[kDevices];
-    int dev = 0, sms = 0;
-    cudaError_t err = cudaGetDevice(&dev);
-    if (err == cudaSuccess) {
-        if (dev < kDevices && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
-        err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    if (status_of(err) != MATCHATTN_OK || sms <= 0) return 148;
-    if (dev < kDevices) known[dev].store(sms, std::memory_order_relaxed);
-    return sms;
-}
-
 inline bool aligned(const void *p, uintptr_t a) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // The matrix-instruction kernel: unsorted (walks the map in tiles) or in sorted order.  In sorted

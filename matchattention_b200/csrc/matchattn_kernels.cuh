@@ -27,6 +27,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/matchattn.h"
 
 namespace matchattn {
@@ -40,6 +42,22 @@ inline int status_of(cudaError_t err)
     if (err == cudaSuccess) return MATCHATTN_OK;
     static_cast<void>(cudaGetLastError());
     return MATCHATTN_ERR_CUDA + static_cast<int>(err);
+}
+
+// SMs of the current device (148 when the query fails); asked once per device
+inline int sm_count()
+{
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
+    int dev = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) {
+        if (dev < kDevices && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+        err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    if (status_of(err) != MATCHATTN_OK || sms <= 0) return 148;
+    if (dev < kDevices) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
 }
 
 // Kernels that follow one another in a stream (programmatic dependent launch): a kernel launched by launch_chained is set

@@ -129,29 +129,105 @@ __device__ __forceinline__ __nv_bfloat162 pair_max(__nv_bfloat162 a, __nv_bfloat
 template <typename P>
 __device__ __forceinline__ uint32_t pair_word(P p) { return *reinterpret_cast<const uint32_t *>(&p); }
 
-constexpr int kPairRows = 2;
+// Nine logits of two cells as loaded: a word of two neighbours, or two values, which stay apart (put into a word first, 2 x 543x541
+// by 4 took 66 us in float16 and 106 in bfloat16, now 62 and 63).
+template <typename T, bool EVEN>
+struct Logits {
+    uint32_t w[9];
+    __device__ __forceinline__ void load(int k, const T *at, int w0, int) { w[k] = *reinterpret_cast<const uint32_t *>(at + w0); }
+    __device__ __forceinline__ float2 get(int k) const { return make_float2(DT<T>::unpack(w[k], 0), DT<T>::unpack(w[k], 1)); }
+    __device__ __forceinline__ float2 top() const
+    {
+        typename DT<T>::Bcast top = word_as_pair<T>(w[0]);
+#pragma unroll
+        for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(w[k]));
+        const uint32_t tw = pair_word(top);
+        return make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
+    }
+};
+template <typename T>
+struct Logits<T, false> {
+    T a[9], b[9];
+    __device__ __forceinline__ void load(int k, const T *at, int w0, int w1)
+    {
+        a[k] = at[w0];
+        b[k] = at[w1];
+    }
+    __device__ __forceinline__ float2 get(int k) const { return make_float2(static_cast<float>(a[k]), static_cast<float>(b[k])); }
+    __device__ __forceinline__ float2 top() const
+    {
+        T ta = a[0], tb = b[0];
+#pragma unroll
+        for (int k = 1; k < 9; ++k) {
+            ta = __hmax(ta, a[k]);
+            tb = __hmax(tb, b[k]);
+        }
+        return make_float2(static_cast<float>(ta), static_cast<float>(tb));
+    }
+};
+
+// One fine row of two cells: softmax of the logits at m0, weighted sums of the neighbours' components, F fine cells to either.
+// (place: gives the row's output, asked for at the end: one row per thread needs no register for it before that)
+template <typename T, int F, bool EVEN, typename Place>
+__device__ __forceinline__ void fine_row(const T *m0, Place place, const uint32_t (&nx)[9], const uint32_t (&ny)[9], int w0, int w1, bool second, int64_t plane)
+{
+    uint32_t o0[F], o1[F];
+#pragma unroll
+    for (int j = 0; j < F; ++j) {
+        Logits<T, EVEN> logits;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) logits.load(k, m0 + static_cast<int64_t>(k * F * F + j) * plane, w0, w1);
+        const float2 mx = logits.top();
+        float2 p[9], den;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            p[k] = weight_exp<T>(logits.get(k), mx);
+            den = k == 0 ? p[0] : add_f32x2(den, p[k]);
+        }
+        const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
+        float sx[2] = {0.f, 0.f}, sy[2] = {0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const float2 q = mul_f32x2(p[k], inv);
+            const typename DT<T>::Bcast w = word_as_pair<T>(DT<T>::aw_from(q.x, q.y));
+            DT<T>::wmul(w, nx[k], sx);
+            DT<T>::wmul(w, ny[k], sy);
+        }
+        o0[j] = DT<T>::aw_from(sx[0], sy[0]);
+        o1[j] = DT<T>::aw_from(sx[1], sy[1]);
+    }
+    uint32_t *row = place();
+    if constexpr (F == 4) {
+        st_128(row + static_cast<int64_t>(w0) * F, o0);
+        if (second) st_128(row + static_cast<int64_t>(w1) * F, o1);
+    } else {
+        st_64(row + static_cast<int64_t>(w0) * F, o0);
+        if (second) st_64(row + static_cast<int64_t>(w1) * F, o1);
+    }
+}
 
 // 16-bit types, two-component fields (the model's), factors 2 and 4, any width.  A thread owns two cells of a row and
-// kPairRows fine rows, one after the other, and takes them through everything in pairs: a weight word holds both cells' weights, multiplied by the
-// pair of their neighbours' components, packed float32 arithmetic in between.  EVEN: the two cells are neighbours and a
-// mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous.  A cell's F fine cells are one aligned store of 8 or 16 bytes.
-// Bound by instruction issue (70 %; integer pipe 55 %).  Measured, float16: 2 x 384x384 by 4: 33 -> 27.9 us (four cells and
-// five blocks per SM before; one fine row per thread 28.5, two without the limit of 64 registers 54); 2 x 200x304 by 2: 8.4 -> 5.0; 2 x 201x303 by 4: 84 us (one cell and all its
-// fine rows per thread) -> 17.7.
-template <typename T, int F, bool EVEN>
-__global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *field, const T *mask, T *__restrict__ out,
+// ROWS fine rows, one after the other, and takes them through everything in pairs: a weight word holds both cells' weights,
+// multiplied by the pair of their neighbours' components, packed float32 arithmetic in between.  EVEN: the two cells are
+// neighbours and a mask read is one word; otherwise they lie 32 apart, so that a warp's 2-byte reads are contiguous.  A cell's
+// F fine cells are one aligned store of 8 or 16 bytes.
+// Two rows share the neighbours and their addresses; one is half as long where the blocks do not fill the chip (pair_rows).
+// Two: issue 65 %, then the latency of the mask reads (4.7 stalls per issue).  Measured, float16, 2 x 384x384 by 4: 27.3 us
+// (one row 28.9, two without the limit of 64 registers 54, four cells and five blocks per SM 33); by 2 9.1 (10.5).
+template <typename T, int F, bool EVEN, int ROWS>
+__global__ void __launch_bounds__(128, ROWS == 1 ? 0 : 8) upsample_pair_kernel(const T *field, const T *mask, T *__restrict__ out,
                                                             int B, int H, int W, int segments)
 {
     chain_begin();
-    constexpr int G = F / kPairRows;               // threads' shares of a cell
+    constexpr int G = F / ROWS;                    // threads' shares of a cell
     constexpr int COLS = EVEN ? 4 : 6;             // columns of neighbours: -1 .. 2 around the pair, or -1 .. 1 around either
     const int lane = threadIdx.x & 31;
     const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5);
-    const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, pair of fine rows
+    const uint32_t line = warp / static_cast<uint32_t>(segments);              // b, ROWS fine rows
     const int w0 = static_cast<int>(warp - line * segments) * 64 + (EVEN ? 2 * lane : lane);
     const uint32_t b = line / static_cast<uint32_t>(H * G);
     if (b >= static_cast<uint32_t>(B) || w0 >= W) return;
-    const int hi = static_cast<int>(line - b * (H * G)), h = hi / G, i0 = (hi - h * G) * kPairRows;
+    const int hi = static_cast<int>(line - b * (H * G)), h = hi / G, i0 = (hi - h * G) * ROWS;
     const int w1 = EVEN ? w0 + 1 : min(w0 + 32, W - 1);
     const bool second = EVEN || w0 + 32 < W;
     const int64_t plane = static_cast<int64_t>(H) * W;
@@ -180,54 +256,13 @@ __global__ void __launch_bounds__(128, 8) upsample_pair_kernel(const T *field, c
     }
 
     const T *m0 = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(i0) * F * plane + static_cast<int64_t>(h) * W;
-    uint32_t *row = reinterpret_cast<uint32_t *>(out) + static_cast<int64_t>(line) * kPairRows * W * F;
+    if constexpr (ROWS == 1) {
+        fine_row<T, F, EVEN>(m0, [&] { return reinterpret_cast<uint32_t *>(out) + static_cast<int64_t>(line) * W * F; }, nx, ny, w0, w1, second, plane);
+    } else {
+        uint32_t *row = reinterpret_cast<uint32_t *>(out) + static_cast<int64_t>(line) * ROWS * W * F;
 #pragma unroll 1
-    for (int i = 0; i < kPairRows; ++i, m0 += F * plane, row += static_cast<int64_t>(W) * F) {
-        uint32_t o0[F], o1[F];
-#pragma unroll
-        for (int j = 0; j < F; ++j) {
-            uint32_t raw[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                const T *at = m0 + static_cast<int64_t>(k * F * F + j) * plane;
-                if constexpr (EVEN) {
-                    raw[k] = *reinterpret_cast<const uint32_t *>(at + w0);
-                } else {
-                    const unsigned short *u = reinterpret_cast<const unsigned short *>(at);
-                    raw[k] = static_cast<uint32_t>(u[w0]) | static_cast<uint32_t>(u[w1]) << 16;
-                }
-            }
-            typename DT<T>::Bcast top = word_as_pair<T>(raw[0]);
-#pragma unroll
-            for (int k = 1; k < 9; ++k) top = pair_max(top, word_as_pair<T>(raw[k]));
-            const uint32_t tw = pair_word(top);
-            const float2 mx = make_float2(DT<T>::unpack(tw, 0), DT<T>::unpack(tw, 1));
-            float2 p[9], den;
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                const float2 l = make_float2(DT<T>::unpack(raw[k], 0), DT<T>::unpack(raw[k], 1));
-                p[k] = weight_exp<T>(l, mx);
-                den = k == 0 ? p[0] : add_f32x2(den, p[k]);
-            }
-            const float2 inv = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
-            float sx[2] = {0.f, 0.f}, sy[2] = {0.f, 0.f};
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                const float2 q = mul_f32x2(p[k], inv);
-                const typename DT<T>::Bcast w = word_as_pair<T>(DT<T>::aw_from(q.x, q.y));
-                DT<T>::wmul(w, nx[k], sx);
-                DT<T>::wmul(w, ny[k], sy);
-            }
-            o0[j] = DT<T>::aw_from(sx[0], sy[0]);
-            o1[j] = DT<T>::aw_from(sx[1], sy[1]);
-        }
-        if constexpr (F == 4) {
-            st_128(row + static_cast<int64_t>(w0) * F, o0);
-            if (second) st_128(row + static_cast<int64_t>(w1) * F, o1);
-        } else {
-            st_64(row + static_cast<int64_t>(w0) * F, o0);
-            if (second) st_64(row + static_cast<int64_t>(w1) * F, o1);
-        }
+        for (int i = 0; i < ROWS; ++i, m0 += F * plane, row += static_cast<int64_t>(W) * F)
+            fine_row<T, F, EVEN>(m0, [row] { return row; }, nx, ny, w0, w1, second, plane);
     }
 }
 
@@ -295,6 +330,18 @@ __global__ void __launch_bounds__(128) upsample_f32_kernel(const float *field, c
     }
 }
 
+// Fine rows per thread of the kernel for pairs; `blocks`: of a launch with one.  Two pay once the chip is full: one row in even
+// widths by 4 is held by 64 registers, eight blocks per SM, in other builds by up to 80, six.  Even by 4, three rounds of one row
+// beat two of two.  Measured, one row / two, us, float16, 2 maps: by 4 48x48 3.4 / 5.2, 192x192 (0.97 rounds) 9.1 / 11.4, 200x304
+// (1.7) 14.5 / 13.9, 272x272 (2.3) 19.1 / 21.3, 352x352 (3.6) 26.9 / 25.7, 544x544 57.4 / 56.0, 161x161 (1.1 of six) 10.6 / 9.3,
+// 96x97 5.3 / 7.0, 543x541 83.7 / 62.4; by 2 192x192 3.5 / 3.7, 240x240 (1.1 of six) 4.8 / 4.5, 96x97 3.4 / 3.9, 201x303 6.2 / 5.6.
+int pair_rows(long long blocks, int factor, bool even)
+{
+    const long long eight = 8LL * sm_count(), held = even && factor == 4 ? eight : eight * 6 / 8;
+    if (blocks <= held || (held == eight && (blocks + eight - 1) / eight == 3)) return 1;
+    return 2;
+}
+
 template <typename T>
 cudaError_t launch(const void *field, const void *mask, void *out, int B, int H, int W, int D, int factor,
                    cudaStream_t stream)
@@ -311,9 +358,14 @@ cudaError_t launch(const void *field, const void *mask, void *out, int B, int H,
         static_cast<int64_t>(H) * W < (1LL << 31) && warps < (1LL << 31)) {
         if constexpr (sizeof(T) == 2) {
             if ((reinterpret_cast<uintptr_t>(f) & 3u) == 0) {
-                const auto kernel = even ? (factor == 4 ? upsample_pair_kernel<T, 4, true> : upsample_pair_kernel<T, 2, true>)
-                                         : (factor == 4 ? upsample_pair_kernel<T, 4, false> : upsample_pair_kernel<T, 2, false>);
-                launch_chained(kernel, (blocks + kPairRows - 1) / kPairRows, 128, 0, stream, f, m, o, B, H, W, seg);
+                const auto go = [&](auto rows) {
+                    constexpr int ROWS = decltype(rows)::value;
+                    const auto kernel = even ? (factor == 4 ? upsample_pair_kernel<T, 4, true, ROWS> : upsample_pair_kernel<T, 2, true, ROWS>)
+                                             : (factor == 4 ? upsample_pair_kernel<T, 4, false, ROWS> : upsample_pair_kernel<T, 2, false, ROWS>);
+                    launch_chained(kernel, (blocks + ROWS - 1) / ROWS, 128, 0, stream, f, m, o, B, H, W, seg);
+                };
+                if (pair_rows(blocks, factor, even) == 2) go(std::integral_constant<int, 2>());
+                else go(std::integral_constant<int, 1>());
                 return cudaGetLastError();
             }
         } else if (even) {

@@ -59,9 +59,11 @@ def test_bad_arguments_raise():
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("factor", [2, 4])
-@pytest.mark.parametrize("H,W", [(1, 1), (2, 2), (3, 31), (2, 33), (1, 63), (3, 64), (2, 65), (5, 98), (2, 129)])
+@pytest.mark.parametrize("H,W", [(1, 1), (2, 2), (3, 31), (2, 33), (1, 63), (3, 64), (2, 65), (5, 98), (2, 129),
+                                 (900, 1), (901, 2), (900, 33), (903, 64), (460, 65), (301, 130)])
 def test_pairs_of_cells_at_the_edges_of_a_warp(H, W, factor, dtype):
-    """Widths around the 32 and 64 cells of a warp, odd and even, down to a map of one cell."""
+    """Widths around the 32 and 64 cells of a warp, odd and even, down to a map of one cell; the high maps fill the chip and
+    take two fine rows per thread."""
     import matchattention_b200 as ma
     import oracle
     g = torch.Generator().manual_seed(H * W + factor)
