@@ -82,6 +82,13 @@ __global__ void __launch_bounds__(128) upsample_field_kernel(const T *field, con
     }
 
     const T *mrow = mask + static_cast<int64_t>(b) * 9 * F * F * plane + static_cast<int64_t>(h) * W + w;
+    // the logits of a fine cell are asked for before the cell ahead of it is stored: loads do not pass stores
+    float next[9];
+    const auto ask = [&](int cell) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) next[k] = load_one<T>(mrow + static_cast<int64_t>(k * F * F + cell) * plane);
+    };
+    ask(0);
     for (int i = 0; i < F; ++i) {
         T *orow = out + ((static_cast<int64_t>(b) * H * F + static_cast<int64_t>(h) * F + i) * W * F + static_cast<int64_t>(w) * F) * D;
 #pragma unroll
@@ -90,9 +97,10 @@ __global__ void __launch_bounds__(128) upsample_field_kernel(const T *field, con
             float mx = -INFINITY;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
-                p[k] = load_one<T>(mrow + static_cast<int64_t>((k * F + i) * F + j) * plane);
+                p[k] = next[k];
                 mx = fmaxf(mx, p[k]);
             }
+            if (i * F + j + 1 < F * F) ask(i * F + j + 1);
             float den = 0.f;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
