@@ -310,8 +310,11 @@ int run(Params &p, const Plan &pl, int r, int tile_w_request, cudaStream_t strea
             // the same queries over more SMs.  With 4 x 4 windows blocks of half the size already pay below ten
             // per SM: an SM holds three of the large ones, and a last round of few costs as much as a full one (104x208
             // tokens, 8 heads x 16, float32 23.2 -> 22.2 us, two maps in float16 24.4 -> 22.9; at 24 per SM smooth centres
-            // lose up to 11 % of the taps' reuse, at two all of this).  6 x 6 windows share more taps within a block and keep
-            // the large ones (96x96 tokens, a layer: 44.4 us, with half of them 47.1).
+            // lose up to 11 % of the taps' reuse).  Smooth and shared random centres gain at every load below ten (float16, 8 x
+            // 16, 104x104 tokens 8.1 -> 7.4, 160x240 22.6 -> 22.1; 4 x 8, 104x208 6.2 -> 5.5); one lane per head with a centre
+            // each gains below four per SM and loses up to 7 % above (8 x 16, 104x208 17.5 -> 18.2; 4 x 8, two maps 12.1 ->
+            // 12.9).  6 x 6 windows share more taps within a block and keep the large ones (96x96 tokens, a layer: 44.4 us,
+            // with half of them 47.1).
             if (threads <= 64 || threads / 2 < p.G || blocks * p.B >= (r == 1 && threads == kThreads ? 5 * fill : fill)) break;
             threads /= 2;
         }

@@ -949,9 +949,9 @@ __device__ __forceinline__ void prefetch_l2(const void *global, int count, uint3
 // of all buckets that the tile needs are staged in shared memory, `batch` at a time: coefficients, q and dout.
 // A slot of coefficients is padded by 16 bytes: neighbouring tokens read the same tap of neighbouring slots.
 // Such narrow heads alone: read straight from global memory, every item of a list is a line of its own for as few bytes
-// (float16, 384x384 tokens, 8 heads x 16, a centre per head: 219 us, the kernel below 260; float32, 2 x 192x192, 4 x 16: 79
-// and 105; 4 x 8 channels: 54 and 50, 4 x 64: 190 and 160).
-// Bound by instruction issue (69 % of the slots; about 57 per token, item and eight channels; two thirds of the lanes busy,
+// (float16, 384x384 tokens, 8 heads x 16, a centre per head: 207 to 219 us on several boards, the kernel below 260 where it
+// took 219; float32, 2 x 192x192, 4 x 16: 79 and 105; 4 x 8 channels: 54 and 50, 4 x 64: 190 and 160).
+// Bound by instruction issue (73 % of the slots; about 57 per token, item and eight channels; two thirds of the lanes busy,
 // lists differ in length); walking a token's four ranges as one list costs as much as it saves.
 template <typename T, int R>
 __global__ void __launch_bounds__(kStagedX * kStagedY * kStagedChunks) gather_sum_staged_kernel(const GatherParams g)
@@ -1051,7 +1051,8 @@ __global__ void __launch_bounds__(kStagedX * kStagedY * kStagedChunks) gather_su
 // float32, 2 x 45x79, 4 x 32, r = 2: 41 to 48 with three, 34 with two)
 template <typename T, int R, int CPT>
 constexpr int sum_min_blocks() { return CPT == 4 ? 0 : CPT == 2 ? 2 : sizeof(T) == 2 && R == 1 ? 4 : sizeof(T) == 4 && R == 2 ? 2 : 3; }
-// blocks ahead whose coefficients a block asks L2 for (600: 173 us, 300: 171, 1000: 176)
+// blocks ahead, in the same list, whose coefficients a block asks L2 for (float16, 384x384 tokens, 8 heads x 16: 600 173 us, 300
+// 171, 1000 176); the first so many blocks of every list, all those of a small map, go without
 constexpr unsigned kPrefetchAhead = 300;
 
 // The same without staging: `lanes` lanes per token, each with CPT chunks of eight channels (chunk = lane + s * lanes),
@@ -1224,7 +1225,7 @@ GatherPlan gather_plan(int B, int H, int W, int h, int hd, int r, int dtype, int
             }
         }
         const int tokens = 8 * tl.per_warp;
-        tl.x = tokens >= 32 ? 8 : tokens >= 16 && tokens % 4 == 0 ? 4 : tokens % 3 == 0 ? 6 : 4;
+        tl.x = tokens >= 32 ? 8 : 4;
         tl.y = tokens / tl.x;
         tl.tiles_x = (W + tl.x - 1) / tl.x;
         return best != 0;

@@ -18,9 +18,9 @@
 // prob and the deciding averages are formed in one fixed order (sums of exponentials in 256 interleaved partial sums
 // per row and four per column, box sums row by row) whatever the split of the work, and only the screening in step 3
 // adds in another.
-// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 0.99 ms = 0.09 + 0.25 +
-// 0.61 + 0.05; with a pooling pass over the stored probabilities and separate statistics passes it was 6.59 ms, of which
-// the pooling took 4.1.  48x48 tokens: 44 us, before 196.
+// Measured on a B200, float16, 128x128 tokens (1.61 GB are the least possible, 3.2 GB move): 1.01 to 1.04 ms in a row of
+// calls = 0.09 + 0.25 + 0.62 + 0.05; with a pooling pass over the stored probabilities and separate statistics passes it was
+// 6.59 ms, of which the pooling took 4.1.  48x48 tokens: 44 us, before 196.
 // Rounding of the 16-bit types as eager PyTorch on the GPU: softmax, pooling and sums accumulate in float32
 // and round once, every elementwise op rounds.
 #include "../../include/matchattn.h"
@@ -729,7 +729,7 @@ __device__ __forceinline__ void pool_cols(const PoolParams &pp, const T *src, T 
 // the softmax runs over (pool_rows, pool_cols); a lane of the second gathers eight rows of its columns and stores
 // them as 16 bytes of a prob row, or, where rows of prob are not 16-byte aligned, through shared memory.
 // Eight consecutive blocks (four of either role) cover one 4-band x 4-chunk region, so the second role finds corr in L2.
-// Bound by instruction issue (about 25 per element and role, a third of them the exponential; 81 % of the slots busy).
+// Bound by instruction issue (about 25 per element and role, a third of them the exponential; 76 % of the slots busy).
 // Measured, float16, 16384 x 16384: 0.61 ms (0.72 with eight rows unrolled and the halo rows apart: the instruction cache
 // ran short, 2.2 of 8 stalls).  With 16-byte stores straight from the registers to 32 rows of prob the
 // second role alone took 0.67 ms; five blocks of four warps hold 20 warps per SM (0.75 ms with four blocks).
