@@ -139,15 +139,22 @@ __global__ void __launch_bounds__(128) backward_kernel(const BwdParams p)
     for (int c = 0; c < p.hd; ++c) {
         const float qc = load_one<T>(qp + c), go = load_one<T>(gop + c);
         float acc = 0.f;
-        for (int m = 0; m < M; ++m) {
-            const int64_t off = static_cast<int64_t>(tok[m]) * p.C + c;
-            const float d = qc - load_one<T>(kb + off);
-            const float sg = d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f);
-            const float g = p.scale * ds[m] * sg;
-            acc -= g;
-            if (g != 0.f) atomicAdd(p.dk + kv_base + off, g);
-            const float gv = a[m] * go;
-            if (gv != 0.f) atomicAdd(p.dv + kv_base + off, gv);
+        for (int m0 = 0; m0 < M; m0 += 4) {       // four loads, then what they lead to: loads do not pass the additions
+            float kv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kv[i] = load_one<T>(kb + static_cast<int64_t>(tok[m0 + i]) * p.C + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int m = m0 + i;
+                const int64_t off = static_cast<int64_t>(tok[m]) * p.C + c;
+                const float d = qc - kv[i];
+                const float sg = d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f);
+                const float g = p.scale * ds[m] * sg;
+                acc -= g;
+                if (g != 0.f) atomicAdd(p.dk + kv_base + off, g);
+                const float gv = a[m] * go;
+                if (gv != 0.f) atomicAdd(p.dv + kv_base + off, gv);
+            }
         }
         store_one<T>(gq + c, acc);
     }
