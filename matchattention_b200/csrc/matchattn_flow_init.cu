@@ -54,11 +54,12 @@ constexpr int kWindowTokens = kFlowWarps;             // tokens per block of the
 constexpr int64_t kLongBands = 5000, kLongBandsOdd = 10000;
 // Column sums: 32-column blocks from so many tokens on, 16-column blocks below, where the wider ones leave SMs without work.
 // Measured, the whole call, wide against narrow: float16 48x48 tokens 45.8 / 45.0 us, 64x64 103.6 / 102.4, 72x72 145.8 / 144.8,
-// 80x80 200.4 / 208.0, 96x96 365.2 / 387.6; float32 64x64 119.9 / 119.5, 76x76 206.3 / 201.8, 88x88 343.4 / 356.2.  Single
-// elements (strided): the narrow blocks read 32 rows ahead, the wide ones 16; float16 96x96 418.2 / 407.9, 96x100 433.3 / 445.5.
+// 80x80 200.4 / 208.0, 96x96 365.2 / 387.6; float32 64x64 119.9 / 119.5, 76x76 206.3 / 201.8, 88x88 343.4 / 356.2; in
+// rows aligned to single elements 70x73 224.1 / 231.6, 78x75 265.7 / 279.3, 79x83 311.2 / 334.3.  Single 16-bit elements
+// (strided): the narrow blocks read 32 rows ahead, the wide ones 16; float16 96x96 418.2 / 407.9, 96x100 433.3 / 445.5.
 template <typename T>
 constexpr int64_t kWideSums = sizeof(T) == 2 ? 5800 : 6600;
-constexpr int64_t kWideStrided = 9400;
+constexpr int64_t kWideStrided = 9400, kWideOdd = 5000;
 
 // Column sums of a block: batches of exponentials, two of them in shared memory.
 template <int COLUMNS>
@@ -934,7 +935,7 @@ cudaError_t run_flow_kernels(const FlowPlan &pl, const T *corr, T *prob, T *flow
         if (N >= kWideStrided) launch_sums(flow_sum_strided_kernel<T, 32, 16>, 32, 32 * kSumGroups, 0);
         else launch_sums(flow_sum_strided_kernel<T, 16, 32>, 16, 16 * kSumGroups, 0);
     } else {
-        if (N >= kWideSums<T>) launch_sums(flow_sum_kernel<T, ALIGN, 32>, 32, kFlowThreads, SumTile<32>::kBytes);
+        if (N >= (ALIGN == 1 ? kWideOdd : kWideSums<T>)) launch_sums(flow_sum_kernel<T, ALIGN, 32>, 32, kFlowThreads, SumTile<32>::kBytes);
         else launch_sums(flow_sum_kernel<T, ALIGN, 16>, 16, kFlowThreads, SumTile<16>::kBytes);
     }
     constexpr int smem = kPoolWarps * kPoolSmemPerWarp;
